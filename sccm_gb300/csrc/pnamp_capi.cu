@@ -54,6 +54,8 @@ struct pnamp_ctx {
     std::vector<uint32_t> r2_quads;
     std::vector<double> r2_tc;
     uint32_t *d_r2q = nullptr;
+    uint2 *d_r2s = nullptr;
+    int r2_off[3] = {0, 0, 0}, r2_ss = -1;
     double *d_r2acc = nullptr, *d_r2out = nullptr;
     long long r2acc_cap = 0, r2out_cap = 0;
     // tensor-core contraction of the two-body energy (contract_tc.cu): bf16 terms per value
@@ -68,6 +70,9 @@ struct pnamp_ctx {
     std::vector<int> tc_src;
     TcGroup *d_tc_groups = nullptr;
     int *d_tc_src = nullptr;
+    unsigned short *d_tc_sp = nullptr;           // species rows of the CTAs' split batches
+    int *d_tc_chunks = nullptr;
+    int tc_choff[3] = {0, 0, 0};
     unsigned short *d_tc_mat[3] = {nullptr, nullptr, nullptr};
     unsigned short *d_tc_x[3] = {nullptr, nullptr, nullptr}, *d_tc_y[3] = {nullptr, nullptr, nullptr};
     double *d_tc_w = nullptr, *d_tc_e2 = nullptr;
@@ -154,13 +159,78 @@ std::vector<dd> to_dd(const std::vector<double> &v) {
     return out;
 }
 
+// Thread groups of the reduced pairs' problems (order N, point_reduced.cuh) in `smem` bytes:
+// as many groups as fit, the CTA's warps shared among them, at most 8 matrix entries per
+// thread. More groups hide the sweep's latency better than more warps per group, which only
+// shorten one problem; an even count serves the two species. ng = 0: nothing fits.
+constexpr int kMaxDynSmem = 227 * 1024 - kMultiSmemTail;
+RedPlan plan_reduced(const Params &p, int N, bool split, int smem) {
+    auto align = [](int x) { return (x + 15) & ~15; };
+    const int T = N * (N - 1) / 2;
+    auto make = [&](int ng) {
+        RedPlan L;
+        memset(&L, 0, sizeof(L));
+        L.ng = ng;
+        L.w = kThreads / 32 / ng;
+        L.ld = N + 1;
+        L.items = split ? std::max(1, ng / 2) : 1;
+        int o = 0;
+        L.off_eph = o;
+        o += align(16 * p.nfom);
+        L.off_acc = o;
+        if (split) o += align(16 * (2 * L.items * p.nfom + 2 * std::max(ng, 2 * L.items)) + 4 * std::max(ng, 2 * L.items));
+        else o += align(16 * 4 * ng + 4 * ng);
+        L.off_z0 = o;
+        o += align((split ? 2 : 1) * N * N * 8);
+        L.off_grp = o;
+        L.off_scr = align(16 * N * (L.ld + std::max(L.ld, 5)));   // A; Rh, in which the pivot rows fit
+        L.grp_bytes = L.off_scr + 16 * (32 + 32 + 16) + 3 * 64 + 16;   // SkewScratch and the norm
+        o += ng * L.grp_bytes;
+        // the Euler point's rotation blocks, the Onishi matrix and the final sums use the same place
+        const int rot = L.items * p.rot_elems * 16;
+        const int fin = L.items * (2 * N * N + 2 * 17 + 8) * 16 + 16 * 32 + (split ? 0 : 16 * (N + 32 + 64));
+        o = std::max(o, L.off_grp + std::max(rot, fin));
+        L.smem_bytes = o;
+        return L;
+    };
+    RedPlan best;
+    memset(&best, 0, sizeof(best));
+    for (int ng = 1; ng <= (split ? 16 : 8); ++ng) {
+        if (split && ng > 1 && ng % 2) continue;
+        const RedPlan L = make(ng);
+        if (L.smem_bytes > smem || (T + 32 * L.w - 1) / (32 * L.w) > 8) continue;
+        // warps in use first, then groups
+        if (best.ng == 0 || L.ng * L.w > best.ng * best.w || (L.ng * L.w == best.ng * best.w && L.ng > best.ng)) best = L;
+    }
+    if (best.ng) {   // register tiles with the fewest passes over the group's threads
+        const int nthr = 32 * best.w;
+        const int rt[5][2] = {{3, 2}, {3, 3}, {4, 2}, {5, 3}, {4, 4}}, kt[4][2] = {{2, 2}, {2, 4}, {3, 3}, {4, 4}};
+        long long cr = -1, ck = -1;
+        int br = 0, bk = 0;
+        for (int q = 0; q < 5; ++q) {
+            const long long nt = (long long)((N + rt[q][0] - 1) / rt[q][0]) * ((N + rt[q][1] - 1) / rt[q][1]);
+            const long long c = ((nt + nthr - 1) / nthr) * (rt[q][0] * rt[q][1] * 8 + rt[q][0] + rt[q][1]);
+            if (cr < 0 || c < cr) { cr = c; br = q; }
+        }
+        for (int q = 0; q < 4; ++q) {
+            long long nt = 0;
+            const int nj = (N + kt[q][1] - 1) / kt[q][1];
+            for (int r = 0; r < (N + kt[q][0] - 1) / kt[q][0]; ++r) nt += std::max(0, nj - (r * kt[q][0] + 1) / kt[q][1]);
+            const long long c = ((nt + nthr - 1) / nthr) * (kt[q][0] * kt[q][1] * 8 + kt[q][0] + kt[q][1]);
+            if (ck < 0 || c < ck) { ck = c; bk = q; }
+        }
+        best.tile = br | (bk << 4);
+    }
+    return best;
+}
+
 int plan_placement(Params &p, int smem_max) {
     const int n = p.n, N = p.N2;
     const long long nn = (long long)n * n;
     Placement &pl = p.place;
     auto align = [](int x) { return (x + 15) & ~15; };
     // fixed shared pieces
-    int fixed = 0, fixed2 = 0;
+    int fixed = 0;
     pl.off_piv = fixed; fixed += align((n + 8) * 4);
     pl.off_inv = fixed; fixed += align(n * 16);
     pl.off_red = fixed; fixed += align(40 * (kThreads / 32) * 8);  // 36 observable slots per warp
@@ -179,24 +249,20 @@ int plan_placement(Params &p, int smem_max) {
     auto total = [&]() { return fixed + flags[0] * bs + flags[1] * bt + flags[2] * by + flags[3] * buv; };
     for (int k = 0; k < 4 && total() > smem_max; ++k) flags[order[k]] = 0;
     if (total() > smem_max) return PNAMP_ERR_UNSUPPORTED;
-    // species-split pairs with two gauge points in flight: after the fixed pieces, the compact
-    // V0^T / U0^T diagonal blocks and two half regions, when they fit (pf: 213 KB)
-    {
-        const int h = n / 2;
-        const int uvc = align(4 * h * h * 8);
-        const long long need = (long long)align(fixed) + uvc + 2LL * half_layout(h).bytes;
-        pl.sp2 = need <= smem_max ? 1 : 0;
-        pl.off_uvc = align(fixed);
-        pl.off_half = pl.off_uvc + uvc;
-        if (pl.sp2) fixed2 = (int)need;
-    }
     int off = fixed;
     pl.s_smem = flags[0]; pl.t_smem = flags[1]; pl.y_smem = flags[2]; pl.uv_smem = flags[3];
     if (pl.s_smem) { pl.off_s = off; off += bs; }
     if (pl.t_smem) { pl.off_t = off; off += bt; }
     if (pl.y_smem) { pl.off_y = off; off += by; }
     if (pl.uv_smem) { pl.off_uv = off; off += buv; }
-    pl.smem_bytes = std::max(off, fixed2);
+    pl.gen = plan_reduced(p, n, false, std::max(off, smem_max));
+    pl.spl = plan_reduced(p, n / 2, true, std::max(off, smem_max));
+    if (!pl.gen.ng || !pl.spl.ng) {   // the least a point needs is held whatever the budget
+        if (!pl.gen.ng) pl.gen = plan_reduced(p, n, false, kMaxDynSmem);
+        if (!pl.spl.ng) pl.spl = plan_reduced(p, n / 2, true, kMaxDynSmem);
+        if (!pl.gen.ng || !pl.spl.ng) return PNAMP_ERR_UNSUPPORTED;
+    }
+    pl.smem_bytes = std::max({off, pl.gen.smem_bytes, pl.spl.smem_bytes});
     long long g = 0;
     pl.g_x = g; g += nn;
     pl.g_b = g; g += 2 * nn;
@@ -513,6 +579,27 @@ int build_tc(pnamp_ctx *c) {
                   cudaMemcpyHostToDevice));
     CK(cudaMalloc(&c->d_tc_src, c->tc_src.size() * sizeof(int)));
     CK(cudaMemcpy(c->d_tc_src, c->tc_src.data(), c->tc_src.size() * sizeof(int), cudaMemcpyHostToDevice));
+    {   // 16-byte chunks of a species row (X entries, then the pair entries again as Y) per species
+        const int npp = c->tc_nk - c->tc_nph, W = c->tc_nk + npp;
+        std::vector<int> ch;
+        for (int s = 0; s < 2; ++s) {
+            c->tc_choff[s] = (int)ch.size();
+            for (int k = 0; k < W / 8; ++k) {
+                bool any = false;
+                for (int q = 8 * k; q < 8 * k + 8; ++q) {
+                    const int src = c->tc_src[q < c->tc_nk ? q : q - c->tc_nk + c->tc_nph];
+                    any = any || (src >= 0 && ((src >> 8) >= n / 2) == (s == 1) && ((src & 255) >= n / 2) == (s == 1));
+                }
+                if (any) ch.push_back(k);
+            }
+        }
+        c->tc_choff[2] = (int)ch.size();
+        CK(cudaMalloc(&c->d_tc_chunks, std::max<size_t>(ch.size(), 1) * sizeof(int)));
+        CK(cudaMemcpy(c->d_tc_chunks, ch.data(), ch.size() * sizeof(int), cudaMemcpyHostToDevice));
+        const size_t bytes = (size_t)c->grid_form[1] * c->p.place.spl.items * 2 * c->p.nfom * 6 * W * sizeof(uint16_t);
+        CK(cudaMalloc(&c->d_tc_sp, bytes));
+        CK(cudaMemset(c->d_tc_sp, 0, bytes));
+    }
     for (int sp = 0; sp < 3; ++sp) {
         CK(cudaMalloc(&c->d_tc_mat[sp], mat.size() * sizeof(uint16_t)));
         CK(cudaMemcpy(c->d_tc_mat[sp], terms[sp].data(), mat.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
@@ -586,6 +673,9 @@ int tc_run(pnamp_ctx *c, int npairs, const double *d_uv, double *d_zres, int *d_
     q.tc_nk = c->tc_nk;
     q.tc_nph = c->tc_nph;
     q.tc_src = c->d_tc_src;
+    q.tc_sp = c->d_tc_sp;
+    q.tc_chunks = c->d_tc_chunks;
+    for (int k = 0; k < 3; ++k) q.tc_choff[k] = c->tc_choff[k];
     for (int sp = 0; sp < 3; ++sp) {
         q.tc_x[sp] = c->d_tc_x[sp];
         q.tc_y[sp] = c->d_tc_y[sp];
@@ -693,7 +783,7 @@ void pnamp_free(pnamp_ctx *ctx) {
     if (!ctx) return;
     for (void *q : ctx->allocs) cudaFree(q);
     if (ctx->d_r1b) cudaFree(ctx->d_r1b);
-    for (void *q : {(void *)ctx->d_r2q, (void *)ctx->d_r2acc, (void *)ctx->d_r2out})
+    for (void *q : {(void *)ctx->d_r2q, (void *)ctx->d_r2s, (void *)ctx->d_r2acc, (void *)ctx->d_r2out})
         if (q) cudaFree(q);
     for (void *q : {(void *)ctx->d_pairbuf, (void *)ctx->d_scratch, (void *)ctx->d_uv, (void *)ctx->d_zres,
                     (void *)ctx->d_status, (void *)ctx->d_proj, (void *)ctx->d_projq})
@@ -701,7 +791,7 @@ void pnamp_free(pnamp_ctx *ctx) {
     for (int sp = 0; sp < 3; ++sp)
         for (void *q : {(void *)ctx->d_tc_mat[sp], (void *)ctx->d_tc_x[sp], (void *)ctx->d_tc_y[sp]})
             if (q) cudaFree(q);
-    for (void *q : {(void *)ctx->d_tc_groups, (void *)ctx->d_tc_src, (void *)ctx->d_tc_w, (void *)ctx->d_tc_e2,
+    for (void *q : {(void *)ctx->d_tc_groups, (void *)ctx->d_tc_src, (void *)ctx->d_tc_sp, (void *)ctx->d_tc_chunks, (void *)ctx->d_tc_w, (void *)ctx->d_tc_e2,
                     (void *)ctx->d_tc_err})
         if (q) cudaFree(q);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
@@ -769,20 +859,27 @@ int pnamp_init(const pnamp_space *sp, const pnamp_hamiltonian *h, const pnamp_me
     }
     // proton-neutron records (a, c protons; b, d neutrons) last: for species-split pairs half
     // of their terms vanish and the point kernel takes a shorter path over that range
-    int nrec_gen = 0;
+    int nrec_gen = 0, rec_off[3] = {0, 0, 0};
     {
-        std::vector<uint32_t> gi, pi;
-        std::vector<double> gv, pv;
+        std::vector<uint32_t> cls[4];
+        std::vector<double> val[4];
         for (int e = 0; e < h->nrec; ++e) {
             const int a = rec_idx[e] & 0xff, b = (rec_idx[e] >> 8) & 0xff, c = (rec_idx[e] >> 16) & 0xff,
                       d = rec_idx[e] >> 24;
+            const int np = (a < hh) + (b < hh) + (c < hh) + (d < hh);
             const bool pn = a < hh && b >= hh && c < hh && d >= hh;
-            (pn ? pi : gi).push_back(rec_idx[e]);
-            (pn ? pv : gv).push_back(rec_v[e]);
+            const int k = pn ? 3 : (np == 4 ? 0 : (np == 0 ? 1 : 2));
+            cls[k].push_back(rec_idx[e]);
+            val[k].push_back(rec_v[e]);
         }
-        nrec_gen = (int)gi.size();
-        gi.insert(gi.end(), pi.begin(), pi.end());
-        gv.insert(gv.end(), pv.begin(), pv.end());
+        std::vector<uint32_t> gi;
+        std::vector<double> gv;
+        for (int k = 0; k < 4; ++k) {
+            gi.insert(gi.end(), cls[k].begin(), cls[k].end());
+            gv.insert(gv.end(), val[k].begin(), val[k].end());
+            if (k < 2) rec_off[k + 1] = (int)gi.size();
+            if (k == 2) nrec_gen = (int)gi.size();
+        }
         rec_idx.swap(gi);
         rec_v.swap(gv);
     }
@@ -858,6 +955,8 @@ int pnamp_init(const pnamp_space *sp, const pnamp_hamiltonian *h, const pnamp_me
     p.rot_elems = rot;
     p.nrec = h->nrec;
     p.nrec_gen = nrec_gen;
+    for (int k = 0; k < 3; ++k) p.rec_off[k] = rec_off[k];
+    p.split_ok = rec_off[2] == nrec_gen;
     p.pl.make(n);
     c->core_prot = sp->core_prot;
     c->core_neut = sp->core_neut;
@@ -1174,6 +1273,14 @@ int pnamp_rho2b_tables(const pnamp_space *sp, int *blocks, int *states, unsigned
 }
 
 namespace {
+void set_r2(const pnamp_ctx *c, Params &q) {
+    q.n_r2q = (int)c->r2_quads.size();
+    q.r2q = c->d_r2q;
+    q.r2s = c->d_r2s;
+    for (int k = 0; k < 3; ++k) q.r2_off[k] = c->r2_off[k];
+    q.r2_ss = c->r2_ss;
+    q.r2acc = c->d_r2acc;
+}
 int ensure_r2(pnamp_ctx *c) {
     if (!c->r2_built) {
         R2Tables r;
@@ -1184,6 +1291,22 @@ int ensure_r2(pnamp_ctx *c) {
         if (r.quads.empty()) return PNAMP_ERR_UNSUPPORTED;
         CK(cudaMalloc(&c->d_r2q, r.quads.size() * sizeof(uint32_t)));
         CK(cudaMemcpy(c->d_r2q, r.quads.data(), r.quads.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+        std::vector<uint2> cls[3], all;
+        bool other = false;
+        for (size_t q = 0; q < r.quads.size(); ++q) {
+            const uint32_t k = r.quads[q];
+            bool nt[4];
+            for (int b = 0; b < 4; ++b) nt[b] = (int)((k >> (8 * b)) & 0xff) >= n / 2;
+            other = other || nt[0] != nt[2] || nt[1] != nt[3];
+            cls[nt[0] != nt[1] ? 2 : (nt[0] ? 1 : 0)].push_back(make_uint2(k, (unsigned)q));
+        }
+        for (int k = 0; k < 3; ++k) {
+            c->r2_off[k] = (int)all.size();
+            all.insert(all.end(), cls[k].begin(), cls[k].end());
+        }
+        c->r2_ss = other ? -1 : (int)std::max(cls[0].size(), cls[1].size());
+        CK(cudaMalloc(&c->d_r2s, all.size() * sizeof(uint2)));
+        CK(cudaMemcpy(c->d_r2s, all.data(), all.size() * sizeof(uint2), cudaMemcpyHostToDevice));
         c->r2_blocks.swap(r.blocks);
         c->r2_states.swap(r.states);
         c->r2_quads.swap(r.quads);
@@ -1192,7 +1315,12 @@ int ensure_r2(pnamp_ctx *c) {
         c->r2_tc.swap(r.tc);
         c->r2_built = true;
     }
-    const long long need = 2LL * (long long)c->r2_quads.size() * c->grid_form[c->p.form];
+    // one set of sums per thread group that runs gauge points of its own, or per unit of a
+    // species-split batch
+    const RedPlan &gn = c->p.place.gen, &sl = c->p.place.spl;
+    const long long need = 2LL * c->grid_form[c->p.form] *
+                           std::max<long long>((long long)c->r2_quads.size() * gn.ng,
+                                               (long long)std::max(c->r2_ss, 0) * std::max(sl.ng, 2 * sl.items));
     if (need > c->r2acc_cap) {
         if (c->d_r2acc) cudaFree(c->d_r2acc);
         c->d_r2acc = nullptr;
@@ -1215,9 +1343,7 @@ int pnamp_batch_rho2b_device(pnamp_ctx *c, int npairs, const double *d_uv, doubl
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;  // NULL: legacy default stream
     Params q = c->p;
-    q.n_r2q = (int)c->r2_quads.size();
-    q.r2q = c->d_r2q;
-    q.r2acc = c->d_r2acc;
+    set_r2(c, q);
     CK(cudaMemsetAsync(d_rho2b, 0, (size_t)npairs * q.n_r2q * 2 * sizeof(double), st));
     CK(launch_setup(q, npairs, d_uv, c->d_pairbuf, st));
     CK(launch_points(q, npairs, c->d_pairbuf, c->d_scratch, c->grid_form[q.form], d_zres, d_status, st, nullptr, 0,
@@ -1272,9 +1398,7 @@ int pnamp_batch_densities_device(pnamp_ctx *c, int npairs, const double *d_uv, d
     cudaStream_t st = (cudaStream_t)stream;  // NULL: legacy default stream
     Params q = c->p;
     if (d_rho2b) {
-        q.n_r2q = (int)c->r2_quads.size();
-        q.r2q = c->d_r2q;
-        q.r2acc = c->d_r2acc;
+            set_r2(c, q);
         CK(cudaMemsetAsync(d_rho2b, 0, (size_t)npairs * q.n_r2q * 2 * sizeof(double), st));
     }
     CK(launch_setup(q, npairs, d_uv, c->d_pairbuf, st));

@@ -21,9 +21,10 @@ constexpr int kSetupThreads = 256;
 constexpr int kMultiSmemTail = 16;       // dynamic shared bytes after the placement: multi kernel's counter
 
 // One pair record (doubles), all matrices row-major n x n:
-// U0 V0 U1 V1 W Z0 ZI then [det0, det1, status-as-double, reduced flag, Pf(-c Z0) re, im, pad, pad].
-// ZI = Z0^-1 = U0 V0^-1; with the reduced flag set the point kernel eliminates the n x n
-// matrix c (D X D - ZI) and multiplies by Pf(-c Z0) instead of eliminating the 2n x 2n one.
+// U0 V0 U1 V1 W Z0 ZI then [det0, det1, status-as-double, Schur flag, Pf re, im, no
+// proton-neutron blocks, reduced flag]. Reduced pairs (point_reduced.cuh): ZI = W^-1 = U1 V1^-1
+// and Pf = Pf(c W). Others with the Schur flag: ZI = Z0^-1 = U0 V0^-1, Pf = Pf(-c Z0), and the
+// point kernel eliminates the n x n matrix c (D X D - ZI) instead of the 2n x 2n one.
 struct PairLayout {
     long long u0, v0, u1, v1, w, z0, zi, dets, pfz, stride;
     __host__ __device__ void make(int n) {
@@ -33,13 +34,29 @@ struct PairLayout {
         stride = 7 * nn + 8;
     }
 };
-// min/max |LU pivot| of V0 for the reduced Pfaffian. A bra with nearly empty levels (small
+// min/max |LU pivot| of V0 for the Schur complement's Pfaffian. A bra with nearly empty levels (small
 // singular values of V0) makes Z0^-1 dominate the Schur complement c (D X D - Z0^-1), whose
 // Pfaffian then carries the point's dependence in its low-order bits: on the shipped Ti48
 // vacua a ratio of 2e-6 cost 2e-9 relative and 8e-5 cost 3e-7, while every bra at >= 3e-2
 // stayed within 6e-13 of the 2n x 2n elimination. Below the bound the pair keeps the
 // 2n x 2n form.
 constexpr double kReducedPivotRatio = 1e-2;
+// The reduced pairs of point_reduced.cuh: pivot ratios of U0 and V1 within the same bound and
+// no entry of W^-1 = U1 V1^-1 above this. Its entries enter K = M^-1 - Z0 with their rounding in
+// the point arithmetic: in a simulation with 24-bit words the densities are as exact as with
+// T22 up to 25 (every synthetic and Ge76 vacuum and Ti48's beta2 = -0.1 ... 0.2 are at 5 to 36)
+// and 10 to 20 times less exact at 76 (Ti48's beta2 = 0.3 as the ket).
+constexpr double kReducedMaxEntry = 40.0;
+
+// Thread groups and shared memory (byte offsets) of the reduced pairs' problems, order N: ng
+// groups of w warps, each with the inverse (then kappa) and rho (N x ld complex each), the
+// factorisation's scratch from off_scr in a region of grp_bytes. tile: the register tiles of
+// the density products (rho in bits 0..3, kappa10 above). items: Euler points per batch of
+// the species-split path.
+struct RedPlan {
+    int ng, w, ld, items, tile;
+    int off_eph, off_acc, off_z0, off_grp, off_scr, grp_bytes, smem_bytes;
+};
 
 // Where the per-point work arrays live: shared memory or the CTA's global slot.
 // Offsets are in bytes (shared) or complex elements (global slot).
@@ -47,41 +64,11 @@ struct Placement {
     int s_smem, t_smem, y_smem, uv_smem;
     int off_s, off_t, off_y, off_uv;     // shared byte offsets (when *_smem)
     int off_piv, off_inv, off_red, off_rot, off_vec;
-    // species-split pairs, two gauge points in flight (when sp2): compact V0^T, U0^T
-    // diagonal blocks at off_uvc, then the two halves' regions (half_layout) from off_half
-    int sp2, off_uvc, off_half;
+    RedPlan gen, spl;                    // reduced pairs: n x n problems, species-split h x h problems
     int smem_bytes;
     long long g_x, g_b, g_p, g_rw, g_zr, g_s, g_t, g_y, g_uv;
     long long slot_elems;
 };
-
-// One half's shared region for the species-split path with two gauge points in flight:
-// byte offsets of the compact densities (rho, kappa10, kappa01, K; each two h x (h + 1)
-// species blocks; the Pfaffian's two h x h blocks come first in the same storage), T22's
-// two blocks, the right-hand sides, the solve's pivot row, the Pfaffian vector and pivots,
-// the accumulators, the final sums, the per-warp partials and the flags.
-constexpr int kHalfThreads = kThreads / 2, kHalfWarps = kHalfThreads / 32;
-struct HalfLayout {
-    int dens, t, y, invd, vec, pfs, acc, fin, pw, sh, bytes;
-};
-__host__ __device__ inline HalfLayout half_layout(int h) {
-    constexpr int zs = 16;   // complex element, both arithmetics
-    HalfLayout L;
-    int o = 0;
-    auto take = [&](int bytes) { const int at = o; o += (bytes + 15) & ~15; return at; };
-    L.dens = take(8 * h * (h + 1) * zs);
-    L.t = take(2 * h * h * zs);
-    L.y = take(4 * h * h * zs);
-    L.invd = take(2 * h * zs);
-    L.vec = take((2 * h + 4) * zs);
-    L.pfs = take(4 * zs);
-    L.acc = take(kNobs * 16);
-    L.fin = take(40 * 8);
-    L.pw = take(4 * kHalfWarps * 8);
-    L.sh = take(16 * 4);
-    L.bytes = o;
-    return L;
-}
 
 // Sparse one-body data used by the observables, built on the host once.
 struct ObsTables {
@@ -125,6 +112,8 @@ struct Params {
     // Hamiltonian two-body list
     int nrec;
     int nrec_gen;              // records [0, nrec_gen): general; [nrec_gen, nrec): a, c protons and b, d neutrons
+    int rec_off[3];            // of the general ones, [0, rec_off[1]): four protons, [.., rec_off[2]): four neutrons
+    int split_ok;              // no other general records and no charge-changing one-body terms
     const uint32_t *rec_idx;   // packed 8-bit a,b,c,d (0-based)
     const double *rec_v;
     const dd *rec_vd;          // rec_v as double-float (df64 form)
@@ -135,6 +124,11 @@ struct Params {
     // per-CTA FP64 accumulators [grid][n_r2q] complex; n_r2q = 0 outside Rho2B launches
     int n_r2q;
     const uint32_t *r2q;
+    // the same quadruples with their index, [r2_off[0], r2_off[1]) four protons, [.., r2_off[2]) four
+    // neutrons, the rest proton-neutron; r2_ss the longer same-species list, -1 when a quadruple
+    // is of another kind
+    const uint2 *r2s;
+    int r2_off[3], r2_ss;
     double *r2acc;
     // tensor-core contraction (contract_tc.cu): tc_splits = 0 runs the record loop here;
     // 2 or 3 makes the point kernel write each gauge point's density rows as that many bf16
@@ -145,6 +139,12 @@ struct Params {
     const int *tc_src;         // [tc_nk]: r << 8 | c (ph entries), i << 8 | j (pp, i < j), -1 padding
     unsigned short *tc_x[3], *tc_y[3];
     double *tc_w;
+    // species-split pairs: per CTA the rows of each species' problems [items][2][NFOM][3 terms][2]
+    // of 2 tc_nk - tc_nph entries, zero outside the 16-byte chunks tc_chunks[tc_choff[s] ..) of
+    // species s
+    unsigned short *tc_sp;
+    const int *tc_chunks;
+    int tc_choff[3];
 };
 
 // One group of the contraction: a contiguous range [off, off + dpad) of the X row (and, for

@@ -4,36 +4,37 @@
 // Work decomposition (one CUDA launch per stage, batched over pairs):
 //   setup_kernel   one CTA per (q,q') pair: W = V1 U1^-1, Z0 = V0 U0^-1, the
 //                  bare-vacuum overlaps det(1 + Z^T Z)^(-1/4) (zbareover,
-//                  Codes/PNAMP/PNAMP_Proj.f90:6-79), and the once-per-pair pieces of
-//                  the reduced Pfaffian (Z0^-1, Pf(-c Z0)) and the species-split flag.
-//   point_kernel   persistent; one CTA per (pair, Euler point) work item at a
-//                  time. Per Euler point it builds the block-diagonal Wigner-D
-//                  rotation R (ROTATION_MAT, PNAMP_Proj.f90:83-136) and the
-//                  gauge-independent pieces X = R W R^T, R V1, R* U1 and the four
-//                  species partials of T22; then for each of the NFOM^2 gauge points:
-//                  the Pfaffian of the point's skew matrix (Pfaf_Over + ZPfaffianF +
-//                  ZExch, PNAMP_Proj.f90:142-392; the n x n Schur complement c (D X D -
-//                  Z0^-1) when V0 is well conditioned, two h x h species blocks for
-//                  charge-conserving pairs, else the 2n x 2n matrix) beside the column
-//                  Gauss-Jordan solve Y T22^-1 on other warps (named barriers), then
-//                  rho, kappa10, kappa01 (ROKAPPAphiomega, :459-551) and the observables
-//                  of Kernel3D.f90:296-358 (ZN_0, the energy of
-//                  PNAMP_Energy_OpenMP.f90:31-90 or the split-bf16 rows for the tensor-
-//                  core contraction in contract_tc.cu, ZJ2_0, ZQ2/ZQ2t), summed into
-//                  ZRES(iang, io) (Kernel3D.f90:385-387). Species-split pairs run two
-//                  gauge points at a time on the two halves of the CTA
-//                  (split_pair_points) with compact species-block densities.
+//                  Codes/PNAMP/PNAMP_Proj.f90:6-79), the once-per-pair pieces of the
+//                  Pfaffians and what kind of points the pair has (pair_kind).
+//   point_kernel   persistent; per Euler point the block-diagonal Wigner-D rotation R
+//                  (ROTATION_MAT, PNAMP_Proj.f90:83-136) and what of it does not depend on
+//                  the gauge angles, then per gauge point the norm (Pfaf_Over + ZPfaffianF +
+//                  ZExch, PNAMP_Proj.f90:142-392), rho, kappa10, kappa01 (ROKAPPAphiomega,
+//                  :459-551) and the observables of Kernel3D.f90:296-358 (ZN_0, the energy of
+//                  PNAMP_Energy_OpenMP.f90:31-90 or the split-bf16 rows for the tensor-core
+//                  contraction in contract_tc.cu, ZJ2_0, ZQ2/ZQ2t), summed into ZRES(iang, io)
+//                  (Kernel3D.f90:385-387). Three bodies by the kind of pair:
+//     split_items    (point_reduced.cuh) no proton-neutron blocks, U0 and V1 well conditioned:
+//                    2 NFOM problems of order n/2 per Euler point, one per species and angle;
+//     reduced_item   (point_reduced.cuh) U0 and V1 well conditioned: NFOM^2 problems of order n;
+//     full_item      the rest (nearly empty or nearly full levels): Pfaffian of the n x n
+//                    Schur complement or the 2n x 2n matrix, Gauss-Jordan solve Y T22^-1.
 //   project_kernel J/K projection of ZRES (Kernel3D.f90:415-751, plain form of
 //                  PNAMP_Kernel3D_v2.f90:477-498).
 //
-// Algebra used instead of the reference's per-point LU inverses (exact in
-// exact arithmetic): with A = D_phi R, D_phi = diag(e^{i phi_p}, e^{i phi_n}),
+// Algebra of full_item instead of the reference's per-point LU inverses (exact in exact
+// arithmetic): with A = D_phi R, D_phi = diag(e^{i phi_p}, e^{i phi_n}),
 //   conj(Vbar1) conj(Ubar1)^-1 = A V1 U1^-1 A^T = D (R W R^T) D,
 //   T22 = V0^T A V1 + U0^T A* U1 = sum_s e^{+-i phi_s} (species partials),
 //   rho = D (R V1 T22^-1) V0^T, kappa10 = D (R V1 T22^-1) U0^T,
 //   kappa01 = -D* (R* U1 T22^-1) V0^T.
+// Measured on GB300, pf shell (n = 40), Euler 10 x 20 x 10, gauge 9 x 9, one pair: charge-conserving
+// FP64 195.3 -> 13.8 ms and double-float 74.7 -> 4.9 ms, proton-neutron mixing with the BF16x6
+// contraction 193.3 -> 69.2 ms, against full_item's algebra for every pair (two points in flight
+// for charge-conserving ones).
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "pnamp_df64.cuh"
@@ -72,7 +73,7 @@ template <> __device__ __forceinline__ double szero<double>() { return 0.0; }
 template <> __device__ __forceinline__ zc szero<zc>() { return mk(0.0, 0.0); }
 // pivot magnitude of a double-float value: the float sum of the high words, compared as a
 // float (the FP64 pipe is narrow on this part, and a float compares the same as its double)
-__device__ __forceinline__ float sabs1(zd a) { return fabsf(a.x.hi) + fabsf(a.y.hi); }
+__device__ __forceinline__ float sabs1(zd a) { return fabsf(f2_a(a.hi)) + fabsf(f2_b(a.hi)); }
 __device__ __forceinline__ zd srecip(zd a) { return zrecip(a); }
 __device__ __forceinline__ zd smul(zd a, zd b) { return a * b; }
 __device__ __forceinline__ zd sfms(zd a, zd b, zd c) { return zfms(a, b, c); }
@@ -90,6 +91,8 @@ template <> struct Ar<zc> {
     static __device__ __forceinline__ bool nz(R a) { return a != 0.0; }
     static __device__ __forceinline__ R pick(const double *d, const dd *, long long i) { return d[i]; }
     static __device__ __forceinline__ R rzero() { return 0.0; }
+    static __device__ __forceinline__ zc neg_real(R a) { return mk(-a, 0.0); }
+    static __device__ __forceinline__ R rneg(R a) { return -a; }
     static __device__ __forceinline__ R rconst(float v) { return (double)v; }   // exact
     static __device__ __forceinline__ R radd(R a, R b) { return a + b; }
     static __device__ __forceinline__ R rfma(R a, R b, R c) { return fma(a, b, c); }
@@ -115,6 +118,8 @@ template <> struct Ar<zd> {
     static __device__ __forceinline__ bool nz(R a) { return a.hi != 0.0f; }
     static __device__ __forceinline__ R pick(const double *, const dd *f, long long i) { return f[i]; }
     static __device__ __forceinline__ R rzero() { return dd_make(0.0f, 0.0f); }
+    static __device__ __forceinline__ zd neg_real(R a) { return mkd(dd_neg(a), dd_make(0.0f, 0.0f)); }
+    static __device__ __forceinline__ R rneg(R a) { return dd_neg(a); }
     static __device__ __forceinline__ R rconst(float v) { return dd_make(v, 0.0f); }   // exact
     static __device__ __forceinline__ R radd(R a, R b) { return dd_add(a, b); }
     static __device__ __forceinline__ R rfma(R a, R b, R c) { return dd_fma(a, b, c); }
@@ -126,8 +131,8 @@ template <> struct Ar<zd> {
         return v;
     }
     static __device__ __forceinline__ unsigned long long key(zd z) {
-        const unsigned int kx = __float_as_uint(z.x.hi) & 0x7fffffffu;
-        const unsigned int ky = __float_as_uint(z.y.hi) & 0x7fffffffu;
+        const unsigned int kx = __float_as_uint(f2_a(z.hi)) & 0x7fffffffu;
+        const unsigned int ky = __float_as_uint(f2_b(z.hi)) & 0x7fffffffu;
         return kx > ky ? kx : ky;
     }
 };
@@ -223,18 +228,16 @@ __device__ bool lu_factor(T *A, int n, int lda, int *perm, T *invd, int *sh) {
 __device__ __forceinline__ unsigned pack_key(float mag, int jrel) {
     return (mag >= 0.0f ? (__float_as_uint(mag) & ~63u) : 0u) | (unsigned)(63 - jrel);
 }
-__device__ __forceinline__ unsigned pack_key_bits(unsigned bits, int jrel) { return (bits & ~63u) | (unsigned)(63 - jrel); }
-// the grouped eliminations search at most n <= PNAMP_MAX_NLEV candidates
 static_assert(PNAMP_MAX_NLEV <= 64, "pivot offsets are packed into 6 bits (7 for the 2n x 2n Pfaffian)");
 
-// A warp-aligned group of the CTA's threads with its own named barrier (bar.sync id,
-// count; id 0 with the whole CTA is __syncthreads). Lets two independent latency-bound
-// eliminations run at the same time on disjoint warps.
+// A warp-aligned group of the CTA's threads that owns one problem, with its named barrier
+// (bar.sync id, count); a one-warp group needs only __syncwarp.
 struct Grp {
-    int tid, nthr, wid, bar;
+    int tid, nthr, bar;
 };
 __device__ __forceinline__ void gsync(const Grp &g) {
-    asm volatile("bar.sync %0, %1;" ::"r"(g.bar), "r"(g.nthr) : "memory");
+    if (g.nthr == 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(g.bar), "r"(g.nthr) : "memory");
 }
 
 // Y <- Y A^-1 (Y: ny x n, A: n x n, both row-major with leading dimension n) by
@@ -351,42 +354,36 @@ __device__ bool gj_right_solve(T *A, int n, T *Y, int ny, T *prow, T *pinv, int 
     return sing;
 }
 
-// gj_right_solve for NB = 1 or 2 independent systems at once, by the thread group g (at
-// least NB warps plus h threads; warp b of the group searches the pivots of system b): A holds
-// NB h x h matrices (compact, the second at A + h*h) and Y NB ny x h blocks (the second at
-// Y + ny*h); Y_b <- Y_b A_b^-1 in h steps of two group barriers. prow holds NB*h scratch
-// values, pinv NB, sh 2*NB ints. Returns true if an exactly zero pivot row was met in any
-// system. NB = 2 serves the two species blocks of a species-split point, NB = 1 the whole
-// n x n system of a general point while other warps eliminate its Pfaffian.
-template <typename T, int NB = 2>
-__device__ bool gj_right_solve_g(const Grp &g, T *A, int h, T *Y, int ny, T *prow, T *pinv, int *sh) {
-    const int lane = g.tid & 31, wid = g.wid;
-    const int hh = h * h, yh = ny * h;
+// gj_right_solve by the thread group g (its first warp searches the pivots): prow holds n
+// scratch values, pinv 1, sh 2 ints. Runs beside the Pfaffian elimination of the same point
+// on other warps.
+template <typename T>
+__device__ bool gj_right_solve_g(const Grp &g, T *A, int n, T *Y, int ny, T *prow, T *pinv, int *sh) {
+    const int lane = g.tid & 31, wid = g.tid >> 5;
     // The search of step k + 1 runs beside each step's updates, on its critical path, so in
     // the double-float form it is one redux.sync; the FP64 form keeps the shuffle search.
     constexpr bool kDF = std::is_same<T, zd>::value;
-    auto search = [&](int b, int k) {  // warp b: pivot column of row k of A_b
-        const T *Ab = A + b * hh;
+    auto search = [&](int k) {  // pivot column of row k
         if constexpr (kDF) {
             unsigned key = 0u;
-            for (int j = k + lane; j < h; j += 32) {
-                const unsigned kk = pack_key(sabs1(Ab[k * h + j]), j - k);
+            for (int j = k + lane; j < n; j += 32) {
+                const unsigned kk = pack_key(sabs1(A[k * n + j]), j - k);
                 key = key > kk ? key : kk;
             }
             const unsigned m = __reduce_max_sync(0xffffffffu, key);
             if (lane == 0) {
                 const int idx = k + 63 - (int)(m & 63u);
                 const bool z = (m >> 6) == 0u;
-                sh[2 * b] = idx;
-                sh[2 * b + 1] = z ? 1 : 0;
-                pinv[b] = z ? szero<T>() : srecip(Ab[k * h + idx]);
+                sh[0] = idx;
+                sh[1] = z ? 1 : 0;
+                pinv[0] = z ? szero<T>() : srecip(A[k * n + idx]);
             }
         } else {
             using Mag = decltype(sabs1(A[0]));
             Mag v = -1;
             int idx = 0x7fffffff;
-            for (int j = k + lane; j < h; j += 32) {
-                const Mag a = sabs1(Ab[k * h + j]);
+            for (int j = k + lane; j < n; j += 32) {
+                const Mag a = sabs1(A[k * n + j]);
                 if (a > v) {
                     v = a;
                     idx = j;
@@ -404,59 +401,51 @@ __device__ bool gj_right_solve_g(const Grp &g, T *A, int h, T *Y, int ny, T *pro
             if (lane == 0) {
                 const bool none = (idx == 0x7fffffff);
                 const bool z = none || v == Mag(0);
-                sh[2 * b] = none ? k : idx;
-                sh[2 * b + 1] = z ? 1 : 0;
-                pinv[b] = z ? szero<T>() : srecip(Ab[k * h + (none ? k : idx)]);
+                sh[0] = none ? k : idx;
+                sh[1] = z ? 1 : 0;
+                pinv[0] = z ? szero<T>() : srecip(A[k * n + (none ? k : idx)]);
             }
         }
     };
     bool sing = false;
-    // phase-2 layout of warps NB..: rpi rows at a time, one column per thread
-    constexpr int kRes = 32 * NB;
-    const int rpi = (g.nthr - kRes) / h, jc = (g.tid - kRes) % h, r0 = (g.tid - kRes) / h;
-    if (wid < NB) search(wid, 0);
+    // phase-2 layout of the other warps: rpi rows at a time, one column per thread
+    const int rpi = (g.nthr - 32) / n, jc = (g.tid - 32) % n, r0 = (g.tid - 32) / n;
+    if (wid == 0) search(0);
     gsync(g);
-    for (int k = 0; k < h; ++k) {
-        const int c0 = sh[0], c1 = NB > 1 ? sh[2] : 0;
-        if (sh[1] || (NB > 1 && sh[3])) sing = true;
-        // phase 1 (all systems): m_r = M[r][c] / A[k][c] into column k, old column k into
-        // column c, the exchanged pivot row into prow
-        const int nrT = h - k - 1, nrows = nrT + ny, per1 = nrows + h;
-        for (int t = g.tid; t < NB * per1; t += g.nthr) {
-            const int b = t >= per1 ? 1 : 0, u = t - b * per1;
-            const int c = b ? c1 : c0;
-            T *Ab = A + b * hh;
-            if (u < nrows) {
-                T *row = u < nrT ? Ab + (k + 1 + u) * h : Y + b * yh + (u - nrT) * h;
+    for (int k = 0; k < n; ++k) {
+        const int c = sh[0];
+        if (sh[1]) sing = true;
+        // phase 1: m_r = M[r][c] / A[k][c] into column k, old column k into column c, the
+        // exchanged pivot row into prow
+        const int nrT = n - k - 1, nrows = nrT + ny;
+        for (int t = g.tid; t < nrows + n; t += g.nthr) {
+            if (t < nrows) {
+                T *row = t < nrT ? A + (k + 1 + t) * n : Y + (t - nrT) * n;
                 const T a = row[c], bb = row[k];
-                row[k] = smul(a, pinv[b]);
+                row[k] = smul(a, pinv[0]);
                 if (c != k) row[c] = bb;
             } else {
-                const int j = u - nrows;
-                prow[b * h + j] = (j == c) ? Ab[k * h + k] : Ab[k * h + j];
+                const int j = t - nrows;
+                prow[j] = (j == c) ? A[k * n + k] : A[k * n + j];
             }
         }
         gsync(g);
-        // phase 2: M[r][j] -= m_r prow[j] for j != k; warp b takes row k + 1 of A_b, then its pivot
-        if (wid < NB) {
-            if (k + 1 < h) {
-                T *row = A + wid * hh + (k + 1) * h;
+        // phase 2: M[r][j] -= m_r prow[j] for j != k; warp 0 takes row k + 1 of A, then its pivot
+        if (wid == 0) {
+            if (k + 1 < n) {
+                T *row = A + (k + 1) * n;
                 const T m = row[k];
-                for (int j = lane; j < h; j += 32)
-                    if (j != k) row[j] = sfms(m, prow[wid * h + j], row[j]);
+                for (int j = lane; j < n; j += 32)
+                    if (j != k) row[j] = sfms(m, prow[j], row[j]);
                 __syncwarp();
-                search(wid, k + 1);
+                search(k + 1);
             }
         } else if (r0 < rpi && jc != k) {
-            // thread (r0, jc): column jc of every rpi-th row of all systems; the pivot-row
-            // values stay in registers and m_r = row[k] is a broadcast load
-            const int nrA = h - k - 2 > 0 ? h - k - 2 : 0;
-            const int rows_b = nrA + ny;
-            const T pj0 = prow[jc], pj1 = NB > 1 ? prow[h + jc] : pj0;
-            for (int R = r0; R < NB * rows_b; R += rpi) {
-                const int b = R >= rows_b ? 1 : 0, rr = R - b * rows_b;
-                T *row = rr < nrA ? A + b * hh + (k + 2 + rr) * h : Y + b * yh + (rr - nrA) * h;
-                row[jc] = sfms(row[k], b ? pj1 : pj0, row[jc]);
+            const int nrA = n - k - 2 > 0 ? n - k - 2 : 0;
+            const T pj = prow[jc];
+            for (int R = r0; R < nrA + ny; R += rpi) {
+                T *row = R < nrA ? A + (k + 2 + R) * n : Y + (R - nrA) * n;
+                row[jc] = sfms(row[k], pj, row[jc]);
             }
         }
         gsync(g);
@@ -548,22 +537,31 @@ template <class Z> struct PfProd;
 template <> struct PfProd<zc> {
     zc v = {1.0, 0.0};
     __device__ __forceinline__ void mul(zc f, bool neg) { v = (neg ? -1.0 : 1.0) * (v * f); }
+    // times the product of the lane o away
+    __device__ __forceinline__ void join(int o) {
+        v = v * mk(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+    }
     __device__ __forceinline__ zc get() const { return v; }
 };
 template <> struct PfProd<zd> {
-    zd m = {{1.0f, 0.0f}, {0.0f, 0.0f}};
+    zd m = {f2_make(1.0f, 0.0f), f2_make(0.0f, 0.0f)};
     int e = 0;
+    __device__ __forceinline__ void join(int o) {
+        zd f;
+        f.hi.u = __shfl_xor_sync(0xffffffffu, m.hi.u, o);
+        f.lo.u = __shfl_xor_sync(0xffffffffu, m.lo.u, o);
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+        mul(f, false);
+    }
     __device__ __forceinline__ void mul(zd f, bool neg) {
         m = m * f;
         if (neg) m = -m;
-        const float a = fmaxf(fabsf(m.x.hi), fabsf(m.y.hi));
+        const float a = fmaxf(fabsf(f2_a(m.hi)), fabsf(f2_b(m.hi)));
         if (a > 0.0f && a <= 3.0e38f) {
             int ex;
             frexpf(a, &ex);
-            m.x.hi = ldexpf(m.x.hi, -ex);
-            m.x.lo = ldexpf(m.x.lo, -ex);
-            m.y.hi = ldexpf(m.y.hi, -ex);
-            m.y.lo = ldexpf(m.y.lo, -ex);
+            m.hi = f2_make(ldexpf(f2_a(m.hi), -ex), ldexpf(f2_b(m.hi), -ex));
+            m.lo = f2_make(ldexpf(f2_a(m.lo), -ex), ldexpf(f2_b(m.lo), -ex));
             e += ex;
         }
     }
@@ -576,7 +574,7 @@ template <> struct PfProd<zd> {
 __device__ __forceinline__ int pivot_flag(zc ss) { return !zfinite(ss) ? 2 : (!(abs2(ss) > 1.0e-26) ? 1 : 0); }
 __device__ __forceinline__ int pivot_flag(zd ss) {
     if (!zfinite(ss)) return 2;
-    const float a = fabsf(ss.x.hi), b = fabsf(ss.y.hi);
+    const float a = fabsf(f2_a(ss.hi)), b = fabsf(f2_b(ss.hi));
     // |ss|^2 > 1e-26 in float (the sum of squares underflows only far below the threshold)
     return (a > 1.0e-13f || b > 1.0e-13f || a * a + b * b > 1.0e-26f) ? 0 : 1;
 }
@@ -675,160 +673,131 @@ __device__ zc pfaffian_upper(Z *S, int N, Z *vec, double *red, int *flag, int &u
     return threadIdx.x == 0 ? pf.get() : mk(0.0, 0.0);
 }
 
-// Pfaffians of two independent skew h x h matrices stored compactly (upper triangles,
-// row-major, ld h, the second at S + h*h), eliminated together by the thread group g:
-// each step takes both 2x2 pivots (row pivoting as in pfaffian_upper; warp b of the group
-// searches matrix b), so the species-split form of a point needs h/2 - 1 steps for both
-// species. Two group barriers per step: (a) the exchange of column c with the pivot column
-// and the scaled pivot row v = S[c][.] / S[r][c] in one pass, (b) the rank-2 update, in
-// which warp b first updates the next pivot row of matrix b and searches it (pivot index,
-// value and reciprocal for the next step), then joins the rest of the update. A small pivot
+// Pfaffian of the skew n x n matrix in the upper triangle of S (row-major) by the thread group
+// g, row pivoting as in pfaffian_upper. Two group barriers per step: (a) the exchange of
+// column c with the pivot column and the scaled pivot row v = S[c][.] / S[r][c] in one pass,
+// (b) the rank-2 update, in which the first warp updates the next pivot row and searches it
+// (pivot index, value and reciprocal for the next step), then joins the rest. A small pivot
 // (|S[r][c]|^2 <= 1e-26, PNAMP_Proj.f90:290,333) or a non-finite one is recorded and the
 // elimination runs on (its values are discarded): the result is 0 with `underflow` set.
-// Returns Pf(first) * Pf(second) and `underflow` in the group's thread 0. `vec` holds 2h
-// scratch values, `pv` 4 (pivots and reciprocals), `flag` 4 ints.
-// NB = 1 is the same elimination of one h x h matrix (a general point's n x n Schur
-// complement, eliminated while the other warps run the Gauss-Jordan solve).
-template <class Z, int NB = 2>
-__device__ zc pfaffian_upper_g(const Grp &g, Z *S, int h, Z *vec, Z *pv, int *flag, int &underflow) {
+// Returns the Pfaffian and `underflow` in the group's thread 0. `vec` holds n scratch values,
+// `pv` 2 (pivot and reciprocal), `flag` 2 ints.
+template <class Z>
+__device__ zc pfaffian_upper_g(const Grp &g, Z *S, int n, Z *vec, Z *pv, int *flag, int &underflow) {
     using A = Ar<Z>;
-    const int lane = g.tid & 31, wid = g.wid;
-    const int hh = h * h;
-    const int nstep = h / 2 - 1;
+    const int lane = g.tid & 31, wid = g.tid >> 5;
+    const int nstep = n / 2 - 1;
     PfProd<Z> pf;
     int uf = 0;
-    // warp b: pivot of row r of matrix b over columns c..h-1 -> flag[b] (index), flag[2 + b]
-    // (0 fine, 1 small, 2 non-finite), pv[b] (value), pv[2 + b] (reciprocal)
-    auto search = [&](int b, int r) {
-        const Z *Sb = S + b * hh;
-        if constexpr (std::is_same<Z, zd>::value) {   // one redux.sync; candidates r + 1 .. h - 1 exist
+    auto search = [&](int r) {   // pivot of row r -> flag[0] index, flag[1] its test, pv
+        int q;
+        bool none = false;
+        if constexpr (std::is_same<Z, zd>::value) {   // one redux.sync; candidates r + 1 .. n - 1 exist
             unsigned key = 0u;
-            for (int j = r + 1 + lane; j < h; j += 32) {
-                const unsigned kk = pack_key_bits((unsigned)A::key(Sb[r * h + j]), j - r - 1);
+            for (int j = r + 1 + lane; j < n; j += 32) {
+                const unsigned kk = ((unsigned)A::key(S[r * n + j]) & ~63u) | (unsigned)(63 - (j - r - 1));
                 key = key > kk ? key : kk;
             }
-            const unsigned m = __reduce_max_sync(0xffffffffu, key);
-            if (lane == 0) {
-                const int q = r + 1 + 63 - (int)(m & 63u);
-                const Z ssz = Sb[r * h + q];
-                const int f = pivot_flag(ssz);
-                flag[b] = q;
-                flag[2 + b] = f;
-                pv[b] = ssz;
-                pv[2 + b] = f ? ssz : zrecip(ssz);
+            q = r + 1 + 63 - (int)(__reduce_max_sync(0xffffffffu, key) & 63u);
+        } else {
+            unsigned long long best = 0ull;
+            int bidx = 0x7fffffff;
+            for (int j = r + 1 + lane; j < n; j += 32) {
+                const unsigned long long key = A::key(S[r * n + j]);
+                if (key > best || bidx == 0x7fffffff) {
+                    best = key;
+                    bidx = j;
+                }
             }
-            return;
-        }
-        unsigned long long best = 0ull;
-        int bidx = 0x7fffffff;
-        for (int j = r + 1 + lane; j < h; j += 32) {
-            const unsigned long long key = A::key(Sb[r * h + j]);
-            if (key > best || bidx == 0x7fffffff) {
-                best = key;
-                bidx = j;
-            }
-        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long ob = __shfl_down_sync(0xffffffffu, best, o);
-            const int oi = __shfl_down_sync(0xffffffffu, bidx, o);
-            if (oi != 0x7fffffff && (bidx == 0x7fffffff || ob > best || (ob == best && oi < bidx))) {
-                best = ob;
-                bidx = oi;
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long ob = __shfl_down_sync(0xffffffffu, best, o);
+                const int oi = __shfl_down_sync(0xffffffffu, bidx, o);
+                if (oi != 0x7fffffff && (bidx == 0x7fffffff || ob > best || (ob == best && oi < bidx))) {
+                    best = ob;
+                    bidx = oi;
+                }
             }
+            none = bidx == 0x7fffffff;
+            q = none ? r + 1 : bidx;
         }
         if (lane == 0) {
-            const int q = (bidx == 0x7fffffff) ? r + 1 : bidx;  // at least one candidate when r + 1 < h
-            const Z ssz = Sb[r * h + q];
-            const int f = (bidx == 0x7fffffff) ? 2 : pivot_flag(ssz);
-            flag[b] = q;
-            flag[2 + b] = f;
-            pv[b] = ssz;
-            pv[2 + b] = f ? ssz : zrecip(ssz);
+            const Z ssz = S[r * n + q];
+            const int f = none ? 2 : pivot_flag(ssz);
+            flag[0] = q;
+            flag[1] = f;
+            pv[0] = ssz;
+            pv[1] = f ? ssz : zrecip(ssz);
         }
     };
-    // warp w serves matrices w, w + nwg, ...: one warp per matrix, or one warp for both
-    const int nwg = g.nthr >> 5;
-    for (int b = wid; nstep > 0 && b < NB; b += nwg) search(b, 0);
+    if (wid == 0 && nstep > 0) search(0);
     gsync(g);
     for (int k = 0; k < nstep; ++k) {
         const int r = 2 * k, c = r + 1;
-        const int q0 = flag[0], q1 = NB > 1 ? flag[1] : 0;
+        const int q = flag[0];
         if (g.tid == 0) {
-            const int fk = (NB > 1 && flag[3] > flag[2]) ? flag[3] : flag[2];
-            if (uf == 0) uf = fk;  // the first failing step decides, as the early return did
-            for (int b = 0; b < NB; ++b) pf.mul(pv[b], (b ? q1 : q0) != c);
+            if (uf == 0) uf = flag[1];  // the first failing step decides, as an early return would
+            pf.mul(pv[0], q != c);
         }
-        // (a) exchange c <-> q (exch_upper on every matrix) and v_i = S'[c][i] / S'[r][c], i > c
-        for (int t = g.tid; t < NB * (h - r); t += g.nthr) {
-            const int b = t / (h - r), i = r + t % (h - r);
-            const int q = b ? q1 : q0;
-            const Z inv = pv[2 + b];
-            Z *Sb = S + b * hh;
-            Z *vb = vec + b * h;
+        // (a) exchange c <-> q (exch_upper) and v_i = S'[c][i] / S'[r][c], i > c
+        for (int i = r + g.tid; i < n; i += g.nthr) {
+            const Z inv = pv[1];
             if (q == c) {
-                if (i > c) vb[i] = Sb[c * h + i] * inv;
+                if (i > c) vec[i] = S[c * n + i] * inv;
                 continue;
             }
             if (i < c) {  // i == r: the pivot moves to column c
-                const Z x = Sb[i * h + c];
-                Sb[i * h + c] = Sb[i * h + q];
-                Sb[i * h + q] = x;
+                const Z x = S[i * n + c];
+                S[i * n + c] = S[i * n + q];
+                S[i * n + q] = x;
             } else if (i > q) {
-                const Z x = Sb[c * h + i];
-                const Z y = Sb[q * h + i];
-                Sb[c * h + i] = y;
-                Sb[q * h + i] = x;
-                vb[i] = y * inv;
+                const Z x = S[c * n + i];
+                const Z y = S[q * n + i];
+                S[c * n + i] = y;
+                S[q * n + i] = x;
+                vec[i] = y * inv;
             } else if (i > c && i < q) {
-                const Z x = Sb[c * h + i];
-                const Z y = -Sb[i * h + q];
-                Sb[c * h + i] = y;
-                Sb[i * h + q] = -x;
-                vb[i] = y * inv;
+                const Z x = S[c * n + i];
+                const Z y = -S[i * n + q];
+                S[c * n + i] = y;
+                S[i * n + q] = -x;
+                vec[i] = y * inv;
             } else if (i == c) {  // S'[c][q] = -S[c][q]; its thread also sets v_q
-                const Z y = -Sb[c * h + q];
-                Sb[c * h + q] = y;
-                vb[q] = y * inv;
+                const Z y = -S[c * n + q];
+                S[c * n + q] = y;
+                vec[q] = y * inv;
             }
         }
         gsync(g);
         // (b) S_ij += v_i S_rj - S_ri v_j for c < i < j; row c + 1 (the next pivot row) first
-        const bool more = k + 1 < nstep;
-        for (int b = wid; b < NB; b += nwg) {
-            Z *Sb = S + b * hh;
-            const Z *vb = vec + b * h;
+        if (wid == 0) {
             const int i = c + 1;
-            const Z vi = vb[i], sri = Sb[r * h + i];
-            for (int j = i + 1 + lane; j < h; j += 32) {
-                Z sv = Sb[i * h + j];
-                sv = zfma(vi, Sb[r * h + j], sv);
-                sv = zfms(sri, vb[j], sv);
-                Sb[i * h + j] = sv;
+            const Z vi = vec[i], sri = S[r * n + i];
+            for (int j = i + 1 + lane; j < n; j += 32) {
+                Z sv = S[i * n + j];
+                sv = zfma(vi, S[r * n + j], sv);
+                sv = zfms(sri, vec[j], sv);
+                S[i * n + j] = sv;
             }
             __syncwarp();
-            if (more) search(b, c + 1);
+            if (k + 1 < nstep) search(c + 1);
         }
-        const int mm = h - c - 2, TT = mm * (mm - 1) / 2;
-        for (int t = g.tid; t < NB * TT; t += g.nthr) {
-            const int b = t / TT;
+        const int mm = n - c - 2, TT = mm * (mm - 1) / 2;
+        for (int t = g.tid; t < TT; t += g.nthr) {
             int i, j;
-            tri_index(t - b * TT, mm, i, j);
+            tri_index(t, mm, i, j);
             i += c + 2;
             j += c + 2;
-            Z *Sb = S + b * hh;
-            const Z *vb = vec + b * h;
-            Z sv = Sb[i * h + j];
-            sv = zfma(vb[i], Sb[r * h + j], sv);
-            sv = zfms(Sb[r * h + i], vb[j], sv);
-            Sb[i * h + j] = sv;
+            Z sv = S[i * n + j];
+            sv = zfma(vec[i], S[r * n + j], sv);
+            sv = zfms(S[r * n + i], vec[j], sv);
+            S[i * n + j] = sv;
         }
         gsync(g);
     }
     zc out = mk(0.0, 0.0);
     if (g.tid == 0) {
-        pf.mul(S[(h - 2) * h + h - 1], false);
-        if (NB > 1) pf.mul(S[hh + (h - 2) * h + h - 1], false);
+        pf.mul(S[(n - 2) * n + n - 1], false);
         if (!uf) out = pf.get();
     }
     underflow = uf;
@@ -836,6 +805,17 @@ __device__ zc pfaffian_upper_g(const Grp &g, Z *S, int h, Z *vec, Z *pv, int *fl
 }
 
 // ------------------------------------------------------------------ setup
+// min |U_kk| >= ratio x max |U_kk| over the pivots of a factored matrix, and max > 0.
+__device__ __forceinline__ bool pivots_within(const double *A, int n, double ratio) {
+    double mx = 0.0, mn = 1e300;
+    for (int k = 0; k < n; ++k) {
+        const double d = fabs(A[k * n + k]);
+        mx = fmax(mx, d);
+        mn = fmin(mn, d);
+    }
+    return mx > 0.0 && mn >= ratio * mx;
+}
+
 __global__ void __launch_bounds__(kSetupThreads)
 setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairbuf) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -858,6 +838,7 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
     }
     __syncthreads();
     int st = 0;
+    bool u0_ok = false;
     for (int which = 0; which < 2; ++which) {
         const double *U = out + (which == 0 ? p.pl.u1 : p.pl.u0);
         const double *V = out + (which == 0 ? p.pl.v1 : p.pl.v0);
@@ -868,6 +849,7 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
         }
         __syncthreads();
         if (lu_factor<double>(A, n, n, perm, invd, sh)) st = 1;
+        if (which == 1) u0_ok = pivots_within(A, n, kReducedPivotRatio);
         row_solve<double>(Yb, n, n, A, n, n, perm, invd);  // Z = V U^-1
         for (long long t = threadIdx.x; t < nn; t += blockDim.x) Z[t] = Yb[t];
         __syncthreads();
@@ -886,62 +868,61 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
         if (threadIdx.x == 0) out[p.pl.dets + (which == 0 ? 1 : 0)] = exp(-0.25 * v[0]);
         __syncthreads();
     }
-    // Reduced Pfaffian data: block elimination of the lower-right block of
-    // S = c [[D X D, -I], [I, -Z0]] gives Pf(S) = Pf(c (D X D - Z0^-1)) Pf(-c Z0), so the point
-    // kernel can eliminate an n x n matrix per point. Kept only when V0 is well conditioned
-    // (Z0^-1 = U0 V0^-1 accurate); otherwise the flag stays 0 and the 2n x 2n form is used.
-    {
-        const double *U0 = out + p.pl.u0, *V0 = out + p.pl.v0, *Z0 = out + p.pl.z0;
+    // Once-per-pair pieces of the Pfaffians. Reduced pairs (V1 and U0 well conditioned): W^-1 and
+    // Pf(c W) for point_reduced.cuh. Others with a well conditioned V0: block elimination of the
+    // lower-right block of S = c [[D X D, -I], [I, -Z0]] gives Pf(S) = Pf(c (D X D - Z0^-1))
+    // Pf(-c Z0). Otherwise both flags stay 0 and the 2n x 2n form is used.
+    double schur = 0.0, reduced = 0.0;
+    zc pf = mk(0.0, 0.0);
+    for (int kind = 0; kind < 2 && schur == 0.0 && reduced == 0.0; ++kind) {
+        if (kind == 0 && !u0_ok) continue;
+        const double *U = out + (kind == 0 ? p.pl.u1 : p.pl.u0), *V = out + (kind == 0 ? p.pl.v1 : p.pl.v0);
+        const double *Z = out + (kind == 0 ? p.pl.w : p.pl.z0);
+        const double f = kind == 0 ? p.cscale : -p.cscale;
         for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
-            A[t] = V0[t];
-            Yb[t] = U0[t];
+            A[t] = V[t];
+            Yb[t] = U[t];
         }
         __syncthreads();
         const bool vsing = lu_factor<double>(A, n, n, perm, invd, sh);
-        if (threadIdx.x == 0) {
-            double mx = 0.0, mn = 1e300;
-            for (int k = 0; k < n; ++k) {
-                const double d = fabs(A[k * n + k]);
-                mx = fmax(mx, d);
-                mn = fmin(mn, d);
-            }
-            red[0] = (!vsing && mx > 0.0 && mn >= kReducedPivotRatio * mx) ? 1.0 : 0.0;
+        const bool well = !vsing && pivots_within(A, n, kReducedPivotRatio);
+        __syncthreads();
+        if (!well) continue;
+        row_solve<double>(Yb, n, n, A, n, n, perm, invd);  // U V^-1
+        int big = 0;
+        for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
+            out[p.pl.zi + t] = Yb[t];
+            if (!(fabs(Yb[t]) <= kReducedMaxEntry)) big = 1;
+        }
+        if (__syncthreads_or(big) && kind == 0) continue;
+        zc *Sz = reinterpret_cast<zc *>(A);  // n^2 complex over A and Yb
+        for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
+            const int i = (int)(t / n), j = (int)(t % n);
+            Sz[t] = mk(i < j ? f * Z[t] : 0.0, 0.0);
         }
         __syncthreads();
-        const bool well = red[0] != 0.0;
-        __syncthreads();
-        double ok = 0.0;
-        zc pf = mk(0.0, 0.0);
-        if (well) {
-            row_solve<double>(Yb, n, n, A, n, n, perm, invd);  // U0 V0^-1
-            for (long long t = threadIdx.x; t < nn; t += blockDim.x) out[p.pl.zi + t] = Yb[t];
-            __syncthreads();
-            zc *Sz = reinterpret_cast<zc *>(A);  // n^2 complex over A and Yb
-            for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
-                const int i = (int)(t / n), j = (int)(t % n);
-                Sz[t] = mk(i < j ? -p.cscale * Z0[t] : 0.0, 0.0);
-            }
-            __syncthreads();
-            int under = 0;
-            pf = pfaffian_upper<zc>(Sz, n, vecz, red, sh, under);
-            ok = (under == 0 && zfinite(pf)) ? 1.0 : 0.0;
-        }
-        // species split: U0, V0, U1, V1 without proton-neutron blocks (charge-conserving vacua)
-        // make every per-point matrix block-diagonal by species (protons first, h = n/2 each)
-        int cross = 0;
-        for (long long t = threadIdx.x; t < 4 * nn; t += blockDim.x) {
-            const long long e = t % nn;
-            const int i = (int)(e / n), j = (int)(e % n);
-            if ((i < p.h) != (j < p.h) && out[t] != 0.0) cross = 1;  // U0, V0, U1, V1 lead the record
-        }
-        cross = __syncthreads_or(cross);
-        if (threadIdx.x == 0) {
-            out[p.pl.dets + 2] = (double)st;
-            out[p.pl.dets + 3] = ok;
-            out[p.pl.pfz] = pf.x;
-            out[p.pl.pfz + 1] = pf.y;
-            out[p.pl.dets + 6] = (ok != 0.0 && !cross) ? 1.0 : 0.0;
-        }
+        int under = 0;
+        pf = pfaffian_upper<zc>(Sz, n, vecz, red, sh, under);   // in thread 0
+        const double ok = __syncthreads_and(threadIdx.x != 0 || (under == 0 && zfinite(pf))) ? 1.0 : 0.0;
+        if (kind == 0) reduced = ok;
+        else schur = ok;
+    }
+    // species split: U0, V0, U1, V1 without proton-neutron blocks (charge-conserving vacua)
+    // make every per-point matrix block-diagonal by species (protons first, h = n/2 each)
+    int cross = 0;
+    for (long long t = threadIdx.x; t < 4 * nn; t += blockDim.x) {
+        const long long e = t % nn;
+        const int i = (int)(e / n), j = (int)(e % n);
+        if ((i < p.h) != (j < p.h) && out[t] != 0.0) cross = 1;  // U0, V0, U1, V1 lead the record
+    }
+    cross = __syncthreads_or(cross);
+    if (threadIdx.x == 0) {
+        out[p.pl.dets + 2] = (double)st;
+        out[p.pl.dets + 3] = schur;
+        out[p.pl.pfz] = pf.x;
+        out[p.pl.pfz + 1] = pf.y;
+        out[p.pl.dets + 6] = cross ? 0.0 : 1.0;
+        out[p.pl.dets + 7] = reduced;
     }
 }
 
@@ -978,8 +959,8 @@ cudaError_t launch_setup(const Params &p, int npairs, const double *uv, double *
 static_assert(sizeof(dd) == sizeof(double), "per-warp double-float partials share the double slots of red");
 constexpr int kNSlot = 36;  // observable sums: slots 0..37 final values, then per-warp partials
 constexpr int kR1BSlot = 128;  // one-body density block sums: red[kR1BSlot + 2b], re and im
+constexpr int kPfScratch = 608;  // point-arithmetic values: the grouped Pfaffian's pivot and reciprocal
 constexpr int kR2Norm = 260;   // the gauge point's norm, re and im, for the two-body density pass
-constexpr int kPfScratch = 608;  // 4 point-arithmetic values (<= 64 B): species Pfaffian pivots
 static_assert(kThreads >= 32 * (kNTrace + 1), "one warp per Q trace plus warp 0");
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -988,382 +969,16 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// ---- species-split pairs, two gauge points in flight --------------------------------------
-// The CTA's two halves (8 warps each) take alternate gauge points of the Euler point and run
-// them independently: in each half warps 0-1 eliminate the two species' Schur-complement
-// blocks while warps 2-7 solve the two T22 systems (named barriers 1 + 3 s and 2 + 3 s for
-// half s), and one half-wide barrier (3 + 3 s) separates the densities, K and the
-// observables; warp 0 of each half accumulates its gauge points. A step of one half that
-// waits on a barrier leaves the SM to the other half, which the single-point path (one CTA
-// of 16 warps per gauge point) cannot do. The densities are stored compactly, two h x (h + 1)
-// species blocks per density (the proton-neutron blocks of a split pair vanish). Thread 0
-// sums the halves' accumulators at the end.
-template <class Z>
-__device__ __forceinline__ void split_pair_points(const Params &p, unsigned char *smem, const Z *X, const Z *P,
-                                                  const Z *B, const Z *CZ, const Z *ephz, zc pfz, double det0,
-                                                  double det1, int pair, int ie, long long pt0, double *gout,
-                                                  double *zout, int *status) {
-    using A = Ar<Z>;
-    using R = typename A::R;
-    const int n = p.n, h = p.h, nn = n * n;
-    const int half = threadIdx.x / kHalfThreads, lt = threadIdx.x % kHalfThreads;
-    const int lane = lt & 31, lw = lt >> 5;
-    const HalfLayout L = half_layout(h);
-    unsigned char *hb = smem + p.place.off_half + half * L.bytes;
-    const int hl = h + 1, bs = h * hl, ds = 2 * bs, hh = h * h;   // compact row stride, block, density
-    Z *Dn = reinterpret_cast<Z *>(hb + L.dens);
-    Z *rhoC = Dn, *k10C = Dn + ds, *k01C = Dn + 2 * ds, *KcC = Dn + 3 * ds;
-    Z *S2 = Dn;
-    Z *T2 = reinterpret_cast<Z *>(hb + L.t), *Y2 = reinterpret_cast<Z *>(hb + L.y);
-    Z *inv2 = reinterpret_cast<Z *>(hb + L.invd), *vec2 = reinterpret_cast<Z *>(hb + L.vec);
-    Z *pfs2 = reinterpret_cast<Z *>(hb + L.pfs);
-    zc *acc2 = reinterpret_cast<zc *>(hb + L.acc);
-    double *fin2 = reinterpret_cast<double *>(hb + L.fin);
-    R *pw2 = reinterpret_cast<R *>(hb + L.pw);
-    int *sh2 = reinterpret_cast<int *>(hb + L.sh);   // [0, 4) Pfaffian, [4, 8) solve, [8] flags
-    // compact V0^T, U0^T: species b, [b][k][j] = V0(b h + j, b h + k)
-    const R *V0c = reinterpret_cast<const R *>(smem + p.place.off_uvc), *U0c = V0c + 2 * hh;
-    const int barH = 3 + 3 * half;
-    // one warp eliminates both species' Pfaffians (it finished at half the solve's time on
-    // two), so the Gauss-Jordan group, the critical path, has seven of the half's eight warps
-    constexpr int kPfW2 = 1;
-    auto hsync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(barH), "r"(kHalfThreads) : "memory"); };
-    // compact index of (r, c), r and c of the same species
-    auto cidx = [&](int r, int c) {
-        const int b = r >= h ? 1 : 0;
-        return b * bs + (r - b * h) * hl + (c - b * h);
-    };
-    const Z zero = A::from(mk(0.0, 0.0));
-    const Z csz = A::from(mk(p.cscale, 0.0));
-    for (int io = lt; io < kNobs; io += kHalfThreads) acc2[io] = mk(0.0, 0.0);
-    if (lt == 0) sh2[8] = 0;
-    hsync();
-    for (int gi = half; gi < p.n_gauge; gi += 2) {
-        const int lp = gi / p.nfom, ln = gi % p.nfom;
-        const Z zep = ephz[lp], zepc = zconj(zep), zen = ephz[ln], zenc = zconj(zen);
-        const Z dpp = csz * (zep * zep), dnn = csz * (zen * zen);
-        int under = 0;
-        zc pf = mk(0.0, 0.0);
-        bool sing = false;
-        if (lw < kPfW2) {   // the two species' Schur-complement blocks and their Pfaffians
-            const Grp g{lt, 32 * kPfW2, lw, 1 + 3 * half};
-            const int Th = h * (h - 1) / 2;
-            for (int t = g.tid; t < 2 * Th; t += g.nthr) {
-                const int b = t >= Th ? 1 : 0;
-                int i, j;
-                tri_index(t - b * Th, h, i, j);
-                const int gi_ = b * h + i, gj_ = b * h + j;
-                S2[b * hh + i * h + j] = X[gi_ * n + gj_] * (b ? dnn : dpp) + CZ[gi_ * n + gj_];
-            }
-            gsync(g);
-            pf = pfaffian_upper_g<Z, 2>(g, S2, h, vec2, pfs2, sh2, under);
-            pf = pf * pfz;   // meaningful in the half's thread 0
-        } else if (!p.norm_only) {   // T22 blocks, right-hand sides, Y T22^-1
-            const Grp g{lt - 32 * kPfW2, kHalfThreads - 32 * kPfW2, lw - kPfW2, 2 + 3 * half};
-            for (int t = g.tid; t < 2 * hh; t += g.nthr) {
-                const int b = t >= hh ? 1 : 0, e = t - b * hh, i = e / h, j = e % h;
-                const int gg = (b * h + i) * n + b * h + j;
-                Z sv = zep * P[gg];
-                sv = zfma(zen, P[nn + gg], sv);
-                sv = zfma(zepc, P[2 * nn + gg], sv);
-                sv = zfma(zenc, P[3 * nn + gg], sv);
-                T2[t] = sv;
-            }
-            for (int t = g.tid; t < 4 * hh; t += g.nthr) {
-                const int b = t >= 2 * hh ? 1 : 0, e = t - 2 * b * hh, r = e / h, j = e % h;
-                const int grow = r < h ? b * h + r : n + b * h + (r - h);
-                Y2[t] = B[grow * n + b * h + j];
-            }
-            gsync(g);
-            const bool sg = gj_right_solve_g<Z, 2>(g, T2, h, Y2, 2 * h, inv2, vec2 + 2 * h, sh2 + 4);
-            if (g.tid == 0) sh2[4] = sg ? 1 : 0;
-        }
-        hsync();
-        if (!p.norm_only) sing = sh2[4] != 0;
-        if (!p.norm_only) {
-            // ---- densities of each species block (rho, kappa10, kappa01 share the loads)
-            for (int t = lt; t < 2 * hh; t += kHalfThreads) {
-                const int b = t >= hh ? 1 : 0, e = t - b * hh, i = e / h, j = e % h;
-                const Z *Yt = Y2 + 2 * b * hh + i * h;
-                const Z *Yb = Yt + hh;
-                const R *Mv = V0c + b * hh + j, *Mu = U0c + b * hh + j;
-                Z sr = zero, s10 = zero, s01 = zero;
-                for (int k = 0; k < h; ++k) {
-                    const Z yt = Yt[k];
-                    const R mv = Mv[k * h];
-                    sr = rfma(mv, yt, sr);
-                    s10 = rfma(Mu[k * h], yt, s10);
-                    s01 = rfma(mv, Yb[k], s01);
-                }
-                const Z di = b ? zen : zep;
-                const int o = b * bs + i * hl + j;
-                rhoC[o] = di * sr;
-                k10C[o] = di * s10;
-                k01C[o] = -(zconj(di) * s01);
-            }
-            hsync();
-            // ---- K01_ij (i < j) at K[i][j], K10_ij at K[j][i], within each block
-            {
-                const int Th = h * (h - 1) / 2;
-                for (int t = lt; t < 2 * Th; t += kHalfThreads) {
-                    const int b = t >= Th ? 1 : 0;
-                    int i, j;
-                    tri_index(t - b * Th, h, i, j);
-                    const int oij = b * bs + i * hl + j, oji = b * bs + j * hl + i;
-                    KcC[oij] = k01C[oij] - k01C[oji];
-                    KcC[oji] = k10C[oij] - k10C[oji];
-                }
-            }
-            hsync();
-            // ---- observables: 13 trace jobs over the half's 8 warps (job = lw, lw + 8); then
-            // the energy (records, or the bf16 rows of the tensor-core forms) and <J^2>
-            for (int job = lw; job < kNTrace + 3; job += kHalfWarps) {
-                if (job == 0 || job == kNTrace + 1 || job == kNTrace + 2) {
-                    R v0 = A::rzero(), v1 = v0, v2 = v0, v3 = v0, v4 = v0, v5 = v0;
-                    if (job == 0) {
-                        for (int a = lane; a < n; a += 32) {
-                            const Z d = rhoC[cidx(a, a)];
-                            if (a < h) { v0 = A::radd(v0, d.x); v1 = A::radd(v1, d.y); }
-                            else { v2 = A::radd(v2, d.x); v3 = A::radd(v3, d.y); }
-                            const R jj = A::pick(p.obs.jj1, p.obs.jj1_d, a);
-                            v4 = A::rfma(jj, d.x, v4);
-                            v5 = A::rfma(jj, d.y, v5);
-                        }
-                    } else if (job == kNTrace + 1) {
-                        for (int a = lane; a < n; a += 32) {
-                            const R jpa = A::pick(p.obs.jp, p.obs.jp_d, a), jma = A::pick(p.obs.jm, p.obs.jm_d, a);
-                            const R mza = A::pick(p.obs.mz, p.obs.mz_d, a);
-                            if (A::nz(jpa)) {
-                                const Z r = rhoC[cidx(a + 1, a)];
-                                v0 = A::rfma(jpa, r.x, v0);
-                                v1 = A::rfma(jpa, r.y, v1);
-                            }
-                            if (A::nz(jma)) {
-                                const Z r = rhoC[cidx(a - 1, a)];
-                                v2 = A::rfma(jma, r.x, v2);
-                                v3 = A::rfma(jma, r.y, v3);
-                            }
-                            const Z d = rhoC[cidx(a, a)];
-                            v4 = A::rfma(mza, d.x, v4);
-                            v5 = A::rfma(mza, d.y, v5);
-                        }
-                    } else {
-                        for (int e = lane; e < p.obs.n_t1b; e += 32) {
-                            const int ix = p.obs.t1b_idx[e], r = ix >> 8, c = ix & 255;
-                            if ((r >= h) != (c >= h)) continue;
-                            const Z rv = rhoC[cidx(r, c)];
-                            const R tv = A::pick(p.obs.t1b_val, p.obs.t1b_val_d, e);
-                            v0 = A::rfma(tv, rv.x, v0);
-                            v1 = A::rfma(tv, rv.y, v1);
-                        }
-                    }
-                    const int s0 = job == 0 ? 0 : (job == kNTrace + 1 ? 10 : 4);
-                    const int cnt = job == kNTrace + 2 ? 2 : 6;
-                    const R vals[6] = {v0, v1, v2, v3, v4, v5};
-#pragma unroll
-                    for (int q = 0; q < 6; ++q) {
-                        if (q >= cnt) break;
-                        const R v = A::wsum(vals[q]);
-                        const int slot = (job == 0 && q >= 4) ? 12 + q : s0 + q;
-                        if (lane == 0) fin2[slot] = A::dbl(v);
-                    }
-                } else if (p.iE2) {   // Q_{2mu} trace job - 1
-                    const int q = job - 1;
-                    R sr = A::rzero(), si = A::rzero();
-                    for (int e = p.obs.q_off[q] + lane; e < p.obs.q_off[q + 1]; e += 32) {
-                        const int ix = p.obs.q_idx[e], r = ix >> 8, c = ix & 255;
-                        if ((r >= h) != (c >= h)) continue;
-                        const Z rv = rhoC[cidx(r, c)];
-                        const R qv = A::pick(p.obs.q_val, p.obs.q_val_d, e);
-                        sr = A::rfma(qv, rv.x, sr);
-                        si = A::rfma(qv, rv.y, si);
-                    }
-                    sr = A::wsum(sr);
-                    si = A::wsum(si);
-                    if (lane == 0) {
-                        fin2[18 + 2 * q] = A::dbl(sr);
-                        fin2[19 + 2 * q] = A::dbl(si);
-                    }
-                }
-            }
-            auto put = [&](int slot, R v) {   // slot 0..3: energy re/im, <J^2> re/im
-                v = A::wsum(v);
-                if (lane == 0) pw2[slot * kHalfWarps + lw] = v;
-            };
-            if (p.tc_splits) {   // the gauge point's split-bf16 rows for the tensor-core contraction
-                const long long pt = pt0 + gi;
-                const int S = p.tc_splits, nk = p.tc_nk, npp = p.tc_nk - p.tc_nph;
-                for (int e = lt; e < nk; e += kHalfThreads) {
-                    const int src = p.tc_src[e];
-                    Z v = zero, y = zero;
-                    if (src >= 0) {
-                        const int r = src >> 8, c = src & 255;
-                        if ((r >= h) == (c >= h)) {   // the proton-neutron entries vanish
-                            if (e < p.tc_nph) {
-                                v = rhoC[cidx(r, c)];
-                            } else {
-                                v = KcC[cidx(c, r)];   // K10_rc, r < c
-                                y = KcC[cidx(r, c)];   // K01_rc
-                            }
-                        }
-                    }
-                    unsigned short tr[3], ti[3];
-                    bf16_terms(as_dd(v.x), S, tr);
-                    bf16_terms(as_dd(v.y), S, ti);
-                    for (int sp = 0; sp < S; ++sp) {
-                        p.tc_x[sp][(2 * pt) * nk + e] = tr[sp];
-                        p.tc_x[sp][(2 * pt + 1) * nk + e] = ti[sp];
-                    }
-                    if (e >= p.tc_nph) {
-                        bf16_terms(as_dd(y.x), S, tr);
-                        bf16_terms(as_dd(y.y), S, ti);
-                        const int ey = e - p.tc_nph;
-                        for (int sp = 0; sp < S; ++sp) {
-                            p.tc_y[sp][(2 * pt) * npp + ey] = tr[sp];
-                            p.tc_y[sp][(2 * pt + 1) * npp + ey] = ti[sp];
-                        }
-                    }
-                }
-                if (lane == 0) {
-                    pw2[lw] = A::rzero();
-                    pw2[kHalfWarps + lw] = A::rzero();
-                }
-            } else {   // two-body energy: the point kernel's record loop on the compact blocks
-                const R quarter = A::rconst(0.25f);
-                Z e2 = zero;
-                // same-species records: all four indices in species block b
-                for (int e = lt; e < p.nrec_gen; e += kHalfThreads) {
-                    const uint32_t pk = p.rec_idx[e];
-                    const R v = A::pick(p.rec_v, p.rec_vd, e);
-                    int i = pk & 0xff, j = (pk >> 8) & 0xff, k = (pk >> 16) & 0xff, l = pk >> 24;
-                    const bool sym = i + j != k + l;
-                    const int b = i >= h ? 1 : 0, o = b * bs;
-                    i -= b * h;
-                    j -= b * h;
-                    k -= b * h;
-                    l -= b * h;
-                    Z t = rhoC[o + k * hl + i] * rhoC[o + l * hl + j];
-                    t = zfms(rhoC[o + l * hl + i], rhoC[o + k * hl + j], t);
-                    Z u = KcC[o + i * hl + j] * KcC[o + l * hl + k];
-                    if (sym) {
-                        t = zfma(rhoC[o + i * hl + k], rhoC[o + j * hl + l], t);
-                        t = zfms(rhoC[o + j * hl + k], rhoC[o + i * hl + l], t);
-                        u = zfma(KcC[o + k * hl + l], KcC[o + j * hl + i], u);
-                    }
-                    t = rfma(quarter, u, t);
-                    e2 = rfma(v, t, e2);
-                }
-                // proton-neutron records: (i, k) protons, (j, l) neutrons; only the direct terms
-                for (int e = p.nrec_gen + lt; e < p.nrec; e += kHalfThreads) {
-                    const uint32_t pk = p.rec_idx[e];
-                    const R v = A::pick(p.rec_v, p.rec_vd, e);
-                    const int i = pk & 0xff, j = ((pk >> 8) & 0xff) - h, k = (pk >> 16) & 0xff, l = (pk >> 24) - h;
-                    Z t = rhoC[k * hl + i] * rhoC[bs + l * hl + j];
-                    if (i + j != k + l) t = zfma(rhoC[i * hl + k], rhoC[bs + j * hl + l], t);
-                    e2 = rfma(v, t, e2);
-                }
-                put(0, e2.x);
-                put(1, e2.y);
-            }
-            {   // <J^2>, the same terms as the single-point path, within the species blocks
-                const R half_ = A::rconst(0.5f);
-                Z rest = zero;
-                for (int t = lt; t < 2 * hh; t += kHalfThreads) {
-                    const int blk = t >= hh ? 1 : 0, e = t - blk * hh;
-                    const int a = blk * h + e / h, c = blk * h + e % h;
-                    const R jpa = A::pick(p.obs.jp, p.obs.jp_d, a), jma = A::pick(p.obs.jm, p.obs.jm_d, a);
-                    const R jpc = A::pick(p.obs.jp, p.obs.jp_d, c), jmc = A::pick(p.obs.jm, p.obs.jm_d, c);
-                    const R mzz = A::rmul(A::pick(p.obs.mz, p.obs.mz_d, a), A::pick(p.obs.mz, p.obs.mz_d, c));
-                    const int ac = cidx(a, c);
-                    Z q = mzz * (k10C[ac] * k01C[ac]);
-                    q = zfms(mzz * rhoC[ac], rhoC[cidx(c, a)], q);
-                    if (A::nz(jpa) && A::nz(jmc))
-                        q = zfms(A::rmul(jpa, jmc) * rhoC[ac + hl], rhoC[cidx(c - 1, a)], q);
-                    if (A::nz(jpa) && A::nz(jpc))
-                        q = zfma(A::rmul(half_, A::rmul(jpa, jpc)) * k10C[ac + hl], k01C[ac + 1], q);
-                    if (A::nz(jma) && A::nz(jmc))
-                        q = zfma(A::rmul(half_, A::rmul(jma, jmc)) * k10C[ac - hl], k01C[ac - 1], q);
-                    rest = rest + q;
-                }
-                put(2, rest.x);
-                put(3, rest.y);
-            }
-        }
-        hsync();
-        if (lw == 0) {   // accumulation over this half's gauge points (single-lane FP64 values)
-            const unsigned full = 0xffffffffu;
-            R ws[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) ws[q] = A::wsum(lane < kHalfWarps ? pw2[q * kHalfWarps + lane] : A::rzero());
-            const bool eval = !p.norm_only && !sing;
-            zc norm = mk(0.0, 0.0);
-            if (lane == 0) {
-                const zc zph = mk(p.gphase[2 * gi], p.gphase[2 * gi + 1]);
-                norm = (p.vacfac * det0 * det1) * (pf * zph);
-            }
-            norm.x = __shfl_sync(full, norm.x, 0);
-            norm.y = __shfl_sync(full, norm.y, 0);
-            zc o = mk(0.0, 0.0), hg = mk(0.0, 0.0);
-            bool use = eval;
-            if ((lane == 6 || (lane == 0 && gout)) && eval)
-                hg = mk(fin2[4] + A::dbl(ws[0]) + p.e0, fin2[5] + A::dbl(ws[1]));
-            if (lane == 1) o = mk(fin2[0], fin2[1]);
-            else if (lane == 2) o = mk(fin2[2], fin2[3]);
-            else if (lane == 3) o = mk(fin2[4], fin2[5]);
-            else if (lane == 6) o = hg;
-            else if (lane == 7) {
-                const zc trp = mk(fin2[10], fin2[11]), trm = mk(fin2[12], fin2[13]), trz = mk(fin2[14], fin2[15]);
-                o = mk(fin2[16] + A::dbl(ws[2]), fin2[17] + A::dbl(ws[3])) + trp * trm + trz * trz;
-            } else if (lane >= 8 && lane < 18 && p.iE2) o = mk(fin2[2 * lane + 2], fin2[2 * lane + 3]);
-            else use = false;
-            if (p.tc_splits && lane == 0) {
-                const long long pt = pt0 + gi;
-                const double inv = 1.0 / ((double)p.nfom * p.nfom);
-                p.tc_w[2 * pt] = eval ? inv * norm.x : 0.0;
-                p.tc_w[2 * pt + 1] = eval ? inv * norm.y : 0.0;
-            }
-            if (lane == 0) {
-                acc2[0] = acc2[0] + norm;
-                if (gout) {
-                    double *g = gout + 4LL * (((long long)pair * p.n_euler + ie) * p.n_gauge + gi);
-                    g[0] = norm.x;
-                    g[1] = norm.y;
-                    g[2] = hg.x;
-                    g[3] = hg.y;
-                }
-                int f = (under == 1) ? 1 : (under == 2 ? 4 : 0);
-                if (!p.norm_only && sing) f |= 2;
-                sh2[8] |= f;
-            }
-            if (use) acc2[lane] = zfma(norm, o, acc2[lane]);
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {   // the two halves' sums
-        const zc *a0 = reinterpret_cast<const zc *>(smem + p.place.off_half + L.acc);
-        const zc *a1 = reinterpret_cast<const zc *>(smem + p.place.off_half + L.bytes + L.acc);
-        const int f0 = reinterpret_cast<const int *>(smem + p.place.off_half + L.sh)[8];
-        const int f1 = reinterpret_cast<const int *>(smem + p.place.off_half + L.bytes + L.sh)[8];
-        const double inv = 1.0 / ((double)p.nfom * p.nfom);
-        int f = f0 | f1;
-        for (int io = 0; io < kNobs; ++io) {
-            const zc v = io == kNobs - 1 ? mk(0.0, 0.0) : inv * (a0[io] + a1[io]);
-            if (!zfinite(v)) f |= 4;
-            zout[2LL * (io * p.n_euler + ie)] = v.x;
-            zout[2LL * (io * p.n_euler + ie) + 1] = v.y;
-        }
-        status[(long long)pair * p.n_euler + ie] = f;
-    }
-    __syncthreads();
-}
+}  // namespace pnamp
+#include "point_reduced.cuh"
+namespace pnamp {
 
-// One work item: Euler point `ie` of pair `pair`, all its gauge points, in the
-// CTA's workspace `slot`. `reload` is set when the previous item of this CTA
-// belonged to another pair (or context): V0^T, U0^T and the phase tables are
-// then (re)loaded.
+// One Euler point of a pair whose V0 is ill conditioned (nearly empty levels in the bra): the
+// 2n x 2n Pfaffian or, for NFOM = 1, the Onishi norm, and an n x n solve, by the whole CTA.
+// `reload` is set when the previous item of this CTA belonged to another pair (or context):
+// V0^T, U0^T and the phase tables are then (re)loaded.
 template <class Z>
-__device__ __forceinline__ void point_item(const Params &p, const double *__restrict__ pairbuf, zc *slot,
+__device__ __noinline__ void full_item(const Params &p, const double *__restrict__ pairbuf, zc *slot,
                                            int pair, int ie, bool reload, double *__restrict__ zres,
                                            int *__restrict__ status, double *__restrict__ gout = nullptr,
                                            double *__restrict__ r1out = nullptr,
@@ -1381,8 +996,8 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
     zc *Bz = slot + pl.g_b;                         // the same storage while it holds FP64 values
     Z *P = reinterpret_cast<Z *>(slot + pl.g_p);    // T22 partials: V0p, V0n, U0p, U0n
     zc *RW = slot + pl.g_rw;                        // R W
-    // -Cscale Z0^-1 (reduced pairs) or -Cscale Z0: the constant block of the Pfaffian matrix,
-    // converted once per pair so that building S takes no FP64 work per gauge point
+    // -Cscale Z0 (or -Cscale Z0^-1): the constant block of the Pfaffian matrix, converted once
+    // per pair so that building S takes no FP64 work per gauge point
     Z *CZ = reinterpret_cast<Z *>(slot + pl.g_zr);
     Z *S = reinterpret_cast<Z *>(pl.s_smem ? (void *)(smem + pl.off_s) : (void *)(slot + pl.g_s));
     Z *T = reinterpret_cast<Z *>(pl.t_smem ? (void *)(smem + pl.off_t) : (void *)(slot + pl.g_t));
@@ -1407,50 +1022,22 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
     {
         const double *pr = pairbuf + (long long)pair * p.pl.stride;
         const double *gU1 = pr + p.pl.u1, *gV1 = pr + p.pl.v1, *gU0 = pr + p.pl.u0, *gV0 = pr + p.pl.v0;
-        const double *gW = pr + p.pl.w, *gZ0 = pr + p.pl.z0;
+        const double *gW = pr + p.pl.w;
         const double det0 = pr[p.pl.dets], det1 = pr[p.pl.dets + 1];
-        const int pst = (int)pr[p.pl.dets + 2];
-        // reduced Pfaffian (set-up kernel): eliminate c (D X D - Z0^-1), n x n, times Pf(-c Z0)
-        const bool reduced = pr[p.pl.dets + 3] != 0.0;
-        const double *gZi = pr + p.pl.zi;
+        // V0 well conditioned: the n x n Schur
+        // complement c (D X D - Z0^-1), times Pf(-c Z0), instead of the 2n x 2n matrix
+        const bool schur = pr[p.pl.dets + 3] != 0.0;
+        const double *gZc = pr + (schur ? p.pl.zi : p.pl.z0);
         const zc pfz = mk(pr[p.pl.pfz], pr[p.pl.pfz + 1]);
-        const int NP = reduced ? n : N;  // order of the eliminated skew matrix
-        // species split (set-up kernel): no proton-neutron blocks, so the Schur complement, T22,
-        // the solve and the densities are block-diagonal; both species are eliminated together
-        // on compact h x h blocks
-        const bool split = reduced && pr[p.pl.dets + 6] != 0.0;
-        // two gauge points in flight (split_pair_points) when the halves' storage fits
-        const bool use2 = pl.sp2 && split && p.nfom > 1 && !r2out && !r1out && blockDim.x == kThreads;
+        const int NP = N;  // order of the skew matrix the whole CTA eliminates
         double *zout = zres + 2LL * (long long)pair * kNobs * p.n_euler;
-        if (pst) {
-            for (int io = threadIdx.x; io < kNobs; io += blockDim.x) {
-                zout[2LL * (io * p.n_euler + ie)] = 0.0;
-                zout[2LL * (io * p.n_euler + ie) + 1] = 0.0;
-            }
-            if (threadIdx.x == 0) status[(long long)pair * p.n_euler + ie] = 8;
-            for (int g = threadIdx.x; g < (p.tc_splits ? p.n_gauge : 0); g += blockDim.x) {
-                p.tc_w[2 * (pt0 + g)] = 0.0;
-                p.tc_w[2 * (pt0 + g) + 1] = 0.0;
-            }
-            return;
-        }
         if (reload) {
             __syncthreads();
             for (int t = threadIdx.x; t < nn; t += blockDim.x) {
                 const int k = t / n, j = t % n;
-                if (!use2) {
-                    V0t[t] = A::real(gV0[j * n + k]);
-                    U0t[t] = A::real(gU0[j * n + k]);
-                }
-                CZ[t] = A::from(mk(-p.cscale * (reduced ? gZi[t] : gZ0[t]), 0.0));
-            }
-            if (use2) {   // the diagonal species blocks only: [b][k][j] = V0(b h + j, b h + k)
-                R *V0c = reinterpret_cast<R *>(smem + pl.off_uvc), *U0c = V0c + 2 * h * h;
-                for (int t = threadIdx.x; t < 2 * h * h; t += blockDim.x) {
-                    const int b = t / (h * h), e = t % (h * h), k = e / h, j = e % h;
-                    V0c[t] = A::real(gV0[(b * h + j) * n + b * h + k]);
-                    U0c[t] = A::real(gU0[(b * h + j) * n + b * h + k]);
-                }
+                V0t[t] = A::real(gV0[j * n + k]);
+                U0t[t] = A::real(gU0[j * n + k]);
+                CZ[t] = A::from(mk(-p.cscale * gZc[t], 0.0));
             }
             for (int l = threadIdx.x; l < p.nfom; l += blockDim.x) {
                 const zc e = expi(p.nfom == 1 ? 0.0 : twopi * l / p.nfom);
@@ -1458,19 +1045,7 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                 ephz[l] = A::from(e);
             }
         }
-        // ---- rotation blocks R_b(i,k) = e^{-i alp m_i} d^j_{m_i m_k}(bet) e^{-i gam m_k}  (FP64)
-        const double alp = p.euler[4 * ie], bet = p.euler[4 * ie + 1], gam = p.euler[4 * ie + 2];
-        double cb, sb;
-        sincos(0.5 * bet, &sb, &cb);
-        for (int b = 0; b < p.nblk; ++b) {
-            const int d = p.blk_size[b], tj = p.blk_tj[b], ro = p.blk_roff[b];
-            for (int e = threadIdx.x; e < d * d; e += blockDim.x) {
-                const int i = e / d, k = e % d;
-                const int mi = tj - 2 * i, mkk = tj - 2 * k;
-                const double dv = wigner_d(tj, mi, mkk, cb, sb, p.fact);
-                rot[ro + e] = dv * expi(-0.5 * (alp * mi + gam * mkk));
-            }
-        }
+        rotation_blocks(p, ie, threadIdx.x, blockDim.x, rot);
         if (threadIdx.x == 0) {
             for (int io = 0; io < kNobs; ++io) acc[io] = mk(0.0, 0.0);
             for (int b = 0; b < (r1out ? p.obs.n_r1b : 0); ++b) acc_r1b[b] = mk(0.0, 0.0);
@@ -1528,10 +1103,6 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
             B[t] = A::from(v);
         }
         __syncthreads();
-        if (use2) {
-            split_pair_points<Z>(p, smem, X, P, B, CZ, ephz, pfz, det0, det1, pair, ie, pt0, gout, zout, status);
-            return;
-        }
 
         int flags = 0;
         const Z zero = A::from(mk(0.0, 0.0));
@@ -1540,28 +1111,18 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
             const Z zep = ephz[lp], zepc = zconj(zep);
             for (int ln = 0; ln < p.nfom; ++ln) {
                 const Z zen = ephz[ln], zenc = zconj(zen);
-                // ---- S = Cscale [[D X D, -I], [I, -Z0]] (upper triangle), or for a reduced
-                // pair its Schur complement Cscale (D X D - Z0^-1) (n x n, row stride n)
+                // ---- S = Cscale [[D X D, -I], [I, -Z0]] (upper triangle)
                 const Z dpp = csz * (zep * zep), dpn = csz * (zep * zen), dnn = csz * (zen * zen);
-                // species split: warps 0-1 build and eliminate the two Schur-complement blocks
-                // while warps 2-15 build T22 and Y and run the Gauss-Jordan solve (named barriers
-                // 1 and 2); both are latency-bound, so running them side by side hides the
-                // Pfaffians behind the solve, which is the longer of the two (per-group clock
-                // marks: the Pfaffian group of 4 warps finished at 60-76 % of the solve; with the
-                // two-barrier Pfaffian 2, 3 and 4 Pfaffian warps time within 0.4 % of each other,
-                // so the solve keeps 14). One CTA barrier joins them before the densities.
-                const bool conc = split && !onishi;
-                // general reduced points (vacua that mix protons and neutrons): the same overlap of
-                // the n x n Schur complement's elimination (warps 0 .. kPfWarpsG-1, named barrier 1)
-                // with the n x n Gauss-Jordan solve on the other warps (named barrier 2)
-                const bool concg = !split && reduced && !onishi;
                 int under = 0;
                 zc pf = mk(0.0, 0.0);
                 bool sing = false;
+                // the Schur complement's elimination (warps 0 .. kPfWarpsG-1, named barrier 1) beside
+                // the Gauss-Jordan solve on the other warps (named barrier 2)
+                const bool concg = schur && !onishi;
                 if (concg) {
                     constexpr int kPfWarpsG = 3;
                     if (wid < kPfWarpsG) {
-                        const Grp g{(int)threadIdx.x, kPfWarpsG * 32, wid, 1};
+                        const Grp g{(int)threadIdx.x, kPfWarpsG * 32, 1};
                         for (int t = g.tid; t < n * (n - 1) / 2; t += g.nthr) {
                             int i, j;
                             tri_index(t, n, i, j);
@@ -1569,11 +1130,10 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                             S[i * n + j] = X[i * n + j] * dd_ + CZ[i * n + j];
                         }
                         gsync(g);
-                        pf = pfaffian_upper_g<Z, 1>(g, S, n, vec, reinterpret_cast<Z *>(red + kPfScratch), sh, under);
+                        pf = pfaffian_upper_g<Z>(g, S, n, vec, reinterpret_cast<Z *>(red + kPfScratch), sh, under);
                         pf = pf * pfz;  // meaningful in thread 0
                     } else if (!p.norm_only) {
-                        const Grp g{(int)threadIdx.x - kPfWarpsG * 32, (int)blockDim.x - kPfWarpsG * 32,
-                                    wid - kPfWarpsG, 2};
+                        const Grp g{(int)threadIdx.x - kPfWarpsG * 32, (int)blockDim.x - kPfWarpsG * 32, 2};
                         for (int t = g.tid; t < nn; t += g.nthr) {
                             Z sv = zep * P[t];
                             sv = zfma(zen, P[nn + t], sv);
@@ -1583,61 +1143,19 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                         }
                         for (int t = g.tid; t < 2 * nn; t += g.nthr) Y[t] = B[t];
                         gsync(g);
-                        const bool sg = gj_right_solve_g<Z, 1>(g, T, n, Y, 2 * n, invd, vec + n, sh + 4);
+                        const bool sg = gj_right_solve_g<Z>(g, T, n, Y, 2 * n, invd, vec + n, sh + 4);
                         if (g.tid == 0) sh[4] = sg ? 1 : 0;
                     }
                     __syncthreads();
                     if (!p.norm_only) sing = sh[4] != 0;
                 }
-                if (conc) {
-                    constexpr int kPfWarps = 2;  // the two pivot searches need one warp each
-                    if (wid < kPfWarps) {
-                        const Grp g{(int)threadIdx.x, kPfWarps * 32, wid, 1};
-                        const int Th = h * (h - 1) / 2;
-                        for (int t = g.tid; t < 2 * Th; t += g.nthr) {
-                            const int b = t >= Th ? 1 : 0;
-                            int i, j;
-                            tri_index(t - b * Th, h, i, j);
-                            const int gi = b * h + i, gj = b * h + j;
-                            Z v = X[gi * n + gj] * (b ? dnn : dpp);
-                            v = v + CZ[gi * n + gj];
-                            S[b * h * h + i * h + j] = v;
-                        }
-                        gsync(g);
-                        pf = pfaffian_upper_g<Z, 2>(g, S, h, vec, reinterpret_cast<Z *>(red + kPfScratch), sh, under);
-                        pf = pf * pfz;  // meaningful in thread 0
-                    } else if (!p.norm_only) {
-                        const Grp g{(int)threadIdx.x - kPfWarps * 32, (int)blockDim.x - kPfWarps * 32,
-                                    wid - kPfWarps, 2};
-                        for (int t = g.tid; t < 2 * h * h; t += g.nthr) {
-                            const int b = t >= h * h ? 1 : 0, e = t - b * h * h, i = e / h, j = e % h;
-                            const int gg = (b * h + i) * n + b * h + j;
-                            Z sv = zep * P[gg];
-                            sv = zfma(zen, P[nn + gg], sv);
-                            sv = zfma(zepc, P[2 * nn + gg], sv);
-                            sv = zfma(zenc, P[3 * nn + gg], sv);
-                            T[t] = sv;
-                        }
-                        for (int t = g.tid; t < 4 * h * h; t += g.nthr) {
-                            const int b = t >= 2 * h * h ? 1 : 0, e = t - 2 * b * h * h, r = e / h, j = e % h;
-                            const int grow = r < h ? b * h + r : n + b * h + (r - h);
-                            Y[t] = B[grow * n + b * h + j];
-                        }
-                        gsync(g);
-                        const bool sg = gj_right_solve_g<Z, 2>(g, T, h, Y, 2 * h, invd, vec + 2 * h, sh + 4);
-                        if (g.tid == 0) sh[4] = sg ? 1 : 0;
-                    }
-                    __syncthreads();
-                    if (!p.norm_only) sing = sh[4] != 0;
-                }
-                for (int t = threadIdx.x; t < (onishi || split || concg ? 0 : NP * (NP - 1) / 2); t += blockDim.x) {
+                for (int t = threadIdx.x; t < (onishi || concg ? 0 : NP * (NP - 1) / 2); t += blockDim.x) {
                     int i, j;
                     tri_index(t, NP, i, j);
                     Z v;
                     if (j < n) {
                         const Z dd_ = (j < h) ? dpp : ((i < h) ? dpn : dnn);
                         v = X[i * n + j] * dd_;
-                        if (reduced) v = v + CZ[i * n + j];
                     } else if (i < n) {
                         v = (j - n == i) ? mcs : zero;
                     } else {
@@ -1645,8 +1163,8 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                     }
                     S[i * NP + j] = v;
                 }
-                if (!conc && !concg) __syncthreads();
-                if (conc || concg) {
+                if (!concg) __syncthreads();
+                if (concg) {
                 } else if (onishi) {
                     // Onishi (PNAMP_Onishi.f90:21-37): sqrt(det(Ubar^T U0 + Vbar^T V0)),
                     // Ubar = R U1, Vbar = conj(R) V1 at phi = 0; LU determinant, principal root
@@ -1679,7 +1197,6 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                     __syncthreads();
                 } else {
                     pf = pfaffian_upper<Z>(S, NP, vec, red, sh + 2, under);
-                    if (reduced) pf = pf * pfz;  // meaningful in thread 0, like pf
                 }
                 // fin: final sums (double); pwR: per-warp energy and <J^2> partials in R (8 bytes,
                 // like a double, in both forms)
@@ -1687,53 +1204,6 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                 R *pwR = reinterpret_cast<R *>(red + kNSlot + 2);
                 if (!p.norm_only) {  // uniform over the block: norm-only launches skip the densities
                 // ---- T22(phi) and right-hand sides
-                if (split) {  // compact species blocks: T_b (h x h), Y_b = [R V1; R* U1] rows and columns of b
-                    for (int t = threadIdx.x; t < (conc ? 0 : 2 * h * h); t += blockDim.x) {
-                        const int b = t >= h * h ? 1 : 0, e = t - b * h * h, i = e / h, j = e % h;
-                        const int g = (b * h + i) * n + b * h + j;
-                        Z s = zep * P[g];
-                        s = zfma(zen, P[nn + g], s);
-                        s = zfma(zepc, P[2 * nn + g], s);
-                        s = zfma(zenc, P[3 * nn + g], s);
-                        T[t] = s;
-                    }
-                    for (int t = threadIdx.x; t < (conc ? 0 : 4 * h * h); t += blockDim.x) {
-                        const int b = t >= 2 * h * h ? 1 : 0, e = t - 2 * b * h * h, r = e / h, j = e % h;
-                        const int grow = r < h ? b * h + r : n + b * h + (r - h);
-                        Y[t] = B[grow * n + b * h + j];
-                    }
-                    if (!conc) {  // (Onishi norm) the whole CTA solves after the norm
-                        __syncthreads();
-                        const Grp gall{(int)threadIdx.x, (int)blockDim.x, wid, 0};
-                        sing = gj_right_solve_g<Z, 2>(gall, T, h, Y, 2 * h, invd, vec, sh);
-                    }
-                    // densities of each species block in one pass (rho, kappa10 and kappa01 of an
-                    // entry share the loads of Y and V0^T), and zeros across the species
-                    for (int t = threadIdx.x; t < 2 * h * h; t += blockDim.x) {
-                        const int b = t >= h * h ? 1 : 0, e = t - b * h * h, i = e / h, j = e % h;
-                        const Z *Yt = Y + 2 * b * h * h + i * h;   // R V1 T22^-1 rows of species b
-                        const Z *Yb = Yt + h * h;                  // R* U1 T22^-1 rows
-                        const R *Mv = V0t + (b * h) * n + b * h + j, *Mu = U0t + (b * h) * n + b * h + j;
-                        Z sr = zero, s10 = zero, s01 = zero;
-                        for (int k = 0; k < h; ++k) {
-                            const Z yt = Yt[k];
-                            const R mv = Mv[k * n];
-                            sr = rfma(mv, yt, sr);
-                            s10 = rfma(Mu[k * n], yt, s10);
-                            s01 = rfma(mv, Yb[k], s01);
-                        }
-                        const Z di = b ? zen : zep;
-                        const int o = (b * h + i) * ld + b * h + j;
-                        S[o] = di * sr;
-                        S[n * ld + o] = di * s10;
-                        S[2 * n * ld + o] = -(zconj(di) * s01);
-                    }
-                    for (int t = threadIdx.x; t < 6 * h * h; t += blockDim.x) {  // cross-species zeros
-                        const int q = t / (2 * h * h), e = t % (2 * h * h), b = e >= h * h ? 1 : 0;
-                        const int i = (e - b * h * h) / h, j = (e - b * h * h) % h;
-                        S[q * n * ld + (b * h + i) * ld + (1 - b) * h + j] = zero;
-                    }
-                } else {
                 if (!concg) {  // (2n x 2n Pfaffian or Onishi norm) the whole CTA solves after the norm
                     for (int t = threadIdx.x; t < nn; t += blockDim.x) {
                         Z s = zep * P[t];
@@ -1770,7 +1240,6 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                         }
                     }
                 }
-                }  // split
                 __syncthreads();
                 // K01_ij (i < j) at Kc[i ld + j], K10_ij at Kc[j ld + i]
                 for (int t = threadIdx.x; t < n * (n - 1) / 2; t += blockDim.x) {
@@ -1791,11 +1260,11 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                     if (wid == 0) {
                         for (int a = lane; a < n; a += 32) {
                             const Z d = rho[a * ld + a];
-                            if (a < h) { v0 = A::radd(v0, d.x); v1 = A::radd(v1, d.y); }
-                            else { v2 = A::radd(v2, d.x); v3 = A::radd(v3, d.y); }
+                            if (a < h) { v0 = A::radd(v0, re(d)); v1 = A::radd(v1, im(d)); }
+                            else { v2 = A::radd(v2, re(d)); v3 = A::radd(v3, im(d)); }
                             const R jj = A::pick(p.obs.jj1, p.obs.jj1_d, a);
-                            v4 = A::rfma(jj, d.x, v4);
-                            v5 = A::rfma(jj, d.y, v5);
+                            v4 = A::rfma(jj, re(d), v4);
+                            v5 = A::rfma(jj, im(d), v5);
                         }
                     } else if (wid == kNTrace + 1) {
                         for (int a = lane; a < n; a += 32) {
@@ -1803,25 +1272,25 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                             const R mza = A::pick(p.obs.mz, p.obs.mz_d, a);
                             if (A::nz(jpa)) {
                                 const Z r = rho[(a + 1) * ld + a];
-                                v0 = A::rfma(jpa, r.x, v0);
-                                v1 = A::rfma(jpa, r.y, v1);
+                                v0 = A::rfma(jpa, re(r), v0);
+                                v1 = A::rfma(jpa, im(r), v1);
                             }
                             if (A::nz(jma)) {
                                 const Z r = rho[(a - 1) * ld + a];
-                                v2 = A::rfma(jma, r.x, v2);
-                                v3 = A::rfma(jma, r.y, v3);
+                                v2 = A::rfma(jma, re(r), v2);
+                                v3 = A::rfma(jma, im(r), v3);
                             }
                             const Z d = rho[a * ld + a];
-                            v4 = A::rfma(mza, d.x, v4);
-                            v5 = A::rfma(mza, d.y, v5);
+                            v4 = A::rfma(mza, re(d), v4);
+                            v5 = A::rfma(mza, im(d), v5);
                         }
                     } else {
                         for (int e = lane; e < p.obs.n_t1b; e += 32) {
                             const int ix = p.obs.t1b_idx[e];
                             const Z r = rho[(ix >> 8) * ld + (ix & 255)];
                             const R tv = A::pick(p.obs.t1b_val, p.obs.t1b_val_d, e);
-                            v0 = A::rfma(tv, r.x, v0);
-                            v1 = A::rfma(tv, r.y, v1);
+                            v0 = A::rfma(tv, re(r), v0);
+                            v1 = A::rfma(tv, im(r), v1);
                         }
                     }
                     // result slots: z 0,1  n 2,3  t1b 4,5  J+ 10,11  J- 12,13  Jz 14,15  j(j+1) 16,17
@@ -1842,8 +1311,8 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                         const int ix = p.obs.q_idx[e];
                         const Z r = rho[(ix >> 8) * ld + (ix & 255)];
                         const R qv = A::pick(p.obs.q_val, p.obs.q_val_d, e);
-                        sr = A::rfma(qv, r.x, sr);
-                        si = A::rfma(qv, r.y, si);
+                        sr = A::rfma(qv, re(r), sr);
+                        si = A::rfma(qv, im(r), si);
                     }
                     sr = A::wsum(sr);
                     si = A::wsum(si);
@@ -1859,8 +1328,8 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                             const int ix = p.obs.r1b_idx[e];
                             const Z r = rho[(ix >> 8) * ld + (ix & 255)];
                             const R bv = A::pick(p.obs.r1b_val, p.obs.r1b_val_d, e);
-                            sr = A::rfma(bv, r.x, sr);
-                            si = A::rfma(bv, r.y, si);
+                            sr = A::rfma(bv, re(r), sr);
+                            si = A::rfma(bv, im(r), si);
                         }
                         sr = A::wsum(sr);
                         si = A::wsum(si);
@@ -1893,15 +1362,15 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                             }
                         }
                         unsigned short tr[3], ti[3];
-                        bf16_terms(as_dd(v.x), S, tr);
-                        bf16_terms(as_dd(v.y), S, ti);
+                        bf16_terms(as_dd(re(v)), S, tr);
+                        bf16_terms(as_dd(im(v)), S, ti);
                         for (int sp = 0; sp < S; ++sp) {
                             p.tc_x[sp][(2 * pt) * nk + e] = tr[sp];
                             p.tc_x[sp][(2 * pt + 1) * nk + e] = ti[sp];
                         }
                         if (e >= p.tc_nph) {
-                            bf16_terms(as_dd(y.x), S, tr);
-                            bf16_terms(as_dd(y.y), S, ti);
+                            bf16_terms(as_dd(re(y)), S, tr);
+                            bf16_terms(as_dd(im(y)), S, ti);
                             const int ey = e - p.tc_nph;
                             for (int sp = 0; sp < S; ++sp) {
                                 p.tc_y[sp][(2 * pt) * npp + ey] = tr[sp];
@@ -1932,38 +1401,19 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                         t = rfma(quarter, u, t);
                         e2 = rfma(v, t, e2);
                     };
-                    // proton-neutron records of a species-split pair: rho_li, rho_kj, rho_jk, rho_il
-                    // and both pairing tensors cross the species and vanish
-                    auto rec_pn = [&](uint32_t pk, R v) {
-                        const int i = pk & 0xff, j = (pk >> 8) & 0xff, k = (pk >> 16) & 0xff, l = pk >> 24;
-                        Z t = rho[k * ld + i] * rho[l * ld + j];
-                        if (i + j != k + l) t = zfma(rho[i * ld + k], rho[j * ld + l], t);
-                        e2 = rfma(v, t, e2);
-                    };
                     const int stride = blockDim.x;
-                    const int ngen = split ? p.nrec_gen : p.nrec;
-                    for (int e = threadIdx.x; e < ngen; e += 2 * stride) {
-                        const int e1 = e + stride;
-                        const uint32_t pk0 = p.rec_idx[e];
-                        const R v0 = A::pick(p.rec_v, p.rec_vd, e);
-                        const bool two = e1 < ngen;
-                        const uint32_t pk1 = two ? p.rec_idx[e1] : 0u;
-                        const R v1 = two ? A::pick(p.rec_v, p.rec_vd, e1) : A::rzero();
-                        rec(pk0, v0);
-                        if (two) rec(pk1, v1);
-                    }
-                    for (int e = ngen + threadIdx.x; e < p.nrec; e += 2 * stride) {
+                    for (int e = threadIdx.x; e < p.nrec; e += 2 * stride) {
                         const int e1 = e + stride;
                         const uint32_t pk0 = p.rec_idx[e];
                         const R v0 = A::pick(p.rec_v, p.rec_vd, e);
                         const bool two = e1 < p.nrec;
                         const uint32_t pk1 = two ? p.rec_idx[e1] : 0u;
                         const R v1 = two ? A::pick(p.rec_v, p.rec_vd, e1) : A::rzero();
-                        rec_pn(pk0, v0);
-                        if (two) rec_pn(pk1, v1);
+                        rec(pk0, v0);
+                        if (two) rec(pk1, v1);
                     }
-                    put(0, e2.x);
-                    put(1, e2.y);
+                    put(0, re(e2));
+                    put(1, im(e2));
                 }
                 {   // <J^2> (ZJ2_0, PNAMP_ME2B.f90:45-147) summed over x, y, z with
                     // Jx, Jy = (J+ +- J-)/(2, 2i):  sum_a j(j+1) rho_aa [above]
@@ -1971,13 +1421,8 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                     // + [Tr(J+ k10 J+ k01^T) + Tr(J- k10 J- k01^T)]/2 + Tr(Jz k10 Jz k01^T)
                     const R half = A::rconst(0.5f);
                     Z rest = zero;
-                    // a species-split pair has no proton-neutron densities and J+-, Jz keep the
-                    // species, so every term with a and c of different species vanishes: only the
-                    // two diagonal h x h blocks are summed (index t -> block, row, column)
-                    const int cnt = split ? 2 * h * h : nn, w = split ? h : n;
-                    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-                        const int blk = split ? t / (h * h) : 0, e = t - blk * h * h;
-                        const int a = blk * h + e / w, c = blk * h + e % w;
+                    for (int t = threadIdx.x; t < nn; t += blockDim.x) {
+                        const int a = t / n, c = t % n;
                         const R jpa = A::pick(p.obs.jp, p.obs.jp_d, a), jma = A::pick(p.obs.jm, p.obs.jm_d, a);
                         const R jpc = A::pick(p.obs.jp, p.obs.jp_d, c), jmc = A::pick(p.obs.jm, p.obs.jm_d, c);
                         const R mzz = A::rmul(A::pick(p.obs.mz, p.obs.mz_d, a), A::pick(p.obs.mz, p.obs.mz_d, c));
@@ -1992,8 +1437,8 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
                             q = zfma(A::rmul(half, A::rmul(jma, jmc)) * k10[ac - ld], k01[ac - 1], q);
                         rest = rest + q;
                     }
-                    put(2, rest.x);
-                    put(3, rest.y);
+                    put(2, re(rest));
+                    put(3, im(rest));
                 }
                 }  // !norm_only
                 __syncthreads();
@@ -2088,14 +1533,14 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
             for (int io = 0; io < kNobs; ++io) {
                 const zc v = inv * acc[io];
                 if (!zfinite(v)) f |= 4;
-                zout[2LL * (io * p.n_euler + ie)] = v.x;
-                zout[2LL * (io * p.n_euler + ie) + 1] = v.y;
+                zout[2LL * (io * p.n_euler + ie)] = re(v);
+                zout[2LL * (io * p.n_euler + ie) + 1] = im(v);
             }
             status[(long long)pair * p.n_euler + ie] = f;
             for (int b = 0; b < (r1out ? p.obs.n_r1b : 0); ++b) {
                 const zc v = inv * acc_r1b[b];
-                r1out[2LL * (((long long)pair * p.obs.n_r1b + b) * p.n_euler + ie)] = v.x;
-                r1out[2LL * (((long long)pair * p.obs.n_r1b + b) * p.n_euler + ie) + 1] = v.y;
+                r1out[2LL * (((long long)pair * p.obs.n_r1b + b) * p.n_euler + ie)] = re(v);
+                r1out[2LL * (((long long)pair * p.obs.n_r1b + b) * p.n_euler + ie) + 1] = im(v);
             }
         }
         if (r2out) {  // Euler weight x gauge mean, added into the pair's sums (ZRho2B_Integral at J = 0)
@@ -2110,16 +1555,90 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
     }
 }
 
+// What a pair's set-up record says about its points.
+enum { kPairBad = 0, kPairFull = 1, kPairReduced = 2, kPairSplit = 3 };
+__device__ __forceinline__ int pair_kind(const Params &p, const double *pr) {
+    if (pr[p.pl.dets + 2] != 0.0) return kPairBad;
+    if (pr[p.pl.dets + 7] == 0.0) return kPairFull;
+    return pr[p.pl.dets + 6] != 0.0 ? kPairSplit : kPairReduced;
+}
+// Species-split pairs factorise (split_items) unless the launch wants what couples the two
+// gauge angles point by point (H/N of every gauge point).
+__device__ __forceinline__ bool split_path(const Params &p, bool gout, bool r2out) {
+    return p.nfom > 1 && p.split_ok && (!p.tc_splits || p.tc_sp) && (!gout || p.norm_only) && (!r2out || p.r2_ss >= 0);
+}
+
+// One Euler point of a pair that does not take split_items.
+template <class Z>
+__device__ __forceinline__ void point_item(const Params &p, const double *__restrict__ pairbuf, zc *slot, int pair,
+                                           int ie, int kind, bool reload, double *__restrict__ zres,
+                                           int *__restrict__ status, double *__restrict__ gout,
+                                           double *__restrict__ r1out, double *__restrict__ r2out, long long pt0) {
+    double *zout = zres + 2LL * (long long)pair * kNobs * p.n_euler;
+    if (kind == kPairBad) {
+        for (int io = threadIdx.x; io < kNobs; io += blockDim.x) {
+            zout[2LL * (io * p.n_euler + ie)] = 0.0;
+            zout[2LL * (io * p.n_euler + ie) + 1] = 0.0;
+        }
+        if (threadIdx.x == 0) status[(long long)pair * p.n_euler + ie] = 8;
+        for (int g = threadIdx.x; g < (p.tc_splits ? p.n_gauge : 0); g += blockDim.x) {
+            p.tc_w[2 * (pt0 + g)] = 0.0;
+            p.tc_w[2 * (pt0 + g) + 1] = 0.0;
+        }
+    } else if (kind == kPairFull) {
+        full_item<Z>(p, pairbuf, slot, pair, ie, reload, zres, status, gout, r1out, r2out, pt0);
+    } else {
+        reduced_item<Z>(p, pairbuf + (long long)pair * p.pl.stride, slot, pair, ie, reload, zout, status, gout, r1out,
+                        r2out, pt0);
+    }
+}
+
 template <class Z>
 __global__ void __launch_bounds__(kThreads, 1)
-point_kernel(Params p, int npairs, const double *__restrict__ pairbuf, zc *scratch,
+point_kernel(const __grid_constant__ Params p, int npairs, const double *__restrict__ pairbuf, zc *scratch,
              double *__restrict__ zres, int *__restrict__ status, const int2 *__restrict__ items,
              long long nitems, double *__restrict__ gout, double *__restrict__ r1out,
-             double *__restrict__ r2out) {
+             double *__restrict__ r2out, int batch) {
     // items == nullptr: every (pair, Euler point) of the batch; else the listed (pair, ie)
     zc *slot = scratch + (long long)blockIdx.x * p.place.slot_elems;
+    int cur_pair = -1, cur_kind = -1;
+    if (split_path(p, gout != nullptr, r2out != nullptr)) {
+        // species-split pairs: `batch` Euler points at a time, runs of one pair
+        const long long per = items ? nitems : p.n_euler, nb = (per + batch - 1) / batch;
+        const long long total = items ? nb : nb * npairs;
+        for (long long b = blockIdx.x; b < total; b += gridDim.x) {
+            const int pair0 = items ? 0 : (int)(b / nb);
+            const long long i0 = (b % nb) * batch;
+            const int cnt = (int)min((long long)batch, per - i0);
+            for (int k = 0; k < cnt;) {
+                int pair = pair0, m = cnt - k;
+                if (items) {
+                    const int2 it = items[i0 + k];
+                    pair = it.x;
+                    if (pair < 0 || pair >= npairs || it.y < 0 || it.y >= p.n_euler) {   // out of range: skipped
+                        ++k;
+                        continue;
+                    }
+                    m = 1;
+                    while (k + m < cnt && items[i0 + k + m].x == pair && items[i0 + k + m].y >= 0 &&
+                           items[i0 + k + m].y < p.n_euler)
+                        ++m;
+                }
+                const double *pr = pairbuf + (long long)pair * p.pl.stride;
+                if (pair_kind(p, pr) == kPairSplit) {
+                    split_items<Z>(p, pr, slot, pair, items ? items + i0 + k : nullptr, (int)(i0 + k), m,
+                                   pair != cur_pair, zres + 2LL * (long long)pair * kNobs * p.n_euler, status, gout,
+                                   r1out, r2out, ((long long)pair0 * p.n_euler + i0 + k) * p.n_gauge);
+                    cur_pair = pair;
+                }
+                k += m;
+            }
+        }
+        cur_pair = -1;
+        cur_kind = kPairSplit;
+    }
+    const bool skip = cur_kind == kPairSplit;
     const long long total = items ? nitems : (long long)npairs * p.n_euler;
-    int cur_pair = -1;
     for (long long item = blockIdx.x; item < total; item += gridDim.x) {
         int pair, ie;
         if (items) {
@@ -2131,30 +1650,33 @@ point_kernel(Params p, int npairs, const double *__restrict__ pairbuf, zc *scrat
             pair = (int)(item / p.n_euler);
             ie = (int)(item % p.n_euler);
         }
-        point_item<Z>(p, pairbuf, slot, pair, ie, pair != cur_pair, zres, status, gout, r1out, r2out,
+        const int kind = pair_kind(p, pairbuf + (long long)pair * p.pl.stride);
+        if (skip && kind == kPairSplit) continue;
+        point_item<Z>(p, pairbuf, slot, pair, ie, kind, pair != cur_pair, zres, status, gout, r1out, r2out,
                       item * p.n_gauge);
         cur_pair = pair;
     }
 }
 
-// Persistent kernel over an uneven batch: work items (context, pair, Euler point)
-// of up to kMultiCtx contexts (model spaces, meshes, placements), taken `grab`
-// at a time from a global counter in the order of `items` (set by the schedule).
-// Every context's parameters travel by value in the launch's parameter space and
-// each context has its own inlined copy of the point body, so the per-point code
-// reads its sizes and table pointers as constant-bank operands exactly as the
-// single-context kernel does (an indexed parameter array would become a load per
-// use inside the hot loops).
+// Persistent kernel over an uneven batch: work items (context, pair, Euler point) of up to
+// kMultiCtx contexts (model spaces, meshes, placements), taken `grab` at a time from a global
+// counter in the order of `items` (set by the schedule). Every context's parameters travel by
+// value in the launch's parameter space. Runs of Euler points of one species-split pair within
+// a grab go through split_items together.
 template <class Z>
-__device__ __forceinline__ void multi_item(const MultiArgs &a, int4 m, zc *slot, bool reload) {
-    switch (m.x) {
-    case 0: point_item<Z>(a.p[0], a.pairbuf[0], slot, m.y, m.z, reload, a.zres[0], a.status[0]); break;
-    case 1: point_item<Z>(a.p[1], a.pairbuf[1], slot, m.y, m.z, reload, a.zres[1], a.status[1]); break;
-    case 2: point_item<Z>(a.p[2], a.pairbuf[2], slot, m.y, m.z, reload, a.zres[2], a.status[2]); break;
-    default: point_item<Z>(a.p[3], a.pairbuf[3], slot, m.y, m.z, reload, a.zres[3], a.status[3]); break;
-    }
+__device__ __forceinline__ void multi_items(const MultiArgs &a, const int4 *items, int cnt, zc *slot, bool reload) {
+    const int4 m = items[0];
+    const Params &p = a.p[m.x];
+    const double *pr = a.pairbuf[m.x] + (long long)m.y * p.pl.stride;
+    const int kind = pair_kind(p, pr);
+    if (kind == kPairSplit && split_path(p, false, false))
+        split_items<Z>(p, pr, slot, m.y, nullptr, m.z, cnt, reload,
+                       a.zres[m.x] + 2LL * (long long)m.y * kNobs * p.n_euler, a.status[m.x], nullptr, nullptr, nullptr, 0);
+    else
+        for (int k = 0; k < cnt; ++k)
+            point_item<Z>(p, a.pairbuf[m.x], slot, m.y, m.z + k, kind, reload && k == 0, a.zres[m.x], a.status[m.x],
+                          nullptr, nullptr, nullptr, 0);
 }
-static_assert(kMultiCtx == 4, "multi_item dispatches four contexts");
 
 template <class Z>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -2173,11 +1695,16 @@ multi_point_kernel(const __grid_constant__ MultiArgs a, const int4 *__restrict__
         __syncthreads();
         if (base >= nitems) break;
         const int end = min(base + grab, nitems);
-        for (int it = base; it < end; ++it) {
-            const int4 m = items[it];  // (context, pair, Euler point, unused)
-            multi_item<Z>(a, m, slot, m.x != cur_ctx || m.y != cur_pair);
+        for (int it = base; it < end;) {
+            const int4 m = items[it];  // (context, pair, first Euler point, unused)
+            int cnt = 1;
+            while (it + cnt < end && cnt < a.p[m.x].place.spl.items && items[it + cnt].x == m.x &&
+                   items[it + cnt].y == m.y && items[it + cnt].z == m.z + cnt)
+                ++cnt;
+            multi_items<Z>(a, items + it, cnt, slot, m.x != cur_ctx || m.y != cur_pair);
             cur_ctx = m.x;
             cur_pair = m.y;
+            it += cnt;
         }
     }
 }
@@ -2222,16 +1749,37 @@ cudaError_t set_point_smem(int form, int bytes) {
     return raise_smem_limit(form == 1 ? point_fn<zd>() : point_fn<zc>());
 }
 
+// Euler points per split_items call: the choice with the fewest rounds of problems, where a
+// batch of m points runs ceil(NFOM / chunks) rounds of one problem per thread group and the
+// launch ceil(batches / grid) batches one after the other.
+static int split_batch(const Params &p, long long nitems, long long per, int grid) {
+    const RedPlan &L = p.place.spl;
+    int best = 1;
+    long long cost = -1;
+    for (int m = 1; m <= L.items; m *= 2) {
+        const int nc = std::max(1, std::min(L.ng / (2 * m), p.nfom));
+        const long long units = 2LL * m * nc, rounds = ((units + L.ng - 1) / L.ng) * ((p.nfom + nc - 1) / nc);
+        const long long batches = per > 0 ? (nitems / per) * ((per + m - 1) / m) : (nitems + m - 1) / m;
+        const long long c = ((batches + grid - 1) / grid) * rounds;
+        if (cost < 0 || c < cost) {
+            cost = c;
+            best = m;
+        }
+    }
+    return best;
+}
+
 cudaError_t launch_points(const Params &p, int npairs, const double *pairbuf, zc *scratch, int grid,
                           double *zres, int *status, cudaStream_t st, const int2 *items, long long nitems,
                           double *gout, double *r1out, double *r2out) {
     if (r2out && (p.n_r2q <= 0 || !p.r2q || !p.r2acc)) return cudaErrorInvalidValue;
+    const int batch = split_batch(p, items ? nitems : (long long)npairs * p.n_euler, items ? 0 : p.n_euler, grid);
     if (p.form == 1)
         point_kernel<zd><<<grid, kThreads, p.place.smem_bytes, st>>>(p, npairs, pairbuf, scratch, zres, status,
-                                                                    items, nitems, gout, r1out, r2out);
+                                                                    items, nitems, gout, r1out, r2out, batch);
     else
         point_kernel<zc><<<grid, kThreads, p.place.smem_bytes, st>>>(p, npairs, pairbuf, scratch, zres, status,
-                                                                    items, nitems, gout, r1out, r2out);
+                                                                    items, nitems, gout, r1out, r2out, batch);
     return cudaGetLastError();
 }
 

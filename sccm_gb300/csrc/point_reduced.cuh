@@ -1,0 +1,1276 @@
+// Points of pairs with a well conditioned U0 (bra) and V1 (ket), the "reduced" pairs of
+// setup_kernel: one skew-symmetric inverse per gauge point instead of a Pfaffian elimination,
+// an n x n solve and three density products.
+//
+// With M = D X D (X = R W R^T, W = V1 U1^-1, D = diag(e^{i phi})), M^-1 = D* Y D* (Y = R* Wi R^+,
+// Wi = W^-1 = U1 V1^-1, real and skew, one per pair) and Z0 = V0 U0^-1 (the same), the
+// transition densities are functions of K = Y - D Z0 D alone:
+//     kappa10 = D K^-1 D,   rho = -kappa10 Z0,   kappa01 = Z0 + Z0 kappa10 Z0,
+// which follows from T22 = U0^T (1 - Z0 M) (D* R* U1): insert D R V1 = M D* R* U1 and rho =
+// -M (1 - Z0 M)^-1 Z0 etc. K is also a Schur complement of the norm's matrix,
+// Pf(c [[M, -1], [1, -Z0]]) = Pf(c M) Pf(c (M^-1 - Z0)) = Pf(c W) Pf(c K) (det R = 1, and the det D of
+// the two factors cancel), so one factorisation by 2 x 2 pivots yields both: N/2 steps each way and N^3/2 complex
+// multiply-adds for the inverse and the Pfaffian, 1.5 N^3 complex x real ones for rho and the
+// upper triangle of kappa01 (skew), where the separate Pfaffian, Gauss-Jordan solve and
+// density products took 4.3 N^3 complex-equivalents and N + N/2 steps. Nothing else of the
+// ket enters, so T22, R V1 and R* U1 are not formed. (The other complement, M - Z0^-1, has the
+// same form with Z0^-1 as the multiplier; its entries are 15 to 80 where those of Z0 are 2 to 20,
+// and its kappa10 loses that factor. The phases stand with Z0 and not with the larger Y for
+// the same reason.)
+#pragma once
+
+namespace pnamp {
+
+// ------------------------------------------------------------------ accumulating arithmetic
+// Sums of products with the factors prepared outside the loop (broadcast and negated words for
+// the packed form). FP64: plain complex FMAs. Double-float: dd2_fma, renormalised after every
+// product; joining the low words only at the end of the sum is 12 operations per product
+// instead of 15, but its error is 3 times larger after 20 terms and 4 times after 40.
+template <class Z> struct Op;
+template <> struct Op<zc> {
+    struct Mul { double x, y; };
+    struct RMul { double r; };
+    struct Rot {};
+    using Acc = zc;
+    static __device__ __forceinline__ Mul mul(zc a) { return {a.x, a.y}; }
+    static __device__ __forceinline__ Mul mul_neg(zc a) { return {-a.x, -a.y}; }
+    static __device__ __forceinline__ RMul rmul(double r) { return {r}; }
+    static __device__ __forceinline__ Rot rot(zc) { return {}; }
+    static __device__ __forceinline__ Acc acc(zc a) { return a; }
+    static __device__ __forceinline__ void cadd(Acc &s, const Mul &a, zc b, Rot) {
+        s.x = fma(a.x, b.x, fma(-a.y, b.y, s.x));
+        s.y = fma(a.x, b.y, fma(a.y, b.x, s.y));
+    }
+    static __device__ __forceinline__ void radd(Acc &s, const RMul &r, zc b) {
+        s.x = fma(r.r, b.x, s.x);
+        s.y = fma(r.r, b.y, s.y);
+    }
+    static __device__ __forceinline__ zc done(const Acc &s) { return s; }
+};
+template <> struct Op<zd> {
+    struct Mul { dd2 x; f2 nx; dd2 y; f2 ny; };
+    struct RMul { dd2 r; f2 nr; };
+    struct Rot { dd2 b; };
+    struct Acc { f2 hi, lo; };
+    static __device__ __forceinline__ Mul mul(zd a) {
+        const dd x = re(a), y = im(a);
+        return {dup(x), f2_dup(-x.hi), dup(y), f2_dup(-y.hi)};
+    }
+    static __device__ __forceinline__ Mul mul_neg(zd a) {
+        const dd x = re(a), y = im(a);
+        return {dup(dd_neg(x)), f2_dup(x.hi), dup(dd_neg(y)), f2_dup(y.hi)};
+    }
+    static __device__ __forceinline__ RMul rmul(dd r) { return {dup(r), f2_dup(-r.hi)}; }
+    // i b = (-im, re)
+    static __device__ __forceinline__ Rot rot(zd b) {
+        return {{f2_make(-f2_b(b.hi), f2_a(b.hi)), f2_make(-f2_b(b.lo), f2_a(b.lo))}};
+    }
+    static __device__ __forceinline__ Acc acc(zd a) { return {a.hi, a.lo}; }
+    // s += a b (both lanes), na = -a.hi
+    static __device__ __forceinline__ void padd(Acc &s, dd2 a, f2 na, f2 bh, f2 bl) {
+        const f2 p = f2_mul(na, bh);              // -(a b) rounded
+        f2 e = f2_fma(a.hi, bh, p);               // its error
+        e = f2_fma(a.hi, bl, e);
+        e = f2_fma(a.lo, bh, e);
+        const f2 t = f2_sub(s.hi, p);             // two_sum(s.hi, -p)
+        const f2 v = f2_sub(t, s.hi);
+        const f2 d = f2_sub(f2_sub(s.hi, f2_sub(t, v)), f2_add(p, v));
+        const dd2 r = quick_two_sum(t, f2_add(d, f2_add(e, s.lo)));
+        s.hi = r.hi;
+        s.lo = r.lo;
+    }
+    static __device__ __forceinline__ void cadd(Acc &s, const Mul &a, zd b, const Rot &ib) {
+        padd(s, a.x, a.nx, b.hi, b.lo);
+        padd(s, a.y, a.ny, ib.b.hi, ib.b.lo);
+    }
+    static __device__ __forceinline__ void radd(Acc &s, const RMul &r, zd b) { padd(s, r.r, r.nr, b.hi, b.lo); }
+    static __device__ __forceinline__ zd done(const Acc &s) { return {s.hi, s.lo}; }
+};
+
+// Magnitude key of a pivot candidate in 26 bits above the 6 index bits.
+__device__ __forceinline__ unsigned sweep_key(zd a, int m) {
+    return (fmaxf(fabsf(f2_a(a.hi)), fabsf(f2_b(a.hi))) >= 0.0f
+                ? (__float_as_uint(fmaxf(fabsf(f2_a(a.hi)), fabsf(f2_b(a.hi)))) & ~63u) : 0u) | (unsigned)(63 - m);
+}
+__device__ __forceinline__ unsigned sweep_key(zc a, int m) {
+    const unsigned x = (unsigned)__double2hiint(a.x) & 0x7fffffffu, y = (unsigned)__double2hiint(a.y) & 0x7fffffffu;
+    const unsigned k = x > y ? x : y;
+    return (k < 0x7ff00000u ? (k & ~63u) : 0u) | (unsigned)(63 - m);
+}
+
+__device__ __forceinline__ zc shfl_xor(zc a, int o) {
+    return mk(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
+}
+__device__ __forceinline__ zd shfl_xor(zd a, int o) {
+    zd r;
+    r.hi.u = __shfl_xor_sync(0xffffffffu, a.hi.u, o);
+    r.lo.u = __shfl_xor_sync(0xffffffffu, a.lo.u, o);
+    return r;
+}
+template <class Z>
+__device__ __forceinline__ Z warp_sum_z(Z v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = v + shfl_xor(v, o);
+    return v;
+}
+// Scratch of one problem's factorisation: the pivots and their values, then byte lists of the
+// remaining indices (two, alternating) and of the pivot order, last step first.
+template <class Z> struct SkewScratch {
+    Z piv[32], s[32], red[16];
+    unsigned char list[2][64], ord[64];
+};
+
+// Pfaffian factorisation of the skew matrix in the upper triangle of A (order N <= 64, even,
+// row stride ld) by a thread group, and (`inverse`) its inverse over all of A.
+//
+// Forward: N/2 steps, each takes the first remaining row r, its largest remaining entry as pivot
+// s = K_rq, and updates the remaining entries K_ij += v_i K_rj - K_ri v_j, v = K_q. / s. Rows
+// move nowhere, the list of remaining indices shrinks instead; the sign of the pivot order goes
+// into the pivots, so Pf(K) = prod piv. Entry t of the remaining triangle is (list[a], list[b])
+// with t = b(b-1)/2 + a, so a thread's (a, b) are the same in every step (ab: a << 8 | b).
+//
+// Backward: with G = [[-v], [K_r. / s]] of a step and Y the inverse over the indices that remain
+// after it, the step's two rows of the inverse are -G Y and its pivot entry is
+// -1/s + (G Y G^T)_rq. Every intermediate is part of the inverse itself. (A sweep that carries
+// the inverse forward, K_rj -> v_j and so on, has the same operation count in one pass over
+// registers but passes through inverses of leading blocks, which can be large: its errors were
+// 4 to 50 times larger.) v is kept at A[.][r], K_r. / s at A[q][.] in between.
+// Returns true if a row had no usable entry (exactly singular or not finite).
+template <class Z, int E>
+__device__ __forceinline__ bool skew_factor(const Grp &g, int N, int ld, const int (&ab)[E], Z *A, Z *buf, int nbuf,
+                                            SkewScratch<Z> &w, bool inverse) {
+    using O = Op<Z>;
+    const int lane = g.tid & 31;
+    Z *Wb = buf, *Vb = buf + N;
+    bool sing = false;
+    for (int t = g.tid; t < N; t += g.nthr) w.list[0][t] = (unsigned char)t;
+    gsync(g);
+    for (int k = 0; k < N / 2; ++k) {
+        const int m = N - 2 * k;
+        const unsigned char *L = w.list[k & 1];
+        unsigned char *Ln = w.list[(k + 1) & 1];
+        const int r = L[0];
+        unsigned key = 0u;
+        for (int t = 1 + lane; t < m; t += 32) {
+            const unsigned kk = sweep_key(A[r * ld + L[t]], t);
+            key = key > kk ? key : kk;
+        }
+        key = __reduce_max_sync(0xffffffffu, key);
+        const bool none = (key >> 6) == 0u;
+        const int pos = none ? 1 : 63 - (int)(key & 63u);
+        sing = sing || none;
+        const int q = L[pos];
+        const Z s = A[r * ld + q];
+        if (g.tid == 0) {
+            w.piv[k] = (pos & 1) ? s : -s;   // pos - 1 remaining indices lie between r and q
+            w.s[k] = s;
+            w.ord[m - 2] = (unsigned char)r;
+            w.ord[m - 1] = (unsigned char)q;
+        }
+        if (m == 2) break;
+        if (1 + g.tid < m) {
+            const Z inv = zrecip(s);
+            for (int t = 1 + g.tid; t < m; t += g.nthr) {
+                if (t == pos) continue;
+                const int c = t - 1 - (t > pos), i = L[t];
+                const Z wi = A[r * ld + i], qi = i > q ? A[q * ld + i] : -A[i * ld + q];
+                const Z vi = qi * inv;
+                Wb[c] = wi;
+                Vb[c] = vi;
+                Ln[c] = (unsigned char)i;
+                if (inverse) {
+                    A[i * ld + r] = vi;
+                    A[q * ld + i] = wi * inv;
+                }
+            }
+        }
+        gsync(g);
+        const int T = (m - 2) * (m - 3) / 2;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            if (g.tid + e * g.nthr >= T) break;
+            const int a = ab[e] >> 8, b = ab[e] & 255;
+            Z *x = A + (int)Ln[a] * ld + (int)Ln[b];
+            const Z wb = Wb[b], vb = Vb[b];
+            typename O::Acc c = O::acc(*x);
+            O::cadd(c, O::mul(Vb[a]), wb, O::rot(wb));
+            O::cadd(c, O::mul_neg(Wb[a]), vb, O::rot(vb));
+            *x = O::done(c);
+        }
+        gsync(g);
+    }
+    if (!inverse) {
+        gsync(g);
+        return sing;
+    }
+    gsync(g);
+    for (int k = N / 2 - 1; k >= 0; --k) {
+        const int m = N - 2 - 2 * k, r = w.ord[m], q = w.ord[m + 1];
+        int parts = 0;
+        if (m > 0) {
+            parts = min(min(g.nthr / m, m), nbuf / (2 * m));
+            const int b = g.tid % m, part = g.tid / m;
+            if (part < parts) {
+                const int jb = w.ord[b];
+                typename O::Acc xp = O::acc(szero<Z>()), xq = xp;
+                for (int a = part; a < m; a += parts) {
+                    const int ia = w.ord[a];
+                    const Z y = A[ia * ld + jb];
+                    const typename O::Rot yr = O::rot(y);
+                    O::cadd(xp, O::mul(A[ia * ld + r]), y, yr);
+                    O::cadd(xq, O::mul_neg(A[q * ld + ia]), y, yr);
+                }
+                buf[(2 * part) * m + b] = O::done(xp);
+                buf[(2 * part + 1) * m + b] = O::done(xq);
+            }
+            gsync(g);
+        }
+        if (g.tid < 32) {
+            typename O::Acc x = O::acc(szero<Z>());
+            for (int b = lane; b < m; b += 32) {
+                Z yr = buf[b], yq = buf[m + b];
+                for (int part = 1; part < parts; ++part) {
+                    yr = yr + buf[(2 * part) * m + b];
+                    yq = yq + buf[(2 * part + 1) * m + b];
+                }
+                const int ib = w.ord[b];
+                O::cadd(x, O::mul(A[q * ld + ib]), yr, O::rot(yr));
+                A[r * ld + ib] = yr;
+                A[ib * ld + r] = -yr;
+                A[q * ld + ib] = yq;
+                A[ib * ld + q] = -yq;
+            }
+            const Z sum = warp_sum_z(O::done(x));
+            if (lane == 0) {
+                const Z y = -(zrecip(w.s[k]) + sum);
+                A[r * ld + q] = y;
+                A[q * ld + r] = -y;
+                A[r * ld + r] = szero<Z>();
+                A[q * ld + q] = szero<Z>();
+            }
+        }
+        gsync(g);
+    }
+    return sing;
+}
+
+// Pf = prod piv[k] (c times each, k < N/2 <= 32) by the lanes of one warp; the reference's
+// pivot test |c piv| <= 1e-13 (or a non-finite pivot) sets `under` to 1 (2). Every lane
+// gets the product.
+template <class Z>
+__device__ __forceinline__ zc pivot_product(const Z *piv, int np, double c, int &under) {
+    const int lane = threadIdx.x & 31;
+    int f = 0;
+    Z v = Ar<Z>::from(mk(1.0, 0.0));
+    if (lane < np) {
+        v = Ar<Z>::from(mk(c, 0.0)) * piv[lane];
+        f = pivot_flag(v);
+    }
+    const unsigned bad = __ballot_sync(0xffffffffu, f != 0);
+    const int first = __shfl_sync(0xffffffffu, f, bad ? __ffs((int)bad) - 1 : 0);
+    PfProd<Z> pf;
+    pf.mul(v, false);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) pf.join(o);
+    under = bad ? first : 0;
+    return under ? mk(0.0, 0.0) : pf.get();
+}
+
+// rho^T = -Z0 K^-1 (A holds K^-1 in full), stored transposed, TI x TJ register tiles over the
+// group. Z: Z0, skew, row stride N.
+template <class Z, int TI, int TJ>
+__device__ __forceinline__ void rho_tiles(const Grp &g, int N, int ld, const typename Ar<Z>::R *Z0, const Z *A, Z *Rh) {
+    using O = Op<Z>;
+    const int nj = (N + TJ - 1) / TJ, nt = ((N + TI - 1) / TI) * nj;
+    for (int t = g.tid; t < nt; t += g.nthr) {
+        const int i0 = (t / nj) * TI, j0 = (t % nj) * TJ;
+        typename O::Acc acc[TI][TJ];
+#pragma unroll
+        for (int a = 0; a < TI; ++a)
+#pragma unroll
+            for (int b = 0; b < TJ; ++b) acc[a][b] = O::acc(szero<Z>());
+        for (int k = 0; k < N; ++k) {
+            Z bv[TJ];
+#pragma unroll
+            for (int b = 0; b < TJ; ++b) bv[b] = A[k * ld + min(j0 + b, N - 1)];
+#pragma unroll
+            for (int a = 0; a < TI; ++a) {   // -Z0_ik = Z0_ki
+                const typename O::RMul m = O::rmul(Z0[k * N + min(i0 + a, N - 1)]);
+#pragma unroll
+                for (int b = 0; b < TJ; ++b) O::radd(acc[a][b], m, bv[b]);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < TI; ++a)
+#pragma unroll
+            for (int b = 0; b < TJ; ++b)
+                if (i0 + a < N && j0 + b < N) Rh[(j0 + b) * ld + i0 + a] = O::done(acc[a][b]);
+    }
+}
+
+// kappa01_ij = Z0_ij - sum_k rho_ki Z0_kj for i < j, stored at A[j][i]: the TI x TJ tiles that
+// reach above the diagonal, in row order.
+template <class Z, int TI, int TJ>
+__device__ __forceinline__ void k01_tiles(const Grp &g, int N, int ld, const typename Ar<Z>::R *Z0, const Z *Rh, Z *A) {
+    using O = Op<Z>;
+    const int ni = (N + TI - 1) / TI, nj = (N + TJ - 1) / TJ;
+    int t = g.tid, row = 0;
+    for (;;) {
+        // tiles of a row start at the first column tile that reaches above its first row
+        int first = (row * TI + 1) / TJ;
+        while (row < ni && t >= nj - first) {
+            t -= max(nj - first, 0);
+            ++row;
+            first = (row * TI + 1) / TJ;
+        }
+        if (row >= ni) break;
+        const int i0 = row * TI, j0 = (first + t) * TJ;
+        typename O::Acc acc[TI][TJ];
+#pragma unroll
+        for (int a = 0; a < TI; ++a)
+#pragma unroll
+            for (int b = 0; b < TJ; ++b)   // Z0_ij = -Z0_ji
+                acc[a][b] = O::acc(Ar<Z>::neg_real(Z0[min(j0 + b, N - 1) * N + min(i0 + a, N - 1)]));
+        for (int k = 0; k < N; ++k) {
+            Z av[TI];
+#pragma unroll
+            for (int a = 0; a < TI; ++a) av[a] = Rh[k * ld + min(i0 + a, N - 1)];
+#pragma unroll
+            for (int b = 0; b < TJ; ++b) {   // -Z0_kj = Z0_jk
+                const typename O::RMul m = O::rmul(Z0[min(j0 + b, N - 1) * N + k]);
+#pragma unroll
+                for (int a = 0; a < TI; ++a) O::radd(acc[a][b], m, av[a]);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < TI; ++a)
+#pragma unroll
+            for (int b = 0; b < TJ; ++b)
+                if (i0 + a < j0 + b && j0 + b < N) A[(j0 + b) * ld + i0 + a] = O::done(acc[a][b]);
+        t += g.nthr;
+    }
+}
+
+// One gauge point's skew matrix K = Y - d Z0 (order N, Y with row stride ldx, phase factors by
+// the species of the row and column: d0 both below h0, d1 mixed, d2 both above), its Pfaffian
+// factors into w and (`inverse`) rho into Rh and (kappa10, kappa01) into A: kappa10_ij =
+// A[i][j] and kappa01_ij = A[j][i] for i < j.
+template <class Z, int E>
+__device__ __forceinline__ bool skew_problem_e(const Grp &g, int N, int ld, int h0, Z d0, Z d1, Z d2, const Z *Y, int ldx,
+                                               const typename Ar<Z>::R *Z0, Z *A, Z *Rh, SkewScratch<Z> &w, bool inverse) {
+    int ab[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int t = g.tid + e * g.nthr;
+        int b = (int)((sqrtf(8.0f * (float)t + 1.0f) + 1.0f) * 0.5f);
+        if (b * (b - 1) / 2 > t) --b;
+        if (b * (b + 1) / 2 <= t) ++b;
+        const int a = t - b * (b - 1) / 2;
+        ab[e] = (a << 8) | b;
+        if (t < N * (N - 1) / 2) {
+            const Z d = b < h0 ? d0 : (a < h0 ? d1 : d2);
+            A[a * ld + b] = rfma(Ar<Z>::rneg(Z0[a * N + b]), d, Y[a * ldx + b]);
+        }
+    }
+    const bool sing = skew_factor<Z, E>(g, N, ld, ab, A, Rh, N * max(ld, 5), w, inverse);
+    if (inverse) {   // kappa10 = D K^-1 D
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            if (g.tid + e * g.nthr >= N * (N - 1) / 2) break;
+            const int a = ab[e] >> 8, b = ab[e] & 255;
+            const Z v = A[a * ld + b] * (b < h0 ? d0 : (a < h0 ? d1 : d2));
+            A[a * ld + b] = v;
+            A[b * ld + a] = -v;
+        }
+        gsync(g);
+    }
+    return sing;
+}
+
+template <class Z>
+__device__ __noinline__ bool skew_problem(const Grp g, int N, int ld, int h0, Z d0, Z d1, Z d2, const Z *Y, int ldx,
+                                          const typename Ar<Z>::R *Z0, Z *A, Z *Rh, SkewScratch<Z> &w, bool inverse,
+                                          int tile) {
+    bool sing = false;
+    switch ((N * (N - 1) / 2 + g.nthr - 1) / g.nthr) {
+#define CASE(E) \
+    case E: sing = skew_problem_e<Z, E>(g, N, ld, h0, d0, d1, d2, Y, ldx, Z0, A, Rh, w, inverse); break;
+        CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8)
+#undef CASE
+    }
+    if (!inverse) return sing;
+    switch (tile & 15) {
+        case 0: rho_tiles<Z, 3, 2>(g, N, ld, Z0, A, Rh); break;
+        case 1: rho_tiles<Z, 3, 3>(g, N, ld, Z0, A, Rh); break;
+        case 2: rho_tiles<Z, 4, 2>(g, N, ld, Z0, A, Rh); break;
+        case 3: rho_tiles<Z, 5, 3>(g, N, ld, Z0, A, Rh); break;
+        default: rho_tiles<Z, 4, 4>(g, N, ld, Z0, A, Rh); break;
+    }
+    gsync(g);
+    switch (tile >> 4) {
+        case 0: k01_tiles<Z, 2, 2>(g, N, ld, Z0, Rh, A); break;
+        case 1: k01_tiles<Z, 2, 4>(g, N, ld, Z0, Rh, A); break;
+        case 2: k01_tiles<Z, 3, 3>(g, N, ld, Z0, Rh, A); break;
+        default: k01_tiles<Z, 4, 4>(g, N, ld, Z0, Rh, A); break;
+    }
+    gsync(g);
+    return sing;
+}
+
+// ------------------------------------------------------------------ observables of one point
+template <class Z> struct PointSums {
+    Z e2, t1, j2, tp, tm, tz;   // two- and one-body energy, <J^2> without its traces, Tr J+, J-, Jz rho
+};
+// Sum over the group, valid in its first warp. red: 16 values.
+template <class Z>
+__device__ __forceinline__ Z group_sum(const Grp &g, Z v, Z *red) {
+    v = warp_sum_z(v);
+    if (g.nthr == 32) return v;
+    const int lane = g.tid & 31, wid = g.tid >> 5, nw = g.nthr >> 5;
+    if (lane == 0) red[wid] = v;
+    gsync(g);
+    if (wid == 0) v = warp_sum_z(lane < nw ? red[lane] : szero<Z>());
+    gsync(g);
+    return v;
+}
+
+// Observables of the densities of skew_problem over the levels [lev0, lev0 + N): the two-body
+// records [rec0, rec1) (exact regrouping of the 8-term sum of PNAMP_Energy_OpenMP.f90:40-78,
+//   V [rho_ki rho_lj - rho_li rho_kj + d (rho_ik rho_jl - rho_jk rho_il)]
+//   + V [kappa01_ij kappa10_kl + d kappa01_kl kappa10_ij],
+// the pairing tensors being skew), the one-body energy, and <J^2> (ZJ2_0, PNAMP_ME2B.f90:45-147;
+// Jx, Jy = (J+ +- J-)/(2, 2i), J-_{a+1,a} = J+_{a,a+1}) without sum_a j(j+1) rho_aa, which is
+// linear in rho, and without the products of traces. Sums are valid in the group's first warp.
+template <class Z>
+__device__ __noinline__ PointSums<Z> point_sums(const Grp g, const Params &p, int N, int ld, int lev0, int rec0,
+                                                int rec1, const Z *A, const Z *Rh, Z *red) {
+    using O = Op<Z>;
+    using Ra = Ar<Z>;
+    using R = typename Ra::R;
+    PointSums<Z> out;
+    typename O::Acc e2 = O::acc(szero<Z>()), t1 = e2, j2 = e2, tp = e2, tm = e2, tz = e2;
+    for (int e = rec0 + g.tid; e < rec1; e += g.nthr) {
+        const uint32_t pk = p.rec_idx[e];
+        const R v = Ra::pick(p.rec_v, p.rec_vd, e);
+        int i = pk & 0xff, j = (pk >> 8) & 0xff, k = (pk >> 16) & 0xff, l = pk >> 24;
+        const bool sym = i + j != k + l;
+        i -= lev0;
+        j -= lev0;
+        k -= lev0;
+        l -= lev0;
+        typename O::Acc t = O::acc(szero<Z>());
+        auto mac = [&](bool neg, Z a, Z b) { O::cadd(t, neg ? O::mul_neg(a) : O::mul(a), b, O::rot(b)); };
+        mac(false, Rh[k * ld + i], Rh[l * ld + j]);
+        mac(true, Rh[l * ld + i], Rh[k * ld + j]);
+        mac(false, A[j * ld + i], A[k * ld + l]);
+        if (sym) {
+            mac(false, Rh[i * ld + k], Rh[j * ld + l]);
+            mac(true, Rh[j * ld + k], Rh[i * ld + l]);
+            mac(false, A[l * ld + k], A[i * ld + j]);
+        }
+        O::radd(e2, O::rmul(v), O::done(t));
+    }
+    for (int e = g.tid; e < p.obs.n_t1b; e += g.nthr) {
+        const int ix = p.obs.t1b_idx[e], r = (ix >> 8) - lev0, c = (ix & 255) - lev0;
+        if ((unsigned)r < (unsigned)N && (unsigned)c < (unsigned)N)
+            O::radd(t1, O::rmul(Ra::pick(p.obs.t1b_val, p.obs.t1b_val_d, e)), Rh[r * ld + c]);
+    }
+    for (int t = g.tid; t < N * N; t += g.nthr) {
+        const int a = t / N, c = t % N;
+        const R jpa = Ra::pick(p.obs.jp, p.obs.jp_d, lev0 + a), jpc = Ra::pick(p.obs.jp, p.obs.jp_d, lev0 + c);
+        const R mza = Ra::pick(p.obs.mz, p.obs.mz_d, lev0 + a), mzc = Ra::pick(p.obs.mz, p.obs.mz_d, lev0 + c);
+        if (a <= c) {
+            const Z rac = Rh[a * ld + c], rca = Rh[c * ld + a];
+            typename O::Acc x = O::acc(szero<Z>());
+            O::cadd(x, O::mul_neg(rac), rca, O::rot(rca));
+            R f = Ra::rmul(mza, mzc);
+            if (a < c) {
+                const Z kk = A[c * ld + a];
+                O::cadd(x, O::mul(A[a * ld + c]), kk, O::rot(kk));
+                f = Ra::radd(f, f);
+            }
+            O::radd(j2, O::rmul(f), O::done(x));
+        }
+        if (Ra::nz(jpa) && Ra::nz(jpc)) {
+            const Z rc = Rh[c * ld + a];
+            typename O::Acc x = O::acc(szero<Z>());
+            O::cadd(x, O::mul_neg(Rh[(a + 1) * ld + c + 1]), rc, O::rot(rc));
+            // kappa10_{a+1,c} kappa01_{a,c+1}
+            if (c > a + 1) {
+                const Z k2 = A[(c + 1) * ld + a];
+                O::cadd(x, O::mul(A[(a + 1) * ld + c]), k2, O::rot(k2));
+            } else if (c < a - 1) {
+                const Z k2 = A[a * ld + c + 1];
+                O::cadd(x, O::mul(A[c * ld + a + 1]), k2, O::rot(k2));
+            } else if (c == a) {
+                const Z k2 = A[(a + 1) * ld + a];
+                O::cadd(x, O::mul_neg(A[a * ld + a + 1]), k2, O::rot(k2));
+            }
+            O::radd(j2, O::rmul(Ra::rmul(jpa, jpc)), O::done(x));
+        }
+        if (a == c) {
+            O::radd(tz, O::rmul(mza), Rh[a * ld + a]);
+            if (Ra::nz(jpa)) {
+                O::radd(tp, O::rmul(jpa), Rh[(a + 1) * ld + a]);
+                O::radd(tm, O::rmul(jpa), Rh[a * ld + a + 1]);
+            }
+        }
+    }
+    out.e2 = group_sum(g, O::done(e2), red);
+    out.t1 = group_sum(g, O::done(t1), red);
+    out.j2 = group_sum(g, O::done(j2), red);
+    out.tp = group_sum(g, O::done(tp), red);
+    out.tm = group_sum(g, O::done(tm), red);
+    out.tz = group_sum(g, O::done(tz), red);
+    return out;
+}
+
+// ZRho2B_Angles (PNAMP_Rho2B.f90:105-112) before its Clebsch-Gordan sums, for the levels (i, j, k, l)
+// of a packed quadruple less lev0: rho_ki rho_lj - rho_li rho_kj + kappa01_ij kappa10_kl.
+template <class Z>
+__device__ __forceinline__ Z quad_product(uint32_t pk, int lev0, int ld, const Z *A, const Z *Rh) {
+    const int i = (int)(pk & 0xff) - lev0, j = (int)((pk >> 8) & 0xff) - lev0, k = (int)((pk >> 16) & 0xff) - lev0,
+              l = (int)(pk >> 24) - lev0;
+    Z t = Rh[k * ld + i] * Rh[l * ld + j];
+    t = zfms(Rh[l * ld + i], Rh[k * ld + j], t);
+    if (i != j && k != l) {
+        const Z u = A[max(i, j) * ld + min(i, j)], v = A[min(k, l) * ld + max(k, l)];
+        t = (i < j) == (k < l) ? zfma(u, v, t) : zfms(u, v, t);
+    }
+    return t;
+}
+
+// The group's part of the tensor-core operand rows of point pt (X: rho entries, then K10 pairs;
+// Y: K01 pairs) as split-bf16 terms; K_xy = kappa_xy - kappa_yx = 2 kappa_xy.
+template <class Z>
+__device__ __noinline__ void tc_rows(const Grp g, const Params &p, int ld, const Z *A, const Z *Rh, long long pt) {
+    const int S = p.tc_splits, nk = p.tc_nk, npp = p.tc_nk - p.tc_nph;
+    for (int e = g.tid; e < nk; e += g.nthr) {
+        const int src = p.tc_src[e];
+        Z v = szero<Z>(), y = v;
+        if (src >= 0) {
+            const int r = src >> 8, c = src & 255;
+            if (e < p.tc_nph) {
+                v = Rh[r * ld + c];
+            } else {
+                v = A[r * ld + c];
+                y = A[c * ld + r];
+                v = v + v;
+                y = y + y;
+            }
+        }
+        unsigned short tr[3], ti[3];
+        bf16_terms(as_dd(re(v)), S, tr);
+        bf16_terms(as_dd(im(v)), S, ti);
+        for (int sp = 0; sp < S; ++sp) {
+            p.tc_x[sp][(2 * pt) * nk + e] = tr[sp];
+            p.tc_x[sp][(2 * pt + 1) * nk + e] = ti[sp];
+        }
+        if (e >= p.tc_nph) {
+            bf16_terms(as_dd(re(y)), S, tr);
+            bf16_terms(as_dd(im(y)), S, ti);
+            const int ey = e - p.tc_nph;
+            for (int sp = 0; sp < S; ++sp) {
+                p.tc_y[sp][(2 * pt) * npp + ey] = tr[sp];
+                p.tc_y[sp][(2 * pt + 1) * npp + ey] = ti[sp];
+            }
+        }
+    }
+}
+
+// The same of one species' problem (levels [lev0, lev0 + N)): a row of the full width, X entries
+// then Y entries, [term][re, im], in which only the 16-byte chunks with entries of that species
+// are written (`chunks`; the rest of the buffer stays zero). A gauge point's operand rows are
+// the bitwise union of its two species' rows (join_rows).
+template <class Z>
+__device__ __noinline__ void species_rows(const Grp g, const Params &p, int s, int N, int ld, const Z *A, const Z *Rh,
+                                          unsigned short *row) {
+    const int S = p.tc_splits, nk = p.tc_nk, W = 2 * nk - p.tc_nph, lev0 = s * N;
+    for (int ci = p.tc_choff[s] + g.tid; ci < p.tc_choff[s + 1]; ci += g.nthr) {
+        const int e0 = 8 * p.tc_chunks[ci];
+        uint32_t o[3][2][4];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int e = e0 + q, src = p.tc_src[e < nk ? e : e - nk + p.tc_nph];
+            const int r = (src >> 8) - lev0, c = (src & 255) - lev0;
+            Z v = szero<Z>();
+            if (src >= 0 && (unsigned)r < (unsigned)N && (unsigned)c < (unsigned)N) {
+                v = e < p.tc_nph ? Rh[r * ld + c] : (e < nk ? A[r * ld + c] : A[c * ld + r]);
+                if (e >= p.tc_nph) v = v + v;   // K_xy = 2 kappa_xy
+            }
+            unsigned short tr[3], ti[3];
+            bf16_terms(as_dd(re(v)), S, tr);
+            bf16_terms(as_dd(im(v)), S, ti);
+#pragma unroll
+            for (int sp = 0; sp < 3; ++sp) {
+                if (q & 1) {
+                    o[sp][0][q >> 1] |= (uint32_t)tr[sp] << 16;
+                    o[sp][1][q >> 1] |= (uint32_t)ti[sp] << 16;
+                } else {
+                    o[sp][0][q >> 1] = tr[sp];
+                    o[sp][1][q >> 1] = ti[sp];
+                }
+            }
+        }
+#pragma unroll
+        for (int sp = 0; sp < 3; ++sp)
+            if (sp < S)
+#pragma unroll
+                for (int ri = 0; ri < 2; ++ri)
+                    *reinterpret_cast<uint4 *>(row + (long long)(2 * sp + ri) * W + e0) =
+                        make_uint4(o[sp][ri][0], o[sp][ri][1], o[sp][ri][2], o[sp][ri][3]);
+    }
+}
+
+// Operand rows of the NFOM^2 gauge points of m Euler points from their species' rows, by the
+// whole CTA: one 16-byte chunk of a proton row against every neutron row. Bound by the stores
+// (40 KB per point for three terms and the pf shell).
+__device__ __noinline__ void join_rows(const Params &p, int m, const unsigned short *rows, long long pt0) {
+    const int S = p.tc_splits, nk = p.tc_nk, npp = nk - p.tc_nph, W = nk + npp, nf = p.nfom, nch = W / 8;
+    const int total = m * S * 2 * nf * nch;
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+        const int c = t % nch;
+        int u = t / nch;
+        const int lp = u % nf;
+        u /= nf;
+        const int ri = u & 1, sp = (u >> 1) % S, it = (u >> 1) / S;
+        const unsigned short *r0 = rows + (long long)it * 2 * nf * 6 * W + (2 * sp + ri) * W + 8 * c;
+        const uint4 a = *reinterpret_cast<const uint4 *>(r0 + (long long)lp * 6 * W);
+        const long long pt = 2 * (pt0 + (long long)it * p.n_gauge + lp * nf) + ri;
+        unsigned short *dst = 8 * c < nk ? p.tc_x[sp] + pt * nk + 8 * c : p.tc_y[sp] + pt * npp + (8 * c - nk);
+        const long long step = 2LL * (8 * c < nk ? nk : npp);
+        for (int ln = 0; ln < nf; ++ln) {
+            const uint4 b = *reinterpret_cast<const uint4 *>(r0 + (long long)(nf + ln) * 6 * W);
+            *reinterpret_cast<uint4 *>(dst + step * ln) = make_uint4(a.x | b.x, a.y | b.y, a.z | b.z, a.w | b.w);
+        }
+    }
+}
+
+// Rotation blocks R_b(i,k) = e^{-i alp m_i} d^j_{m_i m_k}(bet) e^{-i gam m_k} of one Euler point
+// (ROTATION_MAT, PNAMP_Proj.f90:83-136), entries t = tid, tid + nthr, ... of rot.
+__device__ __forceinline__ void rotation_blocks(const Params &p, int ie, int tid, int nthr, zc *rot) {
+    const double alp = p.euler[4 * ie], bet = p.euler[4 * ie + 1], gam = p.euler[4 * ie + 2];
+    double cb, sb;
+    sincos(0.5 * bet, &sb, &cb);
+    for (int b = 0; b < p.nblk; ++b) {
+        const int d = p.blk_size[b], tj = p.blk_tj[b], ro = p.blk_roff[b];
+        for (int e = tid; e < d * d; e += nthr) {
+            const int i = e / d, k = e % d;
+            const int mi = tj - 2 * i, mkk = tj - 2 * k;
+            const double dv = wigner_d(tj, mi, mkk, cb, sb, p.fact);
+            rot[ro + e] = dv * expi(-0.5 * (alp * mi + gam * mkk));
+        }
+    }
+}
+
+// One-body sums over the weighted density (FP64, rows and columns of the levels
+// [lev0, lev0 + N), stored at Sb[(r - lev0) lds + c - lev0]) of one (item, species) or item:
+// slots 0 Tr over protons, 1 over neutrons, 2 one-body energy, 3 sum j(j+1) rho_aa,
+// 4..6 Tr J+, J-, Jz, 7..16 the Q_{2mu} traces (proton rows).
+constexpr int kOneBody = 17;
+template <class Z>
+__device__ __forceinline__ zc one_body(const Params &p, int q, int lane, int lev0, int N, const Z *Sb, int lds) {
+    using Ra = Ar<Z>;
+    zc s = mk(0.0, 0.0);
+    if (q == 0 || q == 1 || q == 3 || q == 6) {
+        for (int a = lane; a < N; a += 32) {
+            const int g = lev0 + a;
+            double f = 1.0;
+            if (q == 0) f = g < p.h ? 1.0 : 0.0;
+            else if (q == 1) f = g < p.h ? 0.0 : 1.0;
+            else if (q == 3) f = p.obs.jj1[g];
+            else f = p.obs.mz[g];
+            if (f != 0.0) s = rfma(f, Ra::to(Sb[a * lds + a]), s);
+        }
+    } else if (q == 4 || q == 5) {
+        for (int a = lane; a < N; a += 32) {
+            const double f = p.obs.jp[lev0 + a];
+            if (f != 0.0) s = rfma(f, Ra::to(q == 4 ? Sb[(a + 1) * lds + a] : Sb[a * lds + a + 1]), s);
+        }
+    } else {
+        const int e0 = q == 2 ? 0 : p.obs.q_off[q - 7], e1 = q == 2 ? p.obs.n_t1b : p.obs.q_off[q - 6];
+        const int *idx = q == 2 ? p.obs.t1b_idx : p.obs.q_idx;
+        const double *val = q == 2 ? p.obs.t1b_val : p.obs.q_val;
+        for (int e = e0 + lane; e < e1; e += 32) {
+            const int ix = idx[e], r = (ix >> 8) - lev0, c = (ix & 255) - lev0;
+            if ((unsigned)r < (unsigned)N && (unsigned)c < (unsigned)N) s = rfma(val[e], Ra::to(Sb[r * lds + c]), s);
+        }
+    }
+    s.x = warp_sum(s.x);
+    s.y = warp_sum(s.y);
+    return s;
+}
+
+// ------------------------------------------------------------------ general reduced points
+// One Euler point of a reduced pair: its NFOM^2 gauge points dealt to the plan's thread
+// groups, which run them independently (n x n problems, named barriers per group). Observables
+// linear in rho are taken once per Euler point from the norm-weighted sum of rho.
+template <class Z>
+__device__ __noinline__ void reduced_item(const Params &p, const double *__restrict__ pr, zc *slot, int pair, int ie,
+                                          bool reload, double *__restrict__ zout, int *__restrict__ status,
+                                          double *__restrict__ gout, double *__restrict__ r1out,
+                                          double *__restrict__ r2out, long long pt0) {
+    using Ra = Ar<Z>;
+    using R = typename Ra::R;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const RedPlan &L = p.place.gen;
+    const int n = p.n, h = p.h, nn = n * n, ld = L.ld;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int ng = L.ng, gthr = 32 * L.w, gid = (int)threadIdx.x / gthr;
+    const bool onishi = p.nfom == 1, inverse = !p.norm_only;
+    Z *ephz = reinterpret_cast<Z *>(smem + L.off_eph);
+    zc *gacc = reinterpret_cast<zc *>(smem + L.off_acc);    // [ng][4]: N, N E2, N J2, N (unused)
+    int *gflag = reinterpret_cast<int *>(gacc + 4 * ng);
+    R *Z0 = reinterpret_cast<R *>(smem + L.off_z0);
+    Z *Y = reinterpret_cast<Z *>(slot);                     // R* Wi R^+
+    zc *RW = slot + nn;                                     // R* Wi
+    Z *Sb = reinterpret_cast<Z *>(slot + nn);               // [ng][n n], after RW is used
+    const double *gU1 = pr + p.pl.u1, *gV1 = pr + p.pl.v1, *gWi = pr + p.pl.zi, *gZ0 = pr + p.pl.z0;
+    const zc pfw = mk(pr[p.pl.pfz], pr[p.pl.pfz + 1]);
+    const double pre = p.vacfac * pr[p.pl.dets] * pr[p.pl.dets + 1];
+    if (reload) {
+        __syncthreads();
+        for (int t = threadIdx.x; t < nn; t += blockDim.x) {   // the skew matrix its upper triangle defines
+            const int i = t / n, j = t % n;
+            Z0[t] = i == j ? Ra::rzero() : Ra::real(i < j ? gZ0[t] : -gZ0[j * n + i]);
+        }
+        const double twopi = 6.283185307179586476925287;
+        for (int l = threadIdx.x; l < p.nfom; l += blockDim.x)
+            ephz[l] = Ra::from(expi(onishi ? 0.0 : twopi * l / p.nfom));
+    }
+    zc *rot = reinterpret_cast<zc *>(smem + L.off_grp);     // before the groups use their storage
+    __syncthreads();
+    rotation_blocks(p, ie, threadIdx.x, blockDim.x, rot);
+    __syncthreads();
+    for (int t = threadIdx.x; t < nn; t += blockDim.x) {
+        const int a = t / n, j = t % n;
+        const int b = p.row_blk[a], s0 = p.blk_start[b], d = p.blk_size[b];
+        const zc *Rr = rot + p.blk_roff[b] + (a - s0) * d;
+        zc rw = mk(0, 0);
+        for (int k = 0; k < d; ++k) rw = rfma(gWi[(s0 + k) * n + j], zconj(Rr[k]), rw);
+        RW[t] = rw;
+    }
+    __syncthreads();
+    // Y = (R* Wi) R^+, upper triangle (Y is skew)
+    for (int t = threadIdx.x; t < n * (n - 1) / 2; t += blockDim.x) {
+        int a, c;
+        tri_index(t, n, a, c);
+        const int b = p.row_blk[c], s0 = p.blk_start[b], d = p.blk_size[b];
+        const zc *Rr = rot + p.blk_roff[b] + (c - s0) * d;
+        zc x = mk(0, 0);
+        for (int k = 0; k < d; ++k) x = zfma(RW[a * n + s0 + k], zconj(Rr[k]), x);
+        Y[a * n + c] = Ra::from(x);
+    }
+    zc nrm1 = mk(0.0, 0.0);
+    if (onishi) {
+        // Onishi (PNAMP_Onishi.f90:21-37): sqrt(det(Ubar^T U0 + Vbar^T V0)), Ubar = R U1,
+        // Vbar = conj(R) V1 at phi = 0; LU determinant, principal root
+        const double *gU0 = pr + p.pl.u0, *gV0 = pr + p.pl.v0;
+        zc *RU = slot + 2 * nn, *RV = slot + 3 * nn;
+        for (int t = threadIdx.x; t < nn; t += blockDim.x) {
+            const int a = t / n, j = t % n;
+            const int b = p.row_blk[a], s0 = p.blk_start[b], d = p.blk_size[b];
+            const zc *Rr = rot + p.blk_roff[b] + (a - s0) * d;
+            zc ru = mk(0, 0), rv = mk(0, 0);
+            for (int k = 0; k < d; ++k) {
+                ru = rfma(gU1[(s0 + k) * n + j], Rr[k], ru);
+                rv = rfma(gV1[(s0 + k) * n + j], zconj(Rr[k]), rv);
+            }
+            RU[t] = ru;
+            RV[t] = rv;
+        }
+        __syncthreads();
+        zc *Bm = reinterpret_cast<zc *>(smem + L.off_grp);   // n x n, one group's A and Rh hold it
+        zc *invz = Bm + nn;
+        int *perm = reinterpret_cast<int *>(invz + n);
+        for (int t = threadIdx.x; t < nn; t += blockDim.x) {
+            const int i = t / n, j = t % n;
+            zc s = mk(0, 0);
+            for (int k = 0; k < n; ++k) {
+                s = rfma(gU0[k * n + j], RU[k * n + i], s);
+                s = rfma(gV0[k * n + j], RV[k * n + i], s);
+            }
+            Bm[t] = s;
+        }
+        __syncthreads();
+        const bool bsing = lu_factor<zc>(Bm, n, n, perm, invz, perm + n);
+        if (threadIdx.x == 0) {
+            zc det = mk(1.0, 0.0);
+            for (int k = 0; k < n; ++k) {
+                det = det * Bm[k * n + k];
+                if (perm[k] != k) det = -det;
+            }
+            if (bsing) det = mk(0.0, 0.0);
+            const double r = sqrt(det.x * det.x + det.y * det.y);
+            nrm1 = mk(sqrt(0.5 * (r + det.x)), copysign(sqrt(0.5 * fmax(r - det.x, 0.0)), det.y));
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    const Grp g{(int)threadIdx.x - gid * gthr, gthr, 1 + gid};
+    if (gid < ng) {
+        unsigned char *gb = smem + L.off_grp + gid * L.grp_bytes;
+        Z *A = reinterpret_cast<Z *>(gb), *Rh = A + n * ld;
+        SkewScratch<Z> &w = *reinterpret_cast<SkewScratch<Z> *>(gb + L.off_scr);
+        zc *nsh = reinterpret_cast<zc *>(gb + L.off_scr + sizeof(SkewScratch<Z>));   // the point's norm
+        Z *sb = Sb + (long long)gid * nn;
+        double *r2acc = r2out ? p.r2acc + 2LL * p.n_r2q * ((long long)blockIdx.x * ng + gid) : nullptr;
+        for (int q = g.tid; q < (r2out ? p.n_r2q : 0); q += g.nthr) {
+            r2acc[2 * q] = 0.0;
+            r2acc[2 * q + 1] = 0.0;
+        }
+        zc aN = mk(0, 0), aE = mk(0, 0), aJ = mk(0, 0);      // the group's thread 0
+        int flags = 0;
+        bool first = true;
+        for (int gi = gid; gi < p.n_gauge; gi += ng) {
+            const int lp = gi / p.nfom, ln = gi % p.nfom;
+            const Z zep = ephz[lp], zen = ephz[ln];
+            const bool sing = skew_problem<Z>(g, n, ld, h, zep * zep, zep * zen, zen * zen, Y, n, Z0, A, Rh, w,
+                                              inverse, L.tile);
+            zc norm = mk(0, 0);
+            if (g.tid < 32) {
+                int under;
+                const zc pf = pivot_product<Z>(w.piv, n / 2, p.cscale, under);
+                if (lane == 0) {
+                    const zc zph = mk(p.gphase[2 * gi], p.gphase[2 * gi + 1]);
+                    norm = onishi ? nrm1 : pre * ((pf * pfw) * zph);
+                    flags |= (onishi ? 0 : (under == 1 ? 1 : (under == 2 ? 4 : 0))) | (inverse && sing ? 2 : 0);
+                    aN = aN + norm;
+                    nsh[0] = norm;
+                }
+            }
+            const bool eval = inverse && !sing;
+            PointSums<Z> s;
+            if (eval) {
+                s = point_sums<Z>(g, p, n, ld, 0, 0, p.tc_splits ? 0 : p.nrec, A, Rh, w.red);
+                if (p.tc_splits) tc_rows<Z>(g, p, ld, A, Rh, pt0 + gi);
+            }
+            if (g.tid == 0) {
+                zc hg = mk(0, 0);
+                if (eval) {
+                    const zc e = Ra::to(s.e2), t = Ra::to(s.t1);
+                    hg = mk(e.x + t.x + p.e0, e.y + t.y);
+                    aE = zfma(norm, hg, aE);
+                    const zc a = Ra::to(s.tp), b = Ra::to(s.tm), c = Ra::to(s.tz);
+                    aJ = zfma(norm, Ra::to(s.j2) + a * b + c * c, aJ);
+                }
+                if (gout) {
+                    double *o = gout + 4LL * (((long long)pair * p.n_euler + ie) * p.n_gauge + gi);
+                    o[0] = norm.x;
+                    o[1] = norm.y;
+                    o[2] = hg.x;
+                    o[3] = hg.y;
+                }
+                if (p.tc_splits) {
+                    const double inv = 1.0 / ((double)p.nfom * p.nfom);
+                    p.tc_w[2 * (pt0 + gi)] = eval ? inv * norm.x : 0.0;
+                    p.tc_w[2 * (pt0 + gi) + 1] = eval ? inv * norm.y : 0.0;
+                }
+            }
+            gsync(g);   // nsh
+            if (eval) {
+                const zc nv = nsh[0];
+                const Z wn = Ra::from(nv);
+                for (int t = g.tid; t < nn; t += g.nthr) {
+                    const Z rv = Rh[(t / n) * ld + t % n];
+                    sb[t] = first ? wn * rv : zfma(wn, rv, sb[t]);
+                }
+                first = false;
+                for (int q = g.tid; q < (r2out ? p.n_r2q : 0); q += g.nthr) {
+                    const zc a = zfma(nv, Ra::to(quad_product<Z>(p.r2q[q], 0, ld, A, Rh)),
+                                      mk(r2acc[2 * q], r2acc[2 * q + 1]));
+                    r2acc[2 * q] = a.x;
+                    r2acc[2 * q + 1] = a.y;
+                }
+            }
+            gsync(g);   // the next point overwrites the densities
+        }
+        if (first && inverse)
+            for (int t = g.tid; t < nn; t += g.nthr) sb[t] = szero<Z>();
+        if (g.tid == 0) {
+            gacc[4 * gid] = aN;
+            gacc[4 * gid + 1] = aE;
+            gacc[4 * gid + 2] = aJ;
+            gflag[gid] = flags;
+        }
+    }
+    __syncthreads();
+    // ---- the groups' sums: weighted density into the first group's storage, one-body traces
+    Z *St = reinterpret_cast<Z *>(smem + L.off_grp);
+    zc *ob = reinterpret_cast<zc *>(smem + L.off_grp + ((nn * (int)sizeof(Z) + 15) & ~15));
+    if (inverse) {
+        for (int t = threadIdx.x; t < nn; t += blockDim.x) {
+            Z s = Sb[t];
+            for (int q = 1; q < ng; ++q) s = s + Sb[(long long)q * nn + t];
+            St[t] = s;
+        }
+        __syncthreads();
+        for (int q = wid; q < kOneBody; q += kThreads / 32) {
+            const zc v = q >= 7 && !p.iE2 ? mk(0, 0) : one_body<Z>(p, q, lane, 0, n, St, n);
+            if (lane == 0) ob[q] = v;
+        }
+        if (r1out) {
+            const double inv = 1.0 / ((double)p.nfom * p.nfom);
+            for (int b = wid; b < p.obs.n_r1b; b += kThreads / 32) {
+                zc s = mk(0, 0);
+                for (int e = p.obs.r1b_off[b] + lane; e < p.obs.r1b_off[b + 1]; e += 32) {
+                    const int ix = p.obs.r1b_idx[e];
+                    s = rfma(p.obs.r1b_val[e], Ra::to(St[(ix >> 8) * n + (ix & 255)]), s);
+                }
+                s.x = warp_sum(s.x);
+                s.y = warp_sum(s.y);
+                if (lane == 0) {
+                    r1out[2LL * (((long long)pair * p.obs.n_r1b + b) * p.n_euler + ie)] = inv * s.x;
+                    r1out[2LL * (((long long)pair * p.obs.n_r1b + b) * p.n_euler + ie) + 1] = inv * s.y;
+                }
+            }
+        }
+        if (r2out) {   // Euler weight x gauge mean, added into the pair's sums (ZRho2B_Integral at J = 0)
+            const double wgt = p.euler[4 * ie + 3] / ((double)p.nfom * p.nfom);
+            double *o = r2out + 2LL * p.n_r2q * pair;
+            const double *a = p.r2acc + 2LL * p.n_r2q * (long long)blockIdx.x * ng;
+            for (int q = threadIdx.x; q < 2 * p.n_r2q; q += blockDim.x) {
+                double s = 0.0;
+                for (int k = 0; k < ng; ++k) s += a[2LL * p.n_r2q * k + q];
+                atomicAdd(o + q, wgt * s);
+            }
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < kNobs) {
+        const int io = threadIdx.x;
+        const double inv = 1.0 / ((double)p.nfom * p.nfom);
+        zc v = mk(0, 0);
+        int f = 0;
+        for (int q = 0; q < ng; ++q) {
+            f |= gflag[q];
+            if (io == 0) v = v + gacc[4 * q];
+            else if (io == 6) v = v + gacc[4 * q + 1];
+            else if (io == 7) v = v + gacc[4 * q + 2];
+        }
+        if (inverse) {
+            if (io >= 1 && io <= 3) v = ob[io - 1];
+            else if (io == 7) v = v + ob[3];
+            else if (io >= 8 && io < 18) v = ob[io - 1];
+        }
+        v = inv * v;
+        const unsigned bad = __ballot_sync((1u << kNobs) - 1u, !zfinite(v));
+        zout[2LL * (io * p.n_euler + ie)] = v.x;
+        zout[2LL * (io * p.n_euler + ie) + 1] = v.y;
+        if (io == 0) status[(long long)pair * p.n_euler + ie] = f | (bad ? 4 : 0);
+    }
+    __syncthreads();
+}
+
+// ------------------------------------------------------------------ species-split pairs
+// A pair without proton-neutron blocks: K is block-diagonal by species and the proton block
+// depends on phi_p only, the neutron block on phi_n only (K_s = Y_s - e^{2 i phi_s} Z0_s). So an
+// Euler point needs 2 NFOM problems of order h = n / 2, not NFOM^2 of order n. With the species'
+// weights a_s(phi) = Pf(c K_s) e^{-i phi N_s}, the norm is the product of the two sums of a_s,
+// observables of one species are its weighted sum times the other's norm sum, and the
+// proton-neutron energy and the cross terms of <J^2> are bilinear in the two weighted densities
+// sum_phi a_s rho_s, one contraction per Euler point.
+//
+// Up to ng / 2 Euler points at a time: a unit (Euler point, species, chunk of the gauge
+// points) per thread group, so that a launch with few Euler points still fills the groups.
+template <class Z>
+__device__ __noinline__ void split_items(const Params &p, const double *__restrict__ pr, zc *slot, int pair,
+                                         const int2 *__restrict__ items, int ie0, int m, bool reload,
+                                         double *__restrict__ zout, int *__restrict__ status,
+                                         double *__restrict__ gout, double *__restrict__ r1out,
+                                         double *__restrict__ r2out, long long pt0) {
+    using Ra = Ar<Z>;
+    using R = typename Ra::R;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const RedPlan &L = p.place.spl;
+    const int h = p.h, n = p.n, hh = h * h, ld = L.ld, nf = p.nfom;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int ng = L.ng, gthr = 32 * L.w, gid = (int)threadIdx.x / gthr;
+    const bool inverse = !p.norm_only;
+    const int nc = max(1, min(ng / (2 * m), nf)), nu = 2 * m * nc;   // chunks per species, units
+    const int tcw = 2 * p.tc_nk - p.tc_nph;                          // width of a species row
+    unsigned short *rows = p.tc_splits ? p.tc_sp + (long long)blockIdx.x * L.items * 2 * nf * 6 * tcw : nullptr;
+    Z *ephz = reinterpret_cast<Z *>(smem + L.off_eph);
+    zc *asum = reinterpret_cast<zc *>(smem + L.off_acc);     // [m][2][nf]: a_s(phi)
+    zc *uacc = asum + 2 * L.items * nf;                      // [unit][2]: sum a E_ss, sum a J2_ss
+    int *uflag = reinterpret_cast<int *>(uacc + 2 * max(ng, 2 * L.items));
+    R *Z0 = reinterpret_cast<R *>(smem + L.off_z0);          // [2][h][h]
+    // per unit: weighted density; per item: the species blocks of Y. R* Wi takes the densities' place
+    Z *Y = reinterpret_cast<Z *>(slot);                      // [m][2][h h]
+    Z *Sb = reinterpret_cast<Z *>(slot + 2LL * L.items * hh);
+    zc *RW = slot + 2LL * L.items * hh;                      // [m][2][h h]
+    const double *gWi = pr + p.pl.zi, *gZ0 = pr + p.pl.z0;
+    auto euler = [&](int k) { return items ? items[k].y : ie0 + k; };
+    if (reload) {
+        __syncthreads();
+        for (int t = threadIdx.x; t < 2 * hh; t += blockDim.x) {
+            const int b = t / hh, i = (t % hh) / h, j = t % h;
+            const int u = (b * h + min(i, j)) * n + b * h + max(i, j);
+            Z0[t] = i == j ? Ra::rzero() : Ra::real(i < j ? gZ0[u] : -gZ0[u]);
+        }
+        const double twopi = 6.283185307179586476925287;
+        for (int l = threadIdx.x; l < nf; l += blockDim.x) {
+            const zc e = expi(twopi * l / nf);
+            ephz[l] = Ra::from(e);
+        }
+    }
+    zc *rot = reinterpret_cast<zc *>(smem + L.off_grp);      // [m][rot_elems], before the groups run
+    __syncthreads();
+    {
+        // warps share the Euler points evenly
+        const int wpi = max(1, (kThreads / 32) / m), item = wid / wpi;
+        if (item < m)
+            rotation_blocks(p, euler(item), (int)threadIdx.x - item * wpi * 32, wpi * 32, rot + (long long)item * p.rot_elems);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 2 * hh * m; t += blockDim.x) {
+        const int it = t / (2 * hh), e = t % (2 * hh), s = e / hh, a = s * h + (e % hh) / h, j = s * h + e % h;
+        const int b = p.row_blk[a], s0 = p.blk_start[b], d = p.blk_size[b];
+        const zc *Rr = rot + (long long)it * p.rot_elems + p.blk_roff[b] + (a - s0) * d;
+        zc rw = mk(0, 0);
+        for (int k = 0; k < d; ++k) rw = rfma(gWi[(s0 + k) * n + j], zconj(Rr[k]), rw);
+        RW[t] = rw;
+    }
+    __syncthreads();
+    const int Th = h * (h - 1) / 2;
+    for (int t = threadIdx.x; t < 2 * Th * m; t += blockDim.x) {
+        const int it = t / (2 * Th), e = t % (2 * Th), s = e / Th;
+        int a, c;
+        tri_index(e % Th, h, a, c);
+        const int b = p.row_blk[s * h + c], s0 = p.blk_start[b], d = p.blk_size[b];
+        const zc *Rr = rot + (long long)it * p.rot_elems + p.blk_roff[b] + (s * h + c - s0) * d;
+        const zc *rw = RW + (long long)(2 * it + s) * hh + a * h + s0 - s * h;
+        zc x = mk(0, 0);
+        for (int k = 0; k < d; ++k) x = zfma(rw[k], zconj(Rr[k]), x);
+        Y[(long long)(2 * it + s) * hh + a * h + c] = Ra::from(x);
+    }
+    __syncthreads();
+    // ---- the problems
+    const Grp g{(int)threadIdx.x - gid * gthr, gthr, 1 + gid};
+    for (int u = gid; gid < ng && u < nu; u += ng) {
+        const int it = u / (2 * nc), s = (u / nc) & 1, chunk = u % nc;
+        unsigned char *gb = smem + L.off_grp + gid * L.grp_bytes;
+        Z *A = reinterpret_cast<Z *>(gb), *Rh = A + h * ld;
+        SkewScratch<Z> &w = *reinterpret_cast<SkewScratch<Z> *>(gb + L.off_scr);
+        zc *ash = reinterpret_cast<zc *>(gb + L.off_scr + sizeof(SkewScratch<Z>));
+        Z *sb = Sb + (long long)u * hh;
+        // two-body density: same-species quadruples, sum over phi of a_s times their products
+        const int q0 = p.r2_off[s], nq = r2out ? p.r2_off[s + 1] - q0 : 0;
+        double *r2acc = nq ? p.r2acc + 2LL * p.r2_ss * ((long long)blockIdx.x * max(ng, 2 * L.items) + u) : nullptr;
+        zc aE = mk(0, 0), aJ = mk(0, 0);   // the group's thread 0
+        int flags = 0;
+        bool first = true;
+        for (int l = chunk; l < nf; l += nc) {
+            const Z d = ephz[l] * ephz[l];
+            const bool sing = skew_problem<Z>(g, h, ld, h, d, d, d, Y + (long long)(2 * it + s) * hh, h, Z0 + s * hh, A,
+                                              Rh, w, inverse, L.tile);
+            if (g.tid < 32) {
+                int under;
+                const zc pf = pivot_product<Z>(w.piv, h / 2, p.cscale, under);
+                if (lane == 0) {
+                    const int o = s ? l : l * nf;   // e^{-i phi N_s}: the other species' angle is 0
+                    const zc a = pf * mk(p.gphase[2 * o], p.gphase[2 * o + 1]);
+                    asum[(2 * it + s) * nf + l] = a;
+                    ash[0] = a;
+                    flags |= (under == 1 ? 1 : (under == 2 ? 4 : 0)) | (inverse && sing ? 2 : 0);
+                }
+            }
+            if (!inverse || sing) continue;   // uniform over the group
+            const PointSums<Z> q = point_sums<Z>(g, p, h, ld, s * h, p.rec_off[s],
+                                                p.tc_splits ? p.rec_off[s] : p.rec_off[s + 1], A, Rh, w.red);
+            if (p.tc_splits) species_rows<Z>(g, p, s, h, ld, A, Rh, rows + ((long long)(2 * it + s) * nf + l) * 6 * tcw);
+            if (g.tid == 0) {
+                const zc a = ash[0];
+                aE = zfma(a, Ra::to(q.e2), aE);
+                const zc tp = Ra::to(q.tp), tm = Ra::to(q.tm), tz = Ra::to(q.tz);
+                aJ = zfma(a, Ra::to(q.j2) + tp * tm + tz * tz, aJ);
+            }
+            gsync(g);
+            const Z wa = Ra::from(ash[0]);
+            for (int t = g.tid; t < hh; t += g.nthr) {
+                const Z rv = Rh[(t / h) * ld + t % h];
+                sb[t] = first ? wa * rv : zfma(wa, rv, sb[t]);
+            }
+            for (int q = g.tid; q < nq; q += g.nthr) {
+                const zc x = Ra::to(quad_product<Z>(p.r2s[q0 + q].x, s * h, ld, A, Rh));
+                const zc v = first ? ash[0] * x : zfma(ash[0], x, mk(r2acc[2 * q], r2acc[2 * q + 1]));
+                r2acc[2 * q] = v.x;
+                r2acc[2 * q + 1] = v.y;
+            }
+            first = false;
+            gsync(g);   // the next problem overwrites the densities
+        }
+        if (first && inverse) {
+            for (int t = g.tid; t < hh; t += g.nthr) sb[t] = szero<Z>();
+            for (int q = g.tid; q < 2 * nq; q += g.nthr) r2acc[q] = 0.0;
+        }
+        if (g.tid == 0) {
+            uacc[2 * u] = aE;
+            uacc[2 * u + 1] = aJ;
+            uflag[u] = flags;
+        }
+    }
+    __syncthreads();
+    // ---- per Euler point: weighted densities of both species side by side, then the sums
+    const double inv = 1.0 / ((double)nf * nf);
+    const zc pre = (p.vacfac * pr[p.pl.dets] * pr[p.pl.dets + 1]) * mk(pr[p.pl.pfz], pr[p.pl.pfz + 1]);
+    Z *St = reinterpret_cast<Z *>(smem + L.off_grp);                      // [m][2][h h]
+    zc *ob = reinterpret_cast<zc *>(St + 2 * hh * m);                     // [m][2][kOneBody]
+    zc *epn = ob + 2 * kOneBody * m;                                      // [m]
+    zc *asm2 = epn + m;                                                   // [m][2] sums of a_s
+    if (inverse) {
+        for (int t = threadIdx.x; t < 2 * hh * m; t += blockDim.x) {
+            const int is = t / hh, e = t % hh;
+            Z v = Sb[(long long)is * nc * hh + e];
+            for (int q = 1; q < nc; ++q) v = v + Sb[((long long)is * nc + q) * hh + e];
+            St[t] = v;
+        }
+        __syncthreads();
+        for (int t = wid; t < 2 * kOneBody * m; t += kThreads / 32) {
+            const int is = t / kOneBody, q = t % kOneBody, s = is & 1;
+            const bool none = (q == 0 && s) || (q == 1 && !s) || (q >= 7 && (s || !p.iE2));
+            const zc v = none ? mk(0, 0) : one_body<Z>(p, q, lane, s * h, h, St + (long long)is * hh, h);
+            if (lane == 0) ob[t] = v;
+        }
+        // proton-neutron records, (i, k) protons, (j, l) neutrons: only the direct terms
+        const int wpi = max(1, (kThreads / 32) / m);
+        zc *part = asm2 + 2 * m;                                          // [warps]
+        if (wid / wpi < m) {
+            const Z *Sp = St + (long long)(wid / wpi) * 2 * hh, *Sn = Sp + hh;
+            using O = Op<Z>;
+            typename O::Acc e2 = O::acc(szero<Z>());
+            for (int e = p.nrec_gen + (wid % wpi) * 32 + lane; e < (p.tc_splits ? 0 : p.nrec); e += wpi * 32) {
+                const uint32_t pk = p.rec_idx[e];
+                const int i = pk & 0xff, j = ((pk >> 8) & 0xff) - h, k = (pk >> 16) & 0xff, l = (pk >> 24) - h;
+                typename O::Acc t = O::acc(szero<Z>());
+                const Z b0 = Sn[l * h + j];
+                O::cadd(t, O::mul(Sp[k * h + i]), b0, O::rot(b0));
+                if (i + j != k + l) {
+                    const Z b1 = Sn[j * h + l];
+                    O::cadd(t, O::mul(Sp[i * h + k]), b1, O::rot(b1));
+                }
+                O::radd(e2, O::rmul(Ra::pick(p.rec_v, p.rec_vd, e)), O::done(t));
+            }
+            const Z v = warp_sum_z(O::done(e2));
+            if (lane == 0) part[wid] = Ra::to(v);
+        }
+        __syncthreads();
+        if (threadIdx.x < m) {
+            zc v = mk(0, 0);
+            for (int q = 0; q < wpi; ++q) v = v + part[threadIdx.x * wpi + q];
+            epn[threadIdx.x] = v;
+        }
+    }
+    if (threadIdx.x >= 64 && threadIdx.x - 64 < 2 * m) {
+        const int is = threadIdx.x - 64;
+        zc v = mk(0, 0);
+        for (int l = 0; l < nf; ++l) v = v + asum[is * nf + l];
+        asm2[is] = v;
+    }
+    __syncthreads();
+    if (p.tc_splits) {
+        join_rows(p, m, rows, pt0);
+        for (int t = threadIdx.x; t < m * p.n_gauge; t += blockDim.x) {   // w = N / NFOM^2
+            const int it = t / p.n_gauge, gi = t % p.n_gauge;
+            const zc v = inv * (pre * (asum[2 * it * nf + gi / nf] * asum[(2 * it + 1) * nf + gi % nf]));
+            p.tc_w[2 * (pt0 + t)] = v.x;
+            p.tc_w[2 * (pt0 + t) + 1] = v.y;
+        }
+    }
+    if (r2out) {   // Euler weight x gauge mean over the batch, added into the pair's sums
+        double *o = r2out + 2LL * p.n_r2q * pair;
+        const long long us = 2LL * p.r2_ss, u0 = (long long)blockIdx.x * max(ng, 2 * L.items);
+        for (int t = threadIdx.x; t < p.n_r2q; t += blockDim.x) {
+            const int s = t < p.r2_off[1] ? 0 : (t < p.r2_off[2] ? 1 : 2);
+            const uint2 qd = p.r2s[t];
+            zc v = mk(0, 0);
+            for (int it = 0; it < m; ++it) {
+                const double wgt = inv * p.euler[4 * euler(it) + 3];
+                zc x = mk(0, 0);
+                if (s < 2) {
+                    for (int q = 0; q < nc; ++q) {
+                        const double *a = p.r2acc + us * (u0 + (2 * it + s) * nc + q) + 2 * (t - p.r2_off[s]);
+                        x = x + mk(a[0], a[1]);
+                    }
+                    x = asm2[2 * it + 1 - s] * x;
+                } else {   // one proton and one neutron density, rho_ki rho_lj
+                    const int i = qd.x & 0xff, j = (qd.x >> 8) & 0xff, k = (qd.x >> 16) & 0xff, l = qd.x >> 24;
+                    const int si = i >= h ? 1 : 0, sj = 1 - si;
+                    const Z *Sa = St + (long long)(2 * it + si) * hh, *Sc = St + (long long)(2 * it + sj) * hh;
+                    x = Ra::to(Sa[(k - si * h) * h + i - si * h]) * Ra::to(Sc[(l - sj * h) * h + j - sj * h]);
+                }
+                v = v + wgt * x;
+            }
+            v = pre * v;
+            atomicAdd(o + 2 * qd.y, v.x);
+            atomicAdd(o + 2 * qd.y + 1, v.y);
+        }
+    }
+    for (int it = wid; it < m; it += kThreads / 32) {
+        const int ie = euler(it);
+        const zc ap = asm2[2 * it], an = asm2[2 * it + 1];
+        zc v = mk(0, 0);
+        int f = 0;
+        if (lane < 2 * nc) f = uflag[2 * it * nc + lane];
+        for (int k = 32 + lane; k < 2 * nc; k += 32) f |= uflag[2 * it * nc + k];
+        f = (int)__reduce_or_sync(0xffffffffu, (unsigned)f);
+        if (lane == 0) v = pre * (ap * an);
+        if (inverse && lane > 0 && lane < 18) {
+            const zc *op = ob + 2 * it * kOneBody, *on = op + kOneBody;
+            if (lane == 1) v = an * op[0];
+            else if (lane == 2) v = ap * on[1];
+            else if (lane == 3) v = an * op[2] + ap * on[2];
+            else if (lane == 6 || lane == 7) {
+                zc sp = mk(0, 0), sn = mk(0, 0);
+                for (int q = 0; q < nc; ++q) {
+                    sp = sp + uacc[2 * (2 * it * nc + q) + lane - 6];
+                    sn = sn + uacc[2 * ((2 * it + 1) * nc + q) + lane - 6];
+                }
+                if (lane == 6) {   // two-body + one-body energy + e0 N
+                    v = an * (sp + op[2]) + ap * (sn + on[2]) + epn[it] + p.e0 * (ap * an);
+                } else {
+                    v = an * (sp + op[3]) + ap * (sn + on[3]) + op[4] * on[5] + on[4] * op[5] +
+                        2.0 * (op[6] * on[6]);
+                }
+            } else if (lane >= 8) v = an * op[lane - 1];
+            v = pre * v;
+        }
+        v = inv * v;
+        const unsigned bad = __ballot_sync(0xffffffffu, !zfinite(v));
+        if (lane < kNobs) {
+            zout[2LL * (lane * p.n_euler + ie)] = v.x;
+            zout[2LL * (lane * p.n_euler + ie) + 1] = v.y;
+        }
+        if (lane == 0) status[(long long)pair * p.n_euler + ie] = f | (bad ? 4 : 0);
+        if (r1out) {
+            for (int b = 0; b < p.obs.n_r1b; ++b) {
+                zc s = mk(0, 0);
+                int sp = 0;
+                for (int e = p.obs.r1b_off[b] + lane; e < p.obs.r1b_off[b + 1]; e += 32) {
+                    const int ix = p.obs.r1b_idx[e], r = ix >> 8, c = ix & 255;
+                    sp = r >= h ? 1 : 0;
+                    s = rfma(p.obs.r1b_val[e], Ra::to(St[(long long)(2 * it + sp) * hh + (r - sp * h) * h + c - sp * h]), s);
+                }
+                s.x = warp_sum(s.x);
+                s.y = warp_sum(s.y);
+                if (lane == 0) {   // a block is one species: lane 0 holds its first entry
+                    const zc o = inv * (pre * ((sp ? ap : an) * s));
+                    r1out[2LL * (((long long)pair * p.obs.n_r1b + b) * p.n_euler + ie)] = o.x;
+                    r1out[2LL * (((long long)pair * p.obs.n_r1b + b) * p.n_euler + ie) + 1] = o.y;
+                }
+            }
+        }
+        if (gout)   // norm-only launches: N at every gauge point
+            for (int gi = lane; gi < p.n_gauge; gi += 32) {
+                const zc w = pre * (asum[2 * it * nf + gi / nf] * asum[(2 * it + 1) * nf + gi % nf]);
+                double *o = gout + 4LL * (((long long)pair * p.n_euler + ie) * p.n_gauge + gi);
+                o[0] = w.x;
+                o[1] = w.y;
+                o[2] = 0.0;
+                o[3] = 0.0;
+            }
+    }
+    __syncthreads();
+}
+
+}  // namespace pnamp
