@@ -18,6 +18,7 @@ constexpr int kNTrace = 10;              // proton traces of Q_{2mu} rho and Q_{
 constexpr int kNJKK = 1 + 25 + 81 + 169; // (J, K1, K2) with even J <= 6
 constexpr int kProjFields = 5;           // njkk, hjkk, nn, zz, j2
 constexpr int kSetupThreads = 256;
+constexpr int kSetupCluster = 4;          // CTAs that share one pair's set-up
 constexpr int kMultiSmemTail = 16;       // dynamic shared bytes after the placement: multi kernel's counter
 
 // One pair record (doubles), all matrices row-major n x n:

@@ -32,6 +32,7 @@
 // FP64 195.3 -> 13.8 ms and double-float 74.7 -> 4.9 ms, proton-neutron mixing with the BF16x6
 // contraction 193.3 -> 69.2 ms, against full_item's algebra for every pair (two points in flight
 // for charge-conserving ones).
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -816,13 +817,23 @@ __device__ __forceinline__ bool pivots_within(const double *A, int n, double rat
     return mx > 0.0 && mn >= ratio * mx;
 }
 
-__global__ void __launch_bounds__(kSetupThreads)
+// One pair per cluster of four CTAs, bra and ket side by side and within each the two independent
+// chains: (0, 1) U = LU, Z = V U^-1 (W or Z0), log|det U| and the Pfaffian of Z; (2, 3) log det of
+// U^T U + V^T V, V = LU and U V^-1. The elimination steps follow one another at the FP64 pipe's
+// latency, so the chains' length is the time: 460 steps in one CTA took 596 us for n = 40,
+// 140 to 160 here.
+//   det(1 + Z^T Z) = det(U^T U + V^T V) / det(U)^2, whose -1/4 power is the vacuum's overlap
+// (the eigenvalue product of zbareover).
+__global__ void __cluster_dims__(kSetupCluster, 1, 1) __launch_bounds__(kSetupThreads)
 setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairbuf) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n = p.n;
-    const long long nn = (long long)n * n;
-    const double *in = uv + (long long)blockIdx.x * 4 * nn;
-    double *out = pairbuf + (long long)blockIdx.x * p.pl.stride;
+    __shared__ double xchg[4];   // this chain's logarithm of a determinant, its flags
+    const int n = p.n, part = (int)cl.block_rank(), ket = (part & 1) == 0, tail = part >= 2;
+    const long long nn = (long long)n * n, pair = blockIdx.x / kSetupCluster;
+    const double *in = uv + pair * 4 * nn;
+    double *out = pairbuf + pair * p.pl.stride;
     double *A = reinterpret_cast<double *>(smem_raw);
     double *Yb = A + nn;
     double *invd = Yb + nn;
@@ -830,99 +841,120 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
     zc *vecz = reinterpret_cast<zc *>(red + 64);    // n complex: the Pfaffian's pivot row
     int *perm = reinterpret_cast<int *>(vecz + n);
     int *sh = perm + n;
-    // column-major input -> row-major pair record (U0, V0, U1, V1)
-    for (long long t = threadIdx.x; t < 4 * nn; t += blockDim.x) {
-        const long long q = t / nn, e = t % nn;
-        const int i = (int)(e / n), j = (int)(e % n);
-        out[q * nn + e] = in[q * nn + i + (long long)j * n];
+    const double *inU = in + (ket ? 2 : 0) * nn, *inV = inU + nn;   // column-major
+    // row-major U0, V0, U1, V1 of the pair record: chain (bra, ket) x (U, V)
+    for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
+        const int i = (int)(t / n), j = (int)(t % n);
+        const double u = inU[i + (long long)j * n], v = inV[i + (long long)j * n];
+        A[t] = tail ? v : u;
+        Yb[t] = tail ? u : v;
+        out[(tail ? (ket ? p.pl.v1 : p.pl.v0) : (ket ? p.pl.u1 : p.pl.u0)) + t] = A[t];
     }
     __syncthreads();
     int st = 0;
-    bool u0_ok = false;
-    for (int which = 0; which < 2; ++which) {
-        const double *U = out + (which == 0 ? p.pl.u1 : p.pl.u0);
-        const double *V = out + (which == 0 ? p.pl.v1 : p.pl.v0);
-        double *Z = out + (which == 0 ? p.pl.w : p.pl.z0);
-        for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
-            A[t] = U[t];
-            Yb[t] = V[t];
+    double logdet = 0.0;
+    if (tail) {   // U^T U + V^T V: both matrices are needed again, so the sum goes through registers
+        constexpr int kMost = (kMaxN * kMaxN + kSetupThreads - 1) / kSetupThreads;
+        double g[kMost];
+#pragma unroll
+        for (int e = 0; e < kMost; ++e) {
+            const int t = threadIdx.x + e * kSetupThreads, i = t / n, j = t % n;
+            double s = 0.0;
+            if (t < n * n)
+                for (int k = 0; k < n; ++k) {
+                    s = fma(A[k * n + i], A[k * n + j], s);
+                    s = fma(Yb[k * n + i], Yb[k * n + j], s);
+                }
+            g[e] = s;
         }
         __syncthreads();
-        if (lu_factor<double>(A, n, n, perm, invd, sh)) st = 1;
-        if (which == 1) u0_ok = pivots_within(A, n, kReducedPivotRatio);
-        row_solve<double>(Yb, n, n, A, n, n, perm, invd);  // Z = V U^-1
-        for (long long t = threadIdx.x; t < nn; t += blockDim.x) Z[t] = Yb[t];
+#pragma unroll
+        for (int e = 0; e < kMost; ++e)
+            if (threadIdx.x + e * kSetupThreads < n * n) A[threadIdx.x + e * kSetupThreads] = g[e];
         __syncthreads();
-        // det(1 + Z^T Z)^(-1/4): the eigenvalue product of zbareover, via LU
-        for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
-            const int i = (int)(t / n), j = (int)(t % n);
-            double s = (i == j) ? 1.0 : 0.0;
-            for (int k = 0; k < n; ++k) s = fma(Yb[k * n + i], Yb[k * n + j], s);
-            A[t] = s;
+        if (lu_factor<double>(A, n, n, perm, invd, sh)) st = 1;
+    }
+    bool ok = false;
+    for (int pass = tail ? 0 : 1; pass < 2; ++pass) {
+        if (pass == 1) {
+            if (tail) {
+                for (long long t = threadIdx.x; t < nn; t += blockDim.x)
+                    A[t] = inV[t / n + (t % n) * n];
+                __syncthreads();
+            }
+            const bool sing = lu_factor<double>(A, n, n, perm, invd, sh);
+            if (sing && !tail) st = 1;
+            ok = !sing && pivots_within(A, n, kReducedPivotRatio);
         }
-        __syncthreads();
-        if (lu_factor<double>(A, n, n, perm, invd, sh)) st = 1;
-        double v[1] = {0.0};
-        for (int k = threadIdx.x; k < n; k += blockDim.x) v[0] += log(fabs(A[k * n + k]));
-        block_sum<1>(v, red);
-        if (threadIdx.x == 0) out[p.pl.dets + (which == 0 ? 1 : 0)] = exp(-0.25 * v[0]);
+        if (pass == 0 || !tail) {
+            double v[1] = {0.0};
+            for (int k = threadIdx.x; k < n; k += blockDim.x) v[0] += log(fabs(A[k * n + k]));
+            block_sum<1>(v, red);
+            logdet = v[0];
+        }
         __syncthreads();
     }
+    if (!tail || ok) row_solve<double>(Yb, n, n, A, n, n, perm, invd);  // V U^-1, or U V^-1
+    int big = 0;
+    for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
+        if (!tail) out[(ket ? p.pl.w : p.pl.z0) + t] = Yb[t];
+        else if (!(fabs(Yb[t]) <= kReducedMaxEntry)) big = 1;
+    }
+    big = __syncthreads_or(big);
+    int cross = 0;   // proton-neutron blocks of this chain's matrix
+    for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
+        const int i = (int)(t / n), j = (int)(t % n);
+        if ((i < p.h) != (j < p.h) && (tail ? inV : inU)[i + (long long)j * n] != 0.0) cross = 1;
+    }
+    cross = __syncthreads_or(cross);
+    if (threadIdx.x == 0) {
+        xchg[0] = logdet;
+        xchg[1] = (double)st;
+        xchg[2] = ok && !(tail && ket && big) ? 1.0 : 0.0;
+        xchg[3] = (double)cross;
+    }
+    cl.sync();
+    double x[4][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[k][q] = *cl.map_shared_rank(&xchg[q], k);
+    cl.sync();   // read before any CTA exits
     // Once-per-pair pieces of the Pfaffians. Reduced pairs (V1 and U0 well conditioned): W^-1 and
     // Pf(c W) for point_reduced.cuh. Others with a well conditioned V0: block elimination of the
     // lower-right block of S = c [[D X D, -I], [I, -Z0]] gives Pf(S) = Pf(c (D X D - Z0^-1))
-    // Pf(-c Z0). Otherwise both flags stay 0 and the 2n x 2n form is used.
-    double schur = 0.0, reduced = 0.0;
+    // Pf(-c Z0). Otherwise both flags stay 0 and the 2n x 2n form is used. (A Pfaffian that
+    // underflows is kept as the 2n x 2n form too.)
+    const bool reduced = x[1][2] != 0.0 && x[2][2] != 0.0, schur = !reduced && x[3][2] != 0.0;
+    if ((reduced && part == 2) || (schur && part == 3))
+        for (long long t = threadIdx.x; t < nn; t += blockDim.x) out[p.pl.zi + t] = Yb[t];
+    const int pfpart = schur ? 1 : 0;
+    if (part != pfpart) return;
+    int under = 0;
     zc pf = mk(0.0, 0.0);
-    for (int kind = 0; kind < 2 && schur == 0.0 && reduced == 0.0; ++kind) {
-        if (kind == 0 && !u0_ok) continue;
-        const double *U = out + (kind == 0 ? p.pl.u1 : p.pl.u0), *V = out + (kind == 0 ? p.pl.v1 : p.pl.v0);
-        const double *Z = out + (kind == 0 ? p.pl.w : p.pl.z0);
-        const double f = kind == 0 ? p.cscale : -p.cscale;
-        for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
-            A[t] = V[t];
-            Yb[t] = U[t];
-        }
-        __syncthreads();
-        const bool vsing = lu_factor<double>(A, n, n, perm, invd, sh);
-        const bool well = !vsing && pivots_within(A, n, kReducedPivotRatio);
-        __syncthreads();
-        if (!well) continue;
-        row_solve<double>(Yb, n, n, A, n, n, perm, invd);  // U V^-1
-        int big = 0;
-        for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
-            out[p.pl.zi + t] = Yb[t];
-            if (!(fabs(Yb[t]) <= kReducedMaxEntry)) big = 1;
-        }
-        if (__syncthreads_or(big) && kind == 0) continue;
+    if (reduced || schur) {
+        const double f = reduced ? p.cscale : -p.cscale;
+        const double *Z = out + (reduced ? p.pl.w : p.pl.z0);   // this CTA's own result
         zc *Sz = reinterpret_cast<zc *>(A);  // n^2 complex over A and Yb
         for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
             const int i = (int)(t / n), j = (int)(t % n);
             Sz[t] = mk(i < j ? f * Z[t] : 0.0, 0.0);
         }
         __syncthreads();
-        int under = 0;
         pf = pfaffian_upper<zc>(Sz, n, vecz, red, sh, under);   // in thread 0
-        const double ok = __syncthreads_and(threadIdx.x != 0 || (under == 0 && zfinite(pf))) ? 1.0 : 0.0;
-        if (kind == 0) reduced = ok;
-        else schur = ok;
     }
-    // species split: U0, V0, U1, V1 without proton-neutron blocks (charge-conserving vacua)
-    // make every per-point matrix block-diagonal by species (protons first, h = n/2 each)
-    int cross = 0;
-    for (long long t = threadIdx.x; t < 4 * nn; t += blockDim.x) {
-        const long long e = t % nn;
-        const int i = (int)(e / n), j = (int)(e % n);
-        if ((i < p.h) != (j < p.h) && out[t] != 0.0) cross = 1;  // U0, V0, U1, V1 lead the record
-    }
-    cross = __syncthreads_or(cross);
     if (threadIdx.x == 0) {
-        out[p.pl.dets + 2] = (double)st;
-        out[p.pl.dets + 3] = schur;
+        const bool fine = under == 0 && zfinite(pf);
+        out[p.pl.dets] = exp(-0.25 * (x[3][0] - 2.0 * x[1][0]));
+        out[p.pl.dets + 1] = exp(-0.25 * (x[2][0] - 2.0 * x[0][0]));
+        out[p.pl.dets + 2] = x[0][1] + x[1][1] + x[2][1] + x[3][1] != 0.0 ? 1.0 : 0.0;
+        out[p.pl.dets + 3] = schur && fine ? 1.0 : 0.0;
         out[p.pl.pfz] = pf.x;
         out[p.pl.pfz + 1] = pf.y;
-        out[p.pl.dets + 6] = cross ? 0.0 : 1.0;
-        out[p.pl.dets + 7] = reduced;
+        // species split: U0, V0, U1, V1 without proton-neutron blocks (charge-conserving vacua)
+        // make every per-point matrix block-diagonal by species (protons first, h = n/2 each)
+        out[p.pl.dets + 6] = x[0][3] + x[1][3] + x[2][3] + x[3][3] != 0.0 ? 0.0 : 1.0;
+        out[p.pl.dets + 7] = reduced && fine ? 1.0 : 0.0;
     }
 }
 
@@ -951,7 +983,7 @@ cudaError_t prepare_setup(int n) {
 // Enqueues only (no attribute calls): usable under stream capture once
 // prepare_setup(n) ran at context creation.
 cudaError_t launch_setup(const Params &p, int npairs, const double *uv, double *pairbuf, cudaStream_t st) {
-    setup_kernel<<<npairs, kSetupThreads, setup_smem_bytes(p.n), st>>>(p, uv, pairbuf);
+    setup_kernel<<<npairs * kSetupCluster, kSetupThreads, setup_smem_bytes(p.n), st>>>(p, uv, pairbuf);
     return cudaGetLastError();
 }
 
@@ -1806,23 +1838,56 @@ __global__ void proj_weights_kernel(Params p, int axial, zc *w) {
     }
 }
 
-__global__ void project_kernel(Params p, const zc *__restrict__ w, const double *__restrict__ zres,
-                               int core_prot, int core_neut, int chop, double *__restrict__ out) {
-    const int pair = blockIdx.x;
-    const int jkk = blockIdx.y * blockDim.x + threadIdx.x;
-    if (jkk >= kNJKK) return;
+// One (pair, tile of 16 (J, K1, K2)) per cluster of 8 CTAs: the CTAs share the Euler points, a CTA's
+// 256 threads are 16 weights x 16 points, partial sums meet in shared memory and then in the
+// cluster's first CTA, in a fixed order. The sums are FP64 multiply-adds (8 complex ones per
+// Euler point and weight) and a lone pair must reach every SM's narrow FP64 pipe: 144 CTAs per
+// pair. One thread per weight over all Euler points took 2.35 ms for a pf pair's 2000 points.
+constexpr int kProjTile = 16, kProjLanes = 16, kProjCluster = 8;
+constexpr int kProjTiles = (kNJKK + kProjTile - 1) / kProjTile;
+__global__ void __cluster_dims__(kProjCluster, 1, 1) __launch_bounds__(kProjTile * kProjLanes)
+project_kernel(Params p, const zc *__restrict__ w, const double *__restrict__ zres, int core_prot, int core_neut,
+               int chop, double *__restrict__ out) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ zc part[8][kProjLanes][kProjTile];
+    __shared__ zc sum[8][kProjTile];
+    const int rank = (int)cl.block_rank();
+    const int unit = (int)(blockIdx.x / kProjCluster);
+    const int pair = unit / kProjTiles, j = threadIdx.x % kProjTile, ln = threadIdx.x / kProjTile;
+    const int jkk = (unit % kProjTiles) * kProjTile + j;
     const double *z = zres + 2LL * pair * kNobs * p.n_euler;
     zc s[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) s[q] = mk(0, 0);
-    for (int ie = 0; ie < p.n_euler; ++ie) {
+    for (int ie = rank * kProjLanes + ln; ie < p.n_euler && jkk < kNJKK; ie += kProjCluster * kProjLanes) {
         const zc wv = w[(long long)ie * kNJKK + jkk];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const zc zv = mk(z[2LL * (q * p.n_euler + ie)], z[2LL * (q * p.n_euler + ie) + 1]);
-            s[q] = zfma(wv, zv, s[q]);
+            if (q > 2 && q < 6) continue;   // not projected
+            s[q] = zfma(wv, mk(z[2LL * (q * p.n_euler + ie)], z[2LL * (q * p.n_euler + ie) + 1]), s[q]);
         }
     }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) part[q][ln][j] = s[q];
+    __syncthreads();
+    if (threadIdx.x < 8 * kProjTile) {
+        const int q = threadIdx.x / kProjTile;
+        zc v = part[q][0][j];
+        for (int k = 1; k < kProjLanes; ++k) v = v + part[q][k][j];
+        sum[q][j] = v;
+    }
+    cl.sync();
+    if (rank == 0 && threadIdx.x < 8 * kProjTile) {
+        const int q = threadIdx.x / kProjTile;
+        zc v = sum[q][j];
+        for (int k = 1; k < kProjCluster; ++k) v = v + *cl.map_shared_rank(&sum[q][j], k);
+        part[q][0][j] = v;
+    }
+    cl.sync();   // the other CTAs' sums are read before they exit
+    if (rank != 0 || threadIdx.x >= kProjTile || jkk >= kNJKK) return;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s[q] = part[q][0][j];
     int J = 0, rem = jkk;
     while (rem >= (2 * J + 1) * (2 * J + 1)) {
         rem -= (2 * J + 1) * (2 * J + 1);
@@ -1845,8 +1910,13 @@ __global__ void project_kernel(Params p, const zc *__restrict__ w, const double 
 
 cudaError_t launch_project(const Params &p, int npairs, const zc *w, const double *zres, int core_prot,
                            int core_neut, int chop, double *out, cudaStream_t st) {
-    dim3 grid(npairs, (kNJKK + 127) / 128);
-    project_kernel<<<grid, 128, 0, st>>>(p, w, zres, core_prot, core_neut, chop, out);
+    const int step = 0x7fffffff / (kProjTiles * kProjCluster);
+    const long long fs = 2LL * kProjFields * (kJJMax + 1) * kNK * kNK;
+    for (int p0 = 0; p0 < npairs; p0 += step) {
+        const int np = std::min(step, npairs - p0);
+        project_kernel<<<np * kProjTiles * kProjCluster, kProjTile * kProjLanes, 0, st>>>(
+            p, w, zres + 2LL * p0 * kNobs * p.n_euler, core_prot, core_neut, chop, out + p0 * fs);
+    }
     return cudaGetLastError();
 }
 
