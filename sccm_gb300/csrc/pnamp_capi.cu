@@ -159,6 +159,167 @@ std::vector<dd> to_dd(const std::vector<double> &v) {
     return out;
 }
 
+// Builder of an EnergyTab: products V y s; `either` when y and s may change places (then the row
+// with fewer entries so far takes the product, which evens out the rows).
+struct TabBuilder {
+    struct Prod {
+        int y, s;
+        double v;
+    };
+    std::vector<Prod> prods;
+    std::vector<int> len;   // entries per row
+    explicit TabBuilder(int elems) : len(elems, 0) {}
+    void add(int y, int s, double v, bool either) {
+        if (either && len[s] < len[y]) std::swap(y, s);
+        ++len[y];
+        prods.push_back({y, s, v});
+    }
+    int upload(pnamp_ctx *c, EnergyTab &t);
+    std::vector<int> steps;   // per slice, after upload
+};
+
+int TabBuilder::upload(pnamp_ctx *c, EnergyTab &t) {
+    std::vector<int> order, first(len.size() + 1, 0);
+    for (size_t r = 0; r < len.size(); ++r) {
+        if (len[r]) order.push_back((int)r);
+        first[r + 1] = first[r] + len[r];
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return len[a] > len[b]; });
+    std::vector<const Prod *> by(prods.size());   // the products by row
+    {
+        std::vector<int> at(first.begin(), first.end() - 1);
+        for (const Prod &q : prods) by[at[q.y]++] = &q;
+    }
+    const int ns = ((int)order.size() + 31) / 32;
+    std::vector<int> start(ns + 1, 0);
+    for (int q = 0; q < ns; ++q) start[q + 1] = start[q] + len[order[(size_t)q * 32]];
+    std::vector<unsigned short> yoff((size_t)ns * 32, 0), off((size_t)start[ns] * 32, 0);
+    std::vector<double> v((size_t)start[ns] * 32, 0.0);
+    std::vector<int> next(prods.size());          // linked lists of a row's products by 16-byte bank group
+    for (int q = 0; q < ns; ++q)
+        for (int g = 0; g < 4; ++g) {             // the 8 lanes of one shared-memory phase
+            int head[8][8], cnt[8][8] = {}, left[8] = {};
+            for (int k = 0; k < 8; ++k) {
+                const size_t r = (size_t)q * 32 + g * 8 + k;
+                for (int b = 0; b < 8; ++b) head[k][b] = -1;
+                if (r >= order.size()) continue;
+                const int row = order[r];
+                yoff[r] = (unsigned short)row;
+                left[k] = len[row];
+                for (int e = first[row]; e < first[row + 1]; ++e) {
+                    const int b = by[e]->s & 7;
+                    next[e] = head[k][b];
+                    head[k][b] = e;
+                    ++cnt[k][b];
+                }
+            }
+            const int steps = start[q + 1] - start[q];
+            for (int st = 0; st < steps; ++st) {
+                unsigned used = 0;
+                int filler = 0;
+                const size_t at = ((size_t)start[q] + st) * 32 + g * 8;
+                for (int k = 0; k < 8; ++k) {
+                    if (!left[k]) {
+                        off[at + k] = (unsigned short)filler;   // the address of another lane: a broadcast
+                        continue;
+                    }
+                    int best = -1;
+                    for (int b = 0; b < 8; ++b)
+                        if (cnt[k][b] && !((used >> b) & 1u) && (best < 0 || cnt[k][b] > cnt[k][best])) best = b;
+                    for (int b = 0; b < 8 && best < 0; ++b)
+                        if (cnt[k][b]) best = b;
+                    const Prod &e = *by[head[k][best]];
+                    head[k][best] = next[head[k][best]];
+                    --cnt[k][best];
+                    --left[k];
+                    used |= 1u << best;
+                    off[at + k] = (unsigned short)e.s;
+                    v[at + k] = e.v;
+                    filler = e.s;
+                }
+            }
+        }
+    t.nslice = ns;
+    for (int q = 0; q < ns; ++q) steps.push_back(start[q + 1] - start[q]);
+    int rc;
+    const std::vector<dd> vd = to_dd(v);
+    if ((rc = dev_upload(c, start, &t.start)) || (rc = dev_upload(c, yoff, &t.yoff)) || (rc = dev_upload(c, off, &t.off)) ||
+        (rc = dev_upload(c, v, &t.v)) || (rc = dev_upload(c, vd, &t.vd)))
+        return rc;
+    return PNAMP_OK;
+}
+
+// The two-body energy, exact regrouping of the 8-term sum of PNAMP_Energy_OpenMP.f90:40-78 with
+// skew pairing tensors,
+//   V [rho_ki rho_lj - rho_li rho_kj + d (rho_ik rho_jl - rho_jk rho_il)]
+//   + V [kappa01_ij kappa10_kl + d kappa01_kl kappa10_ij],
+// over the reduced points' storage: rho_xy at N ld + x ld + y, kappa10_xy at x ld + y and kappa01_xy
+// at y ld + x (x < y), elements from A. Four products of real and complex numbers per record and
+// bilinear form instead of six complex products, and one pass over the table per point.
+int build_energy_tabs(pnamp_ctx *c) {
+    const Params &p = c->p;
+    const int n = p.n, h = p.h, hh = h * h;
+    const int gl = p.place.gen.ld, sl = p.place.spl.ld;
+    TabBuilder b[kTabs] = {TabBuilder(2 * n * gl), TabBuilder(2 * h * sl), TabBuilder(2 * h * sl), TabBuilder(2 * hh)};
+    b[kTabGeneral].prods.reserve(6 * c->h_rec_idx.size());
+    for (size_t e = 0; e < c->h_rec_idx.size(); ++e) {
+        const uint32_t pk = c->h_rec_idx[e];
+        const int i = pk & 0xff, j = (pk >> 8) & 0xff, k = (pk >> 16) & 0xff, l = pk >> 24;
+        const double V = c->h_rec_v[e];
+        const bool d = i + j != k + l;
+        auto put = [&](TabBuilder &t, int N, int ld, int o) {
+            auto rho = [&](int x, int y) { return N * ld + (x - o) * ld + y - o; };
+            auto lo = [&](int x, int y) { return (std::min(x, y) - o) * ld + std::max(x, y) - o; };
+            auto hi = [&](int x, int y) { return (std::max(x, y) - o) * ld + std::min(x, y) - o; };
+            t.add(rho(k, i), rho(l, j), V, true);
+            t.add(rho(l, i), rho(k, j), -V, true);
+            if (d) {
+                t.add(rho(i, k), rho(j, l), V, true);
+                t.add(rho(j, k), rho(i, l), -V, true);
+            }
+            // kappa_xy = -kappa_yx, kappa_xx = 0
+            if (i != j && k != l) {
+                const double s = (i < j) == (k < l) ? V : -V;
+                t.add(hi(i, j), lo(k, l), s, false);
+                if (d) t.add(hi(k, l), lo(i, j), s, false);
+            }
+        };
+        put(b[kTabGeneral], n, gl, 0);
+        const int np = (i < h) + (j < h) + (k < h) + (l < h);
+        if (np == 4) put(b[kTabProton], h, sl, 0);
+        else if (np == 0) put(b[kTabNeutron], h, sl, h);
+        else if (i < h && k < h && j >= h && l >= h) {
+            b[kTabMixed].add(k * h + i, hh + (l - h) * h + j - h, V, false);
+            if (d) b[kTabMixed].add(i * h + k, hh + (j - h) * h + l - h, V, false);
+        }
+    }
+    for (int t = 0; t < kTabs; ++t) {
+        const int rc = b[t].upload(c, c->p.tab[t]);
+        if (rc) return rc;
+    }
+    for (int k = 0; k < 2; ++k) {   // longest slice first to the warp with the least so far
+        constexpr int nw = kThreads / 32;
+        std::vector<std::array<int, 3>> tasks;   // steps, species, slice
+        for (int s = 0; s < (k ? 2 : 1); ++s) {
+            const std::vector<int> &st = b[k ? kTabProton + s : kTabGeneral].steps;
+            for (size_t q = 0; q < st.size(); ++q) tasks.push_back({st[q] + 2, s, (int)q});
+        }
+        std::stable_sort(tasks.begin(), tasks.end(), [](const auto &x, const auto &y) { return x[0] > y[0]; });
+        std::vector<int> bin[2 * nw], sched(1, 0);
+        int load[nw] = {};
+        for (const auto &x : tasks) {
+            const int w = (int)(std::min_element(load, load + nw) - load);
+            load[w] += x[0];
+            bin[2 * w + x[1]].push_back(x[2]);
+        }
+        for (const auto &v : bin) sched.push_back(sched.back() + (int)v.size());
+        for (const auto &v : bin) sched.insert(sched.end(), v.begin(), v.end());
+        const int rc = dev_upload(c, sched, &c->p.sched[k]);
+        if (rc) return rc;
+    }
+    return PNAMP_OK;
+}
+
 // Thread groups of the reduced pairs' problems (order N, point_reduced.cuh) in `smem` bytes:
 // as many groups as fit, the CTA's warps shared among them, at most 8 matrix entries per
 // thread. More groups hide the sweep's latency better than more warps per group, which only
@@ -955,7 +1116,6 @@ int pnamp_init(const pnamp_space *sp, const pnamp_hamiltonian *h, const pnamp_me
     p.rot_elems = rot;
     p.nrec = h->nrec;
     p.nrec_gen = nrec_gen;
-    for (int k = 0; k < 3; ++k) p.rec_off[k] = rec_off[k];
     p.split_ok = rec_off[2] == nrec_gen;
     p.pl.make(n);
     c->core_prot = sp->core_prot;
@@ -1068,6 +1228,10 @@ int pnamp_init(const pnamp_space *sp, const pnamp_hamiltonian *h, const pnamp_me
     }
     // kMultiSmemTail bytes stay free at the end for the multi-context kernel's work counter
     if ((rc = plan_placement(p, smem_optin - kMultiSmemTail)) != PNAMP_OK) {
+        pnamp_free(c);
+        return rc;
+    }
+    if ((rc = build_energy_tabs(c)) != PNAMP_OK) {
         pnamp_free(c);
         return rc;
     }

@@ -94,6 +94,20 @@ struct ObsTables {
 };
 constexpr int kMaxR1B = 64;               // one-body density blocks per model space
 
+// A bilinear form sum_r y_r sum_k V_rk s_rk over densities in shared memory, as slices of 32 rows
+// (one per lane, longest rows first, padded with V = 0 to the slice's longest): slice q's steps are
+// [start[q], start[q + 1]), entry (step, lane) has the element offset off of s and the value v;
+// yoff[q * 32 + lane] is the row's y. The order of a row's entries spreads the 8 lanes that read
+// shared memory together over the 8 16-byte bank groups.
+struct EnergyTab {
+    int nslice;
+    const int *start;
+    const unsigned short *yoff, *off;
+    const double *v;
+    const dd *vd;
+};
+enum { kTabGeneral = 0, kTabProton = 1, kTabNeutron = 2, kTabMixed = 3, kTabs = 4 };
+
 struct Params {
     int n, h, N2;              // n, n/2, 2n
     int nprot, nneut;
@@ -113,11 +127,16 @@ struct Params {
     // Hamiltonian two-body list
     int nrec;
     int nrec_gen;              // records [0, nrec_gen): general; [nrec_gen, nrec): a, c protons and b, d neutrons
-    int rec_off[3];            // of the general ones, [0, rec_off[1]): four protons, [.., rec_off[2]): four neutrons
     int split_ok;              // no other general records and no charge-changing one-body terms
     const uint32_t *rec_idx;   // packed 8-bit a,b,c,d (0-based)
     const double *rec_v;
     const dd *rec_vd;          // rec_v as double-float (df64 form)
+    // the same interaction for the reduced points: over (A, Rh) of the n x n problem, of one
+    // species' h x h problem, and the proton-neutron part over two h x h densities
+    EnergyTab tab[kTabs];
+    // slices dealt to the CTA's warps, general and (proton, neutron): [2 warps + 1] offsets by (warp,
+    // species), then the slice numbers
+    const int *sched[2];
     ObsTables obs;
     PairLayout pl;
     Placement place;

@@ -434,41 +434,112 @@ __device__ __forceinline__ Z group_sum(const Grp &g, Z v, Z *red) {
     return v;
 }
 
+// Slices [first, ..) in steps of `stride` of a bilinear form over the densities at M, added to e2:
+// one row per lane, the row's factor applied at its end.
+template <class Z>
+__device__ __forceinline__ void energy_slices(const EnergyTab &t, int first, int stride, int lane, const Z *M,
+                                              typename Op<Z>::Acc &e2) {
+    using O = Op<Z>;
+    using Ra = Ar<Z>;
+    for (int q = first; q < t.nslice; q += stride) {
+        const int e0 = t.start[q] * 32 + lane, e1 = t.start[q + 1] * 32;
+        typename O::Acc s = O::acc(szero<Z>());
+#pragma unroll 4
+        for (int e = e0; e < e1; e += 32) O::radd(s, O::rmul(Ra::pick(t.v, t.vd, e)), M[t.off[e]]);
+        const Z y = O::done(s);
+        O::cadd(e2, O::mul(M[t.yoff[q * 32 + lane]]), y, O::rot(y));
+    }
+}
+
+// The double-float energies of `cnt` problems at once by the whole CTA: each warp takes the slices
+// that `sched` deals it and applies every table entry to all problems, whose (A, Rh) start at
+// smem + off[k]; its sum for problem k goes to its reduction slot in that problem's scratch. The
+// table (10 bytes per entry, 0.12 MB for a pf species, 0.8 MB for n = 40) comes from L2: read by
+// every problem for itself its latency bound the loop (FP64 and double-float took the same
+// time), shared by the CTA's problems it is read 7 (species-split pf) or 4 (n = 40) times less
+// often. The slices are dealt longest first to the least loaded warp over both species. FP64 is
+// bound by its pipe either way and keeps the groups independent (energy_slices).
+template <class Z, int C>
+__device__ __forceinline__ void energy_round_c(const EnergyTab &t, const int *task, int ntask, unsigned char *smem,
+                                               const int (&off)[8], int scr) {
+    using O = Op<Z>;
+    using Ra = Ar<Z>;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    typename O::Acc sum[C];
+#pragma unroll
+    for (int k = 0; k < C; ++k) sum[k] = O::acc(szero<Z>());
+    for (int i = 0; i < ntask; ++i) {
+        const int q = task[i];
+        const int e0 = t.start[q] * 32 + lane, e1 = t.start[q + 1] * 32;
+        typename O::Acc a[C];
+#pragma unroll
+        for (int k = 0; k < C; ++k) a[k] = O::acc(szero<Z>());
+#pragma unroll 2
+        for (int e = e0; e < e1; e += 32) {
+            const typename O::RMul v = O::rmul(Ra::pick(t.v, t.vd, e));
+            const int o = t.off[e];
+#pragma unroll
+            for (int k = 0; k < C; ++k) O::radd(a[k], v, reinterpret_cast<const Z *>(smem + off[k])[o]);
+        }
+        const int y = t.yoff[q * 32 + lane];
+#pragma unroll
+        for (int k = 0; k < C; ++k) {
+            const Z x = O::done(a[k]);
+            O::cadd(sum[k], O::mul(reinterpret_cast<const Z *>(smem + off[k])[y]), x, O::rot(x));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+        const Z v = warp_sum_z(O::done(sum[k]));
+        if (lane == 0) reinterpret_cast<SkewScratch<Z> *>(smem + off[k] + scr)->red[wid] = v;
+    }
+}
+template <class Z>
+__device__ __noinline__ void energy_round(const EnergyTab &t, const int *sched, int sp, unsigned char *smem, int cnt,
+                                          const int *list, int grp, int grp_bytes, int scr) {
+    const int b = 2 * ((int)threadIdx.x >> 5) + sp, *task = sched + 2 * (kThreads / 32) + 1 + sched[b];
+    const int nt = sched[b + 1] - sched[b];
+    for (int k0 = 0; k0 < cnt; k0 += 8) {
+        int off[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) off[k] = grp + list[min(k0 + k, cnt - 1)] * grp_bytes;
+        switch (min(cnt - k0, 8)) {   // a count without a case of its own repeats its last problem
+            case 1: energy_round_c<Z, 1>(t, task, nt, smem, off, scr); break;
+            case 2: energy_round_c<Z, 2>(t, task, nt, smem, off, scr); break;
+            case 3:
+            case 4: energy_round_c<Z, 4>(t, task, nt, smem, off, scr); break;
+            default: energy_round_c<Z, 8>(t, task, nt, smem, off, scr); break;
+            case 5:
+            case 6:
+            case 7: energy_round_c<Z, 7>(t, task, nt, smem, off, scr); break;
+        }
+    }
+}
+template <class Z> struct Shared { static constexpr bool energies = std::is_same<Z, zd>::value; };
+
 // Observables of the densities of skew_problem over the levels [lev0, lev0 + N): the two-body
-// records [rec0, rec1) (exact regrouping of the 8-term sum of PNAMP_Energy_OpenMP.f90:40-78,
-//   V [rho_ki rho_lj - rho_li rho_kj + d (rho_ik rho_jl - rho_jk rho_il)]
-//   + V [kappa01_ij kappa10_kl + d kappa01_kl kappa10_ij],
-// the pairing tensors being skew), the one-body energy, and <J^2> (ZJ2_0, PNAMP_ME2B.f90:45-147;
+// energy by tab (null: left out; double-float: from energy_round's sums in red), the one-body
+// energy, and <J^2> (ZJ2_0, PNAMP_ME2B.f90:45-147;
 // Jx, Jy = (J+ +- J-)/(2, 2i), J-_{a+1,a} = J+_{a,a+1}) without sum_a j(j+1) rho_aa, which is
 // linear in rho, and without the products of traces. Sums are valid in the group's first warp.
 template <class Z>
-__device__ __noinline__ PointSums<Z> point_sums(const Grp g, const Params &p, int N, int ld, int lev0, int rec0,
-                                                int rec1, const Z *A, const Z *Rh, Z *red) {
+__device__ __noinline__ PointSums<Z> point_sums(const Grp g, const Params &p, int N, int ld, int lev0,
+                                                const EnergyTab *tab, const Z *A, const Z *Rh, Z *red) {
     using O = Op<Z>;
     using Ra = Ar<Z>;
     using R = typename Ra::R;
     PointSums<Z> out;
-    typename O::Acc e2 = O::acc(szero<Z>()), t1 = e2, j2 = e2, tp = e2, tm = e2, tz = e2;
-    for (int e = rec0 + g.tid; e < rec1; e += g.nthr) {
-        const uint32_t pk = p.rec_idx[e];
-        const R v = Ra::pick(p.rec_v, p.rec_vd, e);
-        int i = pk & 0xff, j = (pk >> 8) & 0xff, k = (pk >> 16) & 0xff, l = pk >> 24;
-        const bool sym = i + j != k + l;
-        i -= lev0;
-        j -= lev0;
-        k -= lev0;
-        l -= lev0;
-        typename O::Acc t = O::acc(szero<Z>());
-        auto mac = [&](bool neg, Z a, Z b) { O::cadd(t, neg ? O::mul_neg(a) : O::mul(a), b, O::rot(b)); };
-        mac(false, Rh[k * ld + i], Rh[l * ld + j]);
-        mac(true, Rh[l * ld + i], Rh[k * ld + j]);
-        mac(false, A[j * ld + i], A[k * ld + l]);
-        if (sym) {
-            mac(false, Rh[i * ld + k], Rh[j * ld + l]);
-            mac(true, Rh[j * ld + k], Rh[i * ld + l]);
-            mac(false, A[l * ld + k], A[i * ld + j]);
+    typename O::Acc t1 = O::acc(szero<Z>()), j2 = t1, tp = t1, tm = t1, tz = t1;
+    out.e2 = szero<Z>();
+    if (tab) {
+        if constexpr (Shared<Z>::energies) {
+            if (g.tid < 32) out.e2 = warp_sum_z(g.tid < kThreads / 32 ? red[g.tid] : szero<Z>());
+            gsync(g);
+        } else {
+            typename O::Acc e2 = O::acc(szero<Z>());
+            energy_slices<Z>(*tab, g.tid >> 5, g.nthr >> 5, g.tid & 31, A, e2);   // Rh follows A
+            out.e2 = group_sum(g, O::done(e2), red);
         }
-        O::radd(e2, O::rmul(v), O::done(t));
     }
     for (int e = g.tid; e < p.obs.n_t1b; e += g.nthr) {
         const int ix = p.obs.t1b_idx[e], r = (ix >> 8) - lev0, c = (ix & 255) - lev0;
@@ -516,7 +587,6 @@ __device__ __noinline__ PointSums<Z> point_sums(const Grp g, const Params &p, in
             }
         }
     }
-    out.e2 = group_sum(g, O::done(e2), red);
     out.t1 = group_sum(g, O::done(t1), red);
     out.j2 = group_sum(g, O::done(j2), red);
     out.tp = group_sum(g, O::done(tp), red);
@@ -808,26 +878,31 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
     }
     __syncthreads();
     const Grp g{(int)threadIdx.x - gid * gthr, gthr, 1 + gid};
-    if (gid < ng) {
-        unsigned char *gb = smem + L.off_grp + gid * L.grp_bytes;
-        Z *A = reinterpret_cast<Z *>(gb), *Rh = A + n * ld;
-        SkewScratch<Z> &w = *reinterpret_cast<SkewScratch<Z> *>(gb + L.off_scr);
-        zc *nsh = reinterpret_cast<zc *>(gb + L.off_scr + sizeof(SkewScratch<Z>));   // the point's norm
-        Z *sb = Sb + (long long)gid * nn;
-        double *r2acc = r2out ? p.r2acc + 2LL * p.n_r2q * ((long long)blockIdx.x * ng + gid) : nullptr;
-        for (int q = g.tid; q < (r2out ? p.n_r2q : 0); q += g.nthr) {
-            r2acc[2 * q] = 0.0;
-            r2acc[2 * q + 1] = 0.0;
-        }
-        zc aN = mk(0, 0), aE = mk(0, 0), aJ = mk(0, 0);      // the group's thread 0
-        int flags = 0;
-        bool first = true;
-        for (int gi = gid; gi < p.n_gauge; gi += ng) {
+    const bool mine = gid < ng, energies = inverse && !p.tc_splits;
+    const bool rounds = energies && Shared<Z>::energies;   // spare warps only join energy_round
+    unsigned char *gb = smem + L.off_grp + (mine ? gid : 0) * L.grp_bytes;
+    Z *A = reinterpret_cast<Z *>(gb), *Rh = A + n * ld;
+    SkewScratch<Z> &w = *reinterpret_cast<SkewScratch<Z> *>(gb + L.off_scr);
+    zc *nsh = reinterpret_cast<zc *>(gb + L.off_scr + sizeof(SkewScratch<Z>));   // the point's norm
+    Z *sb = Sb + (long long)gid * nn;
+    double *r2acc = r2out && mine ? p.r2acc + 2LL * p.n_r2q * ((long long)blockIdx.x * ng + gid) : nullptr;
+    for (int q = g.tid; q < (r2acc ? p.n_r2q : 0); q += g.nthr) {
+        r2acc[2 * q] = 0.0;
+        r2acc[2 * q + 1] = 0.0;
+    }
+    zc aN = mk(0, 0), aE = mk(0, 0), aJ = mk(0, 0);      // the group's thread 0
+    int flags = 0, list[8];
+    for (int k = 0; k < 8; ++k) list[k] = k;
+    bool first = true;
+    for (int g0 = 0; g0 < p.n_gauge; g0 += ng) {
+        const int gi = g0 + gid;
+        const bool act = mine && gi < p.n_gauge;
+        bool sing = false;
+        zc norm = mk(0, 0);
+        if (act) {
             const int lp = gi / p.nfom, ln = gi % p.nfom;
             const Z zep = ephz[lp], zen = ephz[ln];
-            const bool sing = skew_problem<Z>(g, n, ld, h, zep * zep, zep * zen, zen * zen, Y, n, Z0, A, Rh, w,
-                                              inverse, L.tile);
-            zc norm = mk(0, 0);
+            sing = skew_problem<Z>(g, n, ld, h, zep * zep, zep * zen, zen * zen, Y, n, Z0, A, Rh, w, inverse, L.tile);
             if (g.tid < 32) {
                 int under;
                 const zc pf = pivot_product<Z>(w.piv, n / 2, p.cscale, under);
@@ -839,60 +914,66 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
                     nsh[0] = norm;
                 }
             }
-            const bool eval = inverse && !sing;
-            PointSums<Z> s;
-            if (eval) {
-                s = point_sums<Z>(g, p, n, ld, 0, 0, p.tc_splits ? 0 : p.nrec, A, Rh, w.red);
-                if (p.tc_splits) tc_rows<Z>(g, p, ld, A, Rh, pt0 + gi);
-            }
-            if (g.tid == 0) {
-                zc hg = mk(0, 0);
-                if (eval) {
-                    const zc e = Ra::to(s.e2), t = Ra::to(s.t1);
-                    hg = mk(e.x + t.x + p.e0, e.y + t.y);
-                    aE = zfma(norm, hg, aE);
-                    const zc a = Ra::to(s.tp), b = Ra::to(s.tm), c = Ra::to(s.tz);
-                    aJ = zfma(norm, Ra::to(s.j2) + a * b + c * c, aJ);
-                }
-                if (gout) {
-                    double *o = gout + 4LL * (((long long)pair * p.n_euler + ie) * p.n_gauge + gi);
-                    o[0] = norm.x;
-                    o[1] = norm.y;
-                    o[2] = hg.x;
-                    o[3] = hg.y;
-                }
-                if (p.tc_splits) {
-                    const double inv = 1.0 / ((double)p.nfom * p.nfom);
-                    p.tc_w[2 * (pt0 + gi)] = eval ? inv * norm.x : 0.0;
-                    p.tc_w[2 * (pt0 + gi) + 1] = eval ? inv * norm.y : 0.0;
-                }
-            }
-            gsync(g);   // nsh
-            if (eval) {
-                const zc nv = nsh[0];
-                const Z wn = Ra::from(nv);
-                for (int t = g.tid; t < nn; t += g.nthr) {
-                    const Z rv = Rh[(t / n) * ld + t % n];
-                    sb[t] = first ? wn * rv : zfma(wn, rv, sb[t]);
-                }
-                first = false;
-                for (int q = g.tid; q < (r2out ? p.n_r2q : 0); q += g.nthr) {
-                    const zc a = zfma(nv, Ra::to(quad_product<Z>(p.r2q[q], 0, ld, A, Rh)),
-                                      mk(r2acc[2 * q], r2acc[2 * q + 1]));
-                    r2acc[2 * q] = a.x;
-                    r2acc[2 * q + 1] = a.y;
-                }
-            }
-            gsync(g);   // the next point overwrites the densities
         }
-        if (first && inverse)
-            for (int t = g.tid; t < nn; t += g.nthr) sb[t] = szero<Z>();
+        if (rounds) {
+            __syncthreads();
+            energy_round<Z>(p.tab[kTabGeneral], p.sched[0], 0, smem, min(ng, p.n_gauge - g0), list, L.off_grp, L.grp_bytes, L.off_scr);
+            __syncthreads();
+        }
+        if (!act) continue;
+        const bool eval = inverse && !sing;
+        PointSums<Z> s;
+        if (eval) {
+            s = point_sums<Z>(g, p, n, ld, 0, energies ? &p.tab[kTabGeneral] : nullptr, A, Rh, w.red);
+            if (p.tc_splits) tc_rows<Z>(g, p, ld, A, Rh, pt0 + gi);
+        }
         if (g.tid == 0) {
-            gacc[4 * gid] = aN;
-            gacc[4 * gid + 1] = aE;
-            gacc[4 * gid + 2] = aJ;
-            gflag[gid] = flags;
+            zc hg = mk(0, 0);
+            if (eval) {
+                const zc e = Ra::to(s.e2), t = Ra::to(s.t1);
+                hg = mk(e.x + t.x + p.e0, e.y + t.y);
+                aE = zfma(norm, hg, aE);
+                const zc a = Ra::to(s.tp), b = Ra::to(s.tm), c = Ra::to(s.tz);
+                aJ = zfma(norm, Ra::to(s.j2) + a * b + c * c, aJ);
+            }
+            if (gout) {
+                double *o = gout + 4LL * (((long long)pair * p.n_euler + ie) * p.n_gauge + gi);
+                o[0] = norm.x;
+                o[1] = norm.y;
+                o[2] = hg.x;
+                o[3] = hg.y;
+            }
+            if (p.tc_splits) {
+                const double inv = 1.0 / ((double)p.nfom * p.nfom);
+                p.tc_w[2 * (pt0 + gi)] = eval ? inv * norm.x : 0.0;
+                p.tc_w[2 * (pt0 + gi) + 1] = eval ? inv * norm.y : 0.0;
+            }
         }
+        gsync(g);   // nsh
+        if (eval) {
+            const zc nv = nsh[0];
+            const Z wn = Ra::from(nv);
+            for (int t = g.tid; t < nn; t += g.nthr) {
+                const Z rv = Rh[(t / n) * ld + t % n];
+                sb[t] = first ? wn * rv : zfma(wn, rv, sb[t]);
+            }
+            first = false;
+            for (int q = g.tid; q < (r2acc ? p.n_r2q : 0); q += g.nthr) {
+                const zc a = zfma(nv, Ra::to(quad_product<Z>(p.r2q[q], 0, ld, A, Rh)),
+                                  mk(r2acc[2 * q], r2acc[2 * q + 1]));
+                r2acc[2 * q] = a.x;
+                r2acc[2 * q + 1] = a.y;
+            }
+        }
+        gsync(g);   // the next point overwrites the densities
+    }
+    if (first && inverse && mine)
+        for (int t = g.tid; t < nn; t += g.nthr) sb[t] = szero<Z>();
+    if (g.tid == 0 && mine) {
+        gacc[4 * gid] = aN;
+        gacc[4 * gid + 1] = aE;
+        gacc[4 * gid + 2] = aJ;
+        gflag[gid] = flags;
     }
     __syncthreads();
     // ---- the groups' sums: weighted density into the first group's storage, one-body traces
@@ -1047,37 +1128,56 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
     __syncthreads();
     // ---- the problems
     const Grp g{(int)threadIdx.x - gid * gthr, gthr, 1 + gid};
-    for (int u = gid; gid < ng && u < nu; u += ng) {
-        const int it = u / (2 * nc), s = (u / nc) & 1, chunk = u % nc;
-        unsigned char *gb = smem + L.off_grp + gid * L.grp_bytes;
+    const bool energies = inverse && !p.tc_splits;
+    const bool rounds = energies && Shared<Z>::energies;   // spare warps only join energy_round
+    for (int u0 = 0; u0 < nu; u0 += ng) {
+        const int u = u0 + gid;
+        const bool mine = gid < ng && u < nu;
+        const int it = mine ? u / (2 * nc) : 0, s = mine ? (u / nc) & 1 : 0, chunk = mine ? u % nc : 0;
+        unsigned char *gb = smem + L.off_grp + (mine ? gid : 0) * L.grp_bytes;
         Z *A = reinterpret_cast<Z *>(gb), *Rh = A + h * ld;
         SkewScratch<Z> &w = *reinterpret_cast<SkewScratch<Z> *>(gb + L.off_scr);
         zc *ash = reinterpret_cast<zc *>(gb + L.off_scr + sizeof(SkewScratch<Z>));
         Z *sb = Sb + (long long)u * hh;
         // two-body density: same-species quadruples, sum over phi of a_s times their products
-        const int q0 = p.r2_off[s], nq = r2out ? p.r2_off[s + 1] - q0 : 0;
+        const int q0 = p.r2_off[s], nq = r2out && mine ? p.r2_off[s + 1] - q0 : 0;
         double *r2acc = nq ? p.r2acc + 2LL * p.r2_ss * ((long long)blockIdx.x * max(ng, 2 * L.items) + u) : nullptr;
         zc aE = mk(0, 0), aJ = mk(0, 0);   // the group's thread 0
         int flags = 0;
         bool first = true;
-        for (int l = chunk; l < nf; l += nc) {
-            const Z d = ephz[l] * ephz[l];
-            const bool sing = skew_problem<Z>(g, h, ld, h, d, d, d, Y + (long long)(2 * it + s) * hh, h, Z0 + s * hh, A,
-                                              Rh, w, inverse, L.tile);
-            if (g.tid < 32) {
-                int under;
-                const zc pf = pivot_product<Z>(w.piv, h / 2, p.cscale, under);
-                if (lane == 0) {
-                    const int o = s ? l : l * nf;   // e^{-i phi N_s}: the other species' angle is 0
-                    const zc a = pf * mk(p.gphase[2 * o], p.gphase[2 * o + 1]);
-                    asum[(2 * it + s) * nf + l] = a;
-                    ash[0] = a;
-                    flags |= (under == 1 ? 1 : (under == 2 ? 4 : 0)) | (inverse && sing ? 2 : 0);
+        for (int l0 = 0; l0 < nf; l0 += nc) {
+            const int l = l0 + chunk;
+            const bool act = mine && l < nf;
+            bool sing = false;
+            if (act) {
+                const Z d = ephz[l] * ephz[l];
+                sing = skew_problem<Z>(g, h, ld, h, d, d, d, Y + (long long)(2 * it + s) * hh, h, Z0 + s * hh, A, Rh, w,
+                                       inverse, L.tile);
+                if (g.tid < 32) {
+                    int under;
+                    const zc pf = pivot_product<Z>(w.piv, h / 2, p.cscale, under);
+                    if (lane == 0) {
+                        const int o = s ? l : l * nf;   // e^{-i phi N_s}: the other species' angle is 0
+                        const zc a = pf * mk(p.gphase[2 * o], p.gphase[2 * o + 1]);
+                        asum[(2 * it + s) * nf + l] = a;
+                        ash[0] = a;
+                        flags |= (under == 1 ? 1 : (under == 2 ? 4 : 0)) | (inverse && sing ? 2 : 0);
+                    }
                 }
             }
-            if (!inverse || sing) continue;   // uniform over the group
-            const PointSums<Z> q = point_sums<Z>(g, p, h, ld, s * h, p.rec_off[s],
-                                                p.tc_splits ? p.rec_off[s] : p.rec_off[s + 1], A, Rh, w.red);
+            if (rounds) {
+                __syncthreads();
+                for (int sp = 0; sp < 2; ++sp) {   // the groups whose problem of this round is of species sp
+                    int list[16], cnt = 0;
+                    for (int k = 0; k < ng && u0 + k < nu; ++k)
+                        if ((((u0 + k) / nc) & 1) == sp && l0 + (u0 + k) % nc < nf) list[cnt++] = k;
+                    energy_round<Z>(p.tab[kTabProton + sp], p.sched[1], sp, smem, cnt, list, L.off_grp, L.grp_bytes, L.off_scr);
+                }
+                __syncthreads();
+            }
+            if (!act || !inverse || sing) continue;   // uniform over the group
+            const PointSums<Z> q = point_sums<Z>(g, p, h, ld, s * h, energies ? &p.tab[kTabProton + s] : nullptr, A, Rh,
+                                                 w.red);
             if (p.tc_splits) species_rows<Z>(g, p, s, h, ld, A, Rh, rows + ((long long)(2 * it + s) * nf + l) * 6 * tcw);
             if (g.tid == 0) {
                 const zc a = ash[0];
@@ -1100,11 +1200,11 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
             first = false;
             gsync(g);   // the next problem overwrites the densities
         }
-        if (first && inverse) {
+        if (first && inverse && mine) {
             for (int t = g.tid; t < hh; t += g.nthr) sb[t] = szero<Z>();
             for (int q = g.tid; q < 2 * nq; q += g.nthr) r2acc[q] = 0.0;
         }
-        if (g.tid == 0) {
+        if (g.tid == 0 && mine) {
             uacc[2 * u] = aE;
             uacc[2 * u + 1] = aJ;
             uflag[u] = flags;
@@ -1132,25 +1232,14 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
             const zc v = none ? mk(0, 0) : one_body<Z>(p, q, lane, s * h, h, St + (long long)is * hh, h);
             if (lane == 0) ob[t] = v;
         }
-        // proton-neutron records, (i, k) protons, (j, l) neutrons: only the direct terms
+        // the proton-neutron energy, bilinear in the two weighted densities
         const int wpi = max(1, (kThreads / 32) / m);
         zc *part = asm2 + 2 * m;                                          // [warps]
         if (wid / wpi < m) {
-            const Z *Sp = St + (long long)(wid / wpi) * 2 * hh, *Sn = Sp + hh;
             using O = Op<Z>;
             typename O::Acc e2 = O::acc(szero<Z>());
-            for (int e = p.nrec_gen + (wid % wpi) * 32 + lane; e < (p.tc_splits ? 0 : p.nrec); e += wpi * 32) {
-                const uint32_t pk = p.rec_idx[e];
-                const int i = pk & 0xff, j = ((pk >> 8) & 0xff) - h, k = (pk >> 16) & 0xff, l = (pk >> 24) - h;
-                typename O::Acc t = O::acc(szero<Z>());
-                const Z b0 = Sn[l * h + j];
-                O::cadd(t, O::mul(Sp[k * h + i]), b0, O::rot(b0));
-                if (i + j != k + l) {
-                    const Z b1 = Sn[j * h + l];
-                    O::cadd(t, O::mul(Sp[i * h + k]), b1, O::rot(b1));
-                }
-                O::radd(e2, O::rmul(Ra::pick(p.rec_v, p.rec_vd, e)), O::done(t));
-            }
+            if (!p.tc_splits)
+                energy_slices<Z>(p.tab[kTabMixed], wid % wpi, wpi, lane, St + (long long)(wid / wpi) * 2 * hh, e2);
             const Z v = warp_sum_z(O::done(e2));
             if (lane == 0) part[wid] = Ra::to(v);
         }
