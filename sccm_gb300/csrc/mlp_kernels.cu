@@ -5,98 +5,147 @@
 // The network predicts the normalised energy kernel H/N at fine-mesh points
 // from cheap inputs; it has no counterpart in the reference, which evaluates
 // every mesh point exactly. All layers are small (width 256) and the batch is
-// large (10^4 - 10^6 rows), so a 64 x 64 register-tiled SIMT GEMM on the FP32
-// pipes is used for every product; the weight gradient (K = rows) is split
-// over row chunks into a workspace and summed in chunk order, so results do
-// not depend on scheduling.
+// large (10^4 - 10^6 rows), so a register-tiled SIMT GEMM on the FP32 pipes is
+// used for every product; the weight gradient (K = rows) is split over row
+// chunks into a workspace and summed in chunk order, so results do not depend
+// on scheduling.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "../../include/pnamp_mlp.h"
+#include "pnamp_df64.cuh"
 
 namespace {
+using pnamp::f2;
+using pnamp::f2_dup;
+using pnamp::f2_fma;
 
-constexpr int BM = 64, BN = 64, BK = 16, TH = 256;  // tile, 16 x 16 threads x (4 x 4) outputs
+// 128 x 64 tile, 128 threads of 8 x 8 outputs each, K in double-buffered steps of 16. Every output
+// is one chain of FP32 fused multiply-adds over K, two neighbouring columns per packed
+// instruction: 64 lane operations for 4 shared-memory loads per thread and k (the 64 x 64 tile of
+// 4 x 4 outputs before it was bound by its loads, 8 for 16), and the next step's tile is on its
+// way from memory meanwhile. Smaller than 128 x 128, so that 16384 x 256 outputs give 512 tiles
+// for 152 SMs. A training step of 16384 rows, width 256, depth 4: see the launchers below.
+constexpr int BM = 128, BN = 64, BK = 16, TH = 128;
+constexpr int LDA = BM + 4, LDB = BN + 4;
+
+// One BR x BK tile of an operand into registers and from there to shared memory as [k][r].
+// KC: contiguous along k (P[r * ld + k]), else along r (P[k * ld + r]); vec: 16-byte loads
+// (leading dimension and base multiples of 4 floats).
+template <int BR, bool KC>
+struct Stage {
+    static constexpr int Q = BR * BK / 4 / TH;   // float4 per thread
+    float4 v[Q];
+    __device__ __forceinline__ void load(const float *__restrict__ P, int ld, int r0, int R, int k0, int k1, bool vec) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int e = threadIdx.x + q * TH;
+            const int r = r0 + (KC ? e / (BK / 4) : 4 * (e % (BR / 4)));
+            const int k = k0 + (KC ? 4 * (e % (BK / 4)) : e / (BR / 4));
+            float x[4] = {0.f, 0.f, 0.f, 0.f};
+            if (vec && (KC ? (r < R && k + 3 < k1) : (k < k1 && r + 3 < R))) {
+                const float4 t = *reinterpret_cast<const float4 *>(KC ? P + (long long)r * ld + k : P + (long long)k * ld + r);
+                x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int rr = KC ? r : r + i, kk = KC ? k + i : k;
+                    if (rr < R && kk < k1) x[i] = KC ? P[(long long)rr * ld + kk] : P[(long long)kk * ld + rr];
+                }
+            }
+            v[q] = make_float4(x[0], x[1], x[2], x[3]);
+        }
+    }
+    __device__ __forceinline__ void store(float *S, int lds) const {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int e = threadIdx.x + q * TH;
+            if (KC) {
+                const int r = e / (BK / 4), k = 4 * (e % (BK / 4));
+                S[k * lds + r] = v[q].x;
+                S[(k + 1) * lds + r] = v[q].y;
+                S[(k + 2) * lds + r] = v[q].z;
+                S[(k + 3) * lds + r] = v[q].w;
+            } else {
+                *reinterpret_cast<float4 *>(S + (e / (BR / 4)) * lds + 4 * (e % (BR / 4))) = v[q];
+            }
+        }
+    }
+};
 
 // C[m][n] = sum_k A(m, k) B(k, n) over k in [k0, k1) of this split
 //   A(m, k) = TA ? A[k * lda + m] : A[m * lda + k]
 //   B(k, n) = TB ? B[n * ldb + k] : B[k * ldb + n]
 // Epilogue: + bias[n] (if bias), tanh (if act == 1). Split z writes C + z * c_split_stride.
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(TH) gemm_kernel(const float *__restrict__ A, int lda, const float *__restrict__ B,
+__global__ void __launch_bounds__(TH, 4) gemm_kernel(const float *__restrict__ A, int lda, const float *__restrict__ B,
                                                   int ldb, float *__restrict__ C, int ldc, int M, int N, int K,
                                                   int kchunk, long long c_split_stride, const float *__restrict__ bias,
-                                                  int act) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Bs[BK][BN + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+                                                  int act, int veca, int vecb) {
+    __shared__ __align__(16) float As[2][BK * LDA];
+    __shared__ __align__(16) float Bs[2][BK * LDB];
+    const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int k0 = blockIdx.z * kchunk, k1 = min(K, k0 + kchunk);
-    float acc[4][4] = {};
-    for (int kt = k0; kt < k1; kt += BK) {
+    f2 acc[8][4];   // rows 4 ty + i, 64 + 4 ty + i; columns 4 tx + 2 j, 32 + 4 tx + 2 j
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {  // A tile: BM x BK, 4 values per thread
-            const int e = threadIdx.x + r * TH;
-            int mm, kk;
-            if (TA) {  // contiguous along m
-                kk = e / BM;
-                mm = e % BM;
-            } else {   // contiguous along k
-                mm = e / BK;
-                kk = e % BK;
-            }
-            const int gm = m0 + mm, gk = kt + kk;
-            float v = 0.f;
-            if (gm < M && gk < k1) v = TA ? A[(long long)gk * lda + gm] : A[(long long)gm * lda + gk];
-            As[kk][mm] = v;
-        }
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {  // B tile: BK x BN
-            const int e = threadIdx.x + r * TH;
-            int nn, kk;
-            if (TB) {  // contiguous along k
-                nn = e / BK;
-                kk = e % BK;
-            } else {   // contiguous along n
-                kk = e / BN;
-                nn = e % BN;
-            }
-            const int gn = n0 + nn, gk = kt + kk;
-            float v = 0.f;
-            if (gn < N && gk < k1) v = TB ? B[(long long)gn * ldb + gk] : B[(long long)gk * ldb + gn];
-            Bs[kk][nn] = v;
+        for (int j = 0; j < 4; ++j) acc[i][j] = f2_dup(0.f);
+    Stage<BM, !TA> sa;
+    Stage<BN, TB> sb;
+    sa.load(A, lda, m0, M, k0, k1, veca);
+    sb.load(B, ldb, n0, N, k0, k1, vecb);
+    sa.store(As[0], LDA);
+    sb.store(Bs[0], LDB);
+    __syncthreads();
+    int cur = 0;
+    for (int kt = k0; kt < k1; kt += BK, cur ^= 1) {
+        const bool more = kt + BK < k1;
+        if (more) {
+            sa.load(A, lda, m0, M, kt + BK, k1, veca);
+            sb.load(B, ldb, n0, N, kt + BK, k1, vecb);
         }
-        __syncthreads();
+        const float *Ac = As[cur], *Bc = Bs[cur];
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
-            float a[4], b[4];
+            const float4 a0 = *reinterpret_cast<const float4 *>(Ac + kk * LDA + 4 * ty);
+            const float4 a1 = *reinterpret_cast<const float4 *>(Ac + kk * LDA + 64 + 4 * ty);
+            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2 *>(Bc + kk * LDB + 4 * tx);
+            const ulonglong2 b1 = *reinterpret_cast<const ulonglong2 *>(Bc + kk * LDB + 32 + 4 * tx);
+            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            const f2 bv[4] = {{b0.x}, {b0.y}, {b1.x}, {b1.y}};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
+            for (int i = 0; i < 8; ++i) {
+                const f2 ad = f2_dup(av[i]);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) acc[i][j] = f2_fma(ad, bv[j], acc[i][j]);
+            }
+        }
+        if (more) {   // the other buffer was last read before the previous barrier
+            sa.store(As[cur ^ 1], LDA);
+            sb.store(Bs[cur ^ 1], LDB);
         }
         __syncthreads();
     }
     float *Cs = C + blockIdx.z * c_split_stride;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gm = m0 + ty + 16 * i;
+    for (int i = 0; i < 8; ++i) {
+        const int gm = m0 + (i < 4 ? 4 * ty + i : 60 + 4 * ty + i);
         if (gm >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gn = n0 + tx + 16 * j;
+        for (int j = 0; j < 8; ++j) {
+            const int gn = n0 + (j < 4 ? 4 * tx + j : 28 + 4 * tx + j);
             if (gn >= N) continue;
-            float v = acc[i][j];
+            float v = j & 1 ? pnamp::f2_b(acc[i][j >> 1]) : pnamp::f2_a(acc[i][j >> 1]);
             if (bias) v += bias[gn];
             if (act == 1) v = tanhf(v);
             Cs[(long long)gm * ldc + gn] = v;
         }
     }
 }
+
+int vec_ok(const float *p, int ld) { return ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // out[i] = sum_s part[s * n + i], s in order
 __global__ void sum_splits(const float *__restrict__ part, int splits, long long n, float *__restrict__ out) {
@@ -107,19 +156,39 @@ __global__ void sum_splits(const float *__restrict__ part, int splits, long long
     }
 }
 
-// dZ = dY * (1 - Y^2) (tanh) in place
-__global__ void tanh_grad(float *__restrict__ dy, const float *__restrict__ y, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        dy[i] *= 1.f - y[i] * y[i];
-}
-
-// partial column sums of dZ [rows][out] over row chunks: part[s][o]
-__global__ void colsum_partial(const float *__restrict__ dz, int rows, int out, int chunk, float *__restrict__ part) {
-    const int s = blockIdx.x;
-    const int r0 = s * chunk, r1 = min(rows, r0 + chunk);
-    for (int o = threadIdx.x; o < out; o += blockDim.x) {
-        float acc = 0.f;
-        for (int r = r0; r < r1; ++r) acc += dz[(long long)r * out + o];
+// dZ = dY * (1 - Y^2) (tanh; y null: dZ = dY) in place, and its column sums over row chunks,
+// part[s][o]: one pass over dY for both. 64 columns x 8 row groups per block, so that a chunk's
+// rows are not one serial chain.
+constexpr int kColLanes = 64, kRowLanes = 8;
+__global__ void __launch_bounds__(kColLanes * kRowLanes)
+grad_colsum(float *__restrict__ dy, const float *__restrict__ y, int rows, int out, int chunk,
+            float *__restrict__ part) {
+    __shared__ float red[kRowLanes][kColLanes];
+    const int s = blockIdx.x, c = threadIdx.x % kColLanes, g = threadIdx.x / kColLanes;
+    const int o = blockIdx.y * kColLanes + c;
+    const int r1 = min(rows, (s + 1) * chunk);
+    float acc = 0.f;
+    for (int r = s * chunk + g; r < r1 && o < out; r += 8 * kRowLanes) {
+        float d[8], v[8];   // 16 loads in flight before the first store
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const long long i = (long long)(r + k * kRowLanes) * out + o;
+            d[k] = r + k * kRowLanes < r1 ? dy[i] : 0.f;
+            v[k] = y && r + k * kRowLanes < r1 ? y[i] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (y && r + k * kRowLanes < r1) {
+                d[k] *= 1.f - v[k] * v[k];
+                dy[(long long)(r + k * kRowLanes) * out + o] = d[k];
+            }
+            acc += d[k];
+        }
+    }
+    red[g][c] = acc;
+    __syncthreads();
+    if (g == 0 && o < out) {
+        for (int k = 1; k < kRowLanes; ++k) acc += red[k][c];
         part[(long long)s * out + o] = acc;
     }
 }
@@ -189,7 +258,8 @@ int pnamp_mlp_linear_forward(const float *X, const float *W, const float *b, flo
     if (rows == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
     dim3 grid((out + BN - 1) / BN, (rows + BM - 1) / BM, 1);
-    gemm_kernel<false, true><<<grid, TH, 0, st>>>(X, in, W, in, Y, out, rows, out, in, in, 0, b, act);
+    gemm_kernel<false, true><<<grid, TH, 0, st>>>(X, in, W, in, Y, out, rows, out, in, in, 0, b, act, vec_ok(X, in),
+                                                  vec_ok(W, in));
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -199,8 +269,6 @@ int pnamp_mlp_linear_backward(const float *X, const float *W, const float *Y, fl
         (act == 1 && !Y))
         return 1;
     cudaStream_t st = (cudaStream_t)stream;
-    const long long nzy = (long long)rows * out;
-    if (act == 1) tanh_grad<<<grid_1d(nzy), 256, 0, st>>>(dY, Y, nzy);
     // split-K over row chunks: chunk a multiple of BK, at most kMaxSplits chunks
     int splits = (rows + kSplitRows - 1) / kSplitRows;
     if (splits > kMaxSplits) splits = kMaxSplits;
@@ -208,16 +276,17 @@ int pnamp_mlp_linear_backward(const float *X, const float *W, const float *Y, fl
     chunk = (chunk + BK - 1) / BK * BK;
     splits = (rows + chunk - 1) / chunk;
     float *partW = work, *partB = work + (long long)splits * in * out;
+    grad_colsum<<<dim3(splits, (out + kColLanes - 1) / kColLanes), kColLanes * kRowLanes, 0, st>>>(dY, act == 1 ? Y : nullptr, rows, out, chunk, partB);
     // dW[o][i] = sum_r dZ[r][o] X[r][i]: A = dZ^T (TA, lda = out), B = X (ldb = in)
     dim3 gw((in + BN - 1) / BN, (out + BM - 1) / BM, splits);
     gemm_kernel<true, false><<<gw, TH, 0, st>>>(dY, out, X, in, partW, in, out, in, rows, chunk,
-                                                (long long)out * in, nullptr, 0);
+                                                (long long)out * in, nullptr, 0, vec_ok(dY, out), vec_ok(X, in));
     sum_splits<<<grid_1d((long long)out * in), 256, 0, st>>>(partW, splits, (long long)out * in, dW);
-    colsum_partial<<<splits, 256, 0, st>>>(dY, rows, out, chunk, partB);
     sum_splits<<<grid_1d(out), 256, 0, st>>>(partB, splits, out, db);
     if (dX) {  // dX[r][i] = sum_o dZ[r][o] W[o][i]
         dim3 gx((in + BN - 1) / BN, (rows + BM - 1) / BM, 1);
-        gemm_kernel<false, false><<<gx, TH, 0, st>>>(dY, out, W, in, dX, in, rows, in, out, out, 0, nullptr, 0);
+        gemm_kernel<false, false><<<gx, TH, 0, st>>>(dY, out, W, in, dX, in, rows, in, out, out, 0, nullptr, 0,
+                                                     vec_ok(dY, out), vec_ok(W, in));
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
