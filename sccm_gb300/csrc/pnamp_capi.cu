@@ -146,6 +146,28 @@ double threej_h(int tj1, int tj2, int tj3, int tm1, int tm2, int tm3) {
     return ph * cg_h(tj1, tj2, tj3, tm1, tm2, -tm3) / std::sqrt(tj3 + 1.0);
 }
 
+// d^j_{m1 m2}(beta) in Edmonds' convention, doubled arguments, from Wigner's sum (as the device's
+// wigner_d).
+double wigner_d_h(int tj, int tm1, int tm2, double beta) {
+    double f[24], c[24], s[24];
+    f[0] = c[0] = s[0] = 1.0;
+    const double cb = std::cos(0.5 * beta), sb = std::sin(0.5 * beta);
+    for (int k = 1; k < 24; ++k) {
+        f[k] = f[k - 1] * k;
+        c[k] = c[k - 1] * cb;
+        s[k] = s[k - 1] * sb;
+    }
+    const int a1 = (tj + tm1) / 2, a2 = (tj - tm1) / 2, a3 = (tj + tm2) / 2, a4 = (tj - tm2) / 2, dm = (tm1 - tm2) / 2;
+    double d = 0.0;
+    for (int k = 0; k <= tj; ++k) {
+        const int a = a3 - k, e = a2 - k, g = k + dm;
+        if (a < 0 || e < 0 || g < 0) continue;
+        const double t = ((g & 1) ? -1.0 : 1.0) / (f[a] * f[k] * f[e] * f[g]);
+        d = std::fma(t * c[tj - 2 * k - dm], s[2 * k + dm], d);
+    }
+    return std::sqrt(f[a1] * f[a2] * f[a3] * f[a4]) * d;
+}
+
 dd host_dd(double x) {
     dd r;
     r.hi = (float)x;
@@ -1136,6 +1158,27 @@ int pnamp_init(const pnamp_space *sp, const pnamp_hamiltonian *h, const pnamp_me
     UP(row_blk, p.row_blk);
     UP(twom, p.twom);
     UP(euler, p.euler);
+    {   // d^j(beta) of every beta node, protons and neutrons with the same orbit alike
+        std::vector<double> wig((size_t)nbu * rot);
+        std::vector<unsigned short> rm(rot);
+        std::map<int, std::vector<double>> done;   // per 2j: [node][d d]
+        for (size_t b = 0; b < blk_tj.size(); ++b) {
+            const int tj = blk_tj[b], d = blk_size[b];
+            std::vector<double> &t = done[tj];
+            if (t.empty())
+                for (int k = 0; k < nbu; ++k)
+                    for (int e = 0; e < d * d; ++e)
+                        t.push_back(wigner_d_h(tj, tj - 2 * (e / d), tj - 2 * (e % d), m->beta[k]));
+            for (int k = 0; k < nbu; ++k)
+                std::copy(t.begin() + (size_t)k * d * d, t.begin() + (size_t)(k + 1) * d * d,
+                          wig.begin() + (size_t)k * rot + blk_roff[b]);
+            for (int e = 0; e < d * d; ++e)
+                rm[blk_roff[b] + e] = (unsigned short)((tj - 2 * (e / d) + 64) | ((tj - 2 * (e % d) + 64) << 8));
+        }
+        UP(wig, p.wigner);
+        UP(rm, p.rot_m);
+        p.n_alpgam = m->nalp * m->ngam;
+    }
     {
         std::vector<double> gph(2 * (size_t)m->nfom * m->nfom);
         const double twopi = 6.283185307179586476925287;

@@ -122,6 +122,9 @@ struct Params {
     int nblk, rot_elems;
     const int *blk_start, *blk_size, *blk_tj, *blk_roff, *row_blk, *twom;
     const double *euler;       // [n_euler][4] alpha, beta, gamma, weight
+    int n_alpgam;              // Euler points per beta node (beta is the outermost loop)
+    const double *wigner;      // [beta nodes][rot_elems] d^j_{m_i m_k}(beta) in the order of the blocks
+    const unsigned short *rot_m;   // [rot_elems] 2 m_i + 64 | (2 m_k + 64) << 8
     const double *gphase;      // [nfom][nfom] complex e^{-i (phi_lp Z + phi_ln N)}, the projection phase
     const double *fact;        // k!, k = 0..23
     // Hamiltonian two-body list

@@ -204,50 +204,73 @@ __device__ __forceinline__ bool skew_factor(const Grp &g, int N, int ld, const i
         return sing;
     }
     gsync(g);
+    // (G Y G^T)_rq as one sum over all threads' pieces in double-float, where the one warp that
+    // finished a step alone held the others up (pf mixing: 10.8 -> 9.0 of 44 Mcycles); in FP64 by
+    // one warp over finished columns, since the extra products cost the narrow pipe more (sd
+    // mixing: 7.0 against 7.8 of 34 Mcycles).
+    constexpr bool kSpread = std::is_same<Z, zd>::value;
+    const int wid = g.tid >> 5, nw = g.nthr >> 5;
     for (int k = N / 2 - 1; k >= 0; --k) {
         const int m = N - 2 - 2 * k, r = w.ord[m], q = w.ord[m + 1];
-        int parts = 0;
-        if (m > 0) {
-            parts = min(min(g.nthr / m, m), nbuf / (2 * m));
-            const int b = g.tid % m, part = g.tid / m;
-            if (part < parts) {
-                const int jb = w.ord[b];
-                typename O::Acc xp = O::acc(szero<Z>()), xq = xp;
-                for (int a = part; a < m; a += parts) {
-                    const int ia = w.ord[a];
-                    const Z y = A[ia * ld + jb];
-                    const typename O::Rot yr = O::rot(y);
-                    O::cadd(xp, O::mul(A[ia * ld + r]), y, yr);
-                    O::cadd(xq, O::mul_neg(A[q * ld + ia]), y, yr);
-                }
-                buf[(2 * part) * m + b] = O::done(xp);
-                buf[(2 * part + 1) * m + b] = O::done(xq);
+        // column b of -G Y in `parts` pieces, and this thread's piece of (G Y G^T)_rq
+        const int parts = m > 0 ? min(min(g.nthr / m, m), nbuf / (2 * m)) : 0;
+        const int b = m > 0 ? g.tid % m : 0, part = m > 0 ? g.tid / m : 0;
+        Z x = szero<Z>();
+        if (part < parts) {
+            const int jb = w.ord[b];
+            typename O::Acc xp = O::acc(szero<Z>()), xq = xp;
+            for (int a = part; a < m; a += parts) {
+                const int ia = w.ord[a];
+                const Z y = A[ia * ld + jb];
+                const typename O::Rot yr = O::rot(y);
+                O::cadd(xp, O::mul(A[ia * ld + r]), y, yr);
+                O::cadd(xq, O::mul_neg(A[q * ld + ia]), y, yr);
             }
-            gsync(g);
+            const Z yp = O::done(xp);
+            buf[(2 * part) * m + b] = yp;
+            buf[(2 * part + 1) * m + b] = O::done(xq);
+            if constexpr (kSpread) x = A[q * ld + jb] * yp;
         }
-        if (g.tid < 32) {
-            typename O::Acc x = O::acc(szero<Z>());
-            for (int b = lane; b < m; b += 32) {
-                Z yr = buf[b], yq = buf[m + b];
-                for (int part = 1; part < parts; ++part) {
-                    yr = yr + buf[(2 * part) * m + b];
-                    yq = yq + buf[(2 * part + 1) * m + b];
+        if constexpr (kSpread) {
+            x = warp_sum_z(x);
+            if (lane == 0) w.red[wid] = x;
+        }
+        gsync(g);
+        if constexpr (kSpread) {
+            for (int t = g.tid; t < 2 * m; t += g.nthr) {
+                const int row = t < m ? 0 : 1, c = t - row * m, i = row ? q : r, j = w.ord[c];
+                Z y = buf[row * m + c];
+                for (int piece = 1; piece < parts; ++piece) y = y + buf[(2 * piece + row) * m + c];
+                A[i * ld + j] = y;
+                A[j * ld + i] = -y;
+            }
+        } else if (wid == 0) {
+            typename O::Acc xs = O::acc(szero<Z>());
+            for (int c = lane; c < m; c += 32) {
+                Z yr = buf[c], yq = buf[m + c];
+                for (int piece = 1; piece < parts; ++piece) {
+                    yr = yr + buf[(2 * piece) * m + c];
+                    yq = yq + buf[(2 * piece + 1) * m + c];
                 }
-                const int ib = w.ord[b];
-                O::cadd(x, O::mul(A[q * ld + ib]), yr, O::rot(yr));
-                A[r * ld + ib] = yr;
-                A[ib * ld + r] = -yr;
-                A[q * ld + ib] = yq;
-                A[ib * ld + q] = -yq;
+                const int j = w.ord[c];
+                O::cadd(xs, O::mul(A[q * ld + j]), yr, O::rot(yr));
+                A[r * ld + j] = yr;
+                A[j * ld + r] = -yr;
+                A[q * ld + j] = yq;
+                A[j * ld + q] = -yq;
             }
-            const Z sum = warp_sum_z(O::done(x));
-            if (lane == 0) {
-                const Z y = -(zrecip(w.s[k]) + sum);
-                A[r * ld + q] = y;
-                A[q * ld + r] = -y;
-                A[r * ld + r] = szero<Z>();
-                A[q * ld + q] = szero<Z>();
+            x = warp_sum_z(O::done(xs));
+        }
+        if (g.tid == (kSpread ? g.nthr - 1 : 0)) {   // the spread form's last thread has no column
+            if (kSpread) {
+                x = w.red[0];
+                for (int c = 1; c < nw; ++c) x = x + w.red[c];
             }
+            const Z y = -(zrecip(w.s[k]) + x);
+            A[r * ld + q] = y;
+            A[q * ld + r] = -y;
+            A[r * ld + r] = szero<Z>();
+            A[q * ld + q] = szero<Z>();
         }
         gsync(g);
     }
@@ -718,18 +741,14 @@ __device__ __noinline__ void join_rows(const Params &p, int m, const unsigned sh
 
 // Rotation blocks R_b(i,k) = e^{-i alp m_i} d^j_{m_i m_k}(bet) e^{-i gam m_k} of one Euler point
 // (ROTATION_MAT, PNAMP_Proj.f90:83-136), entries t = tid, tid + nthr, ... of rot.
+// d^j comes from the context's table, made once per mesh: Wigner's sum at every point was half of
+// a norm-only pass (2.07 -> 1.45 ms for 2 x 1024 Euler points of pf).
 __device__ __forceinline__ void rotation_blocks(const Params &p, int ie, int tid, int nthr, zc *rot) {
-    const double alp = p.euler[4 * ie], bet = p.euler[4 * ie + 1], gam = p.euler[4 * ie + 2];
-    double cb, sb;
-    sincos(0.5 * bet, &sb, &cb);
-    for (int b = 0; b < p.nblk; ++b) {
-        const int d = p.blk_size[b], tj = p.blk_tj[b], ro = p.blk_roff[b];
-        for (int e = tid; e < d * d; e += nthr) {
-            const int i = e / d, k = e % d;
-            const int mi = tj - 2 * i, mkk = tj - 2 * k;
-            const double dv = wigner_d(tj, mi, mkk, cb, sb, p.fact);
-            rot[ro + e] = dv * expi(-0.5 * (alp * mi + gam * mkk));
-        }
+    const double alp = p.euler[4 * ie], gam = p.euler[4 * ie + 2];
+    const double *d = p.wigner + (long long)(ie / p.n_alpgam) * p.rot_elems;
+    for (int e = tid; e < p.rot_elems; e += nthr) {
+        const int mm = p.rot_m[e];   // 2 m_i + 64 | (2 m_k + 64) << 8
+        rot[e] = d[e] * expi(-0.5 * (alp * ((mm & 255) - 64) + gam * ((mm >> 8) - 64)));
     }
 }
 
