@@ -92,9 +92,9 @@ def _pair_paths(wl, pairs):
 
 
 def algorithmic_flops_per_point(wl, n_gauge, pairs=None, records=True):
-    """Algorithmic FP64 work per kernel point of the point kernel, averaged over `pairs`
-    (default: all): the minimal flops of the algorithm it runs (complex multiply-add = 8
-    flops, complex x real = 4), O(n^2) terms left out.
+    """Algorithmic FP64 work per kernel point with a Pfaffian, a solve and density products at every
+    gauge point (the point kernel's full_item), averaged over `pairs` (default: all; complex
+    multiply-add = 8 flops, complex x real = 4), O(n^2) terms left out.
 
     Per Euler point, amortised over the n_gauge gauge points: R W, R V1, conj(R) U1 and
     X = (R W) R^T with the block-diagonal rotation, (3 * 4 + 8) n sum_b d_b^2, and the
@@ -129,6 +129,40 @@ def algorithmic_flops_per_point(wl, n_gauge, pairs=None, records=True):
             rec = 0.0
         tot += (20.0 * n * sd2 + 8.0 * n ** 3) / n_gauge + dense + float(rec)
     return tot / len(paths)
+
+
+def point_flops(wl, n_gauge, pairs=None, records=True):
+    """Algorithmic FP64 work per kernel point of the point kernel as it now runs, averaged over
+    `pairs` (complex multiply-add = 8 flops, complex x real = 4), O(n^2) terms left out.
+
+    Pairs with U0 and V1 well conditioned (LU pivots spanning less than 1e2, no entry of
+    U1 V1^-1 above 40): one skew inverse with its Pfaffian, 4 N^3, and two products with a real
+    matrix, 6 N^3, per problem, and 4 flops per table entry (6 entries per record, 3 when i + j =
+    k + l). NFOM^2 problems of order n per Euler point; for charge-conserving pairs 2 NFOM of
+    order h = n/2 with the same-species records of that species, and the proton-neutron records
+    once per Euler point. Other pairs as `algorithmic_flops_per_point` counts them."""
+    import scipy.linalg as sl
+    n = wl.sp.nlev
+    h = n // 2
+    i, j, k, l = np.asarray(wl.recs).T
+    pn = (i < h) & (j >= h) & (k < h) & (l >= h)
+    ent = np.where((i + j) == (k + l), 3.0, 6.0) if records else np.zeros(len(i))
+    nfom = int(round(n_gauge ** 0.5))
+
+    def well(M):
+        d = np.abs(np.diag(sl.lu_factor(M)[0]))
+        return d.min() >= 1e-2 * d.max()
+    tot = 0.0
+    pairs = pairs if pairs is not None else wl.pairs
+    for a, b in pairs:
+        (U0, V0), (U1, V1) = wl.vacua[a], wl.vacua[b]
+        if nfom == 1 or not (well(U0) and well(V1) and np.abs(U1 @ np.linalg.inv(V1)).max() <= 40.0):
+            tot += algorithmic_flops_per_point(wl, n_gauge, [(a, b)], records)
+        elif _pair_paths(wl, [(a, b)])[0][0]:
+            tot += (2 * nfom * 10.0 * h ** 3 + 4.0 * (nfom * ent[~pn].sum() + ent[pn].sum() / 3.0)) / n_gauge
+        else:
+            tot += 10.0 * n ** 3 + 4.0 * ent.sum()
+    return tot / len(pairs)
 
 
 SMI_FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
@@ -675,7 +709,7 @@ def main():
     rl = {}
     for form, v in res.items():
         tc = form.startswith("tc")
-        flops_pt = algorithmic_flops_per_point(wl, G, timed_pairs, records=not tc)
+        flops_pt = point_flops(wl, G, timed_pairs, records=not tc)
         t_pts = v["stage_ms_per_step"]["points"] / 1e3
         ach = flops_pt * pts_step / t_pts / 1e12
         if form == "fp64":

@@ -224,9 +224,9 @@ int pnamp_rho2b_tables(const pnamp_space *sp, int *blocks, int *states, unsigned
 
 /* pnamp_batch_device that also writes, per pair and quadruple (k_i, k_j, k_k, k_l),
  * sum_e w_e (1/N_FOM^2) sum_phi N(Omega_e, phi) [rho_ki rho_lj - rho_li rho_kj +
- * kappa01_ij kappa10_kl] into d_rho2b [npairs][nquads] complex (overwritten). Each
- * CTA keeps its sums in FP64 in device memory the context owns ([grid][nquads]
- * complex) and adds them into d_rho2b once per Euler point. PNAMP_ERR_STATE in
+ * kappa01_ij kappa10_kl] into d_rho2b [npairs][nquads] complex (overwritten). The
+ * sums of a CTA's thread groups stay in FP64 in device memory the context owns and
+ * are added into d_rho2b once per Euler point or batch of Euler points. PNAMP_ERR_STATE in
  * norm-only mode. */
 int pnamp_batch_rho2b_device(pnamp_ctx *ctx, int npairs, const double *d_uv, double *d_zres,
                              int *d_point_status, double *d_rho2b, void *stream);
@@ -347,7 +347,9 @@ int pnamp_multi_schedule(pnamp_multi *plan, int order, int grab, int grid);
  * global slot) under the budget and the launch holds the largest result,
  * written to *smem_bytes when that is not NULL. What a CTA does not take as
  * shared memory serves as L1, so a smaller budget can be faster when one
- * context's arrays do not fit anyway. Not while a launch of the plan runs. */
+ * context's arrays do not fit anyway. The least that a point of a context needs
+ * (one thread group of the reduced pairs) is held even above the budget. Not
+ * while a launch of the plan runs. */
 int pnamp_multi_placement(pnamp_multi *plan, int smem_budget, int *smem_bytes);
 
 int pnamp_multi_launch(pnamp_multi *plan, void *stream);
