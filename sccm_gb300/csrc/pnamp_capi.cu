@@ -371,7 +371,7 @@ RedPlan plan_reduced(const Params &p, int N, bool split, int smem) {
         o += ng * L.grp_bytes;
         // the Euler point's rotation blocks, the Onishi matrix and the final sums use the same place
         const int rot = L.items * p.rot_elems * 16;
-        const int fin = L.items * (2 * N * N + 2 * 17 + 8) * 16 + 16 * 32 + (split ? 0 : 16 * (N + 32 + 64));
+        const int fin = L.items * ((split ? 4 : 2) * N * N + 2 * 17 + 8) * 16 + 16 * 32 + (split ? 0 : 16 * (N + 32 + 64));
         o = std::max(o, L.off_grp + std::max(rot, fin));
         L.smem_bytes = o;
         return L;

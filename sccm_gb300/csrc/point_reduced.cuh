@@ -767,9 +767,7 @@ __device__ __forceinline__ void rotation_blocks(const Params &p, int ie, int tid
 // slots 0 Tr over protons, 1 over neutrons, 2 one-body energy, 3 sum j(j+1) rho_aa,
 // 4..6 Tr J+, J-, Jz, 7..16 the Q_{2mu} traces (proton rows).
 constexpr int kOneBody = 17;
-template <class Z>
-__device__ __forceinline__ zc one_body(const Params &p, int q, int lane, int lev0, int N, const Z *Sb, int lds) {
-    using Ra = Ar<Z>;
+__device__ __forceinline__ zc one_body(const Params &p, int q, int lane, int lev0, int N, const zc *Sb, int lds) {
     zc s = mk(0.0, 0.0);
     if (q == 0 || q == 1 || q == 3 || q == 6) {
         for (int a = lane; a < N; a += 32) {
@@ -779,12 +777,12 @@ __device__ __forceinline__ zc one_body(const Params &p, int q, int lane, int lev
             else if (q == 1) f = g < p.h ? 0.0 : 1.0;
             else if (q == 3) f = p.obs.jj1[g];
             else f = p.obs.mz[g];
-            if (f != 0.0) s = rfma(f, Ra::to(Sb[a * lds + a]), s);
+            if (f != 0.0) s = rfma(f, Sb[a * lds + a], s);
         }
     } else if (q == 4 || q == 5) {
         for (int a = lane; a < N; a += 32) {
             const double f = p.obs.jp[lev0 + a];
-            if (f != 0.0) s = rfma(f, Ra::to(q == 4 ? Sb[(a + 1) * lds + a] : Sb[a * lds + a + 1]), s);
+            if (f != 0.0) s = rfma(f, q == 4 ? Sb[(a + 1) * lds + a] : Sb[a * lds + a + 1], s);
         }
     } else {
         const int e0 = q == 2 ? 0 : p.obs.q_off[q - 7], e1 = q == 2 ? p.obs.n_t1b : p.obs.q_off[q - 6];
@@ -792,7 +790,7 @@ __device__ __forceinline__ zc one_body(const Params &p, int q, int lane, int lev
         const double *val = q == 2 ? p.obs.t1b_val : p.obs.q_val;
         for (int e = e0 + lane; e < e1; e += 32) {
             const int ix = idx[e], r = (ix >> 8) - lev0, c = (ix & 255) - lev0;
-            if ((unsigned)r < (unsigned)N && (unsigned)c < (unsigned)N) s = rfma(val[e], Ra::to(Sb[r * lds + c]), s);
+            if ((unsigned)r < (unsigned)N && (unsigned)c < (unsigned)N) s = rfma(val[e], Sb[r * lds + c], s);
         }
     }
     s.x = warp_sum(s.x);
@@ -823,7 +821,7 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
     R *Z0 = reinterpret_cast<R *>(smem + L.off_z0);
     Z *Y = reinterpret_cast<Z *>(slot);                     // R* Wi R^+
     zc *RW = slot + nn;                                     // R* Wi
-    Z *Sb = reinterpret_cast<Z *>(slot + nn);               // [ng][n n], after RW is used
+    zc *Sb = slot + nn;                                     // [ng][n n], after RW is used
     const double *gU1 = pr + p.pl.u1, *gV1 = pr + p.pl.v1, *gWi = pr + p.pl.zi, *gZ0 = pr + p.pl.z0;
     const zc pfw = mk(pr[p.pl.pfz], pr[p.pl.pfz + 1]);
     const double pre = p.vacfac * pr[p.pl.dets] * pr[p.pl.dets + 1];
@@ -913,7 +911,7 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
     Z *A = reinterpret_cast<Z *>(gb), *Rh = A + n * ld;
     SkewScratch<Z> &w = *reinterpret_cast<SkewScratch<Z> *>(gb + L.off_scr);
     zc *nsh = reinterpret_cast<zc *>(gb + L.off_scr + sizeof(SkewScratch<Z>));   // the point's norm
-    Z *sb = Sb + (long long)gid * nn;
+    zc *sb = Sb + (long long)gid * nn;
     double *r2acc = r2out && mine ? p.r2acc + 2LL * p.n_r2q * ((long long)blockIdx.x * ng + gid) : nullptr;
     for (int q = g.tid; q < (r2acc ? p.n_r2q : 0); q += g.nthr) {
         r2acc[2 * q] = 0.0;
@@ -981,10 +979,9 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
         gsync(g);   // nsh
         if (eval) {
             const zc nv = nsh[0];
-            const Z wn = Ra::from(nv);
-            for (int t = g.tid; t < nn; t += g.nthr) {
-                const Z rv = Rh[(t / n) * ld + t % n];
-                sb[t] = first ? wn * rv : zfma(wn, rv, sb[t]);
+            for (int t = g.tid; t < nn; t += g.nthr) {   // the sum over gauge points stays FP64
+                const zc rv = Ra::to(Rh[(t / n) * ld + t % n]);
+                sb[t] = first ? nv * rv : zfma(nv, rv, sb[t]);
             }
             first = false;
             for (int q = g.tid; q < (r2acc ? p.n_r2q : 0); q += g.nthr) {
@@ -997,7 +994,7 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
         gsync(g);   // the next point overwrites the densities
     }
     if (first && inverse && mine)
-        for (int t = g.tid; t < nn; t += g.nthr) sb[t] = szero<Z>();
+        for (int t = g.tid; t < nn; t += g.nthr) sb[t] = mk(0.0, 0.0);
     if (g.tid == 0 && mine) {
         gacc[4 * gid] = aN;
         gacc[4 * gid + 1] = aE;
@@ -1006,17 +1003,16 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
     }
     __syncthreads();
     // ---- the groups' sums: weighted density into the first group's storage, one-body traces
-    Z *St = reinterpret_cast<Z *>(smem + L.off_grp);
-    zc *ob = reinterpret_cast<zc *>(smem + L.off_grp + ((nn * (int)sizeof(Z) + 15) & ~15));
+    zc *St = reinterpret_cast<zc *>(smem + L.off_grp), *ob = St + nn;
     if (inverse) {
         for (int t = threadIdx.x; t < nn; t += blockDim.x) {
-            Z s = Sb[t];
+            zc s = Sb[t];
             for (int q = 1; q < ng; ++q) s = s + Sb[(long long)q * nn + t];
             St[t] = s;
         }
         __syncthreads();
         for (int q = wid; q < kOneBody; q += kThreads / 32) {
-            const zc v = q >= 7 && !p.iE2 ? mk(0, 0) : one_body<Z>(p, q, lane, 0, n, St, n);
+            const zc v = q >= 7 && !p.iE2 ? mk(0, 0) : one_body(p, q, lane, 0, n, St, n);
             if (lane == 0) ob[q] = v;
         }
         if (r1out) {
@@ -1025,7 +1021,7 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
                 zc s = mk(0, 0);
                 for (int e = p.obs.r1b_off[b] + lane; e < p.obs.r1b_off[b + 1]; e += 32) {
                     const int ix = p.obs.r1b_idx[e];
-                    s = rfma(p.obs.r1b_val[e], Ra::to(St[(ix >> 8) * n + (ix & 255)]), s);
+                    s = rfma(p.obs.r1b_val[e], St[(ix >> 8) * n + (ix & 255)], s);
                 }
                 s.x = warp_sum(s.x);
                 s.y = warp_sum(s.y);
@@ -1107,7 +1103,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
     R *Z0 = reinterpret_cast<R *>(smem + L.off_z0);          // [2][h][h]
     // per unit: weighted density; per item: the species blocks of Y. R* Wi takes the densities' place
     Z *Y = reinterpret_cast<Z *>(slot);                      // [m][2][h h]
-    Z *Sb = reinterpret_cast<Z *>(slot + 2LL * L.items * hh);
+    zc *Sb = slot + 2LL * L.items * hh;
     zc *RW = slot + 2LL * L.items * hh;                      // [m][2][h h]
     const double *gWi = pr + p.pl.zi, *gZ0 = pr + p.pl.z0;
     auto euler = [&](int k) { return items ? items[k].y : ie0 + k; };
@@ -1167,7 +1163,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
         Z *A = reinterpret_cast<Z *>(gb), *Rh = A + h * ld;
         SkewScratch<Z> &w = *reinterpret_cast<SkewScratch<Z> *>(gb + L.off_scr);
         zc *ash = reinterpret_cast<zc *>(gb + L.off_scr + sizeof(SkewScratch<Z>));
-        Z *sb = Sb + (long long)u * hh;
+        zc *sb = Sb + (long long)u * hh;
         // two-body density: same-species quadruples, sum over phi of a_s times their products
         const int q0 = p.r2_off[s], nq = r2out && mine ? p.r2_off[s + 1] - q0 : 0;
         double *r2acc = nq ? p.r2acc + 2LL * p.r2_ss * ((long long)blockIdx.x * max(ng, 2 * L.items) + u) : nullptr;
@@ -1215,9 +1211,9 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
                 aJ = zfma(a, Ra::to(q.j2) + tp * tm + tz * tz, aJ);
             }
             gsync(g);
-            const Z wa = Ra::from(ash[0]);
-            for (int t = g.tid; t < hh; t += g.nthr) {
-                const Z rv = Rh[(t / h) * ld + t % h];
+            const zc wa = ash[0];
+            for (int t = g.tid; t < hh; t += g.nthr) {   // the sum over gauge points stays FP64
+                const zc rv = Ra::to(Rh[(t / h) * ld + t % h]);
                 sb[t] = first ? wa * rv : zfma(wa, rv, sb[t]);
             }
             for (int q = g.tid; q < nq; q += g.nthr) {
@@ -1230,7 +1226,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
             gsync(g);   // the next problem overwrites the densities
         }
         if (first && inverse && mine) {
-            for (int t = g.tid; t < hh; t += g.nthr) sb[t] = szero<Z>();
+            for (int t = g.tid; t < hh; t += g.nthr) sb[t] = mk(0.0, 0.0);
             for (int q = g.tid; q < 2 * nq; q += g.nthr) r2acc[q] = 0.0;
         }
         if (g.tid == 0 && mine) {
@@ -1243,22 +1239,24 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
     // ---- per Euler point: weighted densities of both species side by side, then the sums
     const double inv = 1.0 / ((double)nf * nf);
     const zc pre = (p.vacfac * pr[p.pl.dets] * pr[p.pl.dets + 1]) * mk(pr[p.pl.pfz], pr[p.pl.pfz + 1]);
-    Z *St = reinterpret_cast<Z *>(smem + L.off_grp);                      // [m][2][h h]
-    zc *ob = reinterpret_cast<zc *>(St + 2 * hh * m);                     // [m][2][kOneBody]
+    zc *St = reinterpret_cast<zc *>(smem + L.off_grp);                    // [m][2][h h]
+    Z *Se = reinterpret_cast<Z *>(St + 2 * hh * m);                       // the same in the point arithmetic
+    zc *ob = reinterpret_cast<zc *>(Se + 2 * hh * m);                     // [m][2][kOneBody]
     zc *epn = ob + 2 * kOneBody * m;                                      // [m]
     zc *asm2 = epn + m;                                                   // [m][2] sums of a_s
     if (inverse) {
         for (int t = threadIdx.x; t < 2 * hh * m; t += blockDim.x) {
             const int is = t / hh, e = t % hh;
-            Z v = Sb[(long long)is * nc * hh + e];
+            zc v = Sb[(long long)is * nc * hh + e];
             for (int q = 1; q < nc; ++q) v = v + Sb[((long long)is * nc + q) * hh + e];
             St[t] = v;
+            Se[t] = Ra::from(v);
         }
         __syncthreads();
         for (int t = wid; t < 2 * kOneBody * m; t += kThreads / 32) {
             const int is = t / kOneBody, q = t % kOneBody, s = is & 1;
             const bool none = (q == 0 && s) || (q == 1 && !s) || (q >= 7 && (s || !p.iE2));
-            const zc v = none ? mk(0, 0) : one_body<Z>(p, q, lane, s * h, h, St + (long long)is * hh, h);
+            const zc v = none ? mk(0, 0) : one_body(p, q, lane, s * h, h, St + (long long)is * hh, h);
             if (lane == 0) ob[t] = v;
         }
         // the proton-neutron energy, bilinear in the two weighted densities
@@ -1268,7 +1266,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
             using O = Op<Z>;
             typename O::Acc e2 = O::acc(szero<Z>());
             if (!p.tc_splits)
-                energy_slices<Z>(p.tab[kTabMixed], wid % wpi, wpi, lane, St + (long long)(wid / wpi) * 2 * hh, e2);
+                energy_slices<Z>(p.tab[kTabMixed], wid % wpi, wpi, lane, Se + (long long)(wid / wpi) * 2 * hh, e2);
             const Z v = warp_sum_z(O::done(e2));
             if (lane == 0) part[wid] = Ra::to(v);
         }
@@ -1314,8 +1312,8 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
                 } else {   // one proton and one neutron density, rho_ki rho_lj
                     const int i = qd.x & 0xff, j = (qd.x >> 8) & 0xff, k = (qd.x >> 16) & 0xff, l = qd.x >> 24;
                     const int si = i >= h ? 1 : 0, sj = 1 - si;
-                    const Z *Sa = St + (long long)(2 * it + si) * hh, *Sc = St + (long long)(2 * it + sj) * hh;
-                    x = Ra::to(Sa[(k - si * h) * h + i - si * h]) * Ra::to(Sc[(l - sj * h) * h + j - sj * h]);
+                    const zc *Sa = St + (long long)(2 * it + si) * hh, *Sc = St + (long long)(2 * it + sj) * hh;
+                    x = Sa[(k - si * h) * h + i - si * h] * Sc[(l - sj * h) * h + j - sj * h];
                 }
                 v = v + wgt * x;
             }
@@ -1367,7 +1365,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
                 for (int e = p.obs.r1b_off[b] + lane; e < p.obs.r1b_off[b + 1]; e += 32) {
                     const int ix = p.obs.r1b_idx[e], r = ix >> 8, c = ix & 255;
                     sp = r >= h ? 1 : 0;
-                    s = rfma(p.obs.r1b_val[e], Ra::to(St[(long long)(2 * it + sp) * hh + (r - sp * h) * h + c - sp * h]), s);
+                    s = rfma(p.obs.r1b_val[e], St[(long long)(2 * it + sp) * hh + (r - sp * h) * h + c - sp * h], s);
                 }
                 s.x = warp_sum(s.x);
                 s.y = warp_sum(s.y);
