@@ -1244,24 +1244,47 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
     zc *ob = reinterpret_cast<zc *>(Se + 2 * hh * m);                     // [m][2][kOneBody]
     zc *epn = ob + 2 * kOneBody * m;                                      // [m]
     zc *asm2 = epn + m;                                                   // [m][2] sums of a_s
+    zc *part = asm2 + 2 * m;                                              // [warps] proton-neutron energies
+    int *sexp = reinterpret_cast<int *>(part + kThreads / 32);            // [m][2] exponents taken from St in Se
     if (inverse) {
         for (int t = threadIdx.x; t < 2 * hh * m; t += blockDim.x) {
             const int is = t / hh, e = t % hh;
             zc v = Sb[(long long)is * nc * hh + e];
             for (int q = 1; q < nc; ++q) v = v + Sb[((long long)is * nc + q) * hh + e];
             St[t] = v;
-            Se[t] = Ra::from(v);
+            if (!Shared<Z>::energies) Se[t] = Ra::from(v);
         }
         __syncthreads();
+        if constexpr (Shared<Z>::energies) {
+            // The weighted densities carry the Pfaffians as they come, sum_phi Pf(c K_s) rho_s: 1e20 for
+            // each species of an sd+pf pair, and c^(h/2) more for another Pfaffian scale c. Two FP32
+            // words hold neither that nor the product of the two species, so each density is
+            // divided by the power of two of its largest entry, which goes back on the energy in FP64.
+            for (int is = wid; is < 2 * m; is += kThreads / 32) {
+                unsigned x = 0u;
+                for (int e = lane; e < hh; e += 32) {
+                    const zc v = St[is * hh + e];
+                    x = max(x, max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu));
+                }
+                const int ex = (int)(__reduce_max_sync(0xffffffffu, x) >> 20);
+                // all zero: any power will do; Inf or NaN: stays so under the largest
+                if (lane == 0) sexp[is] = ex == 0 ? 1023 : min(ex, 2045);
+            }
+        }
         for (int t = wid; t < 2 * kOneBody * m; t += kThreads / 32) {
             const int is = t / kOneBody, q = t % kOneBody, s = is & 1;
             const bool none = (q == 0 && s) || (q == 1 && !s) || (q >= 7 && (s || !p.iE2));
             const zc v = none ? mk(0, 0) : one_body(p, q, lane, s * h, h, St + (long long)is * hh, h);
             if (lane == 0) ob[t] = v;
         }
+        if constexpr (Shared<Z>::energies) {
+            __syncthreads();
+            for (int t = threadIdx.x; t < 2 * hh * m; t += blockDim.x)
+                Se[t] = Ra::from(__hiloint2double((2046 - sexp[t / hh]) << 20, 0) * St[t]);
+            __syncthreads();
+        }
         // the proton-neutron energy, bilinear in the two weighted densities
         const int wpi = max(1, (kThreads / 32) / m);
-        zc *part = asm2 + 2 * m;                                          // [warps]
         if (wid / wpi < m) {
             using O = Op<Z>;
             typename O::Acc e2 = O::acc(szero<Z>());
@@ -1274,6 +1297,10 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
         if (threadIdx.x < m) {
             zc v = mk(0, 0);
             for (int q = 0; q < wpi; ++q) v = v + part[threadIdx.x * wpi + q];
+            if constexpr (Shared<Z>::energies) {
+                const int ex = sexp[2 * threadIdx.x] + sexp[2 * threadIdx.x + 1] - 2046;
+                v = mk(scalbn(v.x, ex), scalbn(v.y, ex));
+            }
             epn[threadIdx.x] = v;
         }
     }
