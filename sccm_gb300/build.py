@@ -18,7 +18,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(LIBDIR, "libpnamp_gb300.so")
-SOURCES = ["point_df64.cu", "point_fp64.cu", "pnamp_kernels.cu", "pnamp_capi.cu", "contract_tc.cu", "mlp_kernels.cu", "learned_kernels.cu", "hw_kernels.cu"]
+SOURCES = ["point_df64.cu", "point_fp64.cu", "point_gauge_df64.cu", "point_gauge_fp64.cu", "pnamp_kernels.cu", "pnamp_capi.cu", "contract_tc.cu", "mlp_kernels.cu", "learned_kernels.cu", "hw_kernels.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

@@ -347,7 +347,10 @@ int build_energy_tabs(pnamp_ctx *c) {
 // thread. More groups hide the sweep's latency better than more warps per group, which only
 // shorten one problem; an even count serves the two species. ng = 0: nothing fits.
 constexpr int kMaxDynSmem = 227 * 1024 - kMultiSmemTail;
-RedPlan plan_reduced(const Params &p, int N, bool split, int smem) {
+// `solve`: split problems by T22, 2 h x h right-hand sides per group, no shared constants, and the
+// matrices of SolveData in the CTA's global slot, whose 9 n^2 elements (36 h^2) bound the Euler
+// points of a batch: 10 h^2 each, 3 h^2 of constants, h^2 per group.
+RedPlan plan_reduced(const Params &p, int N, bool split, bool solve, int smem) {
     auto align = [](int x) { return (x + 15) & ~15; };
     const int T = N * (N - 1) / 2;
     auto make = [&](int ng) {
@@ -356,7 +359,7 @@ RedPlan plan_reduced(const Params &p, int N, bool split, int smem) {
         L.ng = ng;
         L.w = kThreads / 32 / ng;
         L.ld = N + 1;
-        L.items = split ? std::max(1, ng / 2) : 1;
+        L.items = split ? std::max(1, solve ? std::min(ng / 2, (33 - ng) / 10) : ng / 2) : 1;
         int o = 0;
         L.off_eph = o;
         o += align(16 * p.nfom);
@@ -364,10 +367,12 @@ RedPlan plan_reduced(const Params &p, int N, bool split, int smem) {
         if (split) o += align(16 * (2 * L.items * p.nfom + 2 * std::max(ng, 2 * L.items)) + 4 * std::max(ng, 2 * L.items));
         else o += align(16 * 4 * ng + 4 * ng);
         L.off_z0 = o;
-        o += align((split ? 2 : 1) * N * N * 8);
+        if (!solve) o += align((split ? 2 : 1) * N * N * 8);
         L.off_grp = o;
         L.off_scr = align(16 * N * (L.ld + std::max(L.ld, 5)));   // A; Rh, in which the pivot rows fit
         L.grp_bytes = L.off_scr + 16 * (32 + 32 + 16) + 3 * 64 + 16;   // SkewScratch and the norm
+        L.off_y = L.grp_bytes;
+        if (solve) L.grp_bytes += 16 * 2 * N * N;
         o += ng * L.grp_bytes;
         // the Euler point's rotation blocks, the Onishi matrix and the final sums use the same place
         const int rot = L.items * p.rot_elems * 16;
@@ -438,14 +443,16 @@ int plan_placement(Params &p, int smem_max) {
     if (pl.t_smem) { pl.off_t = off; off += bt; }
     if (pl.y_smem) { pl.off_y = off; off += by; }
     if (pl.uv_smem) { pl.off_uv = off; off += buv; }
-    pl.gen = plan_reduced(p, n, false, std::max(off, smem_max));
-    pl.spl = plan_reduced(p, n / 2, true, std::max(off, smem_max));
-    if (!pl.gen.ng || !pl.spl.ng) {   // the least a point needs is held whatever the budget
-        if (!pl.gen.ng) pl.gen = plan_reduced(p, n, false, kMaxDynSmem);
-        if (!pl.spl.ng) pl.spl = plan_reduced(p, n / 2, true, kMaxDynSmem);
-        if (!pl.gen.ng || !pl.spl.ng) return PNAMP_ERR_UNSUPPORTED;
+    pl.smem_bytes = off;
+    for (RedPlan *L : {&pl.gen, &pl.spl, &pl.sol}) {
+        const bool split = L != &pl.gen, solve = L == &pl.sol;
+        const int order = split ? n / 2 : n;
+        *L = plan_reduced(p, order, split, solve, std::max(off, smem_max));
+        if (!L->ng) *L = plan_reduced(p, order, split, solve, kMaxDynSmem);   // the least a point needs is held
+        if (!L->ng) return PNAMP_ERR_UNSUPPORTED;                             // whatever the budget
+        pl.smem_bytes = std::max(pl.smem_bytes, L->smem_bytes);
     }
-    pl.smem_bytes = std::max({off, pl.gen.smem_bytes, pl.spl.smem_bytes});
+    pl.sol.items = std::min(pl.sol.items, pl.spl.items);   // the species rows' buffer is laid out for spl
     long long g = 0;
     pl.g_x = g; g += nn;
     pl.g_b = g; g += 2 * nn;
@@ -1524,10 +1531,11 @@ int ensure_r2(pnamp_ctx *c) {
     }
     // one set of sums per thread group that runs gauge points of its own, or per unit of a
     // species-split batch
-    const RedPlan &gn = c->p.place.gen, &sl = c->p.place.spl;
+    const Placement &pl = c->p.place;
     const long long need = 2LL * c->grid_form[c->p.form] *
-                           std::max<long long>((long long)c->r2_quads.size() * gn.ng,
-                                               (long long)std::max(c->r2_ss, 0) * std::max(sl.ng, 2 * sl.items));
+                           std::max<long long>((long long)c->r2_quads.size() * pl.gen.ng,
+                                               (long long)std::max(c->r2_ss, 0) *
+                                                   std::max({pl.spl.ng, 2 * pl.spl.items, pl.sol.ng, 2 * pl.sol.items}));
     if (need > c->r2acc_cap) {
         if (c->d_r2acc) cudaFree(c->d_r2acc);
         c->d_r2acc = nullptr;

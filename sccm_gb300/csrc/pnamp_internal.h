@@ -54,9 +54,10 @@ constexpr double kReducedMaxEntry = 40.0;
 // factorisation's scratch from off_scr in a region of grp_bytes. tile: the register tiles of
 // the density products (rho in bits 0..3, kappa10 above). items: Euler points per batch of
 // the species-split path.
+// off_y: the right-hand sides of a group that goes by T22.
 struct RedPlan {
     int ng, w, ld, items, tile;
-    int off_eph, off_acc, off_z0, off_grp, off_scr, grp_bytes, smem_bytes;
+    int off_eph, off_acc, off_z0, off_grp, off_scr, off_y, grp_bytes, smem_bytes;
 };
 
 // Where the per-point work arrays live: shared memory or the CTA's global slot.
@@ -66,6 +67,7 @@ struct Placement {
     int off_s, off_t, off_y, off_uv;     // shared byte offsets (when *_smem)
     int off_piv, off_inv, off_red, off_rot, off_vec;
     RedPlan gen, spl;                    // reduced pairs: n x n problems, species-split h x h problems
+    RedPlan sol;                         // other charge-conserving pairs: h x h problems by T22
     int smem_bytes;
     long long g_x, g_b, g_p, g_rw, g_zr, g_s, g_t, g_y, g_uv;
     long long slot_elems;
@@ -169,6 +171,15 @@ struct Params {
     const int *tc_chunks;
     int tc_choff[3];
 };
+
+// Rows of the proton-neutron table per gauge angle, and the chunks of each species' gauge points
+// for which the CTA's slot has room when H/N of every gauge point is wanted (split_items).
+__host__ __device__ inline int gauge_rows(int h) { return (h * h + 31) / 32 * 32; }
+__host__ __device__ inline int gauge_chunks(const Params &p, bool solve) {
+    const long long hh = (long long)p.h * p.h;
+    const long long room = p.place.slot_elems - (solve ? 13 : 2) * hh - (long long)p.nfom * (2 + gauge_rows(p.h));
+    return room > 0 ? (int)(room / (2 * hh)) : 0;
+}
 
 // One group of the contraction: a contiguous range [off, off + dpad) of the X row (and, for
 // a pp group, [yoff, yoff + dpad) of the Y row), whose square matrix occupies rows

@@ -190,18 +190,24 @@ cudaError_t launch_setup(const Params &p, int npairs, const double *uv, double *
     return cudaGetLastError();
 }
 
-// instantiated in point_fp64.cu and point_df64.cu
-#define POINT_FORM(Z)                                                                                                  \
-    extern template cudaError_t launch_points_z<Z>(const Params &, int, const double *, zc *, int, double *, int *,    \
-                                                   cudaStream_t, const int2 *, long long, double *, double *,          \
-                                                   double *, int);                                                     \
+// instantiated in point_fp64.cu and point_df64.cu, with the gauge points' values in point_gauge_*.cu
+#define POINT_FORM(Z, Gauge)                                                                                           \
+    extern template cudaError_t launch_points_z<Z, Gauge>(const Params &, int, const double *, zc *, int, double *,    \
+                                                          int *, cudaStream_t, const int2 *, long long, double *,      \
+                                                          double *, double *, int);                                    \
+    extern template const void *point_fn<Z, Gauge>();
+#define MULTI_FORM(Z)                                                                                                  \
     extern template cudaError_t launch_multi_z<Z>(const MultiArgs &, const int4 *, int, int, int *, zc *, int, int,    \
                                                   cudaStream_t);                                                       \
-    extern template const void *point_fn<Z>();                                                                         \
     extern template const void *multi_fn<Z>();
-POINT_FORM(zc)
-POINT_FORM(zd)
+POINT_FORM(zc, false)
+POINT_FORM(zc, true)
+POINT_FORM(zd, false)
+POINT_FORM(zd, true)
+MULTI_FORM(zc)
+MULTI_FORM(zd)
 #undef POINT_FORM
+#undef MULTI_FORM
 
 cudaError_t multi_blocks_per_sm(int form, int smem_bytes, int *per_sm) {
     const void *f = form == 1 ? multi_fn<zd>() : multi_fn<zc>();
@@ -220,12 +226,13 @@ cudaError_t launch_multi(int form, const MultiArgs &a, const int4 *items, int ni
 
 cudaError_t point_blocks_per_sm(int form, int smem_bytes, int *per_sm) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        per_sm, form == 1 ? point_fn<zd>() : point_fn<zc>(), kThreads, smem_bytes);
+        per_sm, form == 1 ? point_fn<zd, false>() : point_fn<zc, false>(), kThreads, smem_bytes);
 }
 
 cudaError_t set_point_smem(int form, int bytes) {
     (void)bytes;  // checked against the device maximum by the placement planner
-    return raise_smem_limit(form == 1 ? point_fn<zd>() : point_fn<zc>());
+    const cudaError_t e = raise_smem_limit(form == 1 ? point_fn<zd, false>() : point_fn<zc, false>());
+    return e != cudaSuccess ? e : raise_smem_limit(form == 1 ? point_fn<zd, true>() : point_fn<zc, true>());
 }
 
 // Euler points per split_items call: the choice with the fewest rounds of problems, where a
@@ -252,11 +259,11 @@ cudaError_t launch_points(const Params &p, int npairs, const double *pairbuf, zc
                           double *zres, int *status, cudaStream_t st, const int2 *items, long long nitems,
                           double *gout, double *r1out, double *r2out) {
     if (r2out && (p.n_r2q <= 0 || !p.r2q || !p.r2acc)) return cudaErrorInvalidValue;
-    const int batch = split_batch(p, items ? nitems : (long long)npairs * p.n_euler, items ? 0 : p.n_euler, grid);
-    return p.form == 1 ? launch_points_z<zd>(p, npairs, pairbuf, scratch, grid, zres, status, st, items, nitems, gout,
-                                             r1out, r2out, batch)
-                       : launch_points_z<zc>(p, npairs, pairbuf, scratch, grid, zres, status, st, items, nitems, gout,
-                                             r1out, r2out, batch);
+    const bool gauge = gout && !p.norm_only;   // H/N of every gauge point: one Euler point at a time
+    const int batch = gauge ? 1 : split_batch(p, items ? nitems : (long long)npairs * p.n_euler, items ? 0 : p.n_euler, grid);
+    const auto launch = p.form == 1 ? (gauge ? launch_points_z<zd, true> : launch_points_z<zd, false>)
+                                    : (gauge ? launch_points_z<zc, true> : launch_points_z<zc, false>);
+    return launch(p, npairs, pairbuf, scratch, grid, zres, status, st, items, nitems, gout, r1out, r2out, batch);
 }
 
 // ------------------------------------------------------------------ projection

@@ -1406,16 +1406,18 @@ __device__ __noinline__ void full_item(const Params &p, const double *__restrict
 }
 
 // What a pair's set-up record says about its points.
-enum { kPairBad = 0, kPairFull = 1, kPairReduced = 2, kPairSplit = 3 };
+enum { kPairBad = 0, kPairFull = 1, kPairReduced = 2, kPairSplit = 3, kPairSplitSolve = 4 };
 __device__ __forceinline__ int pair_kind(const Params &p, const double *pr) {
     if (pr[p.pl.dets + 2] != 0.0) return kPairBad;
-    if (pr[p.pl.dets + 7] == 0.0) return kPairFull;
-    return pr[p.pl.dets + 6] != 0.0 ? kPairSplit : kPairReduced;
+    const bool conserving = pr[p.pl.dets + 6] != 0.0;
+    if (pr[p.pl.dets + 7] == 0.0) return conserving && pr[p.pl.dets + 3] != 0.0 ? kPairSplitSolve : kPairFull;
+    return conserving ? kPairSplit : kPairReduced;
 }
-// Species-split pairs factorise (split_items) unless the launch wants what couples the two
-// gauge angles point by point (H/N of every gauge point).
+// Charge-conserving pairs factorise by species (split_items); H/N of every gauge point needs room
+// for the neutrons' part in the CTA's slot (NFOM up to 20).
 __device__ __forceinline__ bool split_path(const Params &p, bool gout, bool r2out) {
-    return p.nfom > 1 && p.split_ok && (!p.tc_splits || p.tc_sp) && (!gout || p.norm_only) && (!r2out || p.r2_ss >= 0);
+    return p.nfom > 1 && p.split_ok && (!p.tc_splits || p.tc_sp) && (!r2out || p.r2_ss >= 0) &&
+           (!gout || p.norm_only || (gauge_chunks(p, false) > 0 && gauge_chunks(p, true) > 0));
 }
 
 // One Euler point of a pair that does not take split_items.
@@ -1435,7 +1437,7 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
             p.tc_w[2 * (pt0 + g)] = 0.0;
             p.tc_w[2 * (pt0 + g) + 1] = 0.0;
         }
-    } else if (kind == kPairFull) {
+    } else if (kind == kPairFull || kind == kPairSplitSolve) {
         full_item<Z>(p, pairbuf, slot, pair, ie, reload, zres, status, gout, r1out, r2out, pt0);
     } else {
         reduced_item<Z>(p, pairbuf + (long long)pair * p.pl.stride, slot, pair, ie, reload, zout, status, gout, r1out,
@@ -1443,7 +1445,9 @@ __device__ __forceinline__ void point_item(const Params &p, const double *__rest
     }
 }
 
-template <class Z>
+// Gauge: launches that want H/N of every gauge point, a kernel of their own because the other
+// launches' code is 1 to 2 % slower beside that body (registers of the functions they share).
+template <class Z, bool Gauge>
 __global__ void __launch_bounds__(kThreads, 1)
 point_kernel(const __grid_constant__ Params p, int npairs, const double *__restrict__ pairbuf, zc *scratch,
              double *__restrict__ zres, int *__restrict__ status, const int2 *__restrict__ items,
@@ -1475,10 +1479,21 @@ point_kernel(const __grid_constant__ Params p, int npairs, const double *__restr
                         ++m;
                 }
                 const double *pr = pairbuf + (long long)pair * p.pl.stride;
-                if (pair_kind(p, pr) == kPairSplit) {
-                    split_items<Z>(p, pr, slot, pair, items ? items + i0 + k : nullptr, (int)(i0 + k), m,
-                                   pair != cur_pair, zres + 2LL * (long long)pair * kNobs * p.n_euler, status, gout,
-                                   r1out, r2out, ((long long)pair0 * p.n_euler + i0 + k) * p.n_gauge);
+                const int kind = pair_kind(p, pr);
+                if (kind >= kPairSplit) {
+                    const bool solve = kind == kPairSplitSolve;
+                    if (Gauge) m = 1;
+                    else if (solve) m = min(m, p.place.sol.items);
+                    double *zout = zres + 2LL * (long long)pair * kNobs * p.n_euler;
+                    const int2 *list = items ? items + i0 + k : nullptr;
+                    const int ie0 = (int)(i0 + k);
+                    const long long pt0 = ((long long)pair0 * p.n_euler + i0 + k) * p.n_gauge;
+                    if (solve)
+                        split_items<Z, true, Gauge>(p, pr, slot, pair, list, ie0, m, pair != cur_pair, zout, status, gout,
+                                                    r1out, r2out, pt0);
+                    else
+                        split_items<Z, false, Gauge>(p, pr, slot, pair, list, ie0, m, pair != cur_pair, zout, status, gout,
+                                                     r1out, r2out, pt0);
                     cur_pair = pair;
                 }
                 k += m;
@@ -1501,7 +1516,7 @@ point_kernel(const __grid_constant__ Params p, int npairs, const double *__restr
             ie = (int)(item % p.n_euler);
         }
         const int kind = pair_kind(p, pairbuf + (long long)pair * p.pl.stride);
-        if (skip && kind == kPairSplit) continue;
+        if (skip && kind >= kPairSplit) continue;
         point_item<Z>(p, pairbuf, slot, pair, ie, kind, pair != cur_pair, zres, status, gout, r1out, r2out,
                       item * p.n_gauge);
         cur_pair = pair;
@@ -1519,10 +1534,16 @@ __device__ __forceinline__ void multi_items(const MultiArgs &a, const int4 *item
     const Params &p = a.p[m.x];
     const double *pr = a.pairbuf[m.x] + (long long)m.y * p.pl.stride;
     const int kind = pair_kind(p, pr);
-    if (kind == kPairSplit && split_path(p, false, false))
-        split_items<Z>(p, pr, slot, m.y, nullptr, m.z, cnt, reload,
-                       a.zres[m.x] + 2LL * (long long)m.y * kNobs * p.n_euler, a.status[m.x], nullptr, nullptr, nullptr, 0);
-    else
+    if (kind >= kPairSplit && split_path(p, false, false)) {
+        double *zout = a.zres[m.x] + 2LL * (long long)m.y * kNobs * p.n_euler;
+        if (kind == kPairSplit)
+            split_items<Z, false, false>(p, pr, slot, m.y, nullptr, m.z, cnt, reload, zout, a.status[m.x], nullptr, nullptr,
+                                         nullptr, 0);
+        else
+            for (int k = 0; k < cnt; k += p.place.sol.items)
+                split_items<Z, true, false>(p, pr, slot, m.y, nullptr, m.z + k, min(p.place.sol.items, cnt - k),
+                                            reload && k == 0, zout, a.status[m.x], nullptr, nullptr, nullptr, 0);
+    } else
         for (int k = 0; k < cnt; ++k)
             point_item<Z>(p, a.pairbuf[m.x], slot, m.y, m.z + k, kind, reload && k == 0, a.zres[m.x], a.status[m.x],
                           nullptr, nullptr, nullptr, 0);
@@ -1560,12 +1581,12 @@ multi_point_kernel(const __grid_constant__ MultiArgs a, const int4 *__restrict__
 }
 
 // Launches of one arithmetic form, instantiated in a translation unit of its own.
-template <class Z>
+template <class Z, bool Gauge>
 cudaError_t launch_points_z(const Params &p, int npairs, const double *pairbuf, zc *scratch, int grid, double *zres,
                             int *status, cudaStream_t st, const int2 *items, long long nitems, double *gout,
                             double *r1out, double *r2out, int batch) {
-    point_kernel<Z><<<grid, kThreads, p.place.smem_bytes, st>>>(p, npairs, pairbuf, scratch, zres, status, items, nitems,
-                                                               gout, r1out, r2out, batch);
+    point_kernel<Z, Gauge><<<grid, kThreads, p.place.smem_bytes, st>>>(p, npairs, pairbuf, scratch, zres, status, items,
+                                                                      nitems, gout, r1out, r2out, batch);
     return cudaGetLastError();
 }
 template <class Z>
@@ -1574,7 +1595,7 @@ cudaError_t launch_multi_z(const MultiArgs &a, const int4 *items, int nitems, in
     multi_point_kernel<Z><<<grid, kThreads, smem, st>>>(a, items, nitems, grab, scratch, counter, smem - kMultiSmemTail);
     return cudaGetLastError();
 }
-template <class Z> const void *point_fn() { return reinterpret_cast<const void *>(point_kernel<Z>); }
+template <class Z, bool Gauge> const void *point_fn() { return reinterpret_cast<const void *>(point_kernel<Z, Gauge>); }
 template <class Z> const void *multi_fn() { return reinterpret_cast<const void *>(multi_point_kernel<Z>); }
 
 }  // namespace pnamp

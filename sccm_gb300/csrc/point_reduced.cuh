@@ -120,6 +120,14 @@ template <class Z> struct SkewScratch {
     unsigned char list[2][64], ord[64];
 };
 
+// Entry t = b (b - 1) / 2 + a of an upper triangle, a < b.
+__device__ __forceinline__ void skew_entry(int t, int &a, int &b) {
+    b = (int)((sqrtf(8.0f * (float)t + 1.0f) + 1.0f) * 0.5f);
+    if (b * (b - 1) / 2 > t) --b;
+    if (b * (b + 1) / 2 <= t) ++b;
+    a = t - b * (b - 1) / 2;
+}
+
 // Pfaffian factorisation of the skew matrix in the upper triangle of A (order N <= 64, even,
 // row stride ld) by a thread group, and (`inverse`) its inverse over all of A.
 //
@@ -385,10 +393,8 @@ __device__ __forceinline__ bool skew_problem_e(const Grp &g, int N, int ld, int 
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const int t = g.tid + e * g.nthr;
-        int b = (int)((sqrtf(8.0f * (float)t + 1.0f) + 1.0f) * 0.5f);
-        if (b * (b - 1) / 2 > t) --b;
-        if (b * (b + 1) / 2 <= t) ++b;
-        const int a = t - b * (b - 1) / 2;
+        int a, b;
+        skew_entry(t, a, b);
         ab[e] = (a << 8) | b;
         if (t < N * (N - 1) / 2) {
             const Z d = b < h0 ? d0 : (a < h0 ? d1 : d2);
@@ -438,6 +444,174 @@ __device__ __noinline__ bool skew_problem(const Grp g, int N, int ld, int h0, Z 
     }
     gsync(g);
     return sing;
+}
+
+// ------------------------------------------------------------------ problems by T22
+// Charge-conserving pairs outside the reduced class (nearly empty or nearly full levels, so that Z0
+// or W^-1 is large) whose V0 is well conditioned: one species' densities at one gauge angle from
+// T22 = V0^T (d R V1) + U0^T (d* R* U1), d = e^{i phi}, whose entries are bounded whatever the levels,
+//     rho = d R V1 T22^-1 V0^T,  kappa10 = d R V1 T22^-1 U0^T,  kappa01 = -d* R* U1 T22^-1 V0^T,
+// and the norm from Pf(c (d^2 X - Z0^-1)) Pf(-c Z0), X = R W R^T: the algebra of full_item on a species'
+// h x h block, which depends on its own gauge angle only. About three times the work of the skew
+// inverse (a solve with 2 h right-hand sides and three products). One pf pair, 4 + 4 nucleons, gap
+// 0.2 MeV, 432 Euler x 81 gauge points: FP64 4.3 ms, double-float 2.4 ms; the same pair as n x n points
+// (full_item) 116 and 46.6 ms, species blocks point by point 41.9 and 17.3 ms.
+//
+// One pair's constants and one (Euler point, species)'s matrices, in the CTA's global slot.
+template <class Z> struct SolveData {
+    const typename Ar<Z>::R *V0t, *U0t, *Zi;   // [h][h]: V0(j, k) at k h + j, U0 likewise; Z0^-1
+    const Z *X, *B, *P;                        // [h][h]; [2][h][h] R V1, R* U1; [2][h][h] V0^T R V1, U0^T R* U1
+};
+
+// Y <- Y T^-1 (Y: ny x N, row stride N; T: N x N, row stride ld, destroyed) by column-oriented
+// Gauss-Jordan elimination as gj_right_solve, for a thread group of any size: every warp searches the
+// pivot of row k itself, so a step is two group barriers and all warps share its updates. Row k of
+// T stays as it is in step k, and the columns k and c are exchanged in the rows below and in Y.
+template <class Z>
+__device__ __forceinline__ bool col_solve(const Grp &g, int N, int ld, Z *T, Z *Y, int ny) {
+    using O = Op<Z>;
+    const int lane = g.tid & 31, dq = g.nthr / N, dr = g.nthr % N, t0 = g.tid / N, j0 = g.tid % N;
+    bool sing = false;
+    for (int k = 0; k < N; ++k) {
+        const Z *row = T + k * ld;
+        unsigned key = 0u;
+        for (int j = k + lane; j < N; j += 32) {
+            const unsigned kk = sweep_key(row[j], j - k);
+            key = key > kk ? key : kk;
+        }
+        key = __reduce_max_sync(0xffffffffu, key);
+        const bool none = (key >> 6) == 0u;
+        const int c = none ? k : k + 63 - (int)(key & 63u), nrT = N - k - 1, rows = nrT + ny;
+        sing = sing || none;
+        if (g.tid < rows) {
+            const Z inv = none ? szero<Z>() : zrecip(row[c]);
+            for (int t = g.tid; t < rows; t += g.nthr) {
+                Z *r = t < nrT ? T + (k + 1 + t) * ld : Y + (t - nrT) * N;
+                const Z a = r[c], b = r[k];
+                r[k] = a * inv;
+                if (c != k) r[c] = b;
+            }
+        }
+        gsync(g);
+        int j = j0;
+        for (int t = t0; t < rows;) {
+            if (j != k) {
+                Z *r = t < nrT ? T + (k + 1 + t) * ld : Y + (t - nrT) * N;
+                const Z p = row[j == c ? k : j];
+                typename O::Acc x = O::acc(r[j]);
+                O::cadd(x, O::mul_neg(r[k]), p, O::rot(p));
+                r[j] = O::done(x);
+            }
+            t += dq;
+            j += dr;
+            if (j >= N) {
+                j -= N;
+                ++t;
+            }
+        }
+        gsync(g);
+    }
+    return sing;
+}
+
+// The pivots of d*^2 (d^2 X - Z0^-1) = X - d*^2 Z0^-1 into w and (`inverse`) the densities of the N
+// levels at A and Rh (row stride ld) as skew_problem leaves them, kappa as the skew part. Y: 2 N x N.
+template <class Z>
+__device__ __noinline__ bool solve_problem(const Grp g, int N, int ld, Z d, const SolveData<Z> &S, Z *A, Z *Rh, Z *Y,
+                                           SkewScratch<Z> &w, bool inverse) {
+    using O = Op<Z>;
+    const Z dc = zconj(d), d2 = dc * dc;
+    {   // Y serves as the factorisation's scratch. One form for up to 8 entries per thread, and not a call of
+        // skew_problem: a second caller of that costs it registers (pf double-float 8.49 -> 8.56 ms)
+        int ab[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            int a = 0, b = 1;
+            const int t = g.tid + e * g.nthr;
+            if (t < N * (N - 1) / 2) {
+                skew_entry(t, a, b);
+                A[a * ld + b] = rfma(Ar<Z>::rneg(S.Zi[a * N + b]), d2, S.X[a * N + b]);
+            }
+            ab[e] = (a << 8) | b;
+        }
+        skew_factor<Z, 8>(g, N, ld, ab, A, Y, 2 * N * N, w, false);
+    }
+    if (!inverse) return false;
+    for (int t = g.tid; t < N * N; t += g.nthr) Rh[(t / N) * ld + t % N] = zfma(d, S.P[t], dc * S.P[N * N + t]);
+    for (int t = g.tid; t < 2 * N * N; t += g.nthr) Y[t] = S.B[t];
+    gsync(g);
+    const bool sing = col_solve<Z>(g, N, ld, Rh, Y, 2 * N);
+    const Z *Yu = Y + N * N;
+    const typename Ar<Z>::R half = Ar<Z>::rconst(0.5f);
+    for (int t = g.tid; t < N * N; t += g.nthr) {
+        const int i = t / N, j = t % N;
+        typename O::Acc x = O::acc(szero<Z>());
+        for (int k = 0; k < N; ++k) O::radd(x, O::rmul(S.V0t[k * N + j]), Y[i * N + k]);
+        Rh[i * ld + j] = d * O::done(x);
+        if (i < j) {
+            typename O::Acc a = O::acc(szero<Z>()), b = a;
+            for (int k = 0; k < N; ++k) {
+                O::radd(a, O::rmul(S.U0t[k * N + j]), Y[i * N + k]);
+                O::radd(a, O::rmul(Ar<Z>::rneg(S.U0t[k * N + i])), Y[j * N + k]);
+                O::radd(b, O::rmul(Ar<Z>::rneg(S.V0t[k * N + j])), Yu[i * N + k]);
+                O::radd(b, O::rmul(S.V0t[k * N + i]), Yu[j * N + k]);
+            }
+            A[i * ld + j] = half * (d * O::done(a));
+            A[j * ld + i] = half * (dc * O::done(b));
+        } else if (i == j) {
+            A[i * ld + i] = szero<Z>();
+        }
+    }
+    gsync(g);
+    return sing;
+}
+
+// One pair's constants of SolveData, both species: V0t, U0t, Zi [2][h][h] each from `c` on.
+template <class Z>
+__device__ __noinline__ void solve_constants(const Params &p, const double *__restrict__ pr, typename Ar<Z>::R *c) {
+    const int h = p.h, hh = h * h, n = p.n;
+    for (int t = threadIdx.x; t < 2 * hh; t += blockDim.x) {
+        const int s = t / hh, k = (t % hh) / h, j = t % h, o = (s * h + j) * n + s * h + k;
+        c[t] = Ar<Z>::real(pr[p.pl.v0 + o]);
+        c[2 * hh + t] = Ar<Z>::real(pr[p.pl.u0 + o]);
+        c[4 * hh + t] = Ar<Z>::real(pr[p.pl.zi + (s * h + k) * n + s * h + j]);
+    }
+}
+
+// B and P of SolveData for m Euler points, both species: B[m][2][2][h][h] holds the FP64 values until the
+// products are formed; rot: the Euler points' rotation blocks.
+template <class Z>
+__device__ __noinline__ void solve_setup(const Params &p, const double *__restrict__ pr, int m, const zc *rot, Z *B, Z *P) {
+    const int h = p.h, hh = h * h, n = p.n;
+    const double *gU0 = pr + p.pl.u0, *gV0 = pr + p.pl.v0, *gU1 = pr + p.pl.u1, *gV1 = pr + p.pl.v1;
+    zc *Bz = reinterpret_cast<zc *>(B);
+    __syncthreads();
+    for (int t = threadIdx.x; t < 2 * hh * m; t += blockDim.x) {
+        const int is = t / hh, e = t % hh, s = is & 1, a = s * h + e / h, j = s * h + e % h;
+        const int b = p.row_blk[a], s0 = p.blk_start[b], d = p.blk_size[b];
+        const zc *Rr = rot + (long long)(is >> 1) * p.rot_elems + p.blk_roff[b] + (a - s0) * d;
+        zc v = mk(0, 0), u = mk(0, 0);
+        for (int k = 0; k < d; ++k) {
+            v = rfma(gV1[(s0 + k) * n + j], Rr[k], v);
+            u = rfma(gU1[(s0 + k) * n + j], zconj(Rr[k]), u);
+        }
+        Bz[2 * is * hh + e] = v;
+        Bz[(2 * is + 1) * hh + e] = u;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 4 * hh * m; t += blockDim.x) {
+        const int q = t / hh, e = t % hh, i = e / h, j = e % h, o = ((q >> 1) & 1) * h;
+        const double *M = (q & 1 ? gU0 : gV0) + o * n + o + i;
+        zc s = mk(0, 0);
+        for (int k = 0; k < h; ++k) s = rfma(M[k * n], Bz[q * hh + k * h + j], s);
+        P[t] = Ar<Z>::from(s);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 4 * hh * m; t += blockDim.x) {   // in place
+        const zc v = Bz[t];
+        B[t] = Ar<Z>::from(v);
+    }
+    __syncthreads();
 }
 
 // ------------------------------------------------------------------ observables of one point
@@ -1077,9 +1251,66 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
 // proton-neutron energy and the cross terms of <J^2> are bilinear in the two weighted densities
 // sum_phi a_s rho_s, one contraction per Euler point.
 //
+// H/N of one species' problem at angle l with the other species' angles: the neutrons leave their
+// energy `e` (two- and one-body, in the group's first warp) in En and F in F; the protons, when all
+// neutrons are through, write E_p + E_n + E_pn + e0 for every phi_n whose neutron problem was
+// regular. A is free: the density goes there without its padding.
+template <class Z>
+__device__ __noinline__ void gauge_values(const Grp g, const Params &p, int h, int ld, int s, int l, zc e, Z *A,
+                                          const Z *Rh, zc *En, Z *F, double *gp) {
+    using O = Op<Z>;
+    using Ra = Ar<Z>;
+    const EnergyTab &t = p.tab[kTabMixed];
+    const int lane = g.tid & 31, wid = g.tid >> 5, nw = g.nthr >> 5, hh = h * h, nf = p.nfom, rows = gauge_rows(h);
+    gsync(g);
+    for (int k = g.tid; k < hh; k += g.nthr) A[k] = Rh[(k / h) * ld + k % h];
+    gsync(g);
+    if (s) {
+        for (int q = wid; q < t.nslice; q += nw) {
+            typename O::Acc x = O::acc(szero<Z>());
+            for (int k = t.start[q] * 32 + lane; k < t.start[q + 1] * 32; k += 32)
+                O::radd(x, O::rmul(Ra::pick(t.v, t.vd, k)), A[t.v[k] != 0.0 ? t.off[k] - hh : 0]);
+            F[(long long)l * rows + q * 32 + lane] = O::done(x);
+        }
+        if (g.tid == 0) {
+            En[2 * l] = e;
+            En[2 * l + 1] = mk(1.0, 0.0);
+        }
+        return;
+    }
+    for (int ln = wid; ln < nf; ln += nw) {
+        typename O::Acc x = O::acc(szero<Z>());
+        for (int q = 0; q < t.nslice; ++q) {
+            const Z y = A[t.yoff[q * 32 + lane]];
+            O::cadd(x, O::mul(F[(long long)ln * rows + q * 32 + lane]), y, O::rot(y));
+        }
+        const Z v = warp_sum_z(O::done(x));
+        if (lane == 0 && En[2 * ln + 1].x != 0.0) {
+            const zc r = Ra::to(v) + En[2 * ln];
+            gp[4 * (l * nf + ln) + 2] = r.x;
+            gp[4 * (l * nf + ln) + 3] = r.y;
+        }
+    }
+    gsync(g);
+    if (wid == 0)
+        for (int ln = lane; ln < nf; ln += 32)
+            if (En[2 * ln + 1].x != 0.0) {
+                gp[4 * (l * nf + ln) + 2] += e.x + p.e0;
+                gp[4 * (l * nf + ln) + 3] += e.y;
+            }
+}
+
 // Up to ng / 2 Euler points at a time: a unit (Euler point, species, chunk of the gauge
 // points) per thread group, so that a launch with few Euler points still fills the groups.
-template <class Z>
+//
+// Solve: the pair's problems go by T22 (solve_problem) instead of the skew inverse. Gauge: H/N of
+// every gauge point goes to gout, for one Euler point at a time and the neutrons' problems first.
+// H/N at (phi_p, phi_n) is E_p + E_n + sum_r rho_p,r F_r(phi_n), F_r = sum_k V_rk rho_n,k over the table
+// of the proton-neutron energy: the table is read NFOM times, not NFOM^2 (the pair above with H/N
+// of every gauge point: FP64 6.5 ms, double-float 4.9 ms).
+// Both are compile-time choices: as arguments of one function they cost the plain form 4 to 7 %
+// (spills; pf double-float 8.43 -> 8.84 ms, norm pass 1.46 -> 1.56 ms).
+template <class Z, bool Solve, bool Gauge>
 __device__ __noinline__ void split_items(const Params &p, const double *__restrict__ pr, zc *slot, int pair,
                                          const int2 *__restrict__ items, int ie0, int m, bool reload,
                                          double *__restrict__ zout, int *__restrict__ status,
@@ -1088,14 +1319,17 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
     using Ra = Ar<Z>;
     using R = typename Ra::R;
     extern __shared__ __align__(16) unsigned char smem[];
-    const RedPlan &L = p.place.spl;
+    const RedPlan &L = Solve ? p.place.sol : p.place.spl;
     const int h = p.h, n = p.n, hh = h * h, ld = L.ld, nf = p.nfom;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int ng = L.ng, gthr = 32 * L.w, gid = (int)threadIdx.x / gthr;
     const bool inverse = !p.norm_only;
-    const int nc = max(1, min(ng / (2 * m), nf)), nu = 2 * m * nc;   // chunks per species, units
+    int nc = max(1, min(ng / (2 * m), nf));                          // chunks per species
+    if (Gauge) nc = min(nc, gauge_chunks(p, Solve));
+    const int nu = 2 * m * nc;                                       // units
     const int tcw = 2 * p.tc_nk - p.tc_nph;                          // width of a species row
-    unsigned short *rows = p.tc_splits ? p.tc_sp + (long long)blockIdx.x * L.items * 2 * nf * 6 * tcw : nullptr;
+    unsigned short *rows =
+        p.tc_splits ? p.tc_sp + (long long)blockIdx.x * p.place.spl.items * 2 * nf * 6 * tcw : nullptr;
     Z *ephz = reinterpret_cast<Z *>(smem + L.off_eph);
     zc *asum = reinterpret_cast<zc *>(smem + L.off_acc);     // [m][2][nf]: a_s(phi)
     zc *uacc = asum + 2 * L.items * nf;                      // [unit][2]: sum a E_ss, sum a J2_ss
@@ -1103,13 +1337,21 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
     R *Z0 = reinterpret_cast<R *>(smem + L.off_z0);          // [2][h][h]
     // per unit: weighted density; per item: the species blocks of Y. R* Wi takes the densities' place
     Z *Y = reinterpret_cast<Z *>(slot);                      // [m][2][h h]
-    zc *Sb = slot + 2LL * L.items * hh;
-    zc *RW = slot + 2LL * L.items * hh;                      // [m][2][h h]
-    const double *gWi = pr + p.pl.zi, *gZ0 = pr + p.pl.z0;
+    const int I = Gauge ? 1 : L.items;
+    zc *Sb = slot + 2LL * I * hh;
+    zc *RW = slot + 2LL * I * hh;                            // [m][2][h h]
+    // by T22: Y is X = R W R^T; SolveData's matrices follow the densities
+    Z *SB = reinterpret_cast<Z *>(Sb + (long long)(Gauge ? nu : max(ng, 2 * I)) * hh), *SP = SB + 4LL * I * hh;
+    R *Sc = reinterpret_cast<R *>(SP + 4LL * I * hh);
+    // Gauge: [nf] (neutron energy; 1 once it is there), [nf][rows] F
+    zc *En = reinterpret_cast<zc *>(SB + (Solve ? 11LL * hh : 0));
+    Z *F = reinterpret_cast<Z *>(En + 2 * nf);
+    const double *gWi = pr + (Solve ? p.pl.w : p.pl.zi), *gZ0 = pr + p.pl.z0;
     auto euler = [&](int k) { return items ? items[k].y : ie0 + k; };
     if (reload) {
         __syncthreads();
-        for (int t = threadIdx.x; t < 2 * hh; t += blockDim.x) {
+        if (Solve) solve_constants<Z>(p, pr, Sc);
+        for (int t = threadIdx.x; t < (Solve ? 0 : 2 * hh); t += blockDim.x) {
             const int b = t / hh, i = (t % hh) / h, j = t % h;
             const int u = (b * h + min(i, j)) * n + b * h + max(i, j);
             Z0[t] = i == j ? Ra::rzero() : Ra::real(i < j ? gZ0[u] : -gZ0[u]);
@@ -1134,7 +1376,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
         const int b = p.row_blk[a], s0 = p.blk_start[b], d = p.blk_size[b];
         const zc *Rr = rot + (long long)it * p.rot_elems + p.blk_roff[b] + (a - s0) * d;
         zc rw = mk(0, 0);
-        for (int k = 0; k < d; ++k) rw = rfma(gWi[(s0 + k) * n + j], zconj(Rr[k]), rw);
+        for (int k = 0; k < d; ++k) rw = rfma(gWi[(s0 + k) * n + j], Solve ? Rr[k] : zconj(Rr[k]), rw);
         RW[t] = rw;
     }
     __syncthreads();
@@ -1147,17 +1389,26 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
         const zc *Rr = rot + (long long)it * p.rot_elems + p.blk_roff[b] + (s * h + c - s0) * d;
         const zc *rw = RW + (long long)(2 * it + s) * hh + a * h + s0 - s * h;
         zc x = mk(0, 0);
-        for (int k = 0; k < d; ++k) x = zfma(rw[k], zconj(Rr[k]), x);
+        for (int k = 0; k < d; ++k) x = zfma(rw[k], Solve ? Rr[k] : zconj(Rr[k]), x);
         Y[(long long)(2 * it + s) * hh + a * h + c] = Ra::from(x);
+    }
+    if (Solve && inverse) solve_setup<Z>(p, pr, m, rot, SB, SP);
+    double *gp = Gauge ? gout + 4LL * ((long long)pair * p.n_euler + euler(0)) * p.n_gauge : nullptr;
+    if (Gauge) {
+        for (int l = threadIdx.x; l < nf; l += blockDim.x) En[2 * l + 1] = mk(0.0, 0.0);
+        for (int t = threadIdx.x; t < p.n_gauge; t += blockDim.x) gp[4 * t + 2] = gp[4 * t + 3] = 0.0;
     }
     __syncthreads();
     // ---- the problems
     const Grp g{(int)threadIdx.x - gid * gthr, gthr, 1 + gid};
     const bool energies = inverse && !p.tc_splits;
     const bool rounds = energies && Shared<Z>::energies;   // spare warps only join energy_round
-    for (int u0 = 0; u0 < nu; u0 += ng) {
-        const int u = u0 + gid;
-        const bool mine = gid < ng && u < nu;
+    const int step = Gauge ? nc : ng;
+    for (int u0 = 0; u0 < nu; u0 += step) {
+        if (Gauge) __syncthreads();   // the protons' problems read the neutrons' F
+        const int ub = Gauge ? nc - u0 : u0;   // this round's first unit: neutrons, then protons
+        const int u = ub + gid;
+        const bool mine = gid < step && u < (Gauge ? ub + nc : nu);
         const int it = mine ? u / (2 * nc) : 0, s = mine ? (u / nc) & 1 : 0, chunk = mine ? u % nc : 0;
         unsigned char *gb = smem + L.off_grp + (mine ? gid : 0) * L.grp_bytes;
         Z *A = reinterpret_cast<Z *>(gb), *Rh = A + h * ld;
@@ -1175,15 +1426,23 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
             const bool act = mine && l < nf;
             bool sing = false;
             if (act) {
-                const Z d = ephz[l] * ephz[l];
-                sing = skew_problem<Z>(g, h, ld, h, d, d, d, Y + (long long)(2 * it + s) * hh, h, Z0 + s * hh, A, Rh, w,
-                                       inverse, L.tile);
+                if constexpr (Solve) {
+                    const long long is = 2 * it + s;
+                    const SolveData<Z> D{Sc + s * hh, Sc + (2 + s) * hh, Sc + (4 + s) * hh, Y + is * hh, SB + 2 * is * hh,
+                                         SP + 2 * is * hh};
+                    sing = solve_problem<Z>(g, h, ld, ephz[l], D, A, Rh, reinterpret_cast<Z *>(gb + L.off_y), w, inverse);
+                } else {
+                    const Z d = ephz[l] * ephz[l];
+                    sing = skew_problem<Z>(g, h, ld, h, d, d, d, Y + (long long)(2 * it + s) * hh, h, Z0 + s * hh, A, Rh, w,
+                                           inverse, L.tile);
+                }
                 if (g.tid < 32) {
                     int under;
                     const zc pf = pivot_product<Z>(w.piv, h / 2, p.cscale, under);
                     if (lane == 0) {
                         const int o = s ? l : l * nf;   // e^{-i phi N_s}: the other species' angle is 0
-                        const zc a = pf * mk(p.gphase[2 * o], p.gphase[2 * o + 1]);
+                        zc a = pf * mk(p.gphase[2 * o], p.gphase[2 * o + 1]);
+                        if (Solve) a = a * expi(6.283185307179586476925287 * ((l * h) % nf) / nf);   // det d of d*^2 (...)
                         asum[(2 * it + s) * nf + l] = a;
                         ash[0] = a;
                         flags |= (under == 1 ? 1 : (under == 2 ? 4 : 0)) | (inverse && sing ? 2 : 0);
@@ -1194,8 +1453,8 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
                 __syncthreads();
                 for (int sp = 0; sp < 2; ++sp) {   // the groups whose problem of this round is of species sp
                     int list[16], cnt = 0;
-                    for (int k = 0; k < ng && u0 + k < nu; ++k)
-                        if ((((u0 + k) / nc) & 1) == sp && l0 + (u0 + k) % nc < nf) list[cnt++] = k;
+                    for (int k = 0; k < step && ub + k < nu; ++k)
+                        if ((((ub + k) / nc) & 1) == sp && l0 + (ub + k) % nc < nf) list[cnt++] = k;
                     energy_round<Z>(p.tab[kTabProton + sp], p.sched[1], sp, smem, cnt, list, L.off_grp, L.grp_bytes, L.off_scr);
                 }
                 __syncthreads();
@@ -1210,6 +1469,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
                 const zc tp = Ra::to(q.tp), tm = Ra::to(q.tm), tz = Ra::to(q.tz);
                 aJ = zfma(a, Ra::to(q.j2) + tp * tm + tz * tz, aJ);
             }
+            if constexpr (Gauge) gauge_values<Z>(g, p, h, ld, s, l, Ra::to(q.e2) + Ra::to(q.t1), A, Rh, En, F, gp);
             gsync(g);
             const zc wa = ash[0];
             for (int t = g.tid; t < hh; t += g.nthr) {   // the sum over gauge points stays FP64
@@ -1260,7 +1520,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
             // each species of an sd+pf pair, and c^(h/2) more for another Pfaffian scale c. Two FP32
             // words hold neither that nor the product of the two species, so each density is
             // divided by the power of two of its largest entry, which goes back on the energy in FP64.
-            for (int is = wid; is < 2 * m; is += kThreads / 32) {
+            for (int is = wid; is < (energies ? 2 * m : 0); is += kThreads / 32) {
                 unsigned x = 0u;
                 for (int e = lane; e < hh; e += 32) {
                     const zc v = St[is * hh + e];
@@ -1279,7 +1539,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
         }
         if constexpr (Shared<Z>::energies) {
             __syncthreads();
-            for (int t = threadIdx.x; t < 2 * hh * m; t += blockDim.x)
+            for (int t = threadIdx.x; t < (energies ? 2 * hh * m : 0); t += blockDim.x)
                 Se[t] = Ra::from(__hiloint2double((2046 - sexp[t / hh]) << 20, 0) * St[t]);
             __syncthreads();
         }
@@ -1297,7 +1557,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
         if (threadIdx.x < m) {
             zc v = mk(0, 0);
             for (int q = 0; q < wpi; ++q) v = v + part[threadIdx.x * wpi + q];
-            if constexpr (Shared<Z>::energies) {
+            if (rounds) {
                 const int ex = sexp[2 * threadIdx.x] + sexp[2 * threadIdx.x + 1] - 2046;
                 v = mk(scalbn(v.x, ex), scalbn(v.y, ex));
             }
@@ -1403,14 +1663,13 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
                 }
             }
         }
-        if (gout)   // norm-only launches: N at every gauge point
+        if (gout)   // N at every gauge point
             for (int gi = lane; gi < p.n_gauge; gi += 32) {
                 const zc w = pre * (asum[2 * it * nf + gi / nf] * asum[(2 * it + 1) * nf + gi % nf]);
                 double *o = gout + 4LL * (((long long)pair * p.n_euler + ie) * p.n_gauge + gi);
                 o[0] = w.x;
                 o[1] = w.y;
-                o[2] = 0.0;
-                o[3] = 0.0;
+                if (!Gauge) o[2] = o[3] = 0.0;
             }
     }
     __syncthreads();

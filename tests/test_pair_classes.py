@@ -50,3 +50,119 @@ def test_results_do_not_depend_on_the_pfaffian_scale(shell, nucleons, gap, scale
                 z, st = ctx.batch(pair)
             assert st.max() == 0, (k, form)
             check(z[0], ref[0])
+
+
+# charge-conserving pairs whose V0 is well conditioned and whose V1 has nearly empty levels: outside
+# the class of the single skew inverse, so their problems go by T22, one per species and gauge angle
+WEAK = {"p2": ((2, 2), 0.1), "sd": ((2, 2), 0.2), "pf": ((4, 4), 0.2), "sdpf": ((4, 4), 0.3)}
+
+
+def oracle(args, q2, mesh, pair, **kw):
+    from oracle.pnamp_oracle import Hamiltonian, kernel_triaxial
+    from sccm_gb300.basis import j_operators
+    sp, e0, t1b, recs, vbar = args
+    return kernel_triaxial(sp, Hamiltonian(e0, t1b, recs, vbar, q2, j_operators(sp)), mesh, *pair, **kw)
+
+
+@pytest.mark.parametrize("shell", sorted(WEAK))
+def test_weak_pairs_are_outside_the_reduced_class(shell):
+    _, _, (b, k) = problem(shell, *WEAK[shell], 0)
+    assert np.abs(k[0] @ np.linalg.inv(k[1])).max() > 40.0      # W^-1 = U1 V1^-1
+    assert np.linalg.cond(b[1]) < 1e2                           # V0
+    h = b[0].shape[0] // 2
+    assert max(np.abs(M[:h, h:]).max() for M in (*b, *k)) == 0.0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["fp64", "df64"])
+@pytest.mark.parametrize("shell,mesh", [("p2", (2, 3, 1, 4)), ("sd", (3, 3, 1, 3)), ("pf", (1, 5, 1, 3)),
+                                        ("sdpf", (1, 3, 1, 2)), ("sd", (2, 2, 2, 1))])
+def test_weak_pairs_match_the_oracle(shell, mesh, form):
+    """Plain launches, densities, and the values of every gauge point, H/N or the norm alone."""
+    import torch
+    from oracle.pnamp_oracle import rho1b_table
+    from sccm_gb300.pnamp import PnampContext
+    args, q2, vac = problem(shell, *WEAK[shell], 0)
+    mesh, pair = Mesh(*mesh), (*vac[0], *vac[1])
+    with PnampContext(*args, mesh, q2=q2, form=form) as ctx:
+        z, st = ctx.batch([pair, pair])
+        zd, _, r1, r2 = ctx.batch_densities([pair])
+        P, G = ctx.n_euler, mesh.n_gauge
+        quads = ctx.rho2b_tables()["quads"]
+        uv = torch.from_numpy(ctx.pack_pairs([pair])).cuda()
+        it = torch.tensor([(0, e) for e in range(P)] + [(1, 0), (0, P)], dtype=torch.int32, device="cuda")
+        zi = {}
+        for outputs in ("all", "norm"):
+            za = torch.zeros((1, NOBS, P, 2), dtype=torch.float64, device="cuda")
+            sa = torch.zeros((1, P), dtype=torch.int32, device="cuda")
+            g = torch.zeros((1, P, G, 4), dtype=torch.float64, device="cuda")
+            ctx.set_outputs(outputs)
+            ctx.batch_items_device(1, uv.data_ptr(), P + 2, it.data_ptr(), za.data_ptr(), sa.data_ptr(), g.data_ptr(),
+                                   torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+            assert sa.max() == 0
+            zi[outputs] = torch.view_as_complex(za).cpu().numpy()[0].T, torch.view_as_complex(g.view(P, G, 2, 2)).cpu().numpy()
+        ctx.set_outputs("all")
+    ref, o1, o2 = oracle(args, q2, mesh, pair, rho1b=rho1b_table(args[0]), rho2b=quads)
+    assert st.max() == 0
+    check(z[0], ref)
+    check(z[1], ref)
+    check(zd[0], ref)
+    assert np.abs(r1[0].T - o1).max() <= 1e-9 * np.abs(o1).max()
+    o2 = mesh.euler_points()[:, 3] @ o2
+    assert np.abs(r2[0] - o2).max() <= 1e-9 * np.abs(o2).max()
+    check(zi["all"][0], ref)
+    N, H = (zi["all"][1][:, :, k] for k in (0, 1))
+    assert np.abs((N * H).mean(1) - ref[:, 6]).max() <= 1e-9 * np.abs(ref[:, 6]).max()
+    assert np.abs(zi["norm"][0][:, 0] - ref[:, 0]).max() <= 1e-10 * np.abs(ref[:, 0]).max()
+    assert np.abs(zi["norm"][1][:, :, 0].mean(1) - ref[:, 0]).max() <= 1e-10 * np.abs(ref[:, 0]).max()
+
+
+@pytest.mark.gpu
+def test_weak_and_other_pairs_of_one_batch_in_the_tensor_core_form():
+    """A launch with pairs of both charge-conserving classes, against double-float (energies of BF16x6
+    within 1e-6, all else to rounding)."""
+    from sccm_gb300.pnamp import PnampContext
+    args, q2, vac = problem("pf", *WEAK["pf"], 0)
+    _, _, good = problem("pf", (4, 4), None, 0)
+    pairs = [(*vac[0], *vac[1]), (*good[0], *good[1]), (*vac[1], *vac[0])]
+    with PnampContext(*args, Mesh(2, 3, 3, 5), q2=q2, form="df64") as ctx:
+        zd, st = ctx.batch(pairs)
+        ctx.set_form("tc6")
+        zt, sc = ctx.batch(pairs)
+    assert st.max() == 0 and sc.max() == 0
+    for a, b in zip(zt, zd):
+        for io in range(NOBS):
+            assert np.abs(a[:, io] - b[:, io]).max() <= (1e-6 if io == 6 else 1e-12) * np.abs(b[:, io]).max(), io
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gauge", [False, True])
+@pytest.mark.parametrize("form", ["fp64", "df64"])
+def test_weak_pairs_keep_the_species_split(form, gauge):
+    """A conserving pair takes at most 0.6 of the time of a mixing pair of the same orders (NFOM^2 points
+    of order n against species blocks), with and without the values of every gauge point."""
+    import torch
+    from sccm_gb300.pnamp import PnampContext
+    ms = []
+    for mix in (False, True):
+        args, q2, vac = problem("pf", *WEAK["pf"], 0, mix=mix)
+        with PnampContext(*args, Mesh(4, 8, 4, 5), q2=q2, form=form) as ctx:
+            P = ctx.n_euler
+            uv = torch.from_numpy(ctx.pack_pairs([(*vac[0], *vac[1])])).cuda()
+            it = torch.tensor([(0, e) for e in range(P)], dtype=torch.int32, device="cuda")
+            z = torch.zeros((1, NOBS, P, 2), dtype=torch.float64, device="cuda")
+            st = torch.zeros((1, P), dtype=torch.int32, device="cuda")
+            g = torch.zeros((1, P, 25, 4), dtype=torch.float64, device="cuda")
+            stream = torch.cuda.current_stream().cuda_stream
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            t = []
+            for _ in range(4):
+                a.record()
+                ctx.batch_items_device(1, uv.data_ptr(), P, it.data_ptr(), z.data_ptr(), st.data_ptr(),
+                                       g.data_ptr() if gauge else 0, stream)
+                b.record()
+                torch.cuda.synchronize()
+                t.append(a.elapsed_time(b))
+            ms.append(min(t[1:]))
+    assert ms[0] <= 0.6 * ms[1], ms
