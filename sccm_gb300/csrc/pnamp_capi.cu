@@ -1300,6 +1300,7 @@ int pnamp_init(const pnamp_space *sp, const pnamp_hamiltonian *h, const pnamp_me
     p.n_r2q = 0;  // two-body density launches set their own copy
     p.r2q = nullptr;
     p.r2acc = nullptr;
+    p.r2_stride = 0;
     c->grid = std::max(c->grid_form[0], c->grid_form[1]);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
         pnamp_free(c);
@@ -1487,6 +1488,15 @@ int pnamp_rho2b_tables(const pnamp_space *sp, int *blocks, int *states, unsigned
 }
 
 namespace {
+// Doubles of one CTA's two-body density sums: a set per thread group that runs gauge points of its own
+// or per unit of a species-split batch. CTAs run pairs of different kinds side by side, so the
+// stride between them is the largest that any kind needs.
+long long r2_stride(const pnamp_ctx *c) {
+    const Placement &pl = c->p.place;
+    return 2 * std::max<long long>((long long)c->r2_quads.size() * pl.gen.ng,
+                                   (long long)std::max(c->r2_ss, 0) *
+                                       std::max({pl.spl.ng, 2 * pl.spl.items, pl.sol.ng, 2 * pl.sol.items}));
+}
 void set_r2(const pnamp_ctx *c, Params &q) {
     q.n_r2q = (int)c->r2_quads.size();
     q.r2q = c->d_r2q;
@@ -1494,6 +1504,7 @@ void set_r2(const pnamp_ctx *c, Params &q) {
     for (int k = 0; k < 3; ++k) q.r2_off[k] = c->r2_off[k];
     q.r2_ss = c->r2_ss;
     q.r2acc = c->d_r2acc;
+    q.r2_stride = r2_stride(c);
 }
 int ensure_r2(pnamp_ctx *c) {
     if (!c->r2_built) {
@@ -1529,13 +1540,7 @@ int ensure_r2(pnamp_ctx *c) {
         c->r2_tc.swap(r.tc);
         c->r2_built = true;
     }
-    // one set of sums per thread group that runs gauge points of its own, or per unit of a
-    // species-split batch
-    const Placement &pl = c->p.place;
-    const long long need = 2LL * c->grid_form[c->p.form] *
-                           std::max<long long>((long long)c->r2_quads.size() * pl.gen.ng,
-                                               (long long)std::max(c->r2_ss, 0) *
-                                                   std::max({pl.spl.ng, 2 * pl.spl.items, pl.sol.ng, 2 * pl.sol.items}));
+    const long long need = r2_stride(c) * c->grid_form[c->p.form];
     if (need > c->r2acc_cap) {
         if (c->d_r2acc) cudaFree(c->d_r2acc);
         c->d_r2acc = nullptr;

@@ -146,7 +146,7 @@ struct Params {
     PairLayout pl;
     Placement place;
     // two-body density quadruples (ZRho2B_Angles): packed 8-bit k_i, k_j, k_k, k_l, and the
-    // per-CTA FP64 accumulators [grid][n_r2q] complex; n_r2q = 0 outside Rho2B launches
+    // per-CTA FP64 accumulators [grid][r2_stride]; n_r2q = 0 outside Rho2B launches
     int n_r2q;
     const uint32_t *r2q;
     // the same quadruples with their index, [r2_off[0], r2_off[1]) four protons, [.., r2_off[2]) four
@@ -155,6 +155,7 @@ struct Params {
     const uint2 *r2s;
     int r2_off[3], r2_ss;
     double *r2acc;
+    long long r2_stride;       // doubles of one CTA's sums, the same for pairs of every kind
     // tensor-core contraction (contract_tc.cu): tc_splits = 0 runs the record loop here;
     // 2 or 3 makes the point kernel write each gauge point's density rows as that many bf16
     // terms instead (X: tc_nk entries, ph part first, pp part from tc_nph; Y: the pp

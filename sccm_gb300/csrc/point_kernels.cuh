@@ -902,7 +902,7 @@ __device__ __noinline__ void full_item(const Params &p, const double *__restrict
         }
         // two-body density sums of this Euler point: thread t owns quadruples t, t + blockDim, ...
         // (zeroed, accumulated and flushed by the same thread, so no barrier between the steps)
-        double *r2acc = r2out ? p.r2acc + 2LL * p.n_r2q * blockIdx.x : nullptr;
+        double *r2acc = r2out ? p.r2acc + p.r2_stride * blockIdx.x : nullptr;
         for (int q = threadIdx.x; q < (r2out ? p.n_r2q : 0); q += blockDim.x) {
             r2acc[2 * q] = 0.0;
             r2acc[2 * q + 1] = 0.0;

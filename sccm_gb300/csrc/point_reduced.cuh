@@ -1086,7 +1086,7 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
     SkewScratch<Z> &w = *reinterpret_cast<SkewScratch<Z> *>(gb + L.off_scr);
     zc *nsh = reinterpret_cast<zc *>(gb + L.off_scr + sizeof(SkewScratch<Z>));   // the point's norm
     zc *sb = Sb + (long long)gid * nn;
-    double *r2acc = r2out && mine ? p.r2acc + 2LL * p.n_r2q * ((long long)blockIdx.x * ng + gid) : nullptr;
+    double *r2acc = r2out && mine ? p.r2acc + p.r2_stride * blockIdx.x + 2LL * p.n_r2q * gid : nullptr;
     for (int q = g.tid; q < (r2acc ? p.n_r2q : 0); q += g.nthr) {
         r2acc[2 * q] = 0.0;
         r2acc[2 * q + 1] = 0.0;
@@ -1208,7 +1208,7 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
         if (r2out) {   // Euler weight x gauge mean, added into the pair's sums (ZRho2B_Integral at J = 0)
             const double wgt = p.euler[4 * ie + 3] / ((double)p.nfom * p.nfom);
             double *o = r2out + 2LL * p.n_r2q * pair;
-            const double *a = p.r2acc + 2LL * p.n_r2q * (long long)blockIdx.x * ng;
+            const double *a = p.r2acc + p.r2_stride * blockIdx.x;
             for (int q = threadIdx.x; q < 2 * p.n_r2q; q += blockDim.x) {
                 double s = 0.0;
                 for (int k = 0; k < ng; ++k) s += a[2LL * p.n_r2q * k + q];
@@ -1417,7 +1417,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
         zc *sb = Sb + (long long)u * hh;
         // two-body density: same-species quadruples, sum over phi of a_s times their products
         const int q0 = p.r2_off[s], nq = r2out && mine ? p.r2_off[s + 1] - q0 : 0;
-        double *r2acc = nq ? p.r2acc + 2LL * p.r2_ss * ((long long)blockIdx.x * max(ng, 2 * L.items) + u) : nullptr;
+        double *r2acc = nq ? p.r2acc + p.r2_stride * blockIdx.x + 2LL * p.r2_ss * u : nullptr;
         zc aE = mk(0, 0), aJ = mk(0, 0);   // the group's thread 0
         int flags = 0;
         bool first = true;
@@ -1582,7 +1582,8 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
     }
     if (r2out) {   // Euler weight x gauge mean over the batch, added into the pair's sums
         double *o = r2out + 2LL * p.n_r2q * pair;
-        const long long us = 2LL * p.r2_ss, u0 = (long long)blockIdx.x * max(ng, 2 * L.items);
+        const long long us = 2LL * p.r2_ss;
+        const double *acc = p.r2acc + p.r2_stride * blockIdx.x;
         for (int t = threadIdx.x; t < p.n_r2q; t += blockDim.x) {
             const int s = t < p.r2_off[1] ? 0 : (t < p.r2_off[2] ? 1 : 2);
             const uint2 qd = p.r2s[t];
@@ -1592,7 +1593,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
                 zc x = mk(0, 0);
                 if (s < 2) {
                     for (int q = 0; q < nc; ++q) {
-                        const double *a = p.r2acc + us * (u0 + (2 * it + s) * nc + q) + 2 * (t - p.r2_off[s]);
+                        const double *a = acc + us * ((2 * it + s) * nc + q) + 2 * (t - p.r2_off[s]);
                         x = x + mk(a[0], a[1]);
                     }
                     x = asm2[2 * it + 1 - s] * x;

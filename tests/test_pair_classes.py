@@ -166,3 +166,22 @@ def test_weak_pairs_keep_the_species_split(form, gauge):
                 t.append(a.elapsed_time(b))
             ms.append(min(t[1:]))
     assert ms[0] <= 0.6 * ms[1], ms
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["fp64", "df64"])
+def test_densities_of_a_batch_with_pairs_of_every_kind(form):
+    """CTAs run pairs of different kinds side by side: every pair's densities are those of the pair
+    alone (to the rounding of their order of summation)."""
+    from sccm_gb300.pnamp import PnampContext
+    args, q2, weak = problem("pf", *WEAK["pf"], 0)
+    vac = [weak] + [problem("pf", (4, 4), gap, 0, mix=mix)[2] for gap, mix in ((None, False), (None, True), (0.2, True))]
+    pairs = [(*v[i], *v[1 - i]) for v in vac for i in (0, 1)]
+    with PnampContext(*args, Mesh(4, 8, 4, 3), q2=q2, form=form) as ctx:
+        alone = [ctx.batch_densities([p]) for p in pairs]
+        z, st, r1, r2 = ctx.batch_densities(pairs + pairs[::-1])
+    assert st.max() == 0
+    for k, p in enumerate(list(range(8)) + list(range(7, -1, -1))):
+        za, _, r1a, r2a = alone[p]
+        for got, ref in ((z[k], za[0]), (r1[k], r1a[0]), (r2[k], r2a[0])):
+            assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max(), (k, p)
