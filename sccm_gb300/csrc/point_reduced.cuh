@@ -514,15 +514,17 @@ __device__ __forceinline__ bool col_solve(const Grp &g, int N, int ld, Z *T, Z *
     return sing;
 }
 
-// The pivots of d*^2 (d^2 X - Z0^-1) = X - d*^2 Z0^-1 into w and (`inverse`) the densities of the N
+// The pivots of d^2 X - Z0^-1 into w and (`inverse`) the densities of the N
 // levels at A and Rh (row stride ld) as skew_problem leaves them, kappa as the skew part. Y: 2 N x N.
 template <class Z>
 __device__ __noinline__ bool solve_problem(const Grp g, int N, int ld, Z d, const SolveData<Z> &S, Z *A, Z *Rh, Z *Y,
                                            SkewScratch<Z> &w, bool inverse) {
     using O = Op<Z>;
-    const Z dc = zconj(d), d2 = dc * dc;
-    {   // Y serves as the factorisation's scratch. One form for up to 8 entries per thread, and not a call of
-        // skew_problem: a second caller of that costs it registers (pf double-float 8.49 -> 8.56 ms)
+    const Z dc = zconj(d), d2 = d * d;
+    {   // The phase stands with X, whose entries are smaller than those of Z0^-1 (the norm's error in
+        // double-float is 1.2 to 1.8 times larger the other way). Y serves as the factorisation's scratch.
+        // One form for up to 8 entries per thread, and not a call of skew_problem: a second caller of
+        // that costs it registers (pf double-float 8.49 -> 8.56 ms).
         int ab[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -530,7 +532,7 @@ __device__ __noinline__ bool solve_problem(const Grp g, int N, int ld, Z d, cons
             const int t = g.tid + e * g.nthr;
             if (t < N * (N - 1) / 2) {
                 skew_entry(t, a, b);
-                A[a * ld + b] = rfma(Ar<Z>::rneg(S.Zi[a * N + b]), d2, S.X[a * N + b]);
+                A[a * ld + b] = zfma(d2, S.X[a * N + b], Ar<Z>::neg_real(S.Zi[a * N + b]));
             }
             ab[e] = (a << 8) | b;
         }
@@ -1441,8 +1443,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
                     const zc pf = pivot_product<Z>(w.piv, h / 2, p.cscale, under);
                     if (lane == 0) {
                         const int o = s ? l : l * nf;   // e^{-i phi N_s}: the other species' angle is 0
-                        zc a = pf * mk(p.gphase[2 * o], p.gphase[2 * o + 1]);
-                        if (Solve) a = a * expi(6.283185307179586476925287 * ((l * h) % nf) / nf);   // det d of d*^2 (...)
+                        const zc a = pf * mk(p.gphase[2 * o], p.gphase[2 * o + 1]);
                         asum[(2 * it + s) * nf + l] = a;
                         ash[0] = a;
                         flags |= (under == 1 ? 1 : (under == 2 ? 4 : 0)) | (inverse && sing ? 2 : 0);
