@@ -129,7 +129,11 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
     // Pf(-c Z0). Otherwise both flags stay 0 and the 2n x 2n form is used. (A Pfaffian that
     // underflows is kept as the 2n x 2n form too.)
     const bool reduced = x[1][2] != 0.0 && x[2][2] != 0.0, schur = !reduced && x[3][2] != 0.0;
-    if ((reduced && part == 2) || (schur && part == 3))
+    // (the skew parts of W, W^-1 and Z0 for the reduced pairs, see point_reduced.cuh)
+    if (reduced && part == 2)
+        for (long long t = threadIdx.x; t < nn; t += blockDim.x)
+            out[p.pl.zi + t] = 0.5 * (Yb[t] - Yb[(t % n) * n + t / n]);
+    if (schur && part == 3)
         for (long long t = threadIdx.x; t < nn; t += blockDim.x) out[p.pl.zi + t] = Yb[t];
     const int pfpart = schur ? 1 : 0;
     if (part != pfpart) return;
@@ -141,7 +145,7 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
         zc *Sz = reinterpret_cast<zc *>(A);  // n^2 complex over A and Yb
         for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
             const int i = (int)(t / n), j = (int)(t % n);
-            Sz[t] = mk(i < j ? f * Z[t] : 0.0, 0.0);
+            Sz[t] = mk(i < j ? f * (reduced ? 0.5 * (Z[t] - Z[j * n + i]) : Z[t]) : 0.0, 0.0);
         }
         __syncthreads();
         pf = pfaffian_upper<zc>(Sz, n, vecz, red, sh, under);   // in thread 0

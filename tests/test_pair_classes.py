@@ -185,3 +185,25 @@ def test_densities_of_a_batch_with_pairs_of_every_kind(form):
         za, _, r1a, r2a = alone[p]
         for got, ref in ((z[k], za[0]), (r1[k], r1a[0]), (r2[k], r2a[0])):
             assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max(), (k, p)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shell,mix", [("sd", True), ("sd", False), ("pf", True), ("pf", False)])
+def test_symmetric_errors_of_the_vacua_drop_out_of_the_norm(shell, mix):
+    """V + d S U with S symmetric adds d S to V U^-1, whose skew part stays as it is, so the norm changes
+    at second order only: d = 1e-9 leaves it to 1e-12 (upper triangles would show 1e-9)."""
+    from sccm_gb300.pnamp import PnampContext
+    args, q2, vac = problem(shell, (2, 2), None, 3, mix=mix)
+    rng = np.random.default_rng(4)
+    h = vac[0][0].shape[0] // 2
+    same = np.kron(np.eye(2), np.ones((h, h))) if not mix else 1.0   # charge-conserving pairs stay so
+
+    def moved(U, V):
+        S = rng.standard_normal(U.shape) * same
+        return U, V + 1e-9 * (S + S.T) @ U
+    pairs = [(*vac[0], *vac[1]), (*moved(*vac[0]), *vac[1]), (*vac[0], *moved(*vac[1]))]
+    with PnampContext(*args, Mesh(2, 4, 2, 3), q2=q2) as ctx:
+        z, st = ctx.batch(pairs)
+    assert st.max() == 0
+    for k in (1, 2):
+        assert np.abs(z[k][:, 0] - z[0][:, 0]).max() <= 1e-12 * np.abs(z[0][:, 0]).max(), k
