@@ -44,10 +44,19 @@ struct PairLayout {
 constexpr double kReducedPivotRatio = 1e-2;
 // The reduced pairs of point_reduced.cuh: pivot ratios of U0 and V1 within the same bound and
 // no entry of W^-1 = U1 V1^-1 above this. Its entries enter K = M^-1 - Z0 with their rounding in
-// the point arithmetic: in a simulation with 24-bit words the densities are as exact as with
-// T22 up to 25 (every synthetic and Ge76 vacuum and Ti48's beta2 = -0.1 ... 0.2 are at 5 to 36)
-// and 10 to 20 times less exact at 76 (Ti48's beta2 = 0.3 as the ket).
+// the point arithmetic. Double-float errors against FP64 over those of T22, geometric means over 250 sd and
+// pf pairs of 4 to 32 nucleons and gaps of 0.35 to 1.5 MeV: norm, energy, <J^2> and one-body
+// traces 0.7 to 1.2 up to 25, 1.0 to 2.0 between 25 and 40 (Ti48 pairs, at 18 to 36: 1.2); in a
+// simulation with 24-bit words the densities are 10 to 20 times less exact at 76 (Ti48's beta2 = 0.3
+// as the ket).
 constexpr double kReducedMaxEntry = 40.0;
+// kappa01 = Z0 + Z0 kappa10 Z0 cancels when Z0 is large (nearly full levels in the bra): its largest
+// error, relative to its largest entry, is about Z0 times that of T22. The energy and <J^2>, where it
+// meets kappa10 and the norm's error, do not show it: 0.8 to 1.1 of T22's error for entries of
+// Z0 from 8 to 25, 0.3 to 0.7 from 30 to 130 (nearly full sd and pf shells). The two-body
+// densities do, 1.1 to 1.6 times T22's error from 10 to 25 in the mean and 8 times in single pairs
+// (1.0 below 8), so launches that form them hold Z0 below this.
+constexpr double kReducedMaxZ0Rho2B = 8.0;
 
 // Thread groups and shared memory (byte offsets) of the reduced pairs' problems, order N: ng
 // groups of w warps, each with the inverse (then kappa) and rho (N x ld complex each), the

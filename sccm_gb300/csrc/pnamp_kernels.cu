@@ -98,10 +98,13 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
         __syncthreads();
     }
     if (!tail || ok) row_solve<double>(Yb, n, n, A, n, n, perm, invd);  // V U^-1, or U V^-1
+    // entries of W^-1 and, where two-body densities are wanted, of Z0 (parts 2 and 1)
+    const bool bounded = part == 2 || (part == 1 && p.n_r2q > 0);
+    const double most = part == 2 ? kReducedMaxEntry : kReducedMaxZ0Rho2B;
     int big = 0;
     for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
         if (!tail) out[(ket ? p.pl.w : p.pl.z0) + t] = Yb[t];
-        else if (!(fabs(Yb[t]) <= kReducedMaxEntry)) big = 1;
+        if (!(fabs(Yb[t]) <= most)) big = 1;
     }
     big = __syncthreads_or(big);
     int cross = 0;   // proton-neutron blocks of this chain's matrix
@@ -113,7 +116,7 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
     if (threadIdx.x == 0) {
         xchg[0] = logdet;
         xchg[1] = (double)st;
-        xchg[2] = ok && !(tail && ket && big) ? 1.0 : 0.0;
+        xchg[2] = ok && !(bounded && big) ? 1.0 : 0.0;
         xchg[3] = (double)cross;
     }
     cl.sync();

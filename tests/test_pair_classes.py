@@ -207,3 +207,24 @@ def test_symmetric_errors_of_the_vacua_drop_out_of_the_norm(shell, mix):
     assert st.max() == 0
     for k in (1, 2):
         assert np.abs(z[k][:, 0] - z[0][:, 0]).max() <= 1e-12 * np.abs(z[0][:, 0]).max(), k
+
+
+@pytest.mark.gpu
+def test_two_body_densities_of_half_filled_shells_in_double_float():
+    """Bras with entries of Z0 = V0 U0^-1 from 10 to 19: kappa01 = Z0 + Z0 kappa10 Z0 cancels there, T22
+    does not (4e-14 of the largest element over these pairs; 2e-13 by the single skew inverse)."""
+    from sccm_gb300.pnamp import PnampContext
+    sp = ModelSpace(SHELLS["pf"], 10, 10)
+    rng = np.random.default_rng(7)
+    spe = rng.uniform(-4.0, 0.0, len(sp.orbits))
+    t1b = np.diag([spe[o] for o in sp.orbit]).astype(complex)
+    recs, q2 = mscheme_pairs(sp), q2_operators(sp)
+    v = [deformed_vacuum(sp, spe, 0.05 + 0.06 * k, 25.0, rng, q2=q2, gap=0.4) for k in range(8)]
+    assert min(np.abs(V @ np.linalg.inv(U)).max() for U, V in v) > 8.0
+    pairs = [(*v[i], *v[(i + d) % 8]) for d in (1, 3) for i in range(8)]
+    vbar = 0.5 * np.random.default_rng(1).standard_normal(len(recs))
+    r = []
+    for form in ("fp64", "df64"):
+        with PnampContext(sp, 0.0, t1b, recs, vbar, Mesh(1, 4, 1, 5), q2=q2, form=form) as ctx:
+            r.append(ctx.batch_rho2b(pairs)[2])
+    assert (np.abs(r[1] - r[0]).max(1) / np.abs(r[0]).max(1)).max() <= 1e-13
