@@ -133,9 +133,9 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
     // underflows is kept as the 2n x 2n form too.)
     const bool reduced = x[1][2] != 0.0 && x[2][2] != 0.0, schur = !reduced && x[3][2] != 0.0;
     // (the skew parts of W, W^-1 and Z0 for the reduced pairs, see point_reduced.cuh)
-    if (reduced && part == 2)
+    if (reduced && (part == 1 || part == 2))
         for (long long t = threadIdx.x; t < nn; t += blockDim.x)
-            out[p.pl.zi + t] = 0.5 * (Yb[t] - Yb[(t % n) * n + t / n]);
+            out[(part == 1 ? p.pl.z0 : p.pl.zi) + t] = 0.5 * (Yb[t] - Yb[(t % n) * n + t / n]);
     if (schur && part == 3)
         for (long long t = threadIdx.x; t < nn; t += blockDim.x) out[p.pl.zi + t] = Yb[t];
     const int pfpart = schur ? 1 : 0;

@@ -1009,8 +1009,7 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
     const double pre = p.vacfac * pr[p.pl.dets] * pr[p.pl.dets + 1];
     if (reload) {
         __syncthreads();
-        for (int t = threadIdx.x; t < nn; t += blockDim.x)   // the skew part
-            Z0[t] = Ra::real(0.5 * (gZ0[t] - gZ0[(t % n) * n + t / n]));
+        for (int t = threadIdx.x; t < nn; t += blockDim.x) Z0[t] = Ra::real(gZ0[t]);
         const double twopi = 6.283185307179586476925287;
         for (int l = threadIdx.x; l < p.nfom; l += blockDim.x)
             ephz[l] = Ra::from(expi(onishi ? 0.0 : twopi * l / p.nfom));
@@ -1358,8 +1357,8 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
         __syncthreads();
         if (Solve) solve_constants<Z>(p, pr, Sc);
         for (int t = threadIdx.x; t < (Solve ? 0 : 2 * hh); t += blockDim.x) {
-            const int b = t / hh, i = (t % hh) / h, j = t % h, o = b * h * (n + 1);
-            Z0[t] = Ra::real(0.5 * (gZ0[o + i * n + j] - gZ0[o + j * n + i]));   // the skew part
+            const int b = t / hh, i = (t % hh) / h, j = t % h;
+            Z0[t] = Ra::real(gZ0[(b * h + i) * n + b * h + j]);
         }
         const double twopi = 6.283185307179586476925287;
         for (int l = threadIdx.x; l < nf; l += blockDim.x) {
@@ -1411,9 +1410,9 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
     const int step = Gauge ? nc : ng;
     for (int u0 = 0; u0 < nu; u0 += step) {
         if (Gauge) __syncthreads();   // the protons' problems read the neutrons' F
-        const int ub = Gauge ? nc - u0 : u0;   // this round's first unit: neutrons, then protons
+        const int ub = Gauge ? nc - u0 : u0, cnt_u = min(step, nu - u0);   // this round's first unit, units
         const int u = ub + gid;
-        const bool mine = gid < step && u < (Gauge ? ub + nc : nu);
+        const bool mine = gid < cnt_u;
         const int it = mine ? u / (2 * nc) : 0, s = mine ? (u / nc) & 1 : 0, chunk = mine ? u % nc : 0;
         unsigned char *gb = smem + L.off_grp + (mine ? gid : 0) * L.grp_bytes;
         Z *A = reinterpret_cast<Z *>(gb), *Rh = A + h * ld;
@@ -1431,15 +1430,14 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
             const bool act = mine && l < nf;
             bool sing = false;
             if (act) {
+                const long long is = 2 * it + s;
                 if constexpr (Solve) {
-                    const long long is = 2 * it + s;
                     const SolveData<Z> D{Sc + s * hh, Sc + (2 + s) * hh, Sc + (4 + s) * hh, Y + is * hh, SB + 2 * is * hh,
                                          SP + 2 * is * hh};
                     sing = solve_problem<Z>(g, h, ld, ephz[l], D, A, Rh, reinterpret_cast<Z *>(gb + L.off_y), w, inverse);
                 } else {
                     const Z d = ephz[l] * ephz[l];
-                    sing = skew_problem<Z>(g, h, ld, h, d, d, d, Y + (long long)(2 * it + s) * hh, h, Z0 + s * hh, A, Rh, w,
-                                           inverse, L.tile);
+                    sing = skew_problem<Z>(g, h, ld, h, d, d, d, Y + is * hh, h, Z0 + s * hh, A, Rh, w, inverse, L.tile);
                 }
                 if (g.tid < 32) {
                     int under;
@@ -1457,7 +1455,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
                 __syncthreads();
                 for (int sp = 0; sp < 2; ++sp) {   // the groups whose problem of this round is of species sp
                     int list[16], cnt = 0;
-                    for (int k = 0; k < step && ub + k < nu; ++k)
+                    for (int k = 0; k < cnt_u; ++k)
                         if ((((ub + k) / nc) & 1) == sp && l0 + (ub + k) % nc < nf) list[cnt++] = k;
                     energy_round<Z>(p.tab[kTabProton + sp], p.sched[1], sp, smem, cnt, list, L.off_grp, L.grp_bytes, L.off_scr);
                 }
