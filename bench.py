@@ -59,42 +59,39 @@ FORMS = ("fp64", "df64", "tc3", "tc6")
 # FMAs of 15 FP32 instructions each (pnamp_df64.cuh: one multiply, three FMAs, TwoSum's six
 # additions, three additions, FastTwoSum's two), i.e. 7.5 FP32 instructions per flop.
 FP32_INSTR_PER_FLOP = 7.5
-# DRAM bytes per kernel point of the point kernels (ncu dram__bytes_read + write on launches of
-# this workload, scaled by points): all per-point matrices live in shared memory or an
-# L2-resident slot, so traffic is tiny.
-# DRAM bytes per point (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture, divided
-# by the points of the launch): FP64 point kernel (20,736-point case), double-float point
-# kernel (20,736-point case: cold reads of the pair records and tables only), the
-# tensor-core forms' point kernel (5,184-point case: the bf16 density rows it writes,
-# 32 KB per point, which scale with the points) and the contraction kernel (5,184-point
-# case: those rows read back, plus the L2-resident group matrices)
-TRAFFIC_BYTES_PER_POINT = {"fp64": (553984.0 + 2560.0) / 20736.0, "df64": 43.0,
-                           "tc_point": (0.664064e6 + 166.103552e6) / 5184.0,
-                           "tc_contract": (212.85504e6 + 3.983616e6) / 5184.0}
+# DRAM bytes per point (ncu, dram__bytes of one capture over the launch's points; one pf pair of 34,992
+# points, profiles/): the point kernels on charge-conserving pairs in FP64 and double-float, whose
+# matrices live in shared memory or an L2-resident slot (cold reads of tables and scratch), in the
+# tensor-core forms with the bf16 rows they write (40 KB per point for three terms), and the
+# contraction kernel, which reads those rows back
+TRAFFIC_BYTES_PER_POINT = {"fp64": 336.0, "df64": 433.0, "tc_point": 56.7e3, "tc_contract": 41.0e3}
 
 
-def _pair_paths(wl, pairs):
-    """(species-split, reduced Pfaffian) per pair, as the set-up kernel decides them: split
-    when the four matrices have no proton-neutron blocks, reduced when V0's LU pivots span
-    less than 1e2."""
+def _pair_kind(wl, i, j):
+    """What the set-up kernel makes of a pair (pair_kind in point_kernels.cuh): "split" or "reduced"
+    when U0 and V1 are well conditioned (LU pivots spanning less than 1e2) and no entry of U1 V1^-1
+    is above 40, without and with proton-neutron blocks; "solve" when only V0 is, without such
+    blocks; "full" otherwise. The second value: V0 well conditioned. The third: no blocks."""
     import scipy.linalg as sl
-    n = wl.sp.nlev
-    h = n // 2
-    out = []
-    for i, j in pairs:
-        (U0, V0), (U1, V1) = wl.vacua[i], wl.vacua[j]
-        split = all(not np.any(np.asarray(M)[:h, h:]) and not np.any(np.asarray(M)[h:, :h])
-                    for M in (U0, V0, U1, V1))
-        d = np.abs(np.diag(sl.lu_factor(V0)[0]))
-        reduced = bool(d.min() >= 1e-2 * d.max())
-        out.append((split and reduced, reduced))
-    return out
+    h = wl.sp.nlev // 2
+    (U0, V0), (U1, V1) = wl.vacua[i], wl.vacua[j]
+
+    def well(M):
+        d = np.abs(np.diag(sl.lu_factor(M)[0]))
+        return bool(d.min() >= 1e-2 * d.max())
+    conserving = all(not np.any(np.asarray(M)[:h, h:]) and not np.any(np.asarray(M)[h:, :h])
+                     for M in (U0, V0, U1, V1))
+    v0 = well(V0)
+    if well(U0) and well(V1) and np.abs(U1 @ np.linalg.inv(V1)).max() <= 40.0:
+        return ("split" if conserving else "reduced"), v0, conserving
+    return ("solve" if conserving and v0 else "full"), v0, conserving
 
 
 def algorithmic_flops_per_point(wl, n_gauge, pairs=None, records=True):
     """Algorithmic FP64 work per kernel point with a Pfaffian, a solve and density products at every
-    gauge point (the point kernel's full_item), averaged over `pairs` (default: all; complex
-    multiply-add = 8 flops, complex x real = 4), O(n^2) terms left out.
+    gauge point, averaged over `pairs` (default: all; complex multiply-add = 8 flops, complex x
+    real = 4), O(n^2) terms left out: the algebra of the point kernel's full_item, on the two species
+    blocks for a charge-conserving pair.
 
     Per Euler point, amortised over the n_gauge gauge points: R W, R V1, conj(R) U1 and
     X = (R W) R^T with the block-diagonal rotation, (3 * 4 + 8) n sum_b d_b^2, and the
@@ -102,7 +99,8 @@ def algorithmic_flops_per_point(wl, n_gauge, pairs=None, records=True):
     Per point: the Pfaffian of the n x n Schur complement c (D X D - Z0^-1), (4/3) n^3, or of
     the 2n x 2n matrix, (4/3) (2n)^3, when V0 is ill conditioned; Y T22^-1 for the 2n x n
     right-hand sides counted as LU + solves, (8/3 + 16) n^3; the density products, 12 n^3.
-    For a species-split pair these run on two h x h blocks, h = n/2: a quarter.
+    For a charge-conserving pair with a well conditioned V0 these run on two h x h blocks,
+    h = n/2: a quarter.
     Two-body records (`records`; the tensor-core forms contract them in their own kernel):
     52 flops (28 when i + j = k + l, which halves the terms); for a split pair the proton-
     neutron records keep two of the four density products, 18 (10).
@@ -115,9 +113,11 @@ def algorithmic_flops_per_point(wl, n_gauge, pairs=None, records=True):
     pn = (i < h) & (j >= h) & (k < h) & (l >= h)
     diag = (i + j) == (k + l)
     tot = 0.0
-    paths = _pair_paths(wl, pairs if pairs is not None else wl.pairs)
-    for split, reduced in paths:
-        pfaff = (4.0 / 3.0) * (n if reduced else 2 * n) ** 3
+    pairs = pairs if pairs is not None else wl.pairs
+    for a, b in pairs:
+        _, v0, conserving = _pair_kind(wl, a, b)
+        split = v0 and conserving
+        pfaff = (4.0 / 3.0) * (n if v0 else 2 * n) ** 3
         dense = (pfaff + (8.0 / 3.0 + 16.0 + 12.0) * n ** 3) * (0.25 if split else 1.0)
         if records:
             if split:
@@ -128,40 +128,39 @@ def algorithmic_flops_per_point(wl, n_gauge, pairs=None, records=True):
         else:
             rec = 0.0
         tot += (20.0 * n * sd2 + 8.0 * n ** 3) / n_gauge + dense + float(rec)
-    return tot / len(paths)
+    return tot / len(pairs)
 
 
 def point_flops(wl, n_gauge, pairs=None, records=True):
     """Algorithmic FP64 work per kernel point of the point kernel as it now runs, averaged over
     `pairs` (complex multiply-add = 8 flops, complex x real = 4), O(n^2) terms left out.
 
-    Pairs with U0 and V1 well conditioned (LU pivots spanning less than 1e2, no entry of
-    U1 V1^-1 above 40): one skew inverse with its Pfaffian, 4 N^3, and two products with a real
-    matrix, 6 N^3, per problem, and 4 flops per table entry (6 entries per record, 3 when i + j =
-    k + l). NFOM^2 problems of order n per Euler point; for charge-conserving pairs 2 NFOM of
-    order h = n/2 with the same-species records of that species, and the proton-neutron records
-    once per Euler point. Other pairs as `algorithmic_flops_per_point` counts them."""
-    import scipy.linalg as sl
+    "split" and "reduced" pairs (_pair_kind): one skew inverse with its Pfaffian, 4 N^3, and two products
+    with a real matrix, 6 N^3, per problem, and 4 flops per table entry (6 entries per record, 3
+    when i + j = k + l). NFOM^2 problems of order n per Euler point; for charge-conserving pairs 2 NFOM
+    of order h = n/2 with the same-species records of that species, and the proton-neutron records
+    once per Euler point. "solve" pairs: the same with a Pfaffian, a solve and density products of
+    order h per problem. Others as `algorithmic_flops_per_point` counts mixing pairs."""
     n = wl.sp.nlev
     h = n // 2
     i, j, k, l = np.asarray(wl.recs).T
     pn = (i < h) & (j >= h) & (k < h) & (l >= h)
     ent = np.where((i + j) == (k + l), 3.0, 6.0) if records else np.zeros(len(i))
     nfom = int(round(n_gauge ** 0.5))
-
-    def well(M):
-        d = np.abs(np.diag(sl.lu_factor(M)[0]))
-        return d.min() >= 1e-2 * d.max()
+    rec = np.where((i + j) == (k + l), 28.0, 52.0).sum() if records else 0.0
+    sd2 = sum(d * d for _, d in wl.sp.blocks())
     tot = 0.0
     pairs = pairs if pairs is not None else wl.pairs
     for a, b in pairs:
-        (U0, V0), (U1, V1) = wl.vacua[a], wl.vacua[b]
-        if nfom == 1 or not (well(U0) and well(V1) and np.abs(U1 @ np.linalg.inv(V1)).max() <= 40.0):
-            tot += algorithmic_flops_per_point(wl, n_gauge, [(a, b)], records)
-        elif _pair_paths(wl, [(a, b)])[0][0]:
-            tot += (2 * nfom * 10.0 * h ** 3 + 4.0 * (nfom * ent[~pn].sum() + ent[pn].sum() / 3.0)) / n_gauge
-        else:
+        kind, v0, _ = _pair_kind(wl, a, b)
+        if kind in ("split", "solve") and nfom > 1:
+            per = 10.0 if kind == "split" else 4.0 / 3.0 + 8.0 / 3.0 + 16.0 + 12.0
+            tot += (2 * nfom * per * h ** 3 + 4.0 * (nfom * ent[~pn].sum() + ent[pn].sum() / 3.0)) / n_gauge
+        elif kind in ("split", "reduced"):
             tot += 10.0 * n ** 3 + 4.0 * ent.sum()
+        else:
+            pfaff = (4.0 / 3.0) * (n if v0 else 2 * n) ** 3
+            tot += (20.0 * n * sd2 + 8.0 * n ** 3) / n_gauge + pfaff + (8.0 / 3.0 + 16.0 + 12.0) * n ** 3 + float(rec)
     return tot / len(pairs)
 
 
@@ -409,10 +408,11 @@ def rho2b_main(args):
 
     One step = setup + the point kernel with the per-quadruple Rho2B sums
     (`pnamp_batch_rho2b_device`) over `--pairs-per-step` pairs; beside it the same
-    pairs without densities (`pnamp_batch_device`). Roofline of the Rho2B pass: per
-    point and quadruple one complex product difference, one complex multiply-add
-    and the norm-weighted FP64 accumulation, 30 flops, and a 16-byte read and write
-    of the CTA's accumulator (L2-resident); the kernel is timed whole.
+    pairs without densities (`pnamp_batch_device`). Work of the Rho2B pass on charge-conserving
+    pairs, per Euler point: for each same-species quadruple and gauge angle one complex
+    product difference, one complex multiply-add and the weighted FP64 accumulation, 30
+    flops, and a 16-byte read and write of the group's sum (L2-resident); for each proton-neutron
+    quadruple one product of the weighted densities, 14 flops. The kernel is timed whole.
     """
     import torch
     from sccm_gb300.pnamp import PnampContext
@@ -423,7 +423,9 @@ def rho2b_main(args):
     wl = config(1)
     pps = args.pairs_per_step
     ctx = PnampContext(wl.sp, wl.e0, wl.t1b, wl.recs, wl.vbar, wl.mesh, q2=wl.q2, form=args.form)
-    nq = ctx.rho2b_tables()["quads"].shape[0]
+    quads = ctx.rho2b_tables()["quads"]
+    nq = quads.shape[0]
+    same = int(np.sum((quads[:, 0] < wl.sp.nlev // 2) == (quads[:, 1] < wl.sp.nlev // 2)))
     dev = torch.device("cuda")
     uv = torch.from_numpy(ctx.pack_pairs([(*wl.vacua[i], *wl.vacua[j]) for i, j in wl.pairs[:pps]])).to(dev)
     z = torch.zeros((pps, 19, ctx.n_euler, 2), dtype=torch.float64, device=dev)
@@ -447,6 +449,7 @@ def rho2b_main(args):
     p_ms, _ = time_launches(plain, args.steps, flush=flush.zero_)
     pts = pps * ctx.n_euler * wl.mesh.n_gauge
     extra_s = (d_ms - p_ms) / 1e3
+    flops = (30.0 * same * wl.mesh.nfom + 14.0 * (nq - same)) / wl.mesh.n_gauge
     print(json.dumps({
         "metric": "projected kernel points/s with the two-body transition density (Rho2B)",
         "value": pts / (d_ms / 1e3), "unit": "points/s", "n_gpus": 1, "steps": args.steps,
@@ -456,9 +459,9 @@ def rho2b_main(args):
         "config": {"workload": WORKLOAD, "pairs_per_step": pps, "quadruples": nq, "form": FORM_TEXT[args.form],
                    "l2": "flushed (256 MiB write) before each step"},
         "step_ms": d_all, "without_densities": {"value": pts / (p_ms / 1e3), "ms_per_step": p_ms},
-        "rho2b_pass": {"flops_per_point": 30.0 * nq, "extra_ms_per_step": d_ms - p_ms,
-                       "tflops_of_extra_time": 30.0 * nq * pts / extra_s / 1e12 if extra_s > 0 else None,
-                       "accumulator_bytes_per_point": 32.0 * nq},
+        "rho2b_pass": {"flops_per_point": flops, "extra_ms_per_step": d_ms - p_ms,
+                       "tflops_of_extra_time": flops * pts / extra_s / 1e12 if extra_s > 0 else None,
+                       "accumulator_bytes_per_point": 32.0 * same / wl.mesh.nfom},
         "clocks": clk.summary(0), "gpu_launches": 2}))
     ctx.close()
     return 0
@@ -690,14 +693,13 @@ def main():
             r2, _ = timed_forms(w2, c2, order2, list(dict.fromkeys(forms2)), steps2, 1, tag)
             c2.close()
             pts2 = steps2 * pps * w2.mesh.n_euler * w2.mesh.n_gauge * world
-            paths = _pair_paths(w2, order2[pps:])
+            kinds = [_pair_kind(w2, a, b)[0] for a, b in order2[pps:]]
             secondary[tag] = {
                 "workload": ("pf shell n=40, 20 seeded deformed vacua mixing protons and neutrons, same mesh "
                              "(general path)" if tag == "pf_pnmix" else
                              "Ti48 / KB3G (pf shell, Z=2, N=6 valence), the reference's 8 HFB vacua with "
                              "proton-neutron pairing and its m-scheme interaction file, same mesh (general path)"),
-                "pairs_timed": len(order2) - pps, "species_split_pairs": sum(a for a, _ in paths),
-                "reduced_pfaffian_pairs": sum(b for _, b in paths),
+                "pairs_timed": len(order2) - pps, "pair_kinds": {q: kinds.count(q) for q in sorted(set(kinds))},
                 "forms": {f: {"value": pts2 / v["total_s"], "ms_per_step": v["ms_per_step"],
                               "stage_ms_per_step": v["stage_ms_per_step"]} for f, v in r2.items()}}
 

@@ -342,10 +342,12 @@ int build_energy_tabs(pnamp_ctx *c) {
     return PNAMP_OK;
 }
 
-// Thread groups of the reduced pairs' problems (order N, point_reduced.cuh) in `smem` bytes:
-// as many groups as fit, the CTA's warps shared among them, at most 8 matrix entries per
-// thread. More groups hide the sweep's latency better than more warps per group, which only
-// shorten one problem; an even count serves the two species. ng = 0: nothing fits.
+// Thread groups of the reduced pairs' problems (order N, point_reduced.cuh) in `smem` bytes: of the
+// plans that fit, with at most 8 matrix entries per thread, one that uses the most of the CTA's
+// warps, and among those the most groups, since more problems side by side hide the
+// factorisation's latency better than more warps on one; an even count serves the two species.
+// sd split: 16 groups of one warp, mixing 8 of two; pf 8 of two and 4 of four; n = 64: 4 of four and
+// one of 16. ng = 0: nothing fits.
 constexpr int kMaxDynSmem = 227 * 1024 - kMultiSmemTail;
 // `solve`: split problems by T22, 2 h x h right-hand sides per group, no shared constants, and the
 // matrices of SolveData in the CTA's global slot, whose 9 n^2 elements (36 h^2) bound the Euler
@@ -1047,9 +1049,9 @@ int pnamp_init(const pnamp_space *sp, const pnamp_hamiltonian *h, const pnamp_me
         if (a < 0 || b < 0 || c < 0 || d < 0 || a >= n || b >= n || c >= n || d >= n) return PNAMP_ERR_ARG;
         rec_idx[e] = (uint32_t)a | ((uint32_t)b << 8) | ((uint32_t)c << 16) | ((uint32_t)d << 24);
     }
-    // proton-neutron records (a, c protons; b, d neutrons) last: for species-split pairs half
-    // of their terms vanish and the point kernel takes a shorter path over that range
-    int nrec_gen = 0, rec_off[3] = {0, 0, 0};
+    // by class: four protons, four neutrons, others, proton-neutron (a, c protons; b, d neutrons). The
+    // species factorisation of charge-conserving pairs has no place for the others (split_ok).
+    bool split_ok = true;
     {
         std::vector<uint32_t> cls[4];
         std::vector<double> val[4];
@@ -1067,11 +1069,10 @@ int pnamp_init(const pnamp_space *sp, const pnamp_hamiltonian *h, const pnamp_me
         for (int k = 0; k < 4; ++k) {
             gi.insert(gi.end(), cls[k].begin(), cls[k].end());
             gv.insert(gv.end(), val[k].begin(), val[k].end());
-            if (k < 2) rec_off[k + 1] = (int)gi.size();
-            if (k == 2) nrec_gen = (int)gi.size();
         }
         rec_idx.swap(gi);
         rec_v.swap(gv);
+        split_ok = cls[2].empty();
     }
     std::vector<uint32_t> h_rec_idx = rec_idx;
     std::vector<double> h_rec_v = rec_v;
@@ -1144,8 +1145,7 @@ int pnamp_init(const pnamp_space *sp, const pnamp_hamiltonian *h, const pnamp_me
     p.nblk = (int)blk_start.size();
     p.rot_elems = rot;
     p.nrec = h->nrec;
-    p.nrec_gen = nrec_gen;
-    p.split_ok = rec_off[2] == nrec_gen;
+    p.split_ok = split_ok;
     p.pl.make(n);
     c->core_prot = sp->core_prot;
     c->core_neut = sp->core_neut;
@@ -1618,7 +1618,7 @@ int pnamp_batch_densities_device(pnamp_ctx *c, int npairs, const double *d_uv, d
     cudaStream_t st = (cudaStream_t)stream;  // NULL: legacy default stream
     Params q = c->p;
     if (d_rho2b) {
-            set_r2(c, q);
+        set_r2(c, q);
         CK(cudaMemsetAsync(d_rho2b, 0, (size_t)npairs * q.n_r2q * 2 * sizeof(double), st));
     }
     CK(launch_setup(q, npairs, d_uv, c->d_pairbuf, st));

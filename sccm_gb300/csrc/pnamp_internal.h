@@ -59,11 +59,10 @@ constexpr double kReducedMaxEntry = 40.0;
 constexpr double kReducedMaxZ0Rho2B = 8.0;
 
 // Thread groups and shared memory (byte offsets) of the reduced pairs' problems, order N: ng
-// groups of w warps, each with the inverse (then kappa) and rho (N x ld complex each), the
+// groups of w warps, each with the inverse (then kappa10 above and kappa01 below the diagonal) and rho (N x ld complex each), the
 // factorisation's scratch from off_scr in a region of grp_bytes. tile: the register tiles of
-// the density products (rho in bits 0..3, kappa10 above). items: Euler points per batch of
-// the species-split path.
-// off_y: the right-hand sides of a group that goes by T22.
+// the density products (rho in bits 0..3, kappa01 above). items: Euler points per batch of
+// the species-split path. off_y: the right-hand sides of a group that goes by T22.
 struct RedPlan {
     int ng, w, ld, items, tile;
     int off_eph, off_acc, off_z0, off_grp, off_scr, off_y, grp_bytes, smem_bytes;
@@ -140,8 +139,7 @@ struct Params {
     const double *fact;        // k!, k = 0..23
     // Hamiltonian two-body list
     int nrec;
-    int nrec_gen;              // records [0, nrec_gen): general; [nrec_gen, nrec): a, c protons and b, d neutrons
-    int split_ok;              // no other general records and no charge-changing one-body terms
+    int split_ok;              // every record: four protons, four neutrons, or a, c protons and b, d neutrons
     const uint32_t *rec_idx;   // packed 8-bit a,b,c,d (0-based)
     const double *rec_v;
     const dd *rec_vd;          // rec_v as double-float (df64 form)

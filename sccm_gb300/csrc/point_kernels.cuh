@@ -2,7 +2,7 @@
 // (zd, float pairs on the FP32 pipes), one template.
 //
 // Work decomposition (one CUDA launch per stage, batched over pairs):
-//   setup_kernel   one CTA per (q,q') pair: W = V1 U1^-1, Z0 = V0 U0^-1, the
+//   setup_kernel   four CTAs per (q,q') pair: W = V1 U1^-1, Z0 = V0 U0^-1, the
 //                  bare-vacuum overlaps det(1 + Z^T Z)^(-1/4) (zbareover,
 //                  Codes/PNAMP/PNAMP_Proj.f90:6-79), the once-per-pair pieces of the
 //                  Pfaffians and what kind of points the pair has (pair_kind).
@@ -14,8 +14,9 @@
 //                  PNAMP_Energy_OpenMP.f90:31-90 or the split-bf16 rows for the tensor-core
 //                  contraction in contract_tc.cu, ZJ2_0, ZQ2/ZQ2t), summed into ZRES(iang, io)
 //                  (Kernel3D.f90:385-387). Three bodies by the kind of pair:
-//     split_items    (point_reduced.cuh) no proton-neutron blocks, U0 and V1 well conditioned:
-//                    2 NFOM problems of order n/2 per Euler point, one per species and angle;
+//     split_items    (point_reduced.cuh) no proton-neutron blocks: 2 NFOM problems of order n/2 per
+//                    Euler point, one per species and angle, by one skew inverse where U0 and
+//                    V1 are well conditioned, by T22 where only V0 is;
 //     reduced_item   (point_reduced.cuh) U0 and V1 well conditioned: NFOM^2 problems of order n;
 //     full_item      the rest (nearly empty or nearly full levels): Pfaffian of the n x n
 //                    Schur complement or the 2n x 2n matrix, Gauss-Jordan solve Y T22^-1.
@@ -29,8 +30,8 @@
 //   rho = D (R V1 T22^-1) V0^T, kappa10 = D (R V1 T22^-1) U0^T,
 //   kappa01 = -D* (R* U1 T22^-1) V0^T.
 // Measured on GB300, pf shell (n = 40), Euler 10 x 20 x 10, gauge 9 x 9, one pair: charge-conserving
-// FP64 195.3 -> 13.8 ms and double-float 74.7 -> 4.9 ms, proton-neutron mixing with the BF16x6
-// contraction 193.3 -> 69.2 ms, against full_item's algebra for every pair (two points in flight
+// FP64 195.3 -> 9.1 ms and double-float 74.7 -> 4.2 ms, proton-neutron mixing with the BF16x6
+// contraction 193.3 -> 66.5 ms, against full_item's algebra for every pair (two points in flight
 // for charge-conserving ones).
 #pragma once
 #include <cuda_bf16.h>
@@ -823,8 +824,9 @@ __device__ __forceinline__ double warp_sum(double v) {
 #include "point_reduced.cuh"
 namespace pnamp {
 
-// One Euler point of a pair whose V0 is ill conditioned (nearly empty levels in the bra): the
-// 2n x 2n Pfaffian or, for NFOM = 1, the Onishi norm, and an n x n solve, by the whole CTA.
+// One Euler point of a pair that no other body takes: the Pfaffian of the n x n Schur complement (V0
+// well conditioned) or of the 2n x 2n matrix or, for NFOM = 1, the Onishi norm, and an n x n
+// solve, by the whole CTA.
 // `reload` is set when the previous item of this CTA belonged to another pair (or context):
 // V0^T, U0^T and the phase tables are then (re)loaded.
 template <class Z>
@@ -874,8 +876,8 @@ __device__ __noinline__ void full_item(const Params &p, const double *__restrict
         const double *gU1 = pr + p.pl.u1, *gV1 = pr + p.pl.v1, *gU0 = pr + p.pl.u0, *gV0 = pr + p.pl.v0;
         const double *gW = pr + p.pl.w;
         const double det0 = pr[p.pl.dets], det1 = pr[p.pl.dets + 1];
-        // V0 well conditioned: the n x n Schur
-        // complement c (D X D - Z0^-1), times Pf(-c Z0), instead of the 2n x 2n matrix
+        // V0 well conditioned: the n x n Schur complement c (D X D - Z0^-1), times Pf(-c Z0), instead
+        // of the 2n x 2n matrix
         const bool schur = pr[p.pl.dets + 3] != 0.0;
         const double *gZc = pr + (schur ? p.pl.zi : p.pl.z0);
         const zc pfz = mk(pr[p.pl.pfz], pr[p.pl.pfz + 1]);

@@ -661,8 +661,8 @@ __device__ __forceinline__ void energy_slices(const EnergyTab &t, int first, int
 // smem + off[k]; its sum for problem k goes to its reduction slot in that problem's scratch. The
 // table (10 bytes per entry, 0.12 MB for a pf species, 0.8 MB for n = 40) comes from L2: read by
 // every problem for itself its latency bound the loop (FP64 and double-float took the same
-// time), shared by the CTA's problems it is read 7 (species-split pf) or 4 (n = 40) times less
-// often. The slices are dealt longest first to the least loaded warp over both species. FP64 is
+// time), shared by the CTA's problems it is read 4 times less often (pf, split and mixing; 7 or 8
+// times for split sd). The slices are dealt longest first to the least loaded warp over both species. FP64 is
 // bound by its pipe either way and keeps the groups independent (energy_slices).
 template <class Z, int C>
 __device__ __forceinline__ void energy_round_c(const EnergyTab &t, const int *task, int ntask, unsigned char *smem,
