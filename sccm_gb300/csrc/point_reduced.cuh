@@ -458,8 +458,8 @@ __device__ __noinline__ bool skew_problem(const Grp g, int N, int ld, int h0, Z 
 // T22 = V0^T (d R V1) + U0^T (d* R* U1), d = e^{i phi}, whose entries are bounded whatever the levels,
 //     rho = d R V1 T22^-1 V0^T,  kappa10 = d R V1 T22^-1 U0^T,  kappa01 = -d* R* U1 T22^-1 V0^T,
 // and the norm from Pf(c (d^2 X - Z0^-1)) Pf(-c Z0), X = R W R^T: the algebra of full_item on a species'
-// h x h block, which depends on its own gauge angle only. About three times the work of the skew
-// inverse (a solve with 2 h right-hand sides and three products). One pf pair, 4 + 4 nucleons, gap
+// h x h block, which depends on its own gauge angle only. A solve with 2 h right-hand
+// sides and three products: 1.8 times the time of the skew inverse. One pf pair, 4 + 4 nucleons, gap
 // 0.2 MeV, 432 Euler x 81 gauge points: FP64 4.3 ms, double-float 2.4 ms; the same pair as n x n points
 // (full_item) 116 and 46.6 ms, species blocks point by point 41.9 and 17.3 ms.
 //

@@ -1,4 +1,5 @@
-"""Charge-conserving pairs over the range of Pfaffian scales, gaps and fillings.
+"""The classes of pairs (pair_kind in sccm_gb300/csrc/point_kernels.cuh) over the range of Pfaffian scales,
+gaps and fillings.
 
 Tolerances, as in test_reduced_points.py: 1e-10 of the largest value for the norm, 1e-9 for the
 other observables, in both arithmetic forms.
@@ -119,13 +120,29 @@ def test_weak_pairs_match_the_oracle(shell, mesh, form):
 
 
 @pytest.mark.gpu
-def test_weak_and_other_pairs_of_one_batch_in_the_tensor_core_form():
-    """A launch with pairs of both charge-conserving classes, against double-float (energies of BF16x6
-    within 1e-6, all else to rounding)."""
+@pytest.mark.parametrize("form", ["fp64", "df64"])
+@pytest.mark.parametrize("shell,mix", [("p2", False), ("p2", True), ("sd", True), ("pf", False), ("pf", True)])
+def test_a_single_gauge_point_takes_the_onishi_norm(shell, mix, form):
+    """NFOM = 1 of pairs in the class of the single skew inverse."""
     from sccm_gb300.pnamp import PnampContext
-    args, q2, vac = problem("pf", *WEAK["pf"], 0)
-    _, _, good = problem("pf", (4, 4), None, 0)
-    pairs = [(*vac[0], *vac[1]), (*good[0], *good[1]), (*vac[1], *vac[0])]
+    args, q2, vac = problem(shell, (2, 2), None, 6, mix=mix)
+    mesh, pair = Mesh(2, 2, 1, 1), (*vac[0], *vac[1])
+    with PnampContext(*args, mesh, q2=q2, form=form) as ctx:
+        z, st = ctx.batch([pair])
+    assert st.max() == 0
+    check(z[0], oracle(args, q2, mesh, pair))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shell,nucleons", [("p2", (2, 2)), ("sd", (4, 2)), ("pf", (4, 4))])
+def test_weak_and_other_pairs_of_one_batch_in_the_tensor_core_form(shell, nucleons):
+    """A launch with pairs of several classes, against double-float (energies of BF16x6 within 1e-6, all
+    else to rounding)."""
+    from sccm_gb300.pnamp import PnampContext
+    args, q2, vac = problem(shell, nucleons, WEAK[shell][1], 0)
+    _, _, good = problem(shell, nucleons, None, 0)
+    _, _, mixing = problem(shell, nucleons, None, 0, mix=True)
+    pairs = [(*vac[0], *vac[1]), (*good[0], *good[1]), (*vac[1], *vac[0]), (*mixing[0], *mixing[1])]
     with PnampContext(*args, Mesh(2, 3, 3, 5), q2=q2, form="df64") as ctx:
         zd, st = ctx.batch(pairs)
         ctx.set_form("tc6")
