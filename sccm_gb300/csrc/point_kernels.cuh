@@ -1416,7 +1416,7 @@ __device__ __forceinline__ int pair_kind(const Params &p, const double *pr) {
     return conserving ? kPairSplit : kPairReduced;
 }
 // Charge-conserving pairs factorise by species (split_items); H/N of every gauge point needs room
-// for the neutrons' part in the CTA's slot (NFOM up to 20).
+// for the neutrons' part in the CTA's slot (NFOM up to 18, more at n = 64).
 __device__ __forceinline__ bool split_path(const Params &p, bool gout, bool r2out) {
     return p.nfom > 1 && p.split_ok && (!p.tc_splits || p.tc_sp) && (!r2out || p.r2_ss >= 0) &&
            (!gout || p.norm_only || (gauge_chunks(p, false) > 0 && gauge_chunks(p, true) > 0));

@@ -245,3 +245,33 @@ def test_two_body_densities_of_half_filled_shells_in_double_float():
         with PnampContext(sp, 0.0, t1b, recs, vbar, Mesh(1, 4, 1, 5), q2=q2, form=form) as ctx:
             r.append(ctx.batch_rho2b(pairs)[2])
     assert (np.abs(r[1] - r[0]).max(1) / np.abs(r[0]).max(1)).max() <= 1e-13
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["fp64", "df64"])
+@pytest.mark.parametrize("shell,gap,mesh", [("sd", None, (1, 3, 2, 3)), ("sd", 0.2, (1, 3, 2, 3)), ("p2", None, (2, 2, 1, 5)),
+                                            ("pf", None, (1, 2, 1, 4)), ("pf", 0.2, (1, 2, 1, 4))])
+def test_values_of_every_gauge_point_match_the_oracle(shell, gap, mesh, form):
+    """N and N (H/N) point by point, both kinds of charge-conserving pairs (FP64 rounding of the
+    largest point, as for the sums)."""
+    import torch
+    from sccm_gb300.pnamp import PnampContext
+    args, q2, vac = problem(shell, (2, 2), gap, 8)
+    mesh, pair, log = Mesh(*mesh), (*vac[0], *vac[1]), []
+    with PnampContext(*args, mesh, q2=q2, form=form) as ctx:
+        P, G = ctx.n_euler, mesh.n_gauge
+        uv = torch.from_numpy(ctx.pack_pairs([pair])).cuda()
+        it = torch.tensor([(0, e) for e in range(P)], dtype=torch.int32, device="cuda")
+        z = torch.zeros((1, NOBS, P, 2), dtype=torch.float64, device="cuda")
+        st = torch.zeros((1, P), dtype=torch.int32, device="cuda")
+        g = torch.full((1, P, G, 2, 2), 7.0, dtype=torch.float64, device="cuda")
+        ctx.batch_items_device(1, uv.data_ptr(), P, it.data_ptr(), z.data_ptr(), st.data_ptr(), g.data_ptr(),
+                               torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+    g = torch.view_as_complex(g[0]).cpu().numpy()
+    oracle(args, q2, mesh, pair, point_log=log)
+    N = np.array([o[0] for *_, o in log]).reshape(P, G)
+    NH = np.array([o[6] for *_, o in log]).reshape(P, G)
+    assert st.max() == 0
+    assert np.abs(g[:, :, 0] - N).max() <= 1e-10 * np.abs(N).max()
+    assert np.abs(g[:, :, 0] * g[:, :, 1] - NH).max() <= 1e-9 * np.abs(NH).max()
