@@ -134,7 +134,7 @@ setup_kernel(Params p, const double *__restrict__ uv, double *__restrict__ pairb
     const bool reduced = x[1][2] != 0.0 && x[2][2] != 0.0, schur = !reduced && x[3][2] != 0.0;
     // (the skew parts of W, W^-1 and Z0 for the reduced pairs, see point_reduced.cuh)
     if (reduced && (part == 1 || part == 2))
-        for (long long t = threadIdx.x; t < nn; t += blockDim.x)
+        for (int t = threadIdx.x; t < n * n; t += blockDim.x)
             out[(part == 1 ? p.pl.z0 : p.pl.zi) + t] = 0.5 * (Yb[t] - Yb[(t % n) * n + t / n]);
     if (schur && part == 3)
         for (long long t = threadIdx.x; t < nn; t += blockDim.x) out[p.pl.zi + t] = Yb[t];

@@ -980,6 +980,15 @@ __device__ __forceinline__ zc one_body(const Params &p, int q, int lane, int lev
     return s;
 }
 
+// sb (+)= w rho: the sum over gauge points stays FP64.
+template <class Z>
+__device__ __noinline__ void add_weighted(const Grp g, int N, int ld, zc w, const Z *Rh, zc *sb, bool first) {
+    for (int t = g.tid; t < N * N; t += g.nthr) {
+        const zc rv = Ar<Z>::to(Rh[(t / N) * ld + t % N]);
+        sb[t] = first ? w * rv : zfma(w, rv, sb[t]);
+    }
+}
+
 // ------------------------------------------------------------------ general reduced points
 // One Euler point of a reduced pair: its NFOM^2 gauge points dealt to the plan's thread
 // groups, which run them independently (n x n problems, named barriers per group). Observables
@@ -1158,10 +1167,7 @@ __device__ __noinline__ void reduced_item(const Params &p, const double *__restr
         gsync(g);   // nsh
         if (eval) {
             const zc nv = nsh[0];
-            for (int t = g.tid; t < nn; t += g.nthr) {   // the sum over gauge points stays FP64
-                const zc rv = Ra::to(Rh[(t / n) * ld + t % n]);
-                sb[t] = first ? nv * rv : zfma(nv, rv, sb[t]);
-            }
+            add_weighted<Z>(g, n, ld, nv, Rh, sb, first);
             first = false;
             for (int q = g.tid; q < (r2acc ? p.n_r2q : 0); q += g.nthr) {
                 const zc a = zfma(nv, Ra::to(quad_product<Z>(p.r2q[q], 0, ld, A, Rh)),
@@ -1305,6 +1311,46 @@ __device__ __noinline__ void gauge_values(const Grp g, const Params &p, int h, i
             }
 }
 
+// Like add_weighted a function of its own: inlined in split_items they cost it registers (four pf pairs in
+// BF16x6 30.77 ms, 30.54 ms so).
+// Rotation blocks of m Euler points (listed, or from ie0 on) and the species blocks of
+// Y = (R* Wi) R^+ or (Solve, gWi = W) X = (R W) R^T, upper triangles.
+template <class Z, bool Solve>
+__device__ __noinline__ void split_setup(const Params &p, const double *__restrict__ gWi, const int2 *__restrict__ items,
+                                         int ie0, int m, zc *rot, zc *RW, Z *Y) {
+    using Ra = Ar<Z>;
+    const int h = p.h, n = p.n, hh = h * h, wid = threadIdx.x >> 5;
+    auto euler = [&](int k) { return items ? items[k].y : ie0 + k; };
+    {
+        // warps share the Euler points evenly
+        const int wpi = max(1, (kThreads / 32) / m), item = wid / wpi;
+        if (item < m)
+            rotation_blocks(p, euler(item), (int)threadIdx.x - item * wpi * 32, wpi * 32, rot + (long long)item * p.rot_elems);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 2 * hh * m; t += blockDim.x) {
+        const int it = t / (2 * hh), e = t % (2 * hh), s = e / hh, a = s * h + (e % hh) / h, j = s * h + e % h;
+        const int b = p.row_blk[a], s0 = p.blk_start[b], d = p.blk_size[b];
+        const zc *Rr = rot + (long long)it * p.rot_elems + p.blk_roff[b] + (a - s0) * d;
+        zc rw = mk(0, 0);
+        for (int k = 0; k < d; ++k) rw = rfma(gWi[(s0 + k) * n + j], Solve ? Rr[k] : zconj(Rr[k]), rw);
+        RW[t] = rw;
+    }
+    __syncthreads();
+    const int Th = h * (h - 1) / 2;
+    for (int t = threadIdx.x; t < 2 * Th * m; t += blockDim.x) {
+        const int it = t / (2 * Th), e = t % (2 * Th), s = e / Th;
+        int a, c;
+        tri_index(e % Th, h, a, c);
+        const int b = p.row_blk[s * h + c], s0 = p.blk_start[b], d = p.blk_size[b];
+        const zc *Rr = rot + (long long)it * p.rot_elems + p.blk_roff[b] + (s * h + c - s0) * d;
+        const zc *rw = RW + (long long)(2 * it + s) * hh + a * h + s0 - s * h;
+        zc x = mk(0, 0);
+        for (int k = 0; k < d; ++k) x = zfma(rw[k], Solve ? Rr[k] : zconj(Rr[k]), x);
+        Y[(long long)(2 * it + s) * hh + a * h + c] = Ra::from(x);
+    }
+}
+
 // Up to ng / 2 Euler points at a time: a unit (Euler point, species, chunk of the gauge
 // points) per thread group, so that a launch with few Euler points still fills the groups.
 //
@@ -1368,34 +1414,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
     }
     zc *rot = reinterpret_cast<zc *>(smem + L.off_grp);      // [m][rot_elems], before the groups run
     __syncthreads();
-    {
-        // warps share the Euler points evenly
-        const int wpi = max(1, (kThreads / 32) / m), item = wid / wpi;
-        if (item < m)
-            rotation_blocks(p, euler(item), (int)threadIdx.x - item * wpi * 32, wpi * 32, rot + (long long)item * p.rot_elems);
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < 2 * hh * m; t += blockDim.x) {
-        const int it = t / (2 * hh), e = t % (2 * hh), s = e / hh, a = s * h + (e % hh) / h, j = s * h + e % h;
-        const int b = p.row_blk[a], s0 = p.blk_start[b], d = p.blk_size[b];
-        const zc *Rr = rot + (long long)it * p.rot_elems + p.blk_roff[b] + (a - s0) * d;
-        zc rw = mk(0, 0);
-        for (int k = 0; k < d; ++k) rw = rfma(gWi[(s0 + k) * n + j], Solve ? Rr[k] : zconj(Rr[k]), rw);
-        RW[t] = rw;
-    }
-    __syncthreads();
-    const int Th = h * (h - 1) / 2;
-    for (int t = threadIdx.x; t < 2 * Th * m; t += blockDim.x) {
-        const int it = t / (2 * Th), e = t % (2 * Th), s = e / Th;
-        int a, c;
-        tri_index(e % Th, h, a, c);
-        const int b = p.row_blk[s * h + c], s0 = p.blk_start[b], d = p.blk_size[b];
-        const zc *Rr = rot + (long long)it * p.rot_elems + p.blk_roff[b] + (s * h + c - s0) * d;
-        const zc *rw = RW + (long long)(2 * it + s) * hh + a * h + s0 - s * h;
-        zc x = mk(0, 0);
-        for (int k = 0; k < d; ++k) x = zfma(rw[k], Solve ? Rr[k] : zconj(Rr[k]), x);
-        Y[(long long)(2 * it + s) * hh + a * h + c] = Ra::from(x);
-    }
+    split_setup<Z, Solve>(p, gWi, items, ie0, m, rot, RW, Y);
     if (Solve && inverse) solve_setup<Z>(p, pr, m, rot, SB, SP);
     double *gp = Gauge ? gout + 4LL * ((long long)pair * p.n_euler + euler(0)) * p.n_gauge : nullptr;
     if (Gauge) {
@@ -1473,11 +1492,7 @@ __device__ __noinline__ void split_items(const Params &p, const double *__restri
             }
             if constexpr (Gauge) gauge_values<Z>(g, p, h, ld, s, l, Ra::to(q.e2) + Ra::to(q.t1), A, Rh, En, F, gp);
             gsync(g);
-            const zc wa = ash[0];
-            for (int t = g.tid; t < hh; t += g.nthr) {   // the sum over gauge points stays FP64
-                const zc rv = Ra::to(Rh[(t / h) * ld + t % h]);
-                sb[t] = first ? wa * rv : zfma(wa, rv, sb[t]);
-            }
+            add_weighted<Z>(g, h, ld, ash[0], Rh, sb, first);
             for (int q = g.tid; q < nq; q += g.nthr) {
                 const zc x = Ra::to(quad_product<Z>(p.r2s[q0 + q].x, s * h, ld, A, Rh));
                 const zc v = first ? ash[0] * x : zfma(ash[0], x, mk(r2acc[2 * q], r2acc[2 * q + 1]));
