@@ -1311,10 +1311,9 @@ __device__ __noinline__ void gauge_values(const Grp g, const Params &p, int h, i
             }
 }
 
-// Like add_weighted a function of its own: inlined in split_items they cost it registers (four pf pairs in
-// BF16x6 30.77 ms, 30.54 ms so).
 // Rotation blocks of m Euler points (listed, or from ie0 on) and the species blocks of
-// Y = (R* Wi) R^+ or (Solve, gWi = W) X = (R W) R^T, upper triangles.
+// Y = (R* Wi) R^+ or (Solve, gWi = W) X = (R W) R^T, upper triangles. Like add_weighted a function of its
+// own: inlined in split_items they cost it registers (four pf pairs in BF16x6 30.77 ms, 30.54 ms so).
 template <class Z, bool Solve>
 __device__ __noinline__ void split_setup(const Params &p, const double *__restrict__ gWi, const int2 *__restrict__ items,
                                          int ie0, int m, zc *rot, zc *RW, Z *Y) {
@@ -1358,7 +1357,7 @@ __device__ __noinline__ void split_setup(const Params &p, const double *__restri
 // every gauge point goes to gout, for one Euler point at a time and the neutrons' problems first.
 // H/N at (phi_p, phi_n) is E_p + E_n + sum_r rho_p,r F_r(phi_n), F_r = sum_k V_rk rho_n,k over the table
 // of the proton-neutron energy: the table is read NFOM times, not NFOM^2 (the pair above with H/N
-// of every gauge point: FP64 6.5 ms, double-float 4.9 ms).
+// of every gauge point: FP64 6.1 ms, double-float 4.1 ms).
 // Both are compile-time choices: as arguments of one function they cost the plain form 4 to 7 %
 // (spills; pf double-float 8.43 -> 8.84 ms, norm pass 1.46 -> 1.56 ms).
 template <class Z, bool Solve, bool Gauge>
